@@ -164,29 +164,18 @@ struct UpdSched {
   int num_sms = 0;
   unsigned long long* build_tiles_dev = nullptr;  // tiles of the tensor-core build, packed like `tiles_dev`
   int build_total = 0;
-  std::vector<int> row_totals;      // per step: 128-row tiles ti >= step over all problems (couplings)
-  int* cpl_order_dev = nullptr;     // per step: (problem << 16 | ti) of its row tiles, own row tile first
-  std::vector<size_t> cpl_off;      // offset of each step's order
-  int* cpl_counter_dev = nullptr;   // per step x 3 couplings: tile counters, zeroed per evaluation
-  int ncounters = 0;
-  // a second captured branch: the right-hand-side rows' trailing update runs
-  // beside the next step's panel conversion and quarter-0 factor, joined
-  // before that step's panel solve
-  cudaStream_t side = nullptr;
-  cudaEvent_t fork = nullptr, join = nullptr;
+  std::vector<int> row_totals;      // per step: 128-row tiles ti >= step over all problems
+  int* pan_order_dev = nullptr;     // per step: (problem << 16 | ti) of its row tiles, own row tiles first
+  std::vector<size_t> pan_off;      // offset of each step's order
+  std::vector<int> diag_totals;     // per step: problems with a panel there
+  int* sync_dev = nullptr;          // zeroed per evaluation: PANEL_FLAGS ints per problem, a tile counter per step
+  size_t flag_ints = 0, nsync = 0;  // offset of the counters, ints in all
+  int dot_builds = 0;               // problems the FP64 dot-product build serves
 };
-
-void free_sched_sync(UpdSched& u) {
-  if (u.fork) cudaEventDestroy(u.fork);
-  if (u.join) cudaEventDestroy(u.join);
-  if (u.side) cudaStreamDestroy(u.side);
-  u.fork = u.join = nullptr;
-  u.side = nullptr;
-}
 
 // One problem's device buffers.  They are carved from one block (`base`,
 // owned by a worker; a batch plan carves them from its shared arena instead
-// and leaves `base` null); the TMA tensor maps live in their own 512 bytes
+// and leaves `base` null); the TMA tensor maps live in their own bytes
 // because they must outlive the arena's reuse by later waves of a plan.
 struct Workspace {
   void* base = nullptr;
@@ -196,11 +185,13 @@ struct Workspace {
   double* out = nullptr;
   double* z = nullptr;
   // tensor-core mode
-  int* escale = nullptr;
-  double* pw2 = nullptr;
+  int* kscale = nullptr;
   long long* acc = nullptr;
   unsigned char* slices = nullptr;
-  unsigned char* tmaps = nullptr;  // 4 x 128 B TMA tensor maps over slices (128-, 64-row boxes; 64, 32 rows, planes stacked)
+  unsigned char* tmaps = nullptr;  // TMA tensor maps over slices (128-, 64-row boxes; 64 rows, planes stacked)
+  double* rhs = nullptr;           // right-hand sides
+  PanelBlock* lpub = nullptr;      // the current panel's published diagonal blocks
+  PanelZ* zpub = nullptr;          // and solved right-hand-side entries
   double* splanes = nullptr;       // theta-scaled planes (dot-product build)
   double* norms = nullptr;
   long long* fnorm = nullptr;      // tensor-core build: W_ii of the distance leaves
@@ -348,14 +339,15 @@ void fill_prob(Prob& p, const fgpu_ctx* c, const double* theta_d, const Workspac
   p.z = ws.z;
   p.mode = c->mode;
   p.nt128 = c->nt128;
-  p.escale = ws.escale;
-  p.pw2 = ws.pw2;
+  p.kscale = ws.kscale;
   p.acc = ws.acc;
   p.slices = ws.slices;
   p.tmap_a = ws.tmaps;
   p.tmap_b = ws.tmaps ? ws.tmaps + 128 : nullptr;
   p.tmap_bs = ws.tmaps ? ws.tmaps + 256 : nullptr;
-  p.tmap_bs32 = ws.tmaps ? ws.tmaps + 384 : nullptr;
+  p.rhs = ws.rhs;
+  p.lpub = ws.lpub;
+  p.zpub = ws.zpub;
   p.splanes = ws.splanes;
   p.norms = ws.norms;
   p.plane_max = c->plane_max_d;
@@ -390,40 +382,42 @@ int build_sched(const std::vector<int>& nt128, const std::vector<int>& tc_build,
   int dev = 0;
   CK(cudaGetDevice(&dev));
   CK(cudaDeviceGetAttribute(&u.num_sms, cudaDevAttrMultiProcessorCount, dev));
-  CK(cudaStreamCreateWithFlags(&u.side, cudaStreamNonBlocking));
-  CK(cudaEventCreateWithFlags(&u.fork, cudaEventDisableTiming));
-  CK(cudaEventCreateWithFlags(&u.join, cudaEventDisableTiming));
   CK(cudaMalloc(&u.tiles_dev, sizeof(unsigned long long) * tl.size()));
   if (track) track->push_back(u.tiles_dev);
   CK(cudaMemcpy(u.tiles_dev, tl.data(), sizeof(unsigned long long) * tl.size(), cudaMemcpyHostToDevice));
-  // couplings: the row tiles ti >= step of every problem, in the order the
-  // CTAs take them: every problem's own row tile (which also carries the
-  // next quarter's diagonal factor) first
+  // panels: the row tiles ti >= step of every problem, in the order the CTAs
+  // take them: every problem's own row tile, which the others wait for, first
   {
     std::vector<int> ord;
-    u.cpl_off.assign(std::max(ntmax, 1), 0);
+    u.pan_off.assign(std::max(ntmax, 1), 0);
     u.row_totals.assign(std::max(ntmax, 1), 0);
+    u.diag_totals.assign(std::max(ntmax, 1), 0);
     for (int st = 0; st < ntmax; ++st) {
-      u.cpl_off[st] = ord.size();
-      for (int p = 0; p < nprob; ++p) u.row_totals[st] += std::max(0, nt128[p] - st);
+      u.pan_off[st] = ord.size();
       for (int p = 0; p < nprob; ++p)
         if (nt128[p] > st) ord.push_back((p << 16) | st);
+      u.diag_totals[st] = (int)(ord.size() - u.pan_off[st]);
       for (int p = 0; p < nprob; ++p)
         for (int ti = st + 1; ti < nt128[p]; ++ti) ord.push_back((p << 16) | ti);
+      u.row_totals[st] = (int)(ord.size() - u.pan_off[st]);
     }
     if (ord.empty()) ord.push_back(0);
-    CK(cudaMalloc(&u.cpl_order_dev, sizeof(int) * ord.size()));
-    if (track) track->push_back(u.cpl_order_dev);
-    CK(cudaMemcpy(u.cpl_order_dev, ord.data(), sizeof(int) * ord.size(), cudaMemcpyHostToDevice));
-    u.ncounters = 3 * std::max(ntmax, 1);
-    CK(cudaMalloc(&u.cpl_counter_dev, sizeof(int) * u.ncounters));
-    if (track) track->push_back(u.cpl_counter_dev);
+    CK(cudaMalloc(&u.pan_order_dev, sizeof(int) * ord.size()));
+    if (track) track->push_back(u.pan_order_dev);
+    CK(cudaMemcpy(u.pan_order_dev, ord.data(), sizeof(int) * ord.size(), cudaMemcpyHostToDevice));
+    u.flag_ints = (size_t)PANEL_FLAGS * nprob;
+    u.nsync = u.flag_ints + std::max(ntmax, 1);
+    CK(cudaMalloc(&u.sync_dev, sizeof(int) * u.nsync));
+    if (track) track->push_back(u.sync_dev);
   }
   // tensor-core build: the whole lower triangle, nt128 (nt128 + 1) tiles of
   // 128 x 64 per eligible problem, column-tile pair major, row tile minor
   std::vector<unsigned long long> bl;
   for (int p = 0; p < nprob; ++p) {
-    if (!tc_build[p]) continue;
+    if (!tc_build[p]) {
+      u.dot_builds++;
+      continue;
+    }
     for (int q = 0; q < nt128[p]; ++q)
       for (int half = 0; half < 2; ++half)
         for (int ti = q; ti < nt128[p]; ++ti)
@@ -468,55 +462,19 @@ int enqueue_eval(const Prob* probs_d, int nprob, int max_nsteps, int max_nplanes
   if (mode == 1) {
     // 128-wide panels; max_nsteps counts 64-column tiles
     const int nt = max_nsteps / 2, max_nc = max_nsteps * TB;
-    CK(cudaMemsetAsync(us->cpl_counter_dev, 0, sizeof(int) * us->ncounters, s));
+    CK(cudaMemsetAsync(us->sync_dev, 0, sizeof(int) * us->nsync, s));
     STAGE(0, launch_prep_planes(probs_d, nprob, max_nc, s));
     if (us->build_total > 0) STAGE(0, launch_feat_digits(probs_d, nprob, nt, s));
-    // FP64 dot-product build: every tile of the other problems, the
-    // right-hand-side rows of all
-    STAGE(0, launch_build_dot(probs_d, nprob, max_nsteps, max_nplanes, s));
+    if (us->dot_builds > 0) STAGE(0, launch_build_dot(probs_d, nprob, max_nsteps, max_nplanes, s));
     if (us->build_total > 0)
       STAGE(0, launch_build_tc(probs_d, nprob, us->build_tiles_dev, us->build_total, us->num_sms, s));
-    STAGE(0, launch_scales(probs_d, nprob, max_nc, s));
-    const int max_rows = max_nc + TB;  // the tallest problem's ld: factor rows + right-hand sides
-    bool joins = false;                // a side branch awaits its join
     for (int step = 0; step < nt; ++step) {
-      if (step > 0) STAGE(5, launch_panel_prep(probs_d, nprob, step, max_nc, s));
-      // four 32-column quarters: FP64 diagonal factor, panel solve (which
-      // writes the quarter's digit planes); tensor-core couplings quarter
-      // 0 -> 1, half 0 -> 1, quarter 2 -> 3 before the quarter that needs
-      // them, each of which also factors that quarter's diagonal block
-      const int* order = us->cpl_order_dev + us->cpl_off[step];
-      const int rows_total = us->row_totals[step];
-      int* ctr = us->cpl_counter_dev + 3 * step;
-      for (int q = 0; q < NB / QW; ++q) {
-        if (q == 1) STAGE(8, launch_couple(probs_d, nprob, step, 0, 1, 1, 1, order, rows_total, ctr, us->num_sms, s));
-        if (q == 2) STAGE(8, launch_couple(probs_d, nprob, step, 0, 2, 2, 2, order, rows_total, ctr + 1, us->num_sms, s));
-        if (q == 3) STAGE(8, launch_couple(probs_d, nprob, step, 2, 1, 3, 1, order, rows_total, ctr + 2, us->num_sms, s));
-        if (q == 0) STAGE(1, launch_potf2_quarter(probs_d, nprob, step, q, s));  // q > 0: inside the coupling
-        if (q == 0 && joins) {  // the previous step's right-hand-side rows, before they are solved
-          CK(cudaStreamWaitEvent(s, us->join, 0));
-          joins = false;
-        }
-        STAGE(2, launch_trsm_quarter(probs_d, nprob, step, q, max_rows, s));  // also its digit planes
-      }
-      if (step + 1 < nt) {
+      STAGE(2, launch_panel(probs_d, step, us->pan_order_dev + us->pan_off[step], us->diag_totals[step],
+                            us->row_totals[step], us->sync_dev + us->flag_ints + step, us->sync_dev, us->num_sms, s));
+      if (step + 1 < nt)
         STAGE(3, launch_ozaki_update(probs_d, nprob, step, nt, us->tiles_dev + us->tile_off[step],
                                      us->totals[step], us->num_sms, s));
-        // fork: the right-hand-side rows' FP64 update on the side branch,
-        // beside the next step's panel conversion and quarter-0 factor
-        CK(cudaEventRecord(us->fork, s));
-        CK(cudaStreamWaitEvent(us->side, us->fork, 0));
-        int r_ = mark(pe, 7, us->side, true);
-        if (r_) return r_;
-        CK(launch_border_update(probs_d, nprob, step, max_nc, us->side));
-        r_ = mark(pe, 7, us->side, false);
-        if (r_) return r_;
-        ++n;
-        CK(cudaEventRecord(us->join, us->side));
-        joins = true;
-      }
     }
-    if (joins) CK(cudaStreamWaitEvent(s, us->join, 0));
     STAGE(4, launch_finalize(probs_d, nprob, s));
     if (kernels) *kernels = n;
     return 0;
@@ -636,7 +594,7 @@ int capture_plan(fgpu_plan* p, cudaGraphExec_t* exec, long long* kernels, StageE
 // return the bytes they span; with base == nullptr only the size is
 // computed.  The block needs no clearing: every buffer is written by the
 // evaluation before it is read.
-size_t layout_workspace(const fgpu_ctx* c, unsigned char* base, Workspace& ws) {
+size_t layout_workspace(const fgpu_ctx* c, unsigned char* base, Workspace& ws, bool keep_l) {
   size_t off = 0;
   auto take = [&](auto*& dst, size_t bytes) {
     off = (off + 255) / 256 * 256;
@@ -644,14 +602,18 @@ size_t layout_workspace(const fgpu_ctx* c, unsigned char* base, Workspace& ws) {
     off += bytes;
   };
   const size_t nc = (size_t)c->Nc;
-  take(ws.K, K_elems(c) * sizeof(double));
-  // one log-det part per 64-column block (FP64 mode) or 32-column quarter (tensor-core mode)
-  take(ws.logdet_part, sizeof(double) * 2 * (c->nsteps + 1));
+  // the FP64 matrix: the FP64 mode's working storage, the tensor-core mode's
+  // factor where it is wanted (alpha, the adjoint)
+  if (c->mode == 0 || keep_l) take(ws.K, K_elems(c) * sizeof(double));
+  // one log-det part per 64-column block (FP64 mode) or 128-column panel (tensor-core mode)
+  take(ws.logdet_part, sizeof(double) * (c->nsteps + 1));
   take(ws.out, sizeof(double) * 8);
   take(ws.z, sizeof(double) * nc);
   if (c->mode == 1) {
-    take(ws.escale, sizeof(int) * nc);
-    take(ws.pw2, sizeof(double) * nc);
+    take(ws.kscale, sizeof(int) * 2);
+    take(ws.rhs, sizeof(double) * MAX_RHS * nc);
+    take(ws.lpub, sizeof(PanelBlock) * 8);
+    take(ws.zpub, sizeof(PanelZ) * 8);
     take(ws.acc, sizeof(long long) * acc_tiles(c->nt128) * ACC_TILE_ELEMS);
     take(ws.slices, (size_t)c->nt128 * NSLICE * SLICE_BYTES);
     take(ws.splanes, sizeof(double) * (size_t)std::max(c->spec.nplanes, 1) * nc);
@@ -663,26 +625,26 @@ size_t layout_workspace(const fgpu_ctx* c, unsigned char* base, Workspace& ws) {
   return (off + 255) / 256 * 256;
 }
 
-size_t workspace_bytes(const fgpu_ctx* c) {
+size_t workspace_bytes(const fgpu_ctx* c, bool keep_l) {
   Workspace tmp;
-  return layout_workspace(c, nullptr, tmp);
+  return layout_workspace(c, nullptr, tmp, keep_l);
 }
 
-// Encode the problem's four TMA tensor maps over ws.slices into the 512
+// Encode the problem's TMA tensor maps over ws.slices into the TMAP_BYTES
 // device bytes at `dst` (tensor-core mode only).
 int write_tmaps(const fgpu_ctx* c, const Workspace& ws, unsigned char* dst) {
   if (c->mode != 1) return 0;
-  alignas(64) unsigned char maps[512];
+  alignas(64) unsigned char maps[TMAP_BYTES];
   const int er = encode_slice_maps(maps, ws.slices, c->nt128);
   if (er != 0) return fail(FGPU_ECUDA, "cuTensorMapEncodeTiled failed (%d)", er);
-  CK(cudaMemcpy(dst, maps, 512, cudaMemcpyHostToDevice));
+  CK(cudaMemcpy(dst, maps, TMAP_BYTES, cudaMemcpyHostToDevice));
   return 0;
 }
 
 // A worker's own workspace: one block plus its tensor maps.  On failure
 // nothing stays allocated and ws is left empty.
 int alloc_workspace(const fgpu_ctx* c, Workspace& ws) {
-  const size_t bytes = workspace_bytes(c);
+  const size_t bytes = workspace_bytes(c, true);
   void* base = nullptr;
   cudaError_t e = cudaMalloc(&base, bytes);
   if (e != cudaSuccess) {
@@ -690,10 +652,10 @@ int alloc_workspace(const fgpu_ctx* c, Workspace& ws) {
     return fail(e == cudaErrorMemoryAllocation ? FGPU_ENOMEM : FGPU_ECUDA,
                 "workspace allocation of %zu bytes (N=%d): %s", bytes, c->N, cudaGetErrorString(e));
   }
-  layout_workspace(c, static_cast<unsigned char*>(base), ws);
+  layout_workspace(c, static_cast<unsigned char*>(base), ws, true);
   ws.base = base;
   if (c->mode == 1) {
-    e = cudaMalloc(&ws.tmaps, 512);
+    e = cudaMalloc(&ws.tmaps, TMAP_BYTES);
     int rc = e == cudaSuccess ? write_tmaps(c, ws, ws.tmaps)
                               : fail(FGPU_ENOMEM, "tensor-map allocation: %s", cudaGetErrorString(e));
     if (rc) {
@@ -716,9 +678,8 @@ void free_worker(Worker* w) {
   cudaFree(w->prob_d);
   cudaFree(w->sched.tiles_dev);
   cudaFree(w->sched.build_tiles_dev);
-  cudaFree(w->sched.cpl_order_dev);
-  cudaFree(w->sched.cpl_counter_dev);
-  free_sched_sync(w->sched);
+  cudaFree(w->sched.pan_order_dev);
+  cudaFree(w->sched.sync_dev);
   if (w->h_stage) cudaFreeHost(w->h_stage);
   if (w->stream) cudaStreamDestroy(w->stream);
   delete w;
@@ -744,6 +705,7 @@ int make_worker(fgpu_ctx* c, Worker** out) {
   w->h_status = reinterpret_cast<int*>(w->h_stage + c->ntheta + 8);
   Prob p;
   fill_prob(p, c, w->theta_d, w->ws);
+  p.keep_l = 1;  // alpha and the adjoint read the factor
   if (cudaMemcpy(w->prob_d, &p, sizeof(Prob), cudaMemcpyHostToDevice) != cudaSuccess)
     return bail(fail(FGPU_ECUDA, "desc copy"));
   if (c->mode == 1 &&
@@ -1178,7 +1140,7 @@ int fgpu_plan_create(fgpu_plan** out, fgpu_ctx* const* ctxs, int nprob, int ldth
     p->ctxs.push_back(ctxs[i]);
   }
   if (ldtheta < maxth) return fail(FGPU_EINVAL, "ldtheta=%d < max nparams %d", ldtheta, maxth);
-  // the couplings' row-tile order packs (problem << 16 | row tile) into a
+  // the panels' row-tile order packs (problem << 16 | row tile) into a
   // non-negative int (a negative entry ends a CTA's work)
   if (ctxs[0]->mode == 1 && nprob > 32767)
     return fail(FGPU_EINVAL, "a tensor-core plan holds at most 32767 problems (%d given)", nprob);
@@ -1187,7 +1149,7 @@ int fgpu_plan_create(fgpu_plan** out, fgpu_ctx* const* ctxs, int nprob, int ldth
   CK(cudaSetDevice(p->device));
   // waves under the device-memory budget
   std::vector<size_t> bytes(nprob);
-  for (int i = 0; i < nprob; ++i) bytes[i] = workspace_bytes(ctxs[i]);
+  for (int i = 0; i < nprob; ++i) bytes[i] = workspace_bytes(ctxs[i], false);
   std::vector<std::vector<int>> groups;
   int rc = plan_waves(bytes, plan_memory_budget(), groups);
   if (rc) return rc;
@@ -1232,7 +1194,7 @@ int fgpu_plan_create(fgpu_plan** out, fgpu_ctx* const* ctxs, int nprob, int ldth
   unsigned char* arena = nullptr;
   PL_CK(track_alloc((void**)&arena, p->arena_bytes));
   unsigned char* tmaps = nullptr;
-  if (p->mode == 1) PL_CK(track_alloc((void**)&tmaps, (size_t)512 * nprob));
+  if (p->mode == 1) PL_CK(track_alloc((void**)&tmaps, TMAP_BYTES * nprob));
   PL_CK(cudaMallocHost(&p->h_theta, sizeof(double) * (size_t)nprob * ldtheta));
   PL_CK(cudaMallocHost(&p->h_ll, sizeof(double) * nprob));
   PL_CK(cudaMallocHost(&p->h_info, sizeof(int) * nprob));
@@ -1242,10 +1204,10 @@ int fgpu_plan_create(fgpu_plan** out, fgpu_ctx* const* ctxs, int nprob, int ldth
     for (int k = w.first; k < w.first + w.count; ++k) {
       const int i = p->order[k];
       Workspace ws;
-      off += layout_workspace(ctxs[i], arena + off, ws);
+      off += layout_workspace(ctxs[i], arena + off, ws, false);
       ws.status = p->status_all + 4 * k;
       if (p->mode == 1) {
-        ws.tmaps = tmaps + (size_t)512 * k;
+        ws.tmaps = tmaps + TMAP_BYTES * k;
         if ((rc = write_tmaps(ctxs[i], ws, ws.tmaps)) != 0) return bail(rc);
       }
       fill_prob(p->probs_h[k], ctxs[i], p->theta_d + (size_t)i * ldtheta, ws);
@@ -1280,7 +1242,6 @@ void fgpu_plan_destroy(fgpu_plan* p) {
     delete p->prof;
   }
   for (void* q : p->allocations) cudaFree(q);
-  for (PlanWave& w : p->waves) free_sched_sync(w.sched);
   if (p->h_theta) cudaFreeHost(p->h_theta);
   if (p->h_ll) cudaFreeHost(p->h_ll);
   if (p->h_info) cudaFreeHost(p->h_info);

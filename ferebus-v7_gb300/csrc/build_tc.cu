@@ -384,52 +384,72 @@ __global__ void __launch_bounds__(BLD_THREADS, 1)
         const longlong2* wj2 = reinterpret_cast<const longlong2*>(P.fnorm + (size_t)d * nc + j0);
         // The combination of the leaf values is chosen once per pass, outside
         // the entry loop: a ternary inside it is compiled into both sides,
-        // and every FP64 operation costs this part's narrow FP64 pipe.  A
-        // plain sum of the two leaves (a = d = 0, b = c = 1) is one add, the
-        // same double as the general form.
+        // and every FP64 operation costs this part's narrow FP64 pipe.
         const double ca = P.fcoef[0], cb = P.fcoef[1], cc = P.fcoef[2], cd = P.fcoef[3];
         const int N = P.N;
-        double* K = P.K;
-        const size_t ld = (size_t)P.ld;
-        double kdiag = 0.0;  // this row's diagonal entry, when the tile holds it
-        // entry (i, j0 + q): lower triangle of the N x N block; identity padding
-        auto put = [&](int q, double kv) {
+        const int e2 = 2 * *P.kscale;
+        bool nonfinite = false;
+        // entries (i, j0 + q), in the accumulator layout; the lower triangle of
+        // the N x N block, identity padding (1/4 in the matrix's unit) beyond
+        long long* A = P.acc + acc_tile(ti, tj, P.nt128) * ACC_TILE_ELEMS;
+        auto put = [&](int q, long long F) {
           const int j = j0 + q;
-          if (j == i) kdiag = kv;
-          K[(size_t)j * ld + i] = (j > i || i >= N || j >= N) ? (i == j ? 1.0 : 0.0) : kv;
+          if (j > i || i >= N || j >= N) F = i == j ? 1LL << 60 : 0LL;
+          A[acc_elem(r, h * 16 + q)] = F;
         };
         auto leaf = [&](int q) {
           const longlong2 w2 = __ldg(wj2 + q / 2);
           long long E = wi + ((q & 1) ? w2.y : w2.x) - 2 * W[q];
           E = E < 0 ? 0 : E;
+          return iexp_fixed_parts((unsigned long long)E, esc, tab, fine);
+        };
+        auto leaf_double = [&](int q) {
+          const longlong2 w2 = __ldg(wj2 + q / 2);
+          long long E = wi + ((q & 1) ? w2.y : w2.x) - 2 * W[q];
+          E = E < 0 ? 0 : E;
           return iexp_fixed_tab((unsigned long long)E, esc, tab, fine);
         };
-        double* st = stash + tid;  // the first leaf's values, for the second pass
-        if (d < sp.ndot - 1) {
+        // one leaf, or a plain sum of two: fixed point throughout (K_ii >= 1,
+        // so e2 >= 2 unless the nugget is negative); any other expression
+        // combines in FP64
+        const bool sum = ca == 0.0 && cd == 0.0 && cb == 1.0 && (sp.ndot == 1 || cc == 1.0) && e2 >= 2;
+        constexpr int tstash = BLD_EPI_WARPS * 32;
+        if (sum) {
+          long long* st = reinterpret_cast<long long*>(stash) + tid;  // the first leaf's values, for the second pass
+          if (d < sp.ndot - 1) {
 #pragma unroll
-          for (int q = 0; q < 16; ++q) st[q * (BLD_EPI_WARPS * 32)] = leaf(q);
-        } else if (d == 0 && cb == 1.0 && ca == 0.0) {
+            for (int q = 0; q < 16; ++q) st[q * tstash] = iexp_parts_fixed62(leaf(q), e2);
+          } else if (d == 0) {
 #pragma unroll
-          for (int q = 0; q < 16; ++q) put(q, leaf(q));
-        } else if (d == 0) {
+            for (int q = 0; q < 16; ++q) put(q, iexp_parts_fixed62(leaf(q), e2));
+          } else {
 #pragma unroll
-          for (int q = 0; q < 16; ++q) put(q, fma(cb, leaf(q), ca));
-        } else if (ca == 0.0 && cb == 1.0 && cc == 1.0 && cd == 0.0) {
-#pragma unroll
-          for (int q = 0; q < 16; ++q) put(q, st[q * (BLD_EPI_WARPS * 32)] + leaf(q));
+            for (int q = 0; q < 16; ++q) put(q, st[q * tstash] + iexp_parts_fixed62(leaf(q), e2));
+          }
         } else {
+          double* st = stash + tid;
+          if (d < sp.ndot - 1) {
 #pragma unroll
-          for (int q = 0; q < 16; ++q) {
-            // second distance leaf: k = (d v0 + c) v1 + (b v0 + a)
-            const double v0 = st[q * (BLD_EPI_WARPS * 32)];
-            put(q, fma(fma(cd, v0, cc), leaf(q), fma(cb, v0, ca)));
+            for (int q = 0; q < 16; ++q) st[q * tstash] = leaf_double(q);
+          } else if (d == 0) {
+#pragma unroll
+            for (int q = 0; q < 16; ++q) put(q, to_fixed62(fma(cb, leaf_double(q), ca), e2, &nonfinite));
+          } else {
+#pragma unroll
+            for (int q = 0; q < 16; ++q) {
+              // second distance leaf: k = (d v0 + c) v1 + (b v0 + a)
+              const double v0 = st[q * tstash];
+              put(q, to_fixed62(fma(fma(cd, v0, cc), leaf_double(q), fma(cb, v0, ca)), e2, &nonfinite));
+            }
           }
         }
-        // the nugget on the diagonal (the loop stored the entry without it)
+        // the diagonal entry (every leaf 1), with the nugget
         if (d == sp.ndot - 1 && i >= j0 && i < j0 + 16 && i < N) {
           const double noise = P.optimise_noise ? P.theta[sp.nkparams] : P.noise;
-          K[(size_t)i * ld + i] = kdiag + noise * 1.0;
+          const double kd = sp.ndot == 1 ? cb + ca : (cd + cc) + (cb + ca);
+          A[acc_elem(r, i - j0 + h * 16)] = diag_fixed62(kd, noise, e2, &nonfinite);
         }
+        if (nonfinite) atomicOr(&P.status[3], 1);
       }
       if (stop) break;
     }

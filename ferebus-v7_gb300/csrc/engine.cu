@@ -230,13 +230,58 @@ __global__ void __launch_bounds__(256) k_build(const Prob* __restrict__ probs) {
 // form for the well separated pairs that dominate, and it vanishes on the
 // diagonal, which is set exactly (x_i = x_j gives a factor 1).
 // ---------------------------------------------------------------------------
+// the kernel expression at zero distance
+__device__ double kernel_diagonal(const Spec& sp, const double* theta) {
+  double stk[MAX_LEAF];
+  int top = 0;
+  for (int t = 0; t < sp.npost; ++t) {
+    const int tok = sp.post[t];
+    if (tok >= 0) {
+      const Leaf& L = sp.leaf[tok];
+      double v = 1.0;
+      if (L.type == L_LINEAR) {
+        v = 0.0;
+        for (int k = 0; k < L.n; ++k) v += 1.0 / transform_param(L_LINEAR, theta[L.param0 + k]);
+      } else if (L.type == L_CONSTANT) {
+        v = theta[L.param0];
+      }
+      stk[top++] = v;
+    } else {
+      const double b = stk[--top];
+      const double a = stk[--top];
+      stk[top++] = (tok == P_SUM) ? a + b : a * b;
+    }
+  }
+  return stk[0];
+}
+
 __global__ void __launch_bounds__(256) k_prep_planes(const Prob* __restrict__ probs) {
   const Prob& P = probs[blockIdx.z];
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   const int l = blockIdx.y;
-  if (P.mode != 1 || i >= P.Nc) return;
+  if (P.mode != 1 || (int)(blockIdx.x * blockDim.x) >= P.Nc) return;
   const Spec& sp = *P.spec;
   const size_t nc = (size_t)P.Nc;
+  if (l == 0) {
+    // the scale 2^e > sqrt(K_ii): the kernels are stationary, so K_ii is one
+    // value, the expression with every distance leaf at 1, plus the nugget
+    __shared__ int s_e;
+    if (threadIdx.x == 0) {
+      const double d = kernel_diagonal(sp, P.theta) + (P.optimise_noise ? P.theta[sp.nkparams] : P.noise);
+      int e = 0;
+      if (d > 0.0 && d < 1e300) frexp(sqrt(d) * (1.0 + 0x1p-20), &e);  // sqrt(K_ii) (1 + 2^-20) < 2^e
+      s_e = e;
+      if (blockIdx.x == 0) P.kscale[0] = e;
+    }
+    __syncthreads();
+    // right-hand sides: y - mu (marginal), or y and 1 (concentrated), in the factor's scale; zero on the padding
+    if (i < P.Nc) {
+      const double w = ldexp(1.0, -s_e);
+      P.rhs[i] = i < P.N ? w * (P.likelihood == 1 ? P.y[i] : P.y[i] - P.mu[i]) : 0.0;
+      if (P.nrhs > 1) P.rhs[nc + i] = i < P.N ? w : 0.0;
+    }
+  }
+  if (i >= P.Nc) return;
   // the workspace is not cleared between evaluations (a batch plan reuses
   // it across problems): rows of non-rbf leaves are zeroed here
   if (l >= sp.nleaf || sp.leaf[l].type != L_RBF) P.norms[(size_t)l * nc + i] = 0.0;
@@ -274,9 +319,9 @@ size_t build_dot_smem_bytes(int nplanes) {
 __global__ void __launch_bounds__(256) k_build_dot(const Prob* __restrict__ probs) {
   const Prob& P = probs[blockIdx.z];
   const int ti = blockIdx.x, tj = blockIdx.y;
-  if (P.mode != 1 || tj >= P.nsteps || ti > P.nsteps || ti < tj) return;
+  if (P.mode != 1 || tj >= P.nsteps || ti >= P.nsteps || ti < tj) return;
   const Spec& sp = *P.spec;
-  if (sp.tc_build && ti != P.nsteps) return;  // built on the tensor cores; only its RHS rows here
+  if (sp.tc_build) return;  // built on the tensor cores
   extern __shared__ __align__(128) unsigned char smem_raw[];
   const int np = sp.nplanes;
   const int nl = sp.nleaf;
@@ -289,7 +334,6 @@ __global__ void __launch_bounds__(256) k_build_dot(const Prob* __restrict__ prob
   __shared__ double leaf_c[MAX_LEAF];  // sum of l (periodic) or sum of 1/c (linear)
   __shared__ int s_fail;
   const int tid = threadIdx.x;
-  const bool border = (ti == P.nsteps);
   const int i0 = ti * TB, j0 = tj * TB;
   const size_t nc = (size_t)P.Nc;
   if (tid == 0) {
@@ -301,14 +345,14 @@ __global__ void __launch_bounds__(256) k_build_dot(const Prob* __restrict__ prob
   if (tid == 0) {
     const uint32_t per = TB * sizeof(double);
     const uint32_t nrows = (uint32_t)(np + nl);
-    mbar_expect_tx(bar, per * nrows * (border ? 1 : 2));
+    mbar_expect_tx(bar, per * nrows * 2);
     for (int p = 0; p < np; ++p) {
       bulk_g2s(Pj + p * TB, P.splanes + (size_t)p * nc + j0, per, bar);
-      if (!border) bulk_g2s(Pi + p * TB, P.splanes + (size_t)p * nc + i0, per, bar);
+      bulk_g2s(Pi + p * TB, P.splanes + (size_t)p * nc + i0, per, bar);
     }
     for (int l = 0; l < nl; ++l) {
       bulk_g2s(Nj + l * TB, P.norms + (size_t)l * nc + j0, per, bar);
-      if (!border) bulk_g2s(Ni + l * TB, P.norms + (size_t)l * nc + i0, per, bar);
+      bulk_g2s(Ni + l * TB, P.norms + (size_t)l * nc + i0, per, bar);
     }
   }
   for (int k = tid; k < sp.nkparams; k += blockDim.x) {
@@ -338,21 +382,20 @@ __global__ void __launch_bounds__(256) k_build_dot(const Prob* __restrict__ prob
     }
     return;
   }
+  bool nonfinite = false;
   const double noise = P.optimise_noise ? P.theta[sp.nkparams] : P.noise;
   const int r0 = (tid & 31) * 2;
   const int c0 = (tid >> 5) * 8;
-  double* K = P.K;
-  const size_t ld = (size_t)P.ld;
+  const int e2 = 2 * *P.kscale;
+  // 64 x 64 tile (ti, tj): rows (ti & 1) * 64 .. of the 128 x 64 accumulator tile
+  long long* A = P.acc + acc_tile(ti >> 1, tj, P.nt128) * ACC_TILE_ELEMS;
   for (int cc = 0; cc < 8; ++cc) {
     const int c = c0 + cc, j = j0 + c;
-    double v[2];
+    long long v[2];
     for (int a = 0; a < 2; ++a) {
       const int r = r0 + a, i = i0 + r;
-      double val = 0.0;
-      if (border) {
-        if (j < P.N && r < P.nrhs)
-          val = (r == 0) ? ((P.likelihood == 1) ? P.y[j] : P.y[j] - P.mu[j]) : 1.0;
-      } else if (i < P.N && j < P.N) {
+      long long val = 0;
+      if (i < P.N && j < P.N) {
         if (i >= j) {
           double stk[MAX_LEAF];
           int top = 0;
@@ -381,16 +424,16 @@ __global__ void __launch_bounds__(256) k_build_dot(const Prob* __restrict__ prob
               stk[top++] = (tok == P_SUM) ? a2 + b : a2 * b;
             }
           }
-          val = stk[0];
-          if (i == j) val = val + noise * 1.0;
+          val = i == j ? diag_fixed62(stk[0], noise, e2, &nonfinite) : to_fixed62(stk[0], e2, &nonfinite);
         }
       } else {
-        val = (i == j) ? 1.0 : 0.0;
+        val = (i == j) ? 1LL << 60 : 0LL;  // identity padding, 1/4 in the matrix's unit
       }
       v[a] = val;
     }
-    *reinterpret_cast<double2*>(K + (size_t)j * ld + i0 + r0) = make_double2(v[0], v[1]);
+    *reinterpret_cast<longlong2*>(A + acc_elem((ti & 1) * TB + r0, c)) = make_longlong2(v[0], v[1]);
   }
+  if (nonfinite) atomicOr(&P.status[3], 1);
 }
 
 // ---------------------------------------------------------------------------
@@ -571,12 +614,14 @@ __global__ void __launch_bounds__(256) k_finalize(const Prob* __restrict__ probs
     }
     return;
   }
-  const size_t ld = (size_t)P.ld;
-  const double* z0 = P.K + P.Nc;      // row Nc: r_0 = y - mu (marginal) or y (concentrated)
-  const double* z1 = P.K + P.Nc + 1;  // row Nc+1: ones (concentrated)
+  // L^-1 r_0, r_0 = y - mu (marginal) or y (concentrated), and L^-1 1
+  // (concentrated): border rows of K, or the right-hand-side array
+  const size_t ld = P.mode == 1 ? 1 : (size_t)P.ld;
+  const double* z0 = P.mode == 1 ? P.rhs : P.K + P.Nc;
+  const double* z1 = P.mode == 1 ? P.rhs + P.Nc : P.K + P.Nc + 1;
   double logdet = 0.0;
   if (tid == 0) {
-    const int nparts = P.mode == 1 ? P.Nc / QW : P.nsteps;  // 32-column parts in tensor-core mode
+    const int nparts = P.mode == 1 ? P.nt128 : P.nsteps;  // one part per panel
     for (int s = 0; s < nparts; ++s) logdet += P.logdet_part[s];
     logdet *= 2.0;
   }
@@ -694,19 +739,13 @@ cudaError_t launch_prep_planes(const Prob* probs, int nprob, int max_nc, cudaStr
 cudaError_t launch_build_dot(const Prob* probs, int nprob, int max_nsteps, int max_nplanes, cudaStream_t s) {
   cudaError_t e = ensure_smem_attr((const void*)k_build_dot, SMEM_BUILD_DOT, (int)build_dot_smem_bytes(MAX_PLANES));
   if (e != cudaSuccess) return e;
-  dim3 grid(max_nsteps + 1, max_nsteps, nprob);
+  dim3 grid(max_nsteps, max_nsteps, nprob);
   k_build_dot<<<grid, 256, build_dot_smem_bytes(max_nplanes), s>>>(probs);
   return cudaGetLastError();
 }
 
 cudaError_t launch_potf2(const Prob* probs, int nprob, int step, cudaStream_t s) {
   k_potf2w<TB><<<nprob, TB * 4, 0, s>>>(probs, step * TB, 0, step, 0);
-  return cudaGetLastError();
-}
-
-cudaError_t launch_potf2_quarter(const Prob* probs, int nprob, int step, int q, cudaStream_t s) {
-  // log-det parts indexed by 32-column block
-  k_potf2w<QW><<<nprob, QW * 4, 0, s>>>(probs, step * NB, q * QW, step * (NB / QW), q);
   return cudaGetLastError();
 }
 

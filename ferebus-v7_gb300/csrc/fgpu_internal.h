@@ -13,6 +13,10 @@
 //             Rows [Nc, Nc + nrhs): the right-hand sides r_q^T (border rows);
 //             the Cholesky sweep turns them into (L^-1 r_q)^T, which is all
 //             the log-likelihood needs.  Rows [Nc + nrhs, ld): zero.
+//
+// Tensor-core mode keeps the matrix as 64-bit fixed point instead (acc), the
+// right-hand sides in an array of their own (rhs), and K only where the
+// factor itself is wanted.
 #pragma once
 #include <cuda_runtime.h>
 #include <cstdint>
@@ -55,6 +59,19 @@ struct Spec {
   int dot_u[2];                   // W units: <f_i, f_j> 2^(u - 2 - 2s)
 };
 
+// A 16 x 16 diagonal block of the factor (panel.cu): its entries L'_jc 2^60 as
+// (high, low) 30-bit halves, and 1 / L'_jj = y 2^(sh - 62).
+struct alignas(16) PanelBlock {
+  int2 x[16][16];
+  unsigned long long y[16];
+  int sh[16];
+};
+// 16 entries of each solved right-hand side, z = (x as above) 2^-60 scale
+struct alignas(16) PanelZ {
+  int2 x[MAX_RHS][16];
+  double scale[MAX_RHS];
+};
+
 // Per-problem descriptor, resident in device memory.
 struct Prob {
   int N, Nc, ld, nsteps, nrhs, likelihood, optimise_noise, nkparams;
@@ -74,15 +91,16 @@ struct Prob {
   // tensor-core (split-integer) trailing update; unused in FP64 mode
   int mode;                       // 0: FP64 mma.sync 64-panels, 1: tcgen05 split update, 128-panels
   int nt128;                      // Nc / 128 (mode 1)
-  int* escale;                    // Nc: per-row power-of-two scale e_i, |L_ik| <= 2^e_i
-  double* pw2;                    // Nc: 2^(e_i - 31)
-  long long* acc;                 // lower-triangle 128 x 64 tiles: exact sums of products W, value
-                                  // W 2^(e_i + e_j - 62); |W| < 2^62 (Cauchy-Schwarz with the row scales)
+  int* kscale;                    // [0]: the scale e, K_ii < 2^2e for every i
+  long long* acc;                 // lower-triangle 128 x 64 tiles: K, then its Schur complements, value A 2^(2e - 62)
   unsigned char* slices;          // nt128 x 7 x 32 KB: fp16 digit planes of the current panel
   const void* tmap_a;             // TMA tensor map over slices, box 8 x 128 rows x 2 kgroups x 7 planes
   const void* tmap_b;             // same, box of 64 rows
   const void* tmap_bs;            // box of 64 rows landing as [k-group][plane][row]: the 7 planes stacked along N
-  const void* tmap_bs32;          // same, box of 32 rows
+  double* rhs;                    // MAX_RHS x Nc: right-hand sides times 2^-e, turned into L^-1 r panel by panel
+  PanelBlock* lpub;               // 8: the current panel's diagonal blocks, as its diagonal tile publishes them
+  PanelZ* zpub;                   // 8: and its solved right-hand-side entries
+  int keep_l;                     // K exists and receives the factor (alpha and the adjoint read it)
   // dot-product kernel build (mode 1): planes scaled by sqrt(l_k) per evaluation
   double* splanes;                // nplanes x Nc
   double* norms;                  // MAX_LEAF x Nc: sum_k u_ik^2 of rbf leaves
@@ -102,9 +120,10 @@ struct Prob {
   int* fscale;                    // 2: s of the distance leaves, max |f| < 2^s
 };
 
-// Encode the four 5-D TMA tensor maps of a problem's digit-plane buffer
-// (boxes of 128 and 64 rows, and 64 and 32 rows with the planes stacked)
-// into host memory (4 x 128 bytes).  Returns 0 or a CUDA driver error code.
+// Encode the three 5-D TMA tensor maps of a problem's digit-plane buffer
+// (boxes of 128 and 64 rows, and 64 rows with the planes stacked) into host
+// memory (TMAP_BYTES).  Returns 0 or a CUDA driver error code.
+constexpr size_t TMAP_BYTES = 3 * 128;
 int encode_slice_maps(void* host_maps, const void* slices, int nt128);
 
 // Launch helpers (engine.cu).  All kernels take a device array of problems
@@ -116,13 +135,6 @@ cudaError_t launch_prep_planes(const Prob* probs, int nprob, int max_nc, cudaStr
 cudaError_t launch_build_dot(const Prob* probs, int nprob, int max_nsteps, int max_nplanes, cudaStream_t s);
 size_t build_dot_smem_bytes(int nplanes);
 cudaError_t launch_potf2(const Prob* probs, int nprob, int step, cudaStream_t s);
-// tensor-core mode: the 32 x 32 diagonal block of quarter q of panel step, and
-// the rows below it up to max_rows (the tallest problem's ld), which also
-// writes their fp16 digit planes
-constexpr int QW = 32;
-cudaError_t launch_potf2_quarter(const Prob* probs, int nprob, int step, int q, cudaStream_t s);
-// quarter panel solve (ozaki.cu): FP64 substitution in two 16-column halves coupled on the tensor cores
-cudaError_t launch_trsm_quarter(const Prob* probs, int nprob, int step, int q, int max_rows, cudaStream_t s);
 // max_rowtiles: 64-row tiles of the tallest problem (0 = max_nsteps + 1)
 cudaError_t launch_trsm(const Prob* probs, int nprob, int step, int max_nsteps, cudaStream_t s,
                         int max_rowtiles = 0);
@@ -137,7 +149,7 @@ size_t build_smem_bytes(int nplanes);
 constexpr int NB = 128;
 constexpr int NSLICE = 7;                       // fp16 digit planes per FP64 value
 constexpr size_t SLICE_BYTES = 128 * 128 * 2;   // one digit plane of a 128-row x 128-k tile
-// The exact trailing sums are kept for lower-triangle tiles only (128 rows x
+// The fixed-point matrix is kept for lower-triangle tiles only (128 rows x
 // 64 columns), one int64 per element: column tile tj holds row tiles tj / 2
 // .. nt128 - 1, so a problem stores nt128 (nt128 + 1) tiles instead of
 // (2 nt128) nt128.  acc_tile is the tile's index in that packed order.
@@ -155,24 +167,19 @@ __host__ __device__ inline int acc_elem(int r, int c) {  // row r < 128, column 
 }
 constexpr size_t ACC_TILE_ELEMS = (size_t)NB * TB;
 
-cudaError_t launch_scales(const Prob* probs, int nprob, int max_nc, cudaStream_t s);
-cudaError_t launch_panel_prep(const Prob* probs, int nprob, int step, int max_nc, cudaStream_t s);
+// One panel of the factorisation (panel.cu), of every problem with a panel
+// `step`.  order: the step's row tiles as (problem << 16 | tile), first the
+// ndiag own row tiles, then the others, total_tiles in all; counter: a
+// zeroed int the CTAs take tiles from; flags: PANEL_FLAGS ints per problem,
+// zeroed once per evaluation.
+constexpr int PANEL_FLAGS = 32;            // one 128-byte line per problem
+cudaError_t launch_panel(const Prob* probs, int step, const int* order, int ndiag, int total_tiles, int* counter,
+                         int* flags, int num_sms, cudaStream_t s);
 // prefix: device table of nprob + 1 tile offsets for this step (tiles of
 // problem p at step s: m (m + 1), m = nt128_p - s - 1); total_tiles = prefix[nprob].
 // tiles: the step's trailing tiles, packed (problem << 40 | row tile << 20 | column tile)
 cudaError_t launch_ozaki_update(const Prob* probs, int nprob, int step, int max_nt128,
                                 const unsigned long long* tiles, int total_tiles, int num_sms, cudaStream_t s);
-cudaError_t launch_border_update(const Prob* probs, int nprob, int step, int max_nc, cudaStream_t s);
-// four 32-column quarters per 128-panel (their digit planes are written by
-// the quarter panel solve): the tensor-core coupling of source quarters
-// [sq, sq + ns) into destination quarters [dq, dq + nq), nq = 1 or 2 (with
-// the right-hand-side rows in FP64), which also factors quarter dq's
-// diagonal block.  order: the step's total_tiles row tiles as
-// (problem << 16 | ti), each problem's own row tile first; counter: a zeroed
-// int the CTAs take tiles from.
-cudaError_t launch_couple(const Prob* probs, int nprob, int step, int sq, int ns, int dq, int nq,
-                          const int* order, int total_tiles, int* counter, int num_sms, cudaStream_t s);
-
 // Tensor-core kernel-matrix build (build_tc.cu): feature digit planes and
 // exact self products, then the persistent build of the lower triangle.
 // tiles: the lower triangle's 128 x 64 tiles of every eligible problem,
@@ -195,7 +202,7 @@ constexpr int GRAD_SLOTS = 33;  // parameters per fused pass + noise slot
 // device, or a second thread, sets the attribute for itself.  Devices
 // beyond the first 64 set it on every call.
 enum SmemSlot {
-  SMEM_BUILD, SMEM_BUILD_DOT, SMEM_UPDATE, SMEM_SYRK, SMEM_OZAKI_UPDATE, SMEM_COUPLE1, SMEM_COUPLE2,
+  SMEM_BUILD, SMEM_BUILD_DOT, SMEM_UPDATE, SMEM_SYRK, SMEM_OZAKI_UPDATE, SMEM_PANEL,
   SMEM_BUILD_TC, SMEM_NSLOTS
 };
 cudaError_t ensure_smem_attr(const void* func, int slot, int bytes);

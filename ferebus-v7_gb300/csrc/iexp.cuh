@@ -88,13 +88,22 @@ struct IexpScale {
 };
 __device__ __forceinline__ IexpScale iexp_scale(int e) { return IexpScale{63 - e}; }
 
-__device__ __forceinline__ double iexp_fixed_tab(unsigned long long E, IexpScale sc,
-                                                 const unsigned long long* __restrict__ tab1024,
-                                                 const unsigned long long* __restrict__ fine1024) {
-  if (E == 0) return 1.0;
+// exp(-E 2^e) = Z 2^-62 2^-m, 2^62 <= Z <= 2^63 (m >= 1100: below every double)
+struct IexpParts {
+  unsigned long long Z;
+  int m;
+};
+__device__ __forceinline__ IexpParts iexp_fixed_parts(unsigned long long E, IexpScale sc,
+                                                      const unsigned long long* __restrict__ tab1024,
+                                                      const unsigned long long* __restrict__ fine1024) {
   const int K0 = sc.K0;
-  if (K0 >= 192) return 1.0;                   // y < 2^-64: rounds to 1
-  if (K0 < 64) return iexp_fixed(E, 63 - K0);  // outside this form's range
+  if (E == 0 || K0 >= 192) return IexpParts{1ULL << 62, 0};  // 1, or y < 2^-64: rounds to 1
+  if (K0 < 64) {  // outside this form's range
+    const unsigned long long bits = (unsigned long long)__double_as_longlong(iexp_fixed(E, 63 - K0));
+    const int ef = (int)(bits >> 52);
+    if (ef == 0) return IexpParts{1ULL << 62, 1100};
+    return IexpParts{((bits & 0xFFFFFFFFFFFFFULL) | 0x10000000000000ULL) << 10, 1023 - ef};
+  }
   const unsigned long long plo = E * IEXP_L2E64, phi = __umul64hi(E, IEXP_L2E64);
   unsigned long long yi, yf;  // y = yi + yf 2^-64
   if (K0 >= 128) {
@@ -104,8 +113,7 @@ __device__ __forceinline__ double iexp_fixed_tab(unsigned long long E, IexpScale
     yi = phi >> (K0 - 64);
     yf = K0 == 64 ? plo : ((plo >> (K0 - 64)) | (phi << (128 - K0)));
   }
-  if (yi >= 1100) return 0.0;
-  const unsigned int m = (unsigned int)yi + (yf ? 1u : 0u);
+  const int m = yi >= 1100 ? 1100 : (int)yi + (yf ? 1 : 0);
   const unsigned long long f = 0ULL - yf;  // (m - y) 2^64
   const int j = (int)(f >> 54);
   const int k = (int)(f >> 44) & 1023;
@@ -116,16 +124,30 @@ __device__ __forceinline__ double iexp_fixed_tab(unsigned long long E, IexpScale
   const unsigned long long dk = fine1024[k];                                  // (2^(k/2^20) - 1) 2^64 < 2^53.5
   const unsigned long long de = ((dk >> 22) * (eps >> 12)) >> 30;            // their product, 2^64
   const unsigned long long p = (1ULL << 63) + ((dk + eps + de) >> 1);       // 2^(k/2^20) exp(t) 2^63
-  const unsigned long long Z = __umul64hi(tab1024[j], p);                   // 2^(g) 2^62
-  const int top = (int)(Z >> 63);
+  return IexpParts{__umul64hi(tab1024[j], p), m};                           // 2^(g) 2^62
+}
+
+__device__ __forceinline__ double iexp_fixed_tab(unsigned long long E, IexpScale sc,
+                                                 const unsigned long long* __restrict__ tab1024,
+                                                 const unsigned long long* __restrict__ fine1024) {
+  const IexpParts v = iexp_fixed_parts(E, sc, tab1024, fine1024);
+  if (v.m >= 1100) return 0.0;
+  const int top = (int)(v.Z >> 63);
   const int sh = 10 + top;
-  const int be = 1023 + top - (int)m;
+  const int be = 1023 + top - v.m;
   if (be >= 1) {
-    const unsigned long long mant = (Z + (1ULL << (sh - 1))) >> sh;
+    const unsigned long long mant = (v.Z + (1ULL << (sh - 1))) >> sh;
     return __longlong_as_double((long long)(((unsigned long long)be << 52) + mant - (1ULL << 52)));
   }
   const int tot = sh + 1 - be;
   if (tot > 64) return 0.0;
-  const unsigned long long mant = (tot == 64) ? (Z >> 63) : ((Z + (1ULL << (tot - 1))) >> tot);
+  const unsigned long long mant = (tot == 64) ? (v.Z >> 63) : ((v.Z + (1ULL << (tot - 1))) >> tot);
   return __longlong_as_double((long long)mant);
+}
+
+// round(exp(-E 2^e) 2^(62 - e2)), e2 >= 1: the value straight in the matrix's
+// fixed-point unit
+__device__ __forceinline__ long long iexp_parts_fixed62(IexpParts v, int e2) {
+  const int sh = v.m + e2;
+  return sh > 63 ? 0LL : (long long)((v.Z + (1ULL << ((sh - 1) & 63))) >> (sh & 63));
 }

@@ -1,0 +1,704 @@
+// One panel of the Cholesky factorisation (tensor-core mode): the 128 columns
+// [c0, c0 + 128) of every problem in one launch, from the fixed-point Schur
+// complement to the factor's digit planes.
+//
+// Everything is in the problem's scale 2^e (K_ii < 2^2e; every K_ii of these
+// kernels is the same): the accumulators hold S_ij 2^(62 - 2e), S = K minus the
+// exact products of the earlier panels, and the factor computed here is
+// L' = 2^-e L, so that every value lies in [-1, 1].
+//
+// A CTA owns one 128-row tile of one problem (or a 64- or 32-row part of one)
+// and walks the panel's 128 columns in 8 pieces of 16.  For piece t:
+//
+//   B_ij = S_ij - sum_{k < 16 t} L'_ik L'_jk  in 64-bit integers: the couplings
+//          inside the panel come from tcgen05.mma on the digit planes (7 exact
+//          level sums, as in the trailing update);
+//   x L'_tt^T = B by substitution, one thread per row, in 60-bit fixed point
+//          (below);
+//   x's 7 fp16 digit planes into shared memory (the A operand of the later
+//          pieces' couplings) and to HBM (the trailing update's operands).
+//
+// The tile that holds the panel's own rows (the diagonal tile) factors the
+// 16 x 16 diagonal blocks on the way, and publishes each piece -- the block
+// and its reciprocal pivots, its rows' digits, the solved right-hand-side
+// entries z -- through release/acquire counters in HBM that the problem's
+// other CTAs poll (bounded).  CTAs take their tile from an atomic ticket,
+// diagonal tiles first: whoever waits for a diagonal tile holds a later
+// ticket than it, so the tile is already running, and a diagonal tile itself
+// waits for nobody.  The right-hand sides ride along: each row's thread
+// accumulates sum_k L'_ik z_k while x is in registers.
+//
+// Arithmetic.  This GPU's FP64 unit takes 64 cycles per warp instruction and
+// SM quarter, for dependent and independent operations alike, so a piece's 136
+// multiply-adds per row cost 10k cycles there whatever their order.  In fixed
+// point, X = x 2^60 split as X = Xh 2^30 + Xl (|Xl| <= 2^29),
+//   x l = (Xh Lh + (Xh Ll + Xl Lh) 2^-30) 2^-60 + O(2^-62),
+// is three 32 x 32 + 64-bit multiply-adds on the integer pipe (~10 cycles).
+// The dropped Xl Ll and the final shifts err by a few 2^-61, well below the
+// 2^-56 to which x is rounded for the trailing update.  The 64-bit sums cannot
+// overflow: rows of L' have norm at most 1, so sum |Xh Ll| <= 2^30 2^29 4.
+// Only the right-hand sides' substitution (32 operations per piece, off the
+// critical path) and their running sums (one per row and piece) are FP64.
+//
+// Bounds.  A lone problem is bound by the diagonal tile's chain of 128
+// pivots, a batch by integer issue (one warp per SM quarter: latency).  The 7
+// digit chunks the couplings read (28 KB each) stay in shared memory, hence
+// one CTA per SM.  Measured, against the FP64 panel in ten launches
+// (conversion of the integer sums, 32-column factors, solves and couplings,
+// right-hand-side update) that this replaces: a lone problem 250 -> 95 us
+// per panel (N = 4000, 32 panels), a swarm of 40 at N = 4000 20.7 -> 9.8 ms.
+#include "fgpu_internal.h"
+#include "tc_common.cuh"
+
+#include <cuda_fp16.h>
+
+namespace fgpu {
+namespace {
+
+constexpr int PW = 16;                 // piece width
+constexpr int NPIECE = NB / PW;        // pieces of a panel
+constexpr uint32_t PN_ACHUNK = NSLICE * 4096;       // one piece's digits of 128 rows: [plane][k-group 2][row 128][8 x fp16]
+constexpr uint32_t PN_BCHUNK = NSLICE * 2 * PW * 16;  // one piece's digits of the next piece's 16 rows: [k-group 2][plane][row 16][8 x fp16]
+constexpr uint32_t PN_LBYTES = sizeof(PanelBlock);
+constexpr uint32_t PN_ZBYTES = sizeof(PanelZ);
+static_assert(PN_LBYTES % 16 == 0 && PN_ZBYTES % 16 == 0, "copied 16 bytes at a time");
+constexpr uint32_t PN_OFF_B = (NPIECE - 1) * PN_ACHUNK;
+constexpr uint32_t PN_OFF_L = PN_OFF_B + (NPIECE - 1) * PN_BCHUNK;
+constexpr uint32_t PN_OFF_Z = PN_OFF_L + 2 * PN_LBYTES;
+constexpr uint32_t PN_OFF_R = PN_OFF_Z + 2 * PN_ZBYTES;
+constexpr uint32_t PN_OFF_BAR = PN_OFF_R + MAX_RHS * PW * 8;
+constexpr uint32_t PN_SMEM = PN_OFF_BAR + 64;
+static_assert(PN_SMEM + 1024 <= 227 * 1024, "shared memory per CTA");
+constexpr int PN_MMA_WARP = 4, PN_RHS_WARP = 5;
+constexpr int PN_THREADS = 32 * 6;  // 4 row warps, operand loads and MMA issue, right-hand sides
+constexpr uint32_t PN_TMEM_COLS = 128;  // 7 levels x 16 columns, rounded up
+constexpr int FLAG_L = 0, FLAG_D = 1, FLAG_Z = 2;  // a problem's counters: blocks, digits, z published
+constexpr int FLAG_FAIL = 1 << 30;                  // the diagonal tile met a non-positive pivot (or gave up)
+
+__device__ __forceinline__ int ld_acquire(const int* p) {
+  int v;
+  asm volatile("ld.acquire.gpu.global.s32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
+  return v;
+}
+__device__ __forceinline__ void st_release(int* p, int v) {
+  asm volatile("st.release.gpu.global.s32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
+}
+__device__ __forceinline__ void cp_async16(void* dst, const void* src) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(su32(dst)), "l"(src) : "memory");
+}
+__device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_all;" ::: "memory"); }
+
+// 1 / sqrt(D 2^-62), 0 < D < 2^62, as y 2^(sh - 62) with y in [2^62, 2^63): a
+// single-precision estimate refined once in 64-bit fixed point.  With
+// D 2^-62 = m 4^k, 1 <= m < 4 (k < 0, sh = -k - 1), and y0 ~ m^-1/2 (24 bits):
+// e = 1 - m y0^2 is formed to 2^-61 (|e| < 2^-20) and m^-1/2 =
+// y0 (1 - e)^-1/2 = y0 (1 + e/2 + 3 e^2 / 8 + O(2^-61)).  Relative error below
+// 2^-58.  About 130 cycles of integer latency; the library's FP64 rsqrt
+// takes ~380, and 128 of them follow one another in a panel.
+__device__ __forceinline__ void rsqrt_fixed(long long D, unsigned long long& y, int& sh) {
+  const int lz = __clzll(D);
+  const unsigned long long A = (unsigned long long)D << (lz & 63);  // leading one at bit 63
+  const int E = 1 - lz, r = E & 1;                                  // D 2^-62 = 1.f 2^E
+  sh = -(E >> 1) - 1;
+  const unsigned long long M = A >> (1 - r);  // m 2^62
+  const float mf = __uint_as_float(((unsigned)(127 + r) << 23) | ((unsigned)(A >> 40) & 0x7FFFFFu));
+  float y0;
+  asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(y0) : "f"(mf));
+  const unsigned yb = __float_as_uint(fminf(fmaxf(y0, 0.5f), 1.0f));
+  const unsigned Y = ((yb & 0x7FFFFFu) | 0x800000u) << ((yb >> 23) - 126u);  // y0 2^24
+  const unsigned long long YY = (unsigned long long)Y * Y;
+  const long long e = (long long)((1ULL << 61) - __umul64hi(M, YY << 15));   // e 2^61
+  const int eh = (int)(e >> 10);
+  const unsigned long long e2 = (unsigned long long)((long long)eh * eh);    // e^2 2^102
+  const long long c = (e >> 1) + (long long)((3ULL * e2) >> 44);             // (e/2 + 3 e^2/8) 2^61
+  const unsigned long long v = ((unsigned long long)Y << 39) + (unsigned long long)(((long long)Y * (c >> 2)) >> 20);
+  y = v < 0x7FFFFFFFFFFFFFFFULL ? v : 0x7FFFFFFFFFFFFFFFULL;
+}
+
+// X = x 2^60 of x = T 2^-62 / L'_jj, split in Xh 2^30 + Xl.  |x| <= 1 while
+// the matrix is positive semidefinite, i.e. |T| < 2^(62 - sh); a larger |T|
+// clamps to +-1 (which fails the row's pivot).
+__device__ __forceinline__ void scale_entry(long long T, unsigned long long y, int sh, int& Xh, int& Xl) {
+  const int lim = 1 << (30 - sh);
+  const int th = (int)(T >> 32);
+  long long X = __mul64hi(T << sh, (long long)y);
+  if ((unsigned)(th + lim) >= 2u * (unsigned)lim) X = T < 0 ? -(1LL << 60) : 1LL << 60;
+  Xh = min(max((int)((X + (1LL << 29)) >> 30), -(1 << 30)), 1 << 30);
+  Xl = (int)((unsigned)X - ((unsigned)Xh << 30));
+}
+
+// The 7 fp16 digit planes of 8 entries X = x 2^60 (one k-group of a row),
+// packed: F = x 2^55 rounded has the balanced digits
+// d_p in [-128, 127] (p = 1..6, base 256, lowest last) and d_0 = the rest.
+// G = F + sum_{k<6} 128 256^k turns them into plain bytes: byte 6 - p of G
+// is d_p + 128, and G >> 48 is d_0 (|d_0| <= 128 when |x| <= 1).  A byte
+// u under the fp16 exponent bits 0x64 is the half 1024 + u, so one HSUB2 of
+// 1152 per pair of entries yields the digits exactly, with no conversion
+// instruction; two byte permutes place a pair's bytes under the 0x64 bytes.
+__device__ __forceinline__ void digits8_packed(const int* Xh, const int* Xl, uint4 out[NSLICE]) {
+  unsigned lo[8], hi[8];
+#pragma unroll
+  for (int kk = 0; kk < 8; ++kk) {
+    const long long X = (long long)Xh[kk] * (1LL << 30) + Xl[kk];
+    const long long G = ((X + 16) >> 5) + 0x808080808080LL;
+    lo[kk] = (unsigned)G;
+    hi[kk] = (unsigned)(G >> 32);
+  }
+  const __half2 off = __halves2half2(__ushort_as_half(0x6480), __ushort_as_half(0x6480));  // 1152
+#pragma unroll
+  for (int p = 0; p < NSLICE; ++p) {
+    unsigned w[4];
+#pragma unroll
+    for (int m = 0; m < 4; ++m) {
+      unsigned bits;
+      if (p == 0) {  // d_0 + 128 may be 256: arithmetic, not a byte
+        const unsigned u0 = (unsigned)(((int)hi[2 * m] >> 16) + 128);
+        const unsigned u1 = (unsigned)(((int)hi[2 * m + 1] >> 16) + 128);
+        bits = (0x6400u + u0) | ((0x6400u + u1) << 16);
+      } else {
+        const int q = 6 - p;  // byte of G: byte q & 3 of the low or high word
+        const unsigned wa = q < 4 ? lo[2 * m] : hi[2 * m], wb = q < 4 ? lo[2 * m + 1] : hi[2 * m + 1];
+        const unsigned t = __byte_perm(wa, 0x64646464u, 0x4440u | (unsigned)(q & 3));  // [a_q, 64, 64, 64]
+        bits = __byte_perm(wb, t, 0x7054u | ((unsigned)(q & 3) << 8));                  // [a_q, 64, b_q, 64]
+      }
+      const __half2 h = __hsub2(*reinterpret_cast<const __half2*>(&bits), off);
+      w[m] = *reinterpret_cast<const unsigned*>(&h);
+    }
+    out[p] = make_uint4(w[0], w[1], w[2], w[3]);
+  }
+}
+
+// the whole warp waits for an mbarrier phase (bounded), or until the CTA
+// stops: 0 the phase completed, 1 stopped, 2 gave up (the same in every lane)
+__device__ __forceinline__ int wait_or_stop(uint64_t* bar, uint32_t parity, const int* stop) {
+  int r = 2;
+  for (int it = 0; it < (1 << 22); ++it) {
+    if (mbar_wait_n(bar, parity, 1)) {
+      r = 0;
+      break;
+    }
+    if (*(volatile const int*)stop) {
+      r = 1;
+      break;
+    }
+  }
+  if (__all_sync(0xffffffffu, r == 0)) return 0;
+  return __any_sync(0xffffffffu, r == 2) ? 2 : 1;
+}
+
+__device__ __forceinline__ void tmem_ld8(uint32_t (&v)[8], uint32_t addr) {
+  asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
+               : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7])
+               : "r"(addr));
+}
+__device__ __forceinline__ uint32_t tmem_ld1(uint32_t addr) {
+  uint32_t v;
+  asm volatile("tcgen05.ld.sync.aligned.32x32b.x1.b32 {%0}, [%1];" : "=r"(v) : "r"(addr));
+  return v;
+}
+
+// one lane polls a problem's counter until it reaches `want` (bounded)
+__device__ __forceinline__ int poll_flag(const int* f, int want) {
+  for (int it = 0; it < (1 << 22); ++it) {
+    const int v = ld_acquire(f);
+    if (v >= want) return v;
+    __nanosleep(it < 64 ? 20 : 200);
+  }
+  return -1;
+}
+
+}  // namespace
+
+__global__ void __launch_bounds__(PN_THREADS, 1)
+    k_panel(const Prob* __restrict__ probs, int s, const int* __restrict__ order, int ndiag, int sub_shift,
+            int* __restrict__ counter, int* __restrict__ flags) {
+  extern __shared__ __align__(1024) unsigned char smp[];
+  unsigned char* As = smp;
+  unsigned char* Bs = smp + PN_OFF_B;
+  PanelBlock* Ls = reinterpret_cast<PanelBlock*>(smp + PN_OFF_L);  // [2]: this piece's diagonal block
+  PanelZ* Zs = reinterpret_cast<PanelZ*>(smp + PN_OFF_Z);          // [2]: this piece's z
+  double* Rs = reinterpret_cast<double*>(smp + PN_OFF_R);  // diagonal tile: right-hand-side entries of the piece's rows
+  uint64_t* b_mma = reinterpret_cast<uint64_t*>(smp + PN_OFF_BAR);  // a piece's couplings are in TMEM
+  uint64_t* b_blk = b_mma + 1;                                      // its block is in Ls
+  uint64_t* b_z = b_mma + 2;                                        // its z is in Zs
+  uint64_t* b_drained = b_mma + 3;                                  // the row warps hold its couplings in registers
+  uint64_t* b_digits = b_mma + 4;                                   // the row warps' digits are in As (and in HBM)
+  uint64_t* b_pub = b_mma + 5;                                      // diagonal tile: the digits are in HBM
+  uint64_t* b_quiet = b_mma + 6;                                    // quiescing before an early exit
+  __shared__ int s_tile, s_sub, s_skip, s_stop, s_abort;
+  __shared__ uint32_t s_tmem;
+  __shared__ long long s_D[2][PW];  // the pieces' pivots, in the matrix's unit
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  if (tid == 0) {
+    const int u = atomicAdd(counter, 1);
+    // the order lists every problem's own row tile first, then the others
+    const int v = u - ndiag;
+    const int id = u < ndiag ? order[u] : order[ndiag + (v >> sub_shift)];
+    s_tile = id;
+    s_skip = *(volatile int*)&probs[id >> 16].status[1];  // one read: the exit below is block-uniform
+    s_sub = u < ndiag ? 0 : (v & ((1 << sub_shift) - 1));
+    s_stop = 0;
+    s_abort = 0;
+  }
+  __syncthreads();
+  if (s_skip) return;
+  const int p = s_tile >> 16, ti = s_tile & 0xFFFF;
+  const bool diag = ti == s;
+  const int nrw = diag ? 4 : 4 >> sub_shift;  // row warps
+  const int row0 = ti * NB + s_sub * 32 * nrw;
+  const Prob& P = probs[p];
+  const int c0 = s * NB;
+  int* fl = flags + PANEL_FLAGS * p;
+  const int fbase = s * NPIECE;  // the counters grow through the whole sweep
+  if (tid == 0) {
+    mbar_init(b_mma, 1);
+    mbar_init(b_blk, 1);
+    mbar_init(b_z, 1);
+    mbar_init(b_drained, nrw);
+    mbar_init(b_digits, nrw);
+    mbar_init(b_pub, nrw);
+    mbar_init(b_quiet, 1);
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+  }
+  if (warp == PN_MMA_WARP) {
+    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(su32(&s_tmem)),
+                 "n"(PN_TMEM_COLS));
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;");
+  }
+  asm volatile("tcgen05.fence::before_thread_sync;");
+  __syncthreads();
+  asm volatile("tcgen05.fence::after_thread_sync;");
+  const uint32_t tmem = s_tmem;
+  bool quiet = false;  // MMA warp: its MMAs were waited for after a stop
+
+  if (warp < nrw) {
+    // ---------------- row warps: one thread per row ----------------
+    const int i = row0 + tid;
+    const int rl = i & (NB - 1);  // row inside its 128-row tile
+    const size_t ld = (size_t)P.ld;
+    double* krow = P.K + (size_t)c0 * ld + i;  // read by alpha and the adjoint (keep_l)
+    const int kexp = *P.kscale;
+    // the accumulators of this row, column 0 of the panel (tiles 2 s and 2 s + 1)
+    const long long* acc0 = P.acc + acc_tile(ti, 2 * s, P.nt128) * ACC_TILE_ELEMS + acc_elem(rl, 0);
+    const long long* acc1 = P.acc + acc_tile(ti, 2 * s + 1, P.nt128) * ACC_TILE_ELEMS + acc_elem(rl, 0);
+    unsigned char* gdig = P.slices + (size_t)ti * NSLICE * SLICE_BYTES + (size_t)rl * 16;
+    long long wv[PW];
+    auto load_piece = [&](int t) {
+      const long long* a = (t < 4 ? acc0 : acc1) + (size_t)(t & 3) * 2048;  // 16 columns: 2 groups of 8
+#pragma unroll
+      for (int c = 0; c < PW; ++c) wv[c] = a[(c >> 3) * 1024 + (c & 7) * 32];
+    };
+    load_piece(0);
+    const uint32_t trow = tmem + ((uint32_t)(warp * 32) << 16);  // this warp's TMEM lanes
+    double r0 = 0.0, r1 = 0.0;  // sum_k L_ik z_k; the diagonal tile: the entries themselves
+    const bool two = P.nrhs > 1;
+    const double rhs0 = P.rhs[i], rhs1 = two ? P.rhs[P.Nc + i] : 0.0;
+    bool live = true;
+    auto wait = [&](uint64_t* bar, int parity) -> bool {
+      const int r = wait_or_stop(bar, (uint32_t)parity, &s_stop);
+      if (r == 2) s_abort = s_stop = 1;
+      live = r == 0;
+      return live;
+    };
+#pragma unroll 1
+    for (int t = 0; t < NPIECE; ++t) {
+      const bool done = diag && warp < (t >> 1);  // the diagonal tile: every row of this warp is factored
+      long long T[PW];
+      if (t > 0) {
+        if (!wait(b_mma, (t - 1) & 1)) break;
+        asm volatile("tcgen05.fence::after_thread_sync;");
+      }
+      if (!done) {
+        if (t > 0) {
+          // the couplings' 7 level sums: by the magic add where they lie in
+          // (-2^22, 2^22) (the sum's exponent bits tell), else by F2I
+          uint32_t off = 0;
+#pragma unroll
+          for (int g = 0; g < 2; ++g) {
+            uint32_t v[NSLICE][8];
+#pragma unroll
+            for (int l = 0; l < NSLICE; ++l) tmem_ld8(v[l], trow + (uint32_t)(l * PW + g * 8));
+            asm volatile("tcgen05.wait::ld.sync.aligned;");
+#pragma unroll
+            for (int l = 0; l < NSLICE; ++l)
+#pragma unroll
+              for (int jj = 0; jj < 8; ++jj) {
+                v[l][jj] = level_bits(v[l][jj]);
+                off |= v[l][jj] ^ 0x4B000000u;
+              }
+#pragma unroll
+            for (int jj = 0; jj < 8; ++jj)
+              T[g * 8 + jj] = (long long)((unsigned long long)wv[g * 8 + jj] - (unsigned long long)level_bits_to_w64(v, jj));
+          }
+          if (__any_sync(0xffffffffu, off >> 23)) {
+#pragma unroll 1
+            for (int c = 0; c < PW; ++c) {
+              uint32_t v[NSLICE];
+#pragma unroll
+              for (int l = 0; l < NSLICE; ++l) v[l] = tmem_ld1(trow + (uint32_t)(l * PW + c));
+              asm volatile("tcgen05.wait::ld.sync.aligned;");
+              int S[NSLICE];
+#pragma unroll
+              for (int l = 0; l < NSLICE; ++l) S[l] = __float2int_rn(__uint_as_float(v[l]));
+              const unsigned long long W = (unsigned long long)levels_to_w64(S);
+#pragma unroll
+              for (int k = 0; k < PW; ++k)
+                if (k == c) T[k] = (long long)((unsigned long long)wv[k] - W);
+            }
+          }
+          asm volatile("tcgen05.fence::before_thread_sync;");
+          __syncwarp();
+          if (lane == 0) mbar_arrive(b_drained);
+        } else {
+#pragma unroll
+          for (int c = 0; c < PW; ++c) T[c] = wv[c];
+        }
+        if (t + 1 < NPIECE) load_piece(t + 1);
+      } else if (t > 0 && lane == 0) {
+        mbar_arrive(b_drained);
+      }
+      PanelBlock& Lt = Ls[t & 1];
+      long long* Dj = s_D[t & 1];
+      int Xh[PW], Xl[PW];  // this row's solved entries
+      const int c_own = diag ? rl - t * PW : PW;  // this row's index in the piece's block; < 0: above it
+      if (diag && warp == (t >> 1)) {
+        // the 16 x 16 diagonal block, column by column on the whole warp
+        // (rows below the block in the same warp are solved on the way)
+        const int base = (t & 1) * PW;
+        if (c_own >= 0 && c_own < PW) {
+          Rs[c_own] = rhs0 - r0;
+          Rs[PW + c_own] = rhs1 - r1;
+        }
+        // no branch per column: a non-positive pivot is remembered and what
+        // follows it is discarded
+        int fail = PW;
+#pragma unroll
+        for (int j = 0; j < PW; ++j) {
+          long long S = 0, M = 0;
+#pragma unroll
+          for (int c = 0; c < j; ++c) {
+            const int lh = __shfl_sync(0xffffffffu, Xh[c], base + j), ll = __shfl_sync(0xffffffffu, Xl[c], base + j);
+            S += (long long)Xh[c] * lh;
+            M += (long long)Xh[c] * ll;
+            M += (long long)Xl[c] * lh;
+          }
+          const long long Tj = T[j] - (S << 2) - (M >> 28);
+          const long long D = __shfl_sync(0xffffffffu, Tj, base + j);
+          if (D <= 0 && fail == PW) fail = j;
+          unsigned long long y;
+          int sh;
+          rsqrt_fixed(D, y, sh);
+          sh = min(max(sh, 0), 30);  // discarded columns only
+          scale_entry(Tj, y, sh, Xh[j], Xl[j]);
+          if (lane == 0) {
+            Lt.y[j] = y;
+            Lt.sh[j] = sh;
+            Dj[j] = D;
+          }
+          if (c_own < j) Xh[j] = Xl[j] = 0;  // above the diagonal
+        }
+        if (fail < PW) {
+          if (lane == 0) {
+            P.status[0] = c0 + t * PW + fail + 1;  // LAPACK info: 1-based column
+            P.status[1] = 1;
+            s_stop = 1;
+            __threadfence();
+            for (int f = 0; f < 3; ++f) st_release(&fl[f], FLAG_FAIL);
+          }
+          live = false;
+          break;
+        }
+        if (c_own >= 0 && c_own < PW) {
+#pragma unroll
+          for (int c = 0; c < PW; c += 2)
+            *reinterpret_cast<int4*>(&Lt.x[c_own][c]) = make_int4(Xh[c], Xl[c], Xh[c + 1], Xl[c + 1]);
+        }
+        __syncwarp();
+        if (lane == 0) mbar_arrive(b_blk);
+        {
+          const uint4* src = reinterpret_cast<const uint4*>(&Lt);
+          uint4* dst = reinterpret_cast<uint4*>(P.lpub + t);
+          for (int q = lane; q < (int)PN_LBYTES / 16; q += 32) dst[q] = src[q];
+        }
+        __threadfence();
+        __syncwarp();
+        if (lane == 0) st_release(&fl[FLAG_L], fbase + t + 1);
+      }
+      if (!wait(b_blk, t & 1)) break;
+      if (!done && !(diag && warp == (t >> 1))) {
+        // x L'_tt^T = B
+#pragma unroll
+        for (int k = 0; k < PW; ++k) {
+          long long S = 0, M = 0;
+#pragma unroll
+          for (int c = 0; c < k; ++c) {
+            const int2 l = Lt.x[k][c];
+            S += (long long)Xh[c] * l.x;
+            M += (long long)Xh[c] * l.y;
+            M += (long long)Xl[c] * l.x;
+          }
+          scale_entry(T[k] - (S << 2) - (M >> 28), Lt.y[k], Lt.sh[k], Xh[k], Xl[k]);
+        }
+      }
+      if (!done) {
+#pragma unroll
+        for (int g = 0; g < 2; ++g) {
+          uint4 d[NSLICE];
+          digits8_packed(&Xh[g * 8], &Xl[g * 8], d);
+#pragma unroll
+          for (int q = 0; q < NSLICE; ++q) {
+            if (t + 1 < NPIECE) *reinterpret_cast<uint4*>(As + t * PN_ACHUNK + q * 4096 + g * 2048 + tid * 16) = d[q];
+            *reinterpret_cast<uint4*>(gdig + (size_t)q * SLICE_BYTES + (size_t)(2 * t + g) * 2048) = d[q];
+            // the diagonal tile's own B operand of the next piece
+            if (diag && (rl >> 4) == t + 1)
+              *reinterpret_cast<uint4*>(Bs + t * PN_BCHUNK + g * (NSLICE * PW * 16) + q * (PW * 16) + (rl & 15) * 16) = d[q];
+          }
+        }
+        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");  // digits visible to the tensor cores
+      }
+      __syncwarp();
+      if (lane == 0) mbar_arrive(b_digits);
+      if (diag) {
+        __threadfence();  // digits visible to the device before they are published
+        __syncwarp();
+        if (lane == 0) mbar_arrive(b_pub);
+      }
+      if (!done && P.keep_l) {
+        double ljj = 0.0;  // the row's own L_jj = d d^-1/2
+        if (c_own >= 0 && c_own < PW)
+          ljj = fixed62_to_double(Dj[c_own]) * fixed62_to_double((long long)Lt.y[c_own], Lt.sh[c_own] + kexp);
+#pragma unroll
+        for (int c = 0; c < PW; ++c) {
+          const double x = fixed62_to_double(((long long)Xh[c] * (1LL << 30) + Xl[c]) * 4, kexp);
+          krow[(size_t)(t * PW + c) * ld] = c == c_own ? ljj : x;
+        }
+      }
+      // the right-hand sides: sum_k L'_ik z_k of this piece, z in 60-bit fixed
+      // point of the piece's own scale
+      if (!wait(b_z, t & 1)) break;
+      if (!done) {
+        const PanelZ& Z = Zs[t & 1];
+        long long S = 0, M = 0;
+#pragma unroll
+        for (int c = 0; c < PW; ++c) {
+          const int2 z = Z.x[0][c];
+          S += (long long)Xh[c] * z.x;
+          M += (long long)Xh[c] * z.y;
+          M += (long long)Xl[c] * z.x;
+        }
+        r0 = fma(Z.scale[0], fixed62_to_double((S << 2) + (M >> 28)), r0);
+        if (two) {
+          S = M = 0;
+#pragma unroll
+          for (int c = 0; c < PW; ++c) {
+            const int2 z = Z.x[1][c];
+            S += (long long)Xh[c] * z.x;
+            M += (long long)Xh[c] * z.y;
+            M += (long long)Xl[c] * z.x;
+          }
+          r1 = fma(Z.scale[1], fixed62_to_double((S << 2) + (M >> 28)), r1);
+        }
+      }
+    }
+    if (!diag && live) {
+      P.rhs[i] = rhs0 - r0;
+      if (two) P.rhs[P.Nc + i] = rhs1 - r1;
+    }
+  } else if (warp == PN_MMA_WARP) {
+    // ---------------- operand loads and MMA issue ----------------
+    const uint64_t adesc = smem_desc(su32(As), 2048, 128);
+    const uint64_t bdesc = smem_desc(su32(Bs), NSLICE * PW * 16, 128);
+    // chunk c against the next piece's 16 rows: A plane q against B planes
+    // 0 .. 6 - q stacked along N, levels q .. 6 in one instruction
+    auto issue_chunk = [&](int c) {
+#pragma unroll
+      for (int q = 0; q < NSLICE; ++q)
+        mma_f16_desc(tmem + (uint32_t)q * PW, adesc + (uint64_t)((c * PN_ACHUNK + q * 4096) >> 4),
+                     bdesc + (uint64_t)((c * PN_BCHUNK) >> 4),
+                     (1u << 4) | ((uint32_t)(PW * (NSLICE - q) >> 3) << 17) | ((128u >> 4) << 24),
+                     (c == 0 && q == 0) ? 0u : 1u);
+    };
+    // the digits of rows 16 (t + 1) .. + 15 of the diagonal tile, chunk c
+    auto load_chunk = [&](int t, int c) {
+      const unsigned char* src = P.slices + (size_t)s * NSLICE * SLICE_BYTES + (size_t)(t + 1) * PW * 16;
+      for (int q = lane; q < (int)PN_BCHUNK / 16; q += 32) {
+        const int row = q & 15, pl = (q >> 4) % NSLICE, g = (q >> 4) / NSLICE;
+        cp_async16(Bs + c * PN_BCHUNK + q * 16, src + (size_t)pl * SLICE_BYTES + (size_t)(2 * c + g) * 2048 + row * 16);
+      }
+    };
+    // a problem's counter, as the whole warp sees it: 0 reached, 1 failed, 2 gave up
+    auto wait_flag = [&](int f, int t) -> int {
+      int r = 0;
+      if (lane == 0) {
+        const int v = poll_flag(&fl[f], fbase + t + 1);
+        r = v < 0 ? 2 : (v >= FLAG_FAIL ? 1 : 0);
+      }
+      return __shfl_sync(0xffffffffu, r, 0);
+    };
+    int st = 0;  // 1: the problem failed, 2: a wait gave up
+#pragma unroll 1
+    for (int t = 0; t < NPIECE && !st; ++t) {
+      if (!diag) {
+        if ((st = wait_flag(FLAG_L, t))) break;
+        const unsigned char* pub = reinterpret_cast<const unsigned char*>(P.lpub + t);
+        unsigned char* dst = reinterpret_cast<unsigned char*>(Ls + (t & 1));
+        for (int q = lane; q < (int)PN_LBYTES / 16; q += 32) cp_async16(dst + q * 16, pub + q * 16);
+        cp_async_wait();
+        __syncwarp();
+        if (lane == 0) mbar_arrive(b_blk);
+      }
+      if (t + 1 < NPIECE) {
+        if (t > 0) {
+          // earlier chunks against the next piece, while the rows are solved
+          if ((st = wait_or_stop(b_mma, (t - 1) & 1, &s_stop))) break;  // the couplings of piece t have read Bs
+          for (int c = 0; c < t; ++c) load_chunk(t, c);
+          cp_async_wait();
+          asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+          __syncwarp();
+          if ((st = wait_or_stop(b_drained, (t - 1) & 1, &s_stop))) break;
+          asm volatile("tcgen05.fence::after_thread_sync;");
+          if (lane == 0)
+            for (int c = 0; c < t; ++c) issue_chunk(c);
+          __syncwarp();
+        }
+        if (!diag) {
+          if ((st = wait_flag(FLAG_D, t))) break;
+          load_chunk(t, t);
+          cp_async_wait();
+          asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+          __syncwarp();
+        }
+        if ((st = wait_or_stop(b_digits, t & 1, &s_stop))) break;
+        asm volatile("tcgen05.fence::after_thread_sync;");
+        if (lane == 0) {
+          issue_chunk(t);
+          mma_commit(b_mma);
+        }
+        __syncwarp();
+      }
+      if (!diag) {
+        if ((st = wait_flag(FLAG_Z, t))) break;
+        if (lane < (int)PN_ZBYTES / 16)
+          cp_async16(reinterpret_cast<unsigned char*>(Zs + (t & 1)) + lane * 16,
+                     reinterpret_cast<const unsigned char*>(P.zpub + t) + lane * 16);
+        cp_async_wait();
+        __syncwarp();
+        if (lane == 0) mbar_arrive(b_z);
+      }
+    }
+    if (st) {
+      // the problem failed or a wait gave up: every warp falls out of its
+      // waits, and no MMA still writes TMEM when it is freed
+      if (st == 2) s_abort = 1;
+      s_stop = 1;
+    }
+    __syncwarp();
+    quiet = st != 0;
+    if (quiet && lane == 0) drain_mmas(b_quiet);
+  } else if (warp == PN_RHS_WARP && diag) {
+    // ---------------- right-hand sides and log-determinant of the panel ----------------
+    // lane j + 16 q: entry j of right-hand side q
+    const int j = lane & 15;
+    const bool have = lane < 16 || P.nrhs > 1;
+    double prod = 1.0;  // product of the pivots' significands; their exponents add up in esum
+    int esum = 0;
+    const int ke = *P.kscale;
+    bool ok = true;
+#pragma unroll 1
+    for (int t = 0; t < NPIECE; ++t) {
+      const int w = wait_or_stop(b_blk, t & 1, &s_stop);
+      if (w == 2) s_abort = s_stop = 1;
+      ok = w == 0;
+      if (!ok) break;
+      const PanelBlock& Lt = Ls[t & 1];
+      double r = have ? Rs[lane] : 0.0, z = 0.0;
+      // row j of the block, and 1 / L'_jj = y 2^(sh - 62), as doubles
+      double lrow[PW];
+#pragma unroll
+      for (int c = 0; c < PW; ++c) {
+        const int2 l = Lt.x[j][c];
+        lrow[c] = fixed62_to_double(((long long)l.x * (1LL << 30) + l.y) * 4);
+      }
+      const double rdj = fixed62_to_double((long long)Lt.y[j], Lt.sh[j]);
+#pragma unroll
+      for (int c = 0; c < PW; ++c) {
+        const double b = __shfl_sync(0xffffffffu, r * rdj, (lane & 16) + c);
+        if (j == c) z = b;
+        r = fma(-b, lrow[c], r);
+      }
+      // z in fixed point of the piece's scale, 4 max |z| or more: then |sum x z| <= 1 in that
+      // scale (16 entries, |x| of norm 1) and no 64-bit sum overflows; NaN and infinity go on through the scale
+      int q = (int)((unsigned)__double2hiint(z) >> 20) & 0x7FF;
+      for (int o = 8; o > 0; o >>= 1) q = max(q, __shfl_xor_sync(0xffffffffu, q, o));
+      PanelZ& Z = Zs[t & 1];
+      {
+        bool nf = false;
+        const long long X = (to_fixed62(z, q - 1020, &nf) + 2) >> 2;
+        const int xh = (int)((X + (1LL << 29)) >> 30);
+        const int2 v = make_int2(xh, (int)((unsigned)X - ((unsigned)xh << 30)));
+        // 2^(q - 1020); beyond the double range the sums are infinite anyway
+        const double sc = q == 0x7FF ? nan("") : __longlong_as_double((long long)min(q + 3, 2046) << 52);
+        Z.x[lane >> 4][j] = v;
+        P.zpub[t].x[lane >> 4][j] = v;
+        if (j == 0) {
+          Z.scale[lane >> 4] = sc;
+          P.zpub[t].scale[lane >> 4] = sc;
+        }
+      }
+      if (have) P.rhs[(size_t)(lane >> 4) * P.Nc + c0 + t * PW + j] = z;
+      __threadfence();
+      __syncwarp();
+      if (lane == 0) {
+        mbar_arrive(b_z);
+        st_release(&fl[FLAG_Z], fbase + t + 1);
+      }
+      const int wp = wait_or_stop(b_pub, t & 1, &s_stop);
+      if (wp == 2) s_abort = s_stop = 1;
+      ok = wp == 0;
+      if (!ok) break;
+      if (lane == 0) st_release(&fl[FLAG_D], fbase + t + 1);
+      const long long lb = __double_as_longlong(fixed62_to_double(s_D[t & 1][j]));
+      if (c0 + t * PW + j < P.N) {  // not the identity padding
+        esum += (int)(lb >> 52) - 1023 + 2 * ke;
+        prod *= __longlong_as_double((lb & 0xFFFFFFFFFFFFFLL) | 0x3FF0000000000000LL);
+      }
+    }
+    if (ok) {
+      for (int o = 8; o > 0; o >>= 1) {
+        prod *= __shfl_xor_sync(0xffffffffu, prod, o);
+        esum += __shfl_xor_sync(0xffffffffu, esum, o);
+      }
+      if (lane == 0) P.logdet_part[s] = 0.5 * (log(prod) + (double)esum * 0.69314718055994530942);  // sum of log L_jj
+    }
+  }
+  __syncthreads();
+  if (s_abort && warp == PN_MMA_WARP && lane == 0 && !quiet) drain_mmas(b_quiet);
+  if (tid == 0 && s_abort) {
+    // a bounded wait gave up: report, and release the problem's other CTAs
+    atomicExch(&P.status[2], 1);
+    __threadfence();
+    for (int f = 0; f < 3; ++f) st_release(&fl[f], FLAG_FAIL);
+  }
+  asm volatile("tcgen05.fence::after_thread_sync;");
+  if (warp == PN_MMA_WARP) __syncwarp();
+  if (warp == PN_MMA_WARP)
+    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "n"(PN_TMEM_COLS));
+}
+
+// Rows per CTA: 128, or 64 or 32 while that still gives every tile an SM of
+// its own.  The FP64 pipe is per SM, so a lone problem's substitution runs up to
+// four times faster on four SMs; once the tiles outnumber the SMs, splitting
+// them only repeats the per-CTA work.
+cudaError_t launch_panel(const Prob* probs, int step, const int* order, int ndiag, int total_tiles, int* counter,
+                         int* flags, int num_sms, cudaStream_t s) {
+  cudaError_t e = ensure_smem_attr((const void*)k_panel, SMEM_PANEL, PN_SMEM);
+  if (e != cudaSuccess) return e;
+  if (ndiag <= 0) return cudaSuccess;
+  int sh = 0;
+  const int rest = total_tiles - ndiag;
+  while (sh < 2 && ndiag + (rest << (sh + 1)) <= num_sms) ++sh;
+  k_panel<<<ndiag + (rest << sh), PN_THREADS, PN_SMEM, s>>>(probs, step, order, ndiag, sh, counter, flags);
+  return cudaGetLastError();
+}
+
+}  // namespace fgpu

@@ -55,17 +55,6 @@ __device__ __forceinline__ void drain_ring(uint64_t* full, int nstage, uint32_t 
   }
 }
 
-// one non-blocking probe of an mbarrier phase
-__device__ __forceinline__ bool mbar_test(uint64_t* bar, uint32_t parity) {
-  uint32_t ok;
-  asm volatile(
-      "{\n .reg .pred p;\n mbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\n selp.u32 %0, 1, 0, p;\n}\n"
-      : "=r"(ok)
-      : "r"(su32(bar)), "r"(parity)
-      : "memory");
-  return ok != 0;
-}
-
 // tcgen05 shared-memory descriptor, no swizzle, K-major core matrices
 // (8 rows x 16 bytes): lbo = byte stride between core matrices along K,
 // sbo = along M/N; descriptor version 1 (bits 46-47).
@@ -146,27 +135,50 @@ __device__ __forceinline__ void mbar_arrive(uint64_t* bar) {
   asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(su32(bar)) : "memory");
 }
 
-// W 2^e rounded to the nearest double (ties to even) with integer
-// operations only, W a signed 64-bit integer: the same double as the exact
-// product correctly rounded, without the FP64 pipe.  Results below 2^-1022
-// (never reached by the factor's scales) flush to 0.
-__device__ __forceinline__ double w64_to_double(long long W, int e) {
-  if (W == 0) return 0.0;
-  const unsigned long long sgn = (unsigned long long)W >> 63;
-  unsigned long long a = sgn ? 0ULL - (unsigned long long)W : (unsigned long long)W;
-  const int lz = __clzll((long long)a);
-  a <<= lz;  // leading one at bit 63
-  unsigned long long mant = a >> 11;  // 53 bits
-  const unsigned rb = (unsigned)a & 0x7FFu;
-  if (rb > 0x400u || (rb == 0x400u && (mant & 1))) ++mant;
-  int be = 63 - lz + e + 1023;  // biased exponent of 1.f
-  if (mant >> 53) {
-    mant >>= 1;
-    ++be;
+// round(x 2^(62 - e)) as an integer, for |x| < 2^e.  What does not fit
+// saturates, NaN and infinities too (they also set *nonfinite): an
+// off-diagonal entry like that leaves the matrix not positive semidefinite,
+// and the factorisation stops at its row's pivot, if not before, where
+// dpotrf on the unrounded matrix does.
+__device__ __forceinline__ long long to_fixed62(double x, int e, bool* nonfinite) {
+  const long long bits = __double_as_longlong(x);
+  const int E = (int)((bits >> 52) & 0x7FF);
+  const long long M = (bits & 0xFFFFFFFFFFFFFLL) | (1LL << 52);
+  const int sh = E - 1075 + 62 - e;
+  long long F;
+  if (E == 0x7FF) *nonfinite = true;
+  if (sh > 9) {
+    F = (1LL << 62) - 1;
+  } else if (E == 0 || sh <= -63) {
+    F = 0;
+  } else {
+    F = sh >= 0 ? M << sh : (M + (1LL << (-sh - 1))) >> (-sh);
   }
-  if (be <= 0) return sgn ? -0.0 : 0.0;
-  if (be >= 2047) return __longlong_as_double((long long)((sgn << 63) | 0x7FF0000000000000ULL));
-  return __longlong_as_double((long long)((sgn << 63) | ((unsigned long long)be << 52) | (mant & 0xFFFFFFFFFFFFFULL)));
+  return bits < 0 ? -F : F;
+}
+
+// a diagonal entry: kernel value plus nugget.  NaN becomes negative, which
+// fails that pivot as NaN does in dpotrf.
+__device__ __forceinline__ long long diag_fixed62(double k, double noise, int e, bool* nonfinite) {
+  const double d = k + noise;
+  if (d != d) {
+    *nonfinite = true;
+    return -(1LL << 61);
+  }
+  return to_fixed62(k, e, nonfinite) + to_fixed62(noise, e, nonfinite);
+}
+
+// T 2^(e - 62) rounded to the nearest double (ties away from zero), T a signed
+// 64-bit integer, with integer operations only; the result must be normal or 0
+__device__ __forceinline__ double fixed62_to_double(long long T, int e = 0) {
+  const long long sgn = T >> 63;
+  unsigned long long a = (unsigned long long)((T ^ sgn) - sgn);
+  const int lz = __clzll((long long)a);
+  a <<= (lz & 63);  // leading one at bit 63
+  const unsigned long long mant = (a >> 11) + ((a >> 10) & 1);  // 53 bits; a carry goes on into the exponent
+  const unsigned long long be = lz == 64 ? 0ULL : (unsigned long long)(1024 + e - lz) << 52;
+  const unsigned long long r = lz == 64 ? 0ULL : be - (1ULL << 52) + mant;
+  return __longlong_as_double((long long)(r | ((unsigned long long)sgn & 0x8000000000000000ULL)));
 }
 
 // The exact integer W = sum_l S_l 256^(6 - l) of 7 level sums, in wrapping
@@ -208,11 +220,6 @@ __device__ __forceinline__ long long level_bits_to_w64(const uint32_t (&b)[7][8]
   w += (unsigned long long)p01 << 40;
   return (long long)(w - LEVEL_BITS_BIAS);
 }
-
-// an integer-valued float x with |x| <= 2^22 as an int, exactly, without a
-// conversion instruction: x + 1.5 * 2^23 lies in [2^23, 2^24], where the
-// float's low mantissa bits are x + 2^22 (one FADD and one IADD)
-__device__ __forceinline__ int small_f2i(float x) { return __float_as_int(x + 12582912.0f) - 0x4B400000; }
 
 }  // namespace
 }  // namespace fgpu

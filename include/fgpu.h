@@ -74,10 +74,10 @@ int fgpu_nparams(const fgpu_ctx* ctx);
  * call (process-wide default; returns the previous setting):
  *   FGPU_TRAILING_TCGEN05 (default): 128-wide panels; the O(N^3) update runs
  *     on the tensor cores as exact integer products of 7 fp16 digit planes
- *     per FP64 value, accumulated exactly in int64;
+ *     per entry, accumulated exactly in int64; the matrix is kept as 62-bit
+ *     fixed point and the panels are solved in 60-bit fixed point;
  *   FGPU_TRAILING_FP64: 64-wide panels, FP64 mma.sync on the FP64 pipe.
- * Diagonal blocks, panel solves and the right-hand-side rows are FP64 in
- * both.  The environment variable FGPU_TRAILING=fp64 selects FP64 at load.
+ * The environment variable FGPU_TRAILING=fp64 selects FP64 at load.
  * No counterpart in the reference (which calls LAPACK dpotrf). */
 #define FGPU_TRAILING_FP64 0
 #define FGPU_TRAILING_TCGEN05 1
@@ -200,8 +200,8 @@ int fgpu_loglik_noalloc(int N, int d, const double* X_dev, const double* y_dev, 
  * fgpu_plan_stage_times fills ms[k] with the summed device time of stage k
  * during the LAST replay and count[k] with its launches (k: 0 build,
  * 1 diagonal factor, 2 panel solve, 3 trailing update, 4 likelihood
- * epilogue, 5 panel conversion, 6 digit split, 7 right-hand-side rows,
- * 8 quarter-panel coupling).
+ * epilogue; in tensor-core mode stage 2 is the whole panel; 5 .. 8 are
+ * unused and stay 0).
  * Diagnostic only; the reference has no counterpart. */
 #define FGPU_NSTAGES 9
 int fgpu_plan_set_profiling(fgpu_plan* plan, int enable);
