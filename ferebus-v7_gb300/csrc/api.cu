@@ -242,9 +242,14 @@ struct Worker {
   UpdSched sched;
 };
 
-// Adjoint workspace (FP64 geometry): K with the right-hand-side tile and N
-// identity rows below it, K^-1, per-CTA partials.
+// Adjoint workspace: K^-1, per-CTA partials, and either the tensor-core
+// inverse's buffers (tc) or, in FP64 geometry, K with the right-hand-side tile
+// and N identity rows below it.
 struct GradWS {
+  bool tc = false;
+  InvWorkspace inv;
+  std::vector<InvLevel> levels;
+  int num_sms = 0;
   int Nc = 0, ld = 0, nsteps = 0, nrt = 0;
   Workspace ws;
   double* kinv = nullptr;
@@ -762,7 +767,9 @@ size_t plan_cache_limit() {
 // Frees an adjoint workspace, complete or partly built (unset members are null).
 void free_grad_ws(GradWS* g) {
   if (!g) return;
-  for (void* q : {(void*)g->ws.K, (void*)g->ws.logdet_part, (void*)g->ws.status, (void*)g->ws.out,
+  for (void* q : {(void*)g->inv.V, (void*)g->inv.rowpart, (void*)g->inv.colpart, (void*)g->inv.colpart_p,
+                  (void*)g->inv.exps, (void*)g->inv.dr, (void*)g->inv.dc, (void*)g->inv.tmaps, (void*)g->inv.splits,
+                  (void*)g->inv.tiles, (void*)g->ws.K, (void*)g->ws.logdet_part, (void*)g->ws.status, (void*)g->ws.out,
                   (void*)g->ws.z, (void*)g->kinv, (void*)g->gpart, (void*)g->theta_d, (void*)g->g_d,
                   (void*)g->prob_d})
     cudaFree(q);
@@ -978,21 +985,59 @@ int fgpu_loglik(fgpu_ctx* ctx, const double* theta, int ntheta, double* ll, int*
 }
 
 namespace {
-int make_grad_ws(fgpu_ctx* c, GradWS** out) {
+// The tensor-core inverse's buffers (about 30 N^2 bytes against the FP64
+// sweep's 24 N^2).
+int alloc_inverse(const fgpu_ctx* c, GradWS* g) {
+  InvWorkspace& w = g->inv;
+  const int nt = c->nt128;
+  const size_t nc = (size_t)c->Nc, dig = inv_slots(nt) * NSLICE * SLICE_BYTES;
+  std::vector<InvSplit> splits;
+  std::vector<InvTile> tiles;
+  inv_schedule(nt, splits, tiles, g->levels);
+  CK(cudaMalloc(&g->kinv, sizeof(double) * nc * nc));
+  w.kinv = g->kinv;
+  CK(cudaMalloc(&w.V, sizeof(double) * nc * nc));
+  CK(cudaMalloc(&w.dr, dig));
+  CK(cudaMalloc(&w.dc, dig));
+  CK(cudaMalloc(&w.rowpart, sizeof(float) * nc / 16 * nc));
+  CK(cudaMalloc(&w.colpart, sizeof(float) * nc / 32 * nc));
+  CK(cudaMalloc(&w.colpart_p, sizeof(float) * nc / 32 * nc));
+  CK(cudaMalloc(&w.exps, sizeof(int) * 4 * nc));
+  CK(cudaMalloc(&w.splits, sizeof(InvSplit) * splits.size()));
+  CK(cudaMalloc(&w.tiles, sizeof(InvTile) * tiles.size()));
+  CK(cudaMalloc(&w.tmaps, 2 * TMAP_BYTES));
+  CK(cudaMemcpy(w.splits, splits.data(), sizeof(InvSplit) * splits.size(), cudaMemcpyHostToDevice));
+  CK(cudaMemcpy(w.tiles, tiles.data(), sizeof(InvTile) * tiles.size(), cudaMemcpyHostToDevice));
+  alignas(64) unsigned char maps[2 * TMAP_BYTES];
+  int er = encode_slice_maps(maps, w.dr, (int)inv_slots(nt));
+  if (er == 0) er = encode_slice_maps(maps + TMAP_BYTES, w.dc, (int)inv_slots(nt));
+  if (er != 0) return fail(FGPU_ECUDA, "cuTensorMapEncodeTiled failed (%d)", er);
+  CK(cudaMemcpy(w.tmaps, maps, 2 * TMAP_BYTES, cudaMemcpyHostToDevice));
+  CK(cudaDeviceGetAttribute(&g->num_sms, cudaDevAttrMultiProcessorCount, c->device));
+  return 0;
+}
+
+int make_grad_ws(fgpu_ctx* c, bool tc, GradWS** out) {
   std::unique_ptr<GradWS, GradWSDeleter> g(new (std::nothrow) GradWS());  // freed whole on failure
   if (!g) return fail(FGPU_ENOMEM, "adjoint workspace");
+  g->tc = tc;
   g->Nc = round_up(c->N, TB);
   g->nsteps = g->Nc / TB;
   g->ld = 2 * g->Nc + TB;
   g->nrt = g->ld / TB;
   const size_t nc = (size_t)g->Nc;
   CK(cudaStreamCreateWithFlags(&g->stream, cudaStreamNonBlocking));
-  CK(cudaMalloc(&g->ws.K, sizeof(double) * (size_t)g->ld * nc));
+  if (tc) {
+    int rc = alloc_inverse(c, g.get());
+    if (rc) return rc;
+  } else {
+    CK(cudaMalloc(&g->ws.K, sizeof(double) * (size_t)g->ld * nc));
+    CK(cudaMalloc(&g->kinv, sizeof(double) * nc * nc));
+  }
   CK(cudaMalloc(&g->ws.logdet_part, sizeof(double) * (g->nsteps + 1)));
   CK(cudaMalloc(&g->ws.status, sizeof(int) * 4));
   CK(cudaMalloc(&g->ws.out, sizeof(double) * 8));
   CK(cudaMalloc(&g->ws.z, sizeof(double) * nc));
-  CK(cudaMalloc(&g->kinv, sizeof(double) * nc * nc));
   CK(cudaMalloc(&g->gpart, sizeof(double) * (size_t)g->nsteps * g->nsteps * GRAD_SLOTS));
   CK(cudaMalloc(&g->theta_d, sizeof(double) * (c->ntheta + 1)));
   CK(cudaMalloc(&g->g_d, sizeof(double) * (c->ntheta + 1)));
@@ -1023,6 +1068,7 @@ int make_grad_ws(fgpu_ctx* c, GradWS** out) {
   p.z = g->ws.z;
   p.mode = 0;
   p.kinv = g->kinv;
+  p.ldkinv = tc ? c->Nc : g->Nc;
   p.gpart = g->gpart;
   CK(cudaMemcpy(g->prob_d, &p, sizeof(Prob), cudaMemcpyHostToDevice));
   *out = g.release();
@@ -1041,7 +1087,14 @@ int fgpu_grad(fgpu_ctx* ctx, const double* theta, int ntheta, double* ll, double
   std::lock_guard<std::mutex> lk(ctx->grad_mu);
   if (!ctx->grad) {
     GradWS* g = nullptr;
-    int rc = make_grad_ws(ctx, &g);
+    // tensor-core contexts invert on the tensor cores; where that workspace
+    // does not fit the device, the smaller FP64 sweep still serves
+    int rc = make_grad_ws(ctx, ctx->mode == 1, &g);
+    if (rc == FGPU_ENOMEM && ctx->mode == 1) {
+      cudaGetLastError();
+      t_err.clear();
+      rc = make_grad_ws(ctx, false, &g);
+    }
     if (rc) return rc;
     ctx->grad = g;
   }
@@ -1058,11 +1111,10 @@ int fgpu_grad(fgpu_ctx* ctx, const double* theta, int ntheta, double* ll, double
   cudaStream_t s = g->stream;
   if (ctx->mode == 1) {
     // Tensor-core context: the evaluation itself (factor, log-likelihood,
-    // alpha) is the plain path's graph; its factor L, alpha, the likelihood
-    // epilogue's scalars and status are copied into the adjoint workspace,
-    // whose FP64 sweep then only turns the identity rows into L^-T.  Every
-    // step runs on the worker's stream; the worker is released after the
-    // final synchronisation.
+    // alpha) is the plain path's graph, and K^-1 comes from its factor; alpha,
+    // the likelihood epilogue's scalars and the status are copied into the
+    // adjoint workspace.  Every step runs on the worker's stream; the worker
+    // is released after the final synchronisation.
     int rc = 0;
     w = acquire(ctx, &rc);
     if (!w) return rc;
@@ -1073,8 +1125,11 @@ int fgpu_grad(fgpu_ctx* ctx, const double* theta, int ntheta, double* ll, double
     CK(cudaGraphLaunch(w->graph, s));
     n += w->graph_kernels;
     CK(launch_backsolve(w->prob_d, 1, ctx->nsteps, nullptr, s, &n));
-    CK(cudaMemcpy2DAsync(g->ws.K, sizeof(double) * g->ld, w->ws.K, sizeof(double) * ctx->ld,
-                         sizeof(double) * g->Nc, g->Nc, cudaMemcpyDeviceToDevice, s));
+    if (g->tc)
+      CK(enqueue_inverse(w->prob_d, ctx->nt128, g->inv, g->levels, g->num_sms, s, &n));
+    else
+      CK(cudaMemcpy2DAsync(g->ws.K, sizeof(double) * g->ld, w->ws.K, sizeof(double) * ctx->ld,
+                           sizeof(double) * g->Nc, g->Nc, cudaMemcpyDeviceToDevice, s));
     CK(cudaMemcpyAsync(g->ws.z, w->ws.z, sizeof(double) * g->Nc, cudaMemcpyDeviceToDevice, s));
     CK(cudaMemcpyAsync(g->ws.out, w->ws.out, sizeof(double) * 8, cudaMemcpyDeviceToDevice, s));
     CK(cudaMemcpyAsync(g->ws.status, w->ws.status, sizeof(int) * 4, cudaMemcpyDeviceToDevice, s));
@@ -1086,24 +1141,28 @@ int fgpu_grad(fgpu_ctx* ctx, const double* theta, int ntheta, double* ll, double
     CK(launch_build(g->prob_d, 1, g->nsteps, ctx->spec.nplanes, s));
     ++n;
   }
-  CK(launch_identity_border(g->prob_d, g->Nc, s));
-  ++n;
-  for (int step = 0; step < g->nsteps; ++step) {
-    if (ctx->mode != 1) {
-      CK(launch_potf2(g->prob_d, 1, step, s));
-      ++n;
+  if (!g->tc) {
+    CK(launch_identity_border(g->prob_d, g->Nc, s));
+    ++n;
+    for (int step = 0; step < g->nsteps; ++step) {
+      if (ctx->mode != 1) {
+        CK(launch_potf2(g->prob_d, 1, step, s));
+        ++n;
+      }
+      CK(launch_trsm(g->prob_d, 1, step, g->nsteps, s, g->nrt));
+      CK(launch_update(g->prob_d, 1, step, g->nsteps, s, g->nrt));
+      n += 2;
     }
-    CK(launch_trsm(g->prob_d, 1, step, g->nsteps, s, g->nrt));
-    CK(launch_update(g->prob_d, 1, step, g->nsteps, s, g->nrt));
-    n += 2;
   }
   if (ctx->mode != 1) {
     CK(launch_finalize(g->prob_d, 1, s));
     ++n;
     CK(launch_backsolve(g->prob_d, 1, g->nsteps, nullptr, s, &n));
   }
-  CK(launch_syrk_inv(g->prob_d, g->nsteps, s));
-  ++n;
+  if (!g->tc) {
+    CK(launch_syrk_inv(g->prob_d, g->nsteps, s));
+    ++n;
+  }
   CK(enqueue_grad_passes(g->prob_d, g->nsteps, ctx->nkparams, ctx->optimise_noise, g->g_d, s, &n));
   double* h_out = g->h_stage;
   double* h_g = g->h_stage + 8;

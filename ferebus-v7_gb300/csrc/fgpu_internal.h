@@ -111,7 +111,8 @@ struct Prob {
   // (from the tensor-core evaluation), so the FP64 sweep works only on the
   // identity rows below the right-hand-side tile
   int border_only;
-  double* kinv;                   // adjoint: K^-1 (Nc x Nc, lower)
+  double* kinv;                   // adjoint: K^-1 (ldkinv x Nc, lower)
+  int ldkinv;
   double* gpart;                  // adjoint: per-CTA partial sums
   // tensor-core build
   const double* plane_max;        // nplanes: max_i |planes[p][i]|
@@ -188,6 +189,40 @@ cudaError_t launch_feat_digits(const Prob* probs, int nprob, int max_nt128, cuda
 cudaError_t launch_build_tc(const Prob* probs, int nprob, const unsigned long long* tiles, int total_tiles,
                             int num_sms, cudaStream_t s);
 
+// K^-1 of a tensor-core context's factor (inv.cu).  A split task turns a
+// 128 x 128 operand tile into digit planes: kind 0 rows of L', 1 rows of V, 2
+// columns of V, 3 columns of P = L'_21 V_11; row = its operand-row tile, k = its
+// k tile, g0 .. g1 the partial sums of squares its rows' scales add up.  A tile
+// task is one 128 x 64 output tile: the first slots of its operands' k blocks
+// and their strides, the k blocks, row tile (128) and column tile (64).
+struct InvSplit {
+  int slot, kind, row, k, g0, g1;
+};
+struct InvTile {
+  int a0, astep, b0, bstep, nkb, row, col, pad;
+};
+struct InvLevel {
+  int split1, nsplit1, tile1, ntile1;  // L'_21, V_22, V_11; P
+  int split2, nsplit2, tile2, ntile2;  // P; V_21
+};
+struct InvWorkspace {
+  double* V = nullptr;                 // Nc x Nc, lower
+  double* kinv = nullptr;              // Nc x Nc, lower: P on the way, then K^-1
+  float* rowpart = nullptr;            // sums of squares of V: 16-column groups (Nc / 16) x rows
+  float* colpart = nullptr;            // 32-row groups (Nc / 32) x columns
+  float* colpart_p = nullptr;          // of P
+  int* exps = nullptr;                 // 4 kinds x Nc: scales of the operand rows
+  unsigned char* dr = nullptr;         // digit planes: row operands (kinds 0, 1)
+  unsigned char* dc = nullptr;         // column operands (kinds 2, 3)
+  unsigned char* tmaps = nullptr;      // tensor maps over dr, dc
+  InvSplit* splits = nullptr;
+  InvTile* tiles = nullptr;
+};
+size_t inv_slots(int nt128);  // 128 x 128 operand tiles each of dr, dc holds
+void inv_schedule(int nt128, std::vector<InvSplit>& splits, std::vector<InvTile>& tiles, std::vector<InvLevel>& levels);
+cudaError_t enqueue_inverse(const Prob* p, int nt128, const InvWorkspace& w, const std::vector<InvLevel>& levels,
+                            int num_sms, cudaStream_t s, long long* nlaunch);
+
 // Adjoint (grad.cu): identity rows below the right-hand-side tile turn into
 // L^-T during the sweep; K^-1 = L^-T (L^-T)^T; fused dK/dtheta pass.
 cudaError_t launch_identity_border(const Prob* p, int nc, cudaStream_t s);
@@ -203,7 +238,7 @@ constexpr int GRAD_SLOTS = 33;  // parameters per fused pass + noise slot
 // beyond the first 64 set it on every call.
 enum SmemSlot {
   SMEM_BUILD, SMEM_BUILD_DOT, SMEM_UPDATE, SMEM_SYRK, SMEM_OZAKI_UPDATE, SMEM_PANEL,
-  SMEM_BUILD_TC, SMEM_NSLOTS
+  SMEM_BUILD_TC, SMEM_INV_GEMM, SMEM_NSLOTS
 };
 cudaError_t ensure_smem_attr(const void* func, int slot, int bytes);
 

@@ -128,7 +128,7 @@ __global__ void __launch_bounds__(256) k_grad(const Prob* __restrict__ pp, int q
       for (int a = 0; a < 2; ++a) {
         const int i = ti * TB + r0 + a, j = tj * TB + c0 + cc;
         if (i < j || i >= P.N || j >= P.N) continue;
-        const double w = (P.z[i] * P.z[j] / s2 - P.kinv[(size_t)j * nc + i]) * (i == j ? 1.0 : 2.0);
+        const double w = (P.z[i] * P.z[j] / s2 - P.kinv[(size_t)j * P.ldkinv + i]) * (i == j ? 1.0 : 2.0);
         if (i == j) acc[GCHUNK] += w;
         // forward: leaf values
         double val[MAX_POST], adj[MAX_POST];

@@ -45,7 +45,7 @@ namespace fgpu {
 // TMEM columns.  Warp 16 (one lane) streams the digit planes of each
 // k-chunk of 16 by 5-D TMA into a 4-stage ring; warp 17 (one lane) issues
 // the chunk's 28 digit pairs as 10 tcgen05.mma with B's planes stacked
-// along N (upd_issue_chunk); warps 0-15 drain TMEM into registers (16
+// along N (issue_chunk_128x64); warps 0-15 drain TMEM into registers (16
 // columns per thread, two rounds of TMEM loads), release it (so the next
 // tile's MMAs start), then stage each 8-column piece of the tile's exact
 // sums (2 KB, contiguous in the accumulator layout) in shared memory and
@@ -81,32 +81,6 @@ static_assert(UPD_SMEM <= 227 * 1024, "shared memory per CTA");
 // MMA-issuing warp of digit level l (one warp issues all levels)
 __host__ __device__ constexpr int upd_level_warp(int) { return 0; }
 static_assert(UPD_MMA_WARPS == 1, "the update epilogue converts all 7 levels of a column group in one pass");
-
-// one k-chunk of a tile with the B planes stacked along N: for A plane pp
-// the pairs (pp, q), q = 0 .. 6 - pp, accumulate into levels pp .. 6, whose
-// TMEM blocks of 64 columns are contiguous, so they are one MMA over B
-// planes 0 .. 6 - pp (N = 64 (7 - pp), above N = 256 in two equal halves): 10 MMAs instead of
-// 28, and A plane pp is read from shared memory once or twice instead of
-// 7 - pp times.  N >= 128 MMAs run at the tensor pipe's full rate; N = 64
-// ones are bound by shared-memory operand bandwidth.
-__device__ __forceinline__ void upd_issue_chunk(uint32_t tbase, uint64_t adesc, uint64_t bdesc, bool first) {
-#pragma unroll
-  for (int pp = 0; pp < NSLICE; ++pp) {
-    // N = 64 (7 - pp) in one MMA, or, above the 256 limit, in two equal
-    // halves (224 + 224, 192 + 192, 160 + 160): an N = 64 remainder would
-    // be bound by the A operand's shared-memory read rather than the tensor
-    // pipe.  The stacked B rows and the TMEM columns are both contiguous, so
-    // a split at any multiple of 8 rows is one offset in each.
-    const int n = 64 * (NSLICE - pp);
-    const int nh = n <= 256 ? n : n / 2;
-#pragma unroll
-    for (int off = 0; off < n; off += nh) {
-      const uint32_t idesc = (1u << 4) | ((uint32_t)(nh >> 3) << 17) | ((128u >> 4) << 24);
-      mma_f16_desc(tbase + (uint32_t)(pp * 64 + off), adesc + (uint64_t)(pp * 4096 >> 4),
-                   bdesc + (uint64_t)((off * 16) >> 4), idesc, (first && pp == 0) ? 0u : 1u);
-    }
-  }
-}
 
 __global__ void __launch_bounds__(UPD_THREADS, 1)
     k_ozaki_update(const Prob* __restrict__ probs, int nprob, int s, const unsigned long long* __restrict__ tiles,
@@ -200,7 +174,7 @@ __global__ void __launch_bounds__(UPD_THREADS, 1)
           }
           asm volatile("tcgen05.fence::after_thread_sync;");
           const uint64_t soff = (uint64_t)((st * STAGE) >> 4);
-          upd_issue_chunk(tbase, adesc0 + soff, bdesc0 + soff, c == 0);
+          issue_chunk_128x64(tbase, adesc0 + soff, bdesc0 + soff, c == 0);
           mma_commit(&empty[st]);
         }
         if (!ok) {

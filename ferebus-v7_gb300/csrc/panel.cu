@@ -127,45 +127,12 @@ __device__ __forceinline__ void scale_entry(long long T, unsigned long long y, i
   Xl = (int)((unsigned)X - ((unsigned)Xh << 30));
 }
 
-// The 7 fp16 digit planes of 8 entries X = x 2^60 (one k-group of a row),
-// packed: F = x 2^55 rounded has the balanced digits
-// d_p in [-128, 127] (p = 1..6, base 256, lowest last) and d_0 = the rest.
-// G = F + sum_{k<6} 128 256^k turns them into plain bytes: byte 6 - p of G
-// is d_p + 128, and G >> 48 is d_0 (|d_0| <= 128 when |x| <= 1).  A byte
-// u under the fp16 exponent bits 0x64 is the half 1024 + u, so one HSUB2 of
-// 1152 per pair of entries yields the digits exactly, with no conversion
-// instruction; two byte permutes place a pair's bytes under the 0x64 bytes.
+// the digit planes of 8 entries X = x 2^60 of a row
 __device__ __forceinline__ void digits8_packed(const int* Xh, const int* Xl, uint4 out[NSLICE]) {
-  unsigned lo[8], hi[8];
+  long long F[8];
 #pragma unroll
-  for (int kk = 0; kk < 8; ++kk) {
-    const long long X = (long long)Xh[kk] * (1LL << 30) + Xl[kk];
-    const long long G = ((X + 16) >> 5) + 0x808080808080LL;
-    lo[kk] = (unsigned)G;
-    hi[kk] = (unsigned)(G >> 32);
-  }
-  const __half2 off = __halves2half2(__ushort_as_half(0x6480), __ushort_as_half(0x6480));  // 1152
-#pragma unroll
-  for (int p = 0; p < NSLICE; ++p) {
-    unsigned w[4];
-#pragma unroll
-    for (int m = 0; m < 4; ++m) {
-      unsigned bits;
-      if (p == 0) {  // d_0 + 128 may be 256: arithmetic, not a byte
-        const unsigned u0 = (unsigned)(((int)hi[2 * m] >> 16) + 128);
-        const unsigned u1 = (unsigned)(((int)hi[2 * m + 1] >> 16) + 128);
-        bits = (0x6400u + u0) | ((0x6400u + u1) << 16);
-      } else {
-        const int q = 6 - p;  // byte of G: byte q & 3 of the low or high word
-        const unsigned wa = q < 4 ? lo[2 * m] : hi[2 * m], wb = q < 4 ? lo[2 * m + 1] : hi[2 * m + 1];
-        const unsigned t = __byte_perm(wa, 0x64646464u, 0x4440u | (unsigned)(q & 3));  // [a_q, 64, 64, 64]
-        bits = __byte_perm(wb, t, 0x7054u | ((unsigned)(q & 3) << 8));                  // [a_q, 64, b_q, 64]
-      }
-      const __half2 h = __hsub2(*reinterpret_cast<const __half2*>(&bits), off);
-      w[m] = *reinterpret_cast<const unsigned*>(&h);
-    }
-    out[p] = make_uint4(w[0], w[1], w[2], w[3]);
-  }
+  for (int kk = 0; kk < 8; ++kk) F[kk] = ((long long)Xh[kk] * (1LL << 30) + Xl[kk] + 16) >> 5;
+  digits8_of_fixed55(F, out);
 }
 
 // the whole warp waits for an mbarrier phase (bounded), or until the CTA
@@ -186,11 +153,6 @@ __device__ __forceinline__ int wait_or_stop(uint64_t* bar, uint32_t parity, cons
   return __any_sync(0xffffffffu, r == 2) ? 2 : 1;
 }
 
-__device__ __forceinline__ void tmem_ld8(uint32_t (&v)[8], uint32_t addr) {
-  asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
-               : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7])
-               : "r"(addr));
-}
 __device__ __forceinline__ uint32_t tmem_ld1(uint32_t addr) {
   uint32_t v;
   asm volatile("tcgen05.ld.sync.aligned.32x32b.x1.b32 {%0}, [%1];" : "=r"(v) : "r"(addr));

@@ -221,5 +221,76 @@ __device__ __forceinline__ long long level_bits_to_w64(const uint32_t (&b)[7][8]
   return (long long)(w - LEVEL_BITS_BIAS);
 }
 
+__device__ __forceinline__ void tmem_ld8(uint32_t (&v)[8], uint32_t addr) {
+  asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
+               : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7])
+               : "r"(addr));
+}
+// one k-chunk of a tile with the B planes stacked along N: for A plane pp
+// the pairs (pp, q), q = 0 .. 6 - pp, accumulate into levels pp .. 6, whose
+// TMEM blocks of 64 columns are contiguous, so they are one MMA over B
+// planes 0 .. 6 - pp (N = 64 (7 - pp), above N = 256 in two equal halves): 10 MMAs instead of
+// 28, and A plane pp is read from shared memory once or twice instead of
+// 7 - pp times.  N >= 128 MMAs run at the tensor pipe's full rate; N = 64
+// ones are bound by shared-memory operand bandwidth.
+__device__ __forceinline__ void issue_chunk_128x64(uint32_t tbase, uint64_t adesc, uint64_t bdesc, bool first) {
+#pragma unroll
+  for (int pp = 0; pp < NSLICE; ++pp) {
+    // N = 64 (7 - pp) in one MMA, or, above the 256 limit, in two equal
+    // halves (224 + 224, 192 + 192, 160 + 160): an N = 64 remainder would
+    // be bound by the A operand's shared-memory read rather than the tensor
+    // pipe.  The stacked B rows and the TMEM columns are both contiguous, so
+    // a split at any multiple of 8 rows is one offset in each.
+    const int n = 64 * (NSLICE - pp);
+    const int nh = n <= 256 ? n : n / 2;
+#pragma unroll
+    for (int off = 0; off < n; off += nh) {
+      const uint32_t idesc = (1u << 4) | ((uint32_t)(nh >> 3) << 17) | ((128u >> 4) << 24);
+      mma_f16_desc(tbase + (uint32_t)(pp * 64 + off), adesc + (uint64_t)(pp * 4096 >> 4),
+                   bdesc + (uint64_t)((off * 16) >> 4), idesc, (first && pp == 0) ? 0u : 1u);
+    }
+  }
+}
+
+// The 7 fp16 digit planes of 8 entries F = x 2^55, |x| <= 1 (one k-group of a
+// row), packed: F has the balanced digits
+// d_p in [-128, 127] (p = 1..6, base 256, lowest last) and d_0 = the rest.
+// G = F + sum_{k<6} 128 256^k turns them into plain bytes: byte 6 - p of G
+// is d_p + 128, and G >> 48 is d_0 (|d_0| <= 128 when |x| <= 1).  A byte
+// u under the fp16 exponent bits 0x64 is the half 1024 + u, so one HSUB2 of
+// 1152 per pair of entries yields the digits exactly, with no conversion
+// instruction; two byte permutes place a pair's bytes under the 0x64 bytes.
+__device__ __forceinline__ void digits8_of_fixed55(const long long (&F)[8], uint4 out[NSLICE]) {
+  unsigned lo[8], hi[8];
+#pragma unroll
+  for (int kk = 0; kk < 8; ++kk) {
+    const long long G = F[kk] + 0x808080808080LL;
+    lo[kk] = (unsigned)G;
+    hi[kk] = (unsigned)(G >> 32);
+  }
+  const __half2 off = __halves2half2(__ushort_as_half(0x6480), __ushort_as_half(0x6480));  // 1152
+#pragma unroll
+  for (int p = 0; p < NSLICE; ++p) {
+    unsigned w[4];
+#pragma unroll
+    for (int m = 0; m < 4; ++m) {
+      unsigned bits;
+      if (p == 0) {  // d_0 + 128 may be 256: arithmetic, not a byte
+        const unsigned u0 = (unsigned)(((int)hi[2 * m] >> 16) + 128);
+        const unsigned u1 = (unsigned)(((int)hi[2 * m + 1] >> 16) + 128);
+        bits = (0x6400u + u0) | ((0x6400u + u1) << 16);
+      } else {
+        const int q = 6 - p;  // byte of G: byte q & 3 of the low or high word
+        const unsigned wa = q < 4 ? lo[2 * m] : hi[2 * m], wb = q < 4 ? lo[2 * m + 1] : hi[2 * m + 1];
+        const unsigned t = __byte_perm(wa, 0x64646464u, 0x4440u | (unsigned)(q & 3));  // [a_q, 64, 64, 64]
+        bits = __byte_perm(wb, t, 0x7054u | ((unsigned)(q & 3) << 8));                  // [a_q, 64, b_q, 64]
+      }
+      const __half2 h = __hsub2(*reinterpret_cast<const __half2*>(&bits), off);
+      w[m] = *reinterpret_cast<const unsigned*>(&h);
+    }
+    out[p] = make_uint4(w[0], w[1], w[2], w[3]);
+  }
+}
+
 }  // namespace
 }  // namespace fgpu
