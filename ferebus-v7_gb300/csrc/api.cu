@@ -234,6 +234,7 @@ struct Worker {
   Workspace ws;
   double* theta_d = nullptr;
   Prob* prob_d = nullptr;
+  int* bsync = nullptr;       // the back-substitution's ticket and counter
   double* h_stage = nullptr;  // pinned: theta | out(4) | status(4 ints as doubles)
   int* h_status = nullptr;
   cudaGraphExec_t graph = nullptr;
@@ -257,6 +258,7 @@ struct GradWS {
   double* theta_d = nullptr;
   double* g_d = nullptr;
   Prob* prob_d = nullptr;
+  int* bsync = nullptr;       // the back-substitution's ticket and counter
   cudaStream_t stream = nullptr;
   double* h_stage = nullptr;  // pinned: out(8) | g(ntheta) | status (as ints)
 };
@@ -681,6 +683,7 @@ void free_worker(Worker* w) {
   cudaFree(w->ws.tmaps);
   cudaFree(w->theta_d);
   cudaFree(w->prob_d);
+  cudaFree(w->bsync);
   cudaFree(w->sched.tiles_dev);
   cudaFree(w->sched.build_tiles_dev);
   cudaFree(w->sched.pan_order_dev);
@@ -705,6 +708,7 @@ int make_worker(fgpu_ctx* c, Worker** out) {
   if (cudaMalloc(&w->theta_d, sizeof(double) * (c->ntheta + 1)) != cudaSuccess)
     return bail(fail(FGPU_ENOMEM, "theta alloc"));
   if (cudaMalloc(&w->prob_d, sizeof(Prob)) != cudaSuccess) return bail(fail(FGPU_ENOMEM, "desc alloc"));
+  if (cudaMalloc(&w->bsync, sizeof(int) * 2) != cudaSuccess) return bail(fail(FGPU_ENOMEM, "back-substitution alloc"));
   if (cudaMallocHost(&w->h_stage, sizeof(double) * (c->ntheta + 16)) != cudaSuccess)
     return bail(fail(FGPU_ENOMEM, "pinned alloc"));
   w->h_status = reinterpret_cast<int*>(w->h_stage + c->ntheta + 8);
@@ -771,7 +775,7 @@ void free_grad_ws(GradWS* g) {
                   (void*)g->inv.exps, (void*)g->inv.dr, (void*)g->inv.dc, (void*)g->inv.tmaps, (void*)g->inv.splits,
                   (void*)g->inv.tiles, (void*)g->ws.K, (void*)g->ws.logdet_part, (void*)g->ws.status, (void*)g->ws.out,
                   (void*)g->ws.z, (void*)g->kinv, (void*)g->gpart, (void*)g->theta_d, (void*)g->g_d,
-                  (void*)g->prob_d})
+                  (void*)g->prob_d, (void*)g->bsync})
     cudaFree(q);
   if (g->h_stage) cudaFreeHost(g->h_stage);
   if (g->stream) cudaStreamDestroy(g->stream);
@@ -969,7 +973,8 @@ int fgpu_loglik(fgpu_ctx* ctx, const double* theta, int ntheta, double* ll, int*
   CK(cudaGraphLaunch(w->graph, w->stream));
   t_launches = w->graph_kernels;
   if (alpha) {
-    CK(launch_backsolve(w->prob_d, 1, ctx->nsteps, nullptr, w->stream, &t_launches));
+    CK(launch_backsolve(w->prob_d, ctx->nsteps, w->bsync, w->stream));
+    ++t_launches;
   }
   double* h_out = w->h_stage + ctx->ntheta;
   CK(cudaMemcpyAsync(h_out, w->ws.out, sizeof(double) * 4, cudaMemcpyDeviceToHost, w->stream));
@@ -1042,6 +1047,7 @@ int make_grad_ws(fgpu_ctx* c, bool tc, GradWS** out) {
   CK(cudaMalloc(&g->theta_d, sizeof(double) * (c->ntheta + 1)));
   CK(cudaMalloc(&g->g_d, sizeof(double) * (c->ntheta + 1)));
   CK(cudaMalloc(&g->prob_d, sizeof(Prob)));
+  CK(cudaMalloc(&g->bsync, sizeof(int) * 2));
   CK(cudaMallocHost(&g->h_stage, sizeof(double) * (c->ntheta + 16)));
   Prob p;
   memset(&p, 0, sizeof(p));
@@ -1124,7 +1130,8 @@ int fgpu_grad(fgpu_ctx* ctx, const double* theta, int ntheta, double* ll, double
     CK(cudaMemcpyAsync(w->theta_d, w->h_stage, sizeof(double) * ntheta, cudaMemcpyHostToDevice, s));
     CK(cudaGraphLaunch(w->graph, s));
     n += w->graph_kernels;
-    CK(launch_backsolve(w->prob_d, 1, ctx->nsteps, nullptr, s, &n));
+    CK(launch_backsolve(w->prob_d, ctx->nsteps, w->bsync, s));
+    ++n;
     if (g->tc)
       CK(enqueue_inverse(w->prob_d, ctx->nt128, g->inv, g->levels, g->num_sms, s, &n));
     else
@@ -1157,7 +1164,8 @@ int fgpu_grad(fgpu_ctx* ctx, const double* theta, int ntheta, double* ll, double
   if (ctx->mode != 1) {
     CK(launch_finalize(g->prob_d, 1, s));
     ++n;
-    CK(launch_backsolve(g->prob_d, 1, g->nsteps, nullptr, s, &n));
+    CK(launch_backsolve(g->prob_d, g->nsteps, g->bsync, s));
+    ++n;
   }
   if (!g->tc) {
     CK(launch_syrk_inv(g->prob_d, g->nsteps, s));

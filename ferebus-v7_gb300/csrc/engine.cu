@@ -668,41 +668,94 @@ __global__ void __launch_bounds__(256) k_finalize(const Prob* __restrict__ probs
 }
 
 // ---------------------------------------------------------------------------
-// alpha = L^-T z by blocked back-substitution (dpotrs's second half)
+// alpha = L^-T z (dpotrs's second half) in one launch: CTA k of the ticket order
+// owns the 64-row block b = nsteps - 1 - k, adds up L_rb^T alpha_r as the blocks
+// r > b below it are published, and solves its own triangle.  Whoever waits
+// for a block holds a later ticket than it, so that block's CTA is running.
+// The chain is nsteps triangles of 64 dependent FP64 steps, ~6 us each; the
+// tiles of L are read beside it.  (Two launches per block, with a division per
+// step and everything re-read in order, took 34 us per block.)
+// sync[0]: ticket, sync[1]: blocks solved; both zeroed before the launch.
 // ---------------------------------------------------------------------------
-__global__ void __launch_bounds__(TB) k_bs_diag(const Prob* __restrict__ probs, int blk) {
-  const Prob& P = probs[blockIdx.x];
-  if (blk >= P.nsteps || P.status[1] || P.status[2]) return;
-  __shared__ double L[TB * (TB + 1)];
-  __shared__ double z[TB];
-  const int tid = threadIdx.x;
-  const size_t ld = (size_t)P.ld;
-  const double* Ld = P.K + (size_t)(blk * TB) * ld + blk * TB;
-  for (int c = 0; c < TB; ++c) L[c * (TB + 1) + tid] = Ld[(size_t)c * ld + tid];
-  z[tid] = P.z[blk * TB + tid];
+__global__ void __launch_bounds__(256) k_backsolve(const Prob* __restrict__ pp, int* __restrict__ sync) {
+  const Prob& P = *pp;
+  if (P.status[1] || P.status[2]) return;
+  extern __shared__ __align__(16) double Ms[];  // [c][r], c > r: L_cr / L_rr
+  __shared__ double rd[TB], w[TB];
+  __shared__ int s_b, s_done;
+  const int tid = threadIdx.x, c = tid >> 2, part = tid & 3;
+  if (tid == 0) s_b = P.nsteps - 1 - atomicAdd(&sync[0], 1);
   __syncthreads();
-  for (int c = TB - 1; c >= 0; --c) {
-    if (tid == 0) z[c] = z[c] / L[c * (TB + 1) + c];
-    __syncthreads();
-    if (tid < c) z[tid] = fma(-L[tid * (TB + 1) + c], z[c], z[tid]);
-    __syncthreads();
-  }
-  P.z[blk * TB + tid] = z[tid];
-}
-
-// z[0 : blk*TB) -= L[blk rows, 0 : blk*TB)^T alpha_blk; one warp per column.
-__global__ void __launch_bounds__(256) k_bs_update(const Prob* __restrict__ probs, int blk) {
-  const Prob& P = probs[blockIdx.y];
-  if (blk >= P.nsteps || P.status[1] || P.status[2]) return;
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int col = blockIdx.x * 8 + warp;
-  if (col >= blk * TB) return;
+  const int b = s_b;
   const size_t ld = (size_t)P.ld;
-  const double* Lc = P.K + (size_t)col * ld + blk * TB;
-  const double* ab = P.z + blk * TB;
-  double s = fma(Lc[lane], ab[lane], Lc[lane + 32] * ab[lane + 32]);
-  for (int o = 16; o > 0; o >>= 1) s += __shfl_down_sync(0xffffffffu, s, o);
-  if (lane == 0) P.z[col] -= s;
+  const double* Ld = P.K + (size_t)(b * TB) * ld + b * TB;
+  if (tid < TB) rd[tid] = 1.0 / Ld[(size_t)tid * ld + tid];
+  __syncthreads();
+  for (int q = tid; q < TB * TB; q += blockDim.x) {
+    const int row = q % TB, col = q / TB;
+    if (row > col) Ms[row * (TB + 1) + col] = Ld[(size_t)col * ld + row] * rd[col];
+  }
+  const double* Lc = P.K + (size_t)(b * TB + c) * ld + part * 16;  // this thread's column and 16 of every 64 rows
+  double acc[4] = {0.0, 0.0, 0.0, 0.0};
+  int done = 0;  // blocks known to be solved
+  for (int r = P.nsteps - 1; r > b; --r) {
+    double2 l[8];
+    const double2* src = reinterpret_cast<const double2*>(Lc + (size_t)r * TB);
+#pragma unroll
+    for (int k = 0; k < 8; ++k) l[k] = src[k];
+    if (done < P.nsteps - r) {
+      if (tid == 0) {
+        int v = 0;
+        for (int it = 0; it < (1 << 22); ++it) {
+          asm volatile("ld.acquire.gpu.global.s32 %0, [%1];" : "=r"(v) : "l"(&sync[1]) : "memory");
+          if (v >= P.nsteps - r) break;
+          __nanosleep(20);
+        }
+        s_done = v;
+      }
+      __syncthreads();
+      done = s_done;
+      __syncthreads();
+      if (done < P.nsteps - r) {  // gave up (block-uniform): the blocks above give up in turn
+        if (tid == 0) atomicExch(&P.status[2], 1);
+        return;
+      }
+    }
+    const double2* ar = reinterpret_cast<const double2*>(P.z + r * TB + part * 16);
+#pragma unroll
+    for (int k = 0; k < 8; ++k) {
+      const double2 v = __ldcg(ar + k);  // written in this launch: from the L2
+      acc[(2 * k) & 3] = fma(l[k].x, v.x, acc[(2 * k) & 3]);
+      acc[(2 * k + 1) & 3] = fma(l[k].y, v.y, acc[(2 * k + 1) & 3]);
+    }
+  }
+  double s = (acc[0] + acc[1]) + (acc[2] + acc[3]);
+  s += __shfl_xor_sync(0xffffffffu, s, 1);
+  s += __shfl_xor_sync(0xffffffffu, s, 2);
+  if (part == 0) w[c] = (P.z[b * TB + c] - s) * rd[c];
+  __syncthreads();
+  if (tid < 32) {
+    // alpha_r = w_r - sum_{k > r} M_kr alpha_k: lane holds rows r and r + 32
+    double w0 = w[tid], w1 = w[tid + 32];
+#pragma unroll 8
+    for (int k = TB - 1; k >= 32; --k) {
+      const double x = __shfl_sync(0xffffffffu, w1, k - 32);
+      const double m1 = tid < k - 32 ? Ms[k * (TB + 1) + tid + 32] : 0.0;
+      w1 = fma(-m1, x, w1);
+      w0 = fma(-Ms[k * (TB + 1) + tid], x, w0);
+    }
+#pragma unroll 8
+    for (int k = 31; k > 0; --k) {
+      const double x = __shfl_sync(0xffffffffu, w0, k);
+      const double m0 = tid < k ? Ms[k * (TB + 1) + tid] : 0.0;
+      w0 = fma(-m0, x, w0);
+    }
+    P.z[b * TB + tid] = w0;
+    P.z[b * TB + tid + 32] = w1;
+    __threadfence();
+    __syncwarp();
+    if (tid == 0) asm volatile("st.release.gpu.global.s32 [%0], %1;" ::"l"(&sync[1]), "r"(P.nsteps - b) : "memory");
+  }
 }
 
 // ---------------------------------------------------------------------------
@@ -776,16 +829,11 @@ cudaError_t launch_finalize(const Prob* probs, int nprob, cudaStream_t s) {
   return cudaGetLastError();
 }
 
-cudaError_t launch_backsolve(const Prob* probs, int nprob, int max_nsteps, double* /*alpha_out*/,
-                             cudaStream_t s, long long* nlaunch) {
-  for (int b = max_nsteps - 1; b >= 0; --b) {
-    k_bs_diag<<<nprob, TB, 0, s>>>(probs, b);
-    if (nlaunch) ++*nlaunch;
-    if (b > 0) {
-      k_bs_update<<<dim3((b * TB + 7) / 8, nprob), 256, 0, s>>>(probs, b);
-      if (nlaunch) ++*nlaunch;
-    }
-  }
+cudaError_t launch_backsolve(const Prob* prob, int nsteps, int* sync, cudaStream_t s) {
+  const int smem = TB * (TB + 1) * (int)sizeof(double);
+  cudaError_t e = cudaMemsetAsync(sync, 0, 2 * sizeof(int), s);
+  if (e != cudaSuccess) return e;
+  k_backsolve<<<nsteps, 256, smem, s>>>(prob, sync);
   return cudaGetLastError();
 }
 

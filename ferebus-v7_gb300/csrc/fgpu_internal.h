@@ -142,8 +142,8 @@ cudaError_t launch_trsm(const Prob* probs, int nprob, int step, int max_nsteps, 
 cudaError_t launch_update(const Prob* probs, int nprob, int step, int max_nsteps, cudaStream_t s,
                           int max_rowtiles = 0);
 cudaError_t launch_finalize(const Prob* probs, int nprob, cudaStream_t s);
-cudaError_t launch_backsolve(const Prob* probs, int nprob, int max_nsteps, double* alpha_out,
-                             cudaStream_t s, long long* nlaunch);
+// alpha of one problem; sync: two ints of scratch
+cudaError_t launch_backsolve(const Prob* prob, int nsteps, int* sync, cudaStream_t s);
 size_t build_smem_bytes(int nplanes);
 
 // Split-integer tensor-core path (ozaki.cu): 128-wide panels.
