@@ -255,6 +255,10 @@ struct GradWS {
   Workspace ws;
   double* kinv = nullptr;
   double* gpart = nullptr;
+  bool fast = false;          // the dK/dtheta pass of enqueue_grad_fast
+  int extra = 0;              // linear or constant leaves
+  long long* fx = nullptr;    // its fixed-point features
+  double* sums = nullptr;     // its total sums (in gpart's block)
   double* theta_d = nullptr;
   double* g_d = nullptr;
   Prob* prob_d = nullptr;
@@ -774,7 +778,7 @@ void free_grad_ws(GradWS* g) {
   for (void* q : {(void*)g->inv.V, (void*)g->inv.rowpart, (void*)g->inv.colpart, (void*)g->inv.colpart_p,
                   (void*)g->inv.exps, (void*)g->inv.dr, (void*)g->inv.dc, (void*)g->inv.tmaps, (void*)g->inv.splits,
                   (void*)g->inv.tiles, (void*)g->ws.K, (void*)g->ws.logdet_part, (void*)g->ws.status, (void*)g->ws.out,
-                  (void*)g->ws.z, (void*)g->kinv, (void*)g->gpart, (void*)g->theta_d, (void*)g->g_d,
+                  (void*)g->ws.z, (void*)g->fx, (void*)g->kinv, (void*)g->gpart, (void*)g->theta_d, (void*)g->g_d,
                   (void*)g->prob_d, (void*)g->bsync})
     cudaFree(q);
   if (g->h_stage) cudaFreeHost(g->h_stage);
@@ -1043,7 +1047,17 @@ int make_grad_ws(fgpu_ctx* c, bool tc, GradWS** out) {
   CK(cudaMalloc(&g->ws.status, sizeof(int) * 4));
   CK(cudaMalloc(&g->ws.out, sizeof(double) * 8));
   CK(cudaMalloc(&g->ws.z, sizeof(double) * nc));
-  CK(cudaMalloc(&g->gpart, sizeof(double) * (size_t)g->nsteps * g->nsteps * GRAD_SLOTS));
+  g->fast = tc && c->spec.tc_build;
+  if (g->fast) {
+    const size_t n = grad_fast_partials(g->nsteps, c->nkparams);
+    CK(cudaMalloc(&g->gpart, sizeof(double) * n));
+    g->sums = g->gpart + n - (c->nkparams + 5);
+    CK(cudaMalloc(&g->fx, sizeof(long long) * (size_t)c->spec.nplanes * c->Nc));
+    for (int l = 0; l < c->spec.nleaf; ++l)
+      g->extra |= c->spec.leaf[l].type == FGPU_LINEAR || c->spec.leaf[l].type == FGPU_CONSTANT;
+  } else {
+    CK(cudaMalloc(&g->gpart, sizeof(double) * (size_t)g->nsteps * g->nsteps * GRAD_SLOTS));
+  }
   CK(cudaMalloc(&g->theta_d, sizeof(double) * (c->ntheta + 1)));
   CK(cudaMalloc(&g->g_d, sizeof(double) * (c->ntheta + 1)));
   CK(cudaMalloc(&g->prob_d, sizeof(Prob)));
@@ -1171,7 +1185,11 @@ int fgpu_grad(fgpu_ctx* ctx, const double* theta, int ntheta, double* ll, double
     CK(launch_syrk_inv(g->prob_d, g->nsteps, s));
     ++n;
   }
-  CK(enqueue_grad_passes(g->prob_d, g->nsteps, ctx->nkparams, ctx->optimise_noise, g->g_d, s, &n));
+  if (g->fast)
+    CK(enqueue_grad_fast(g->prob_d, w->prob_d, g->nsteps, ctx->Nc, ctx->spec.nplanes, ctx->nkparams, g->extra,
+                         ctx->optimise_noise, g->fx, g->sums, g->g_d, s, &n));
+  else
+    CK(enqueue_grad_passes(g->prob_d, g->nsteps, ctx->nkparams, ctx->optimise_noise, g->g_d, s, &n));
   double* h_out = g->h_stage;
   double* h_g = g->h_stage + 8;
   int* h_status = reinterpret_cast<int*>(g->h_stage + 8 + ctx->ntheta + 1);

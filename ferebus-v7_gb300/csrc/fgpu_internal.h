@@ -230,6 +230,14 @@ cudaError_t launch_syrk_inv(const Prob* p, int nsteps, cudaStream_t s);
 cudaError_t enqueue_grad_passes(const Prob* p, int nsteps, int nk, int optimise_noise, double* g_out,
                                 cudaStream_t s, long long* nlaunch);
 constexpr int GRAD_SLOTS = 33;  // parameters per fused pass + noise slot
+// The dK/dtheta pass of kernels the tensor-core build serves: eval is the
+// evaluation's descriptor (its scaled features and coefficients), fx nplanes x
+// nc_eval int64 of scratch; extra: the kernel has linear or constant leaves.
+// grad_fast_partials: doubles of partial and total sums.
+size_t grad_fast_partials(int nsteps, int nk);
+cudaError_t enqueue_grad_fast(const Prob* p, const Prob* eval, int nsteps, int nc_eval, int nplanes, int nk, int extra,
+                              int optimise_noise, long long* fx, double* sums, double* g_out, cudaStream_t s,
+                              long long* nlaunch);
 
 // Opt kernel `func` into `bytes` of dynamic shared memory on the CURRENT
 // device.  cudaFuncSetAttribute acts per device, so the record of what was
@@ -238,7 +246,7 @@ constexpr int GRAD_SLOTS = 33;  // parameters per fused pass + noise slot
 // beyond the first 64 set it on every call.
 enum SmemSlot {
   SMEM_BUILD, SMEM_BUILD_DOT, SMEM_UPDATE, SMEM_SYRK, SMEM_OZAKI_UPDATE, SMEM_PANEL,
-  SMEM_BUILD_TC, SMEM_INV_GEMM, SMEM_NSLOTS
+  SMEM_BUILD_TC, SMEM_INV_GEMM, SMEM_GRAD_FAST, SMEM_NSLOTS
 };
 cudaError_t ensure_smem_attr(const void* func, int slot, int bytes);
 

@@ -11,6 +11,7 @@
 // tile, exactly as the kernel-matrix build does.
 #include "fgpu_internal.h"
 #include "iexp.cuh"
+#include "tc_common.cuh"
 
 #include <cmath>
 
@@ -240,6 +241,317 @@ __global__ void k_grad_reduce(const Prob* __restrict__ pp, int nblocks, int q0, 
   for (int b = 0; b < nblocks; ++b) v += P.gpart[(size_t)b * (GCHUNK + 1) + q];
   if (q < GCHUNK && q0 + q < nk) g[q0 + q] = 0.5 * v;
   if (q == GCHUNK && noise_slot >= 0) g[noise_slot] = 0.5 * v;
+}
+
+// ---------------------------------------------------------------------------
+// the same pass for kernels with one or two rbf / periodic leaves besides
+// linear and constant ones (those of the tensor-core build), k = a + b v0 +
+// c v1 + d v0 v1.
+//
+// FP64 costs 64 cycles per warp instruction here, so it is kept to what the
+// gradient's own sums need: per entry w_ij = W_ij and its products with the leaf
+// values, and per entry and feature the squared difference times that (3
+// operations for an rbf feature, 4 for a periodic one).  The leaf values come
+// from exact integer distances: the evaluation's scaled features f (v = exp(-|f_i
+// - f_j|^2 / 2)) as 54-bit fixed point in the leaf's scale 2^s, a difference
+// D = h 2^27 + l squared as h^2 + 2 h l 2^-27 + l^2 2^-54 on the integer
+// multiply-add pipe, and the fixed-point exponential.  One CTA per 64 x 64 lower
+// tile, 2 rows x 8 columns per thread, the features staged 16 planes at a time.
+// N = 4000, d = 24: 2.1 ms, against 4.9 ms for k_grad (all FP64, leaf values and
+// differences formed twice) and 0.34 ms for its one-block reduction.
+// ---------------------------------------------------------------------------
+namespace {
+constexpr int GF_CH = 16;  // planes per chunk
+constexpr int GF_SMEM = (2 * GF_CH * TB + 256 * GF_CH) * 8;
+}  // namespace
+
+// features of the distance leaves in fixed point: F = f 2^(54 - s)
+__global__ void __launch_bounds__(256) k_grad_fixed(const Prob* __restrict__ pe, long long* __restrict__ fx) {
+  const Prob& P = *pe;
+  const Spec& sp = *P.spec;
+  const int i = blockIdx.x * blockDim.x + threadIdx.x, p = blockIdx.y;
+  if (i >= P.Nc) return;
+  for (int d = 0; d < sp.ndot; ++d) {
+    const Leaf& L = sp.leaf[sp.dot_leaf[d]];
+    const int nf = L.type == L_PERIODIC ? 2 * L.n : L.n;
+    if (p >= L.plane0 && p < L.plane0 + nf)
+      fx[(size_t)p * P.Nc + i] = to_fixed54(P.splanes[(size_t)p * P.Nc + i], P.fscale[d]);
+  }
+}
+
+__global__ void __launch_bounds__(256)
+    k_grad_fast(const Prob* __restrict__ pp, const Prob* __restrict__ pe, const long long* __restrict__ fx,
+                int nslots, int extra) {
+  const Prob& P = *pp;   // adjoint: planes, alpha, K^-1
+  const Prob& Q = *pe;   // evaluation: scales and expression coefficients
+  const Spec& sp = *P.spec;
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  // lower tile (ti, tj) of the linear index
+  int ti = (int)((sqrtf(8.0f * (float)blockIdx.x + 1.0f) - 1.0f) * 0.5f);
+  while ((ti + 1) * (ti + 2) / 2 <= (int)blockIdx.x) ++ti;
+  while (ti * (ti + 1) / 2 > (int)blockIdx.x) --ti;
+  const int tj = (int)blockIdx.x - ti * (ti + 1) / 2;
+  double* gp = P.gpart + (size_t)blockIdx.x * nslots;
+  if (P.status[1]) {
+    for (int q = tid; q < nslots; q += 256) gp[q] = 0.0;
+    return;
+  }
+  extern __shared__ __align__(16) unsigned char smraw[];
+  double* Xi = reinterpret_cast<double*>(smraw);  // [plane of the chunk][64]
+  double* Xj = Xi + GF_CH * TB;
+  double* red = Xj + GF_CH * TB;  // [plane of the chunk][thread]
+  long long* Fi = reinterpret_cast<long long*>(Xi);
+  long long* Fj = reinterpret_cast<long long*>(Xj);
+  const int r0 = lane * 2, c0 = warp * 8;
+  const size_t nc = (size_t)P.Nc, ncq = (size_t)Q.Nc;
+  double v[2][16];  // leaf values, then the leaves' weights
+#pragma unroll
+  for (int d = 0; d < 2; ++d) {
+#pragma unroll
+    for (int e = 0; e < 16; ++e) v[d][e] = 0.0;
+    if (d < sp.ndot) {
+      const Leaf& L = sp.leaf[sp.dot_leaf[d]];
+      const int nf = L.type == L_PERIODIC ? 2 * L.n : L.n;
+      long long H[16], M[16];
+#pragma unroll
+      for (int e = 0; e < 16; ++e) H[e] = M[e] = 0;
+      for (int k0 = 0; k0 < nf; k0 += GF_CH) {
+        const int kn = min(GF_CH, nf - k0);
+        __syncthreads();
+        for (int q = tid; q < kn * TB; q += 256) {
+          const long long* src = fx + (size_t)(L.plane0 + k0 + q / TB) * ncq;
+          Fi[q] = src[ti * TB + q % TB];
+          Fj[q] = src[tj * TB + q % TB];
+        }
+        __syncthreads();
+        for (int k = 0; k < kn; ++k) {
+          const longlong2 fi = *reinterpret_cast<const longlong2*>(Fi + k * TB + r0);
+#pragma unroll
+          for (int c = 0; c < 8; ++c) {
+            const long long fj = Fj[k * TB + c0 + c];
+#pragma unroll
+            for (int a = 0; a < 2; ++a) {
+              const long long D = (a ? fi.y : fi.x) - fj;
+              const int h = (int)((D + (1LL << 26)) >> 27);
+              const int l = (int)D - (int)((unsigned)h << 27);
+              H[c * 2 + a] += (long long)h * h;
+              M[c * 2 + a] += (long long)h * l + (((long long)l * l) >> 28);
+            }
+          }
+        }
+      }
+      // |f_i - f_j|^2 = (H + M 2^-26) 2^(2 s - 54)
+      const IexpScale sc = iexp_scale(2 * Q.fscale[d] - 55);
+#pragma unroll
+      for (int e = 0; e < 16; ++e)
+        v[d][e] = iexp_fixed_tab((unsigned long long)(H[e] + (M[e] >> 26)), sc, g_iexp_tab1024, g_iexp_fine1024);
+    }
+  }
+  // weights: w dk/dv_d v_d, and the sums the linear and constant leaves need
+  double s[5] = {0.0, 0.0, 0.0, 0.0, 0.0};  // sum w, w v0, w v1, w v0 v1, trace of w
+  {
+    const double is2 = P.likelihood == 1 ? 1.0 / P.out[3] : 1.0;
+    const double cb = Q.fcoef[1], cc = Q.fcoef[2], cd = Q.fcoef[3];
+    const bool plain = cb == 1.0 && cd == 0.0 && (sp.ndot == 1 || cc == 1.0);
+    const double zi[2] = {P.z[ti * TB + r0] * is2, P.z[ti * TB + r0 + 1] * is2};
+#pragma unroll
+    for (int e = 0; e < 16; ++e) {
+      const int a = e & 1, i = ti * TB + r0 + a, j = tj * TB + c0 + (e >> 1);
+      double w = 0.0;
+      if (i >= j && i < P.N) {
+        w = fma(zi[a], P.z[j], -P.kinv[(size_t)j * P.ldkinv + i]);
+        if (i == j)
+          s[4] += w;
+        else
+          w = 2.0 * w;
+      }
+      const double v0 = v[0][e], v1 = v[1][e];
+      double m0 = w * v0, m1 = sp.ndot > 1 ? w * v1 : 0.0;
+      if (extra) {
+        s[0] += w;
+        s[1] += m0;
+        s[2] += m1;
+        s[3] = fma(m0, v1, s[3]);
+      }
+      if (!plain) {
+        const double m01 = cd * (m0 * v1);
+        m0 = fma(cb, m0, m01);
+        m1 = fma(cc, m1, m01);
+      }
+      v[0][e] = m0;
+      v[1][e] = m1;
+    }
+  }
+  // per-feature sums of weight x squared difference
+#pragma unroll
+  for (int d = 0; d < 2; ++d) {
+    if (d < sp.ndot) {
+      const Leaf& L = sp.leaf[sp.dot_leaf[d]];
+      const int per = L.type == L_PERIODIC ? 2 : 1;
+      for (int k0 = 0; k0 < L.n; k0 += GF_CH / per) {
+        const int kn = min(GF_CH / per, L.n - k0);
+        __syncthreads();
+        for (int q = tid; q < kn * per * TB; q += 256) {
+          const double* src = P.planes + (size_t)(L.plane0 + k0 * per + q / TB) * nc;
+          Xi[q] = src[ti * TB + q % TB];
+          Xj[q] = src[tj * TB + q % TB];
+        }
+        __syncthreads();
+        for (int k = 0; k < kn; ++k) {
+          double acc = 0.0;
+          if (per == 1) {
+            const double2 xi = *reinterpret_cast<const double2*>(Xi + k * TB + r0);
+#pragma unroll
+            for (int c = 0; c < 8; ++c) {
+              const double xj = Xj[k * TB + c0 + c];
+#pragma unroll
+              for (int a = 0; a < 2; ++a) {
+                const double df = (a ? xi.y : xi.x) - xj;
+                acc = fma(v[d][c * 2 + a] * df, df, acc);
+              }
+            }
+          } else {
+            const double2 si = *reinterpret_cast<const double2*>(Xi + (2 * k) * TB + r0);
+            const double2 ci = *reinterpret_cast<const double2*>(Xi + (2 * k + 1) * TB + r0);
+#pragma unroll
+            for (int c = 0; c < 8; ++c) {
+              const double sj = Xj[(2 * k) * TB + c0 + c], cj = Xj[(2 * k + 1) * TB + c0 + c];
+#pragma unroll
+              for (int a = 0; a < 2; ++a) {
+                const double t = fma(a ? si.y : si.x, cj, -((a ? ci.y : ci.x) * sj));
+                acc = fma(v[d][c * 2 + a] * t, t, acc);
+              }
+            }
+          }
+          red[k * 256 + tid] = acc;
+        }
+        __syncthreads();
+        // 16 threads per feature, in a fixed order
+        const int k = tid >> 4;
+        double t = 0.0;
+        if (k < kn)
+          for (int q = tid & 15; q < 256; q += 16) t += red[k * 256 + q];
+        for (int o = 8; o > 0; o >>= 1) t += __shfl_down_sync(0xffffffffu, t, o, 16);
+        if (k < kn && (tid & 15) == 0) gp[L.param0 + k0 + k] = t;
+      }
+    }
+  }
+  __syncthreads();
+#pragma unroll
+  for (int q = 0; q < 5; ++q) red[q * 256 + tid] = s[q];
+  __syncthreads();
+  const int k = tid >> 4;
+  double t = 0.0;
+  if (k < 5)
+    for (int q = tid & 15; q < 256; q += 16) t += red[k * 256 + q];
+  for (int o = 8; o > 0; o >>= 1) t += __shfl_down_sync(0xffffffffu, t, o, 16);
+  if (k < 5 && (tid & 15) == 0) gp[nslots - 5 + k] = t;
+}
+
+// sums of the tiles' partials (one CTA per slot, in a fixed order), then d logL /
+// d theta: the distance leaves' from their features' sums, the linear and
+// constant leaves' through the expression's coefficients
+__global__ void __launch_bounds__(256)
+    k_grad_fast_reduce(const Prob* __restrict__ pp, int ntiles, int nslots, double* __restrict__ sums) {
+  __shared__ double red[256];
+  const int q = blockIdx.x, tid = threadIdx.x;
+  double t = 0.0;
+  for (int b = tid; b < ntiles; b += 256) t += pp->gpart[(size_t)b * nslots + q];
+  red[tid] = t;
+  __syncthreads();
+  for (int o = 128; o > 0; o >>= 1) {
+    if (tid < o) red[tid] += red[tid + o];
+    __syncthreads();
+  }
+  if (tid == 0) sums[q] = red[0];
+}
+__global__ void __launch_bounds__(256)
+    k_grad_fast_out(const Prob* __restrict__ pp, const double* __restrict__ sums, int nslots, int noise_slot,
+                    double* __restrict__ g) {
+  const Prob& P = *pp;
+  const Spec& sp = *P.spec;
+  const double* s = sums + nslots - 5;
+  const int q = threadIdx.x;  // parameter
+  if (q == 0 && noise_slot >= 0) g[noise_slot] = 0.5 * s[4];
+  if (q >= sp.nkparams) return;
+  int leaf = 0;
+  for (int l = 0; l < sp.nleaf; ++l) {
+    const int cnt = sp.leaf[l].type == L_CONSTANT ? 1 : sp.leaf[l].n;
+    if (q >= sp.leaf[l].param0 && q < sp.leaf[l].param0 + cnt) leaf = l;
+  }
+  const int type = sp.leaf[leaf].type;
+  const double t = P.theta[q];
+  if (type == L_RBF) {  // dv/dtheta = -v l (x_i - x_j)^2 / 2
+    g[q] = 0.5 * (-0.5 * exp(t)) * sums[q];
+  } else if (type == L_PERIODIC) {  // 4 v l sin^2(d / 2)
+    const double il = 1.0 / exp(t);
+    g[q] = 0.5 * (4.0 * (il * il)) * sums[q];
+  } else {
+    // the expression's coefficients (1, v0, v1, v0 v1) and their derivative by this leaf
+    double c[MAX_POST][4], dc[MAX_POST][4];
+    int top = 0;
+    for (int k = 0; k < sp.npost; ++k) {
+      const int tok = sp.post[k];
+      if (tok >= 0) {
+        const Leaf& L = sp.leaf[tok];
+        for (int m = 0; m < 4; ++m) c[top][m] = dc[top][m] = 0.0;
+        if (L.type == L_RBF || L.type == L_PERIODIC) {
+          c[top][tok == sp.dot_leaf[0] ? 1 : 2] = 1.0;
+        } else if (L.type == L_LINEAR) {
+          for (int m = 0; m < L.n; ++m) c[top][0] += 1.0 / exp(-P.theta[L.param0 + m]);
+          if (tok == leaf) dc[top][0] = 1.0 / exp(-t);
+        } else {
+          c[top][0] = P.theta[L.param0];
+          if (tok == leaf) dc[top][0] = 1.0;
+        }
+        ++top;
+      } else {
+        const double* b = c[top - 1];
+        const double* db = dc[top - 1];
+        --top;
+        double* a = c[top - 1];
+        double* da = dc[top - 1];
+        if (tok == P_SUM) {
+          for (int m = 0; m < 4; ++m) {
+            a[m] += b[m];
+            da[m] += db[m];
+          }
+        } else {  // each leaf occurs once: no squared terms
+          double r[4], dr[4];
+          r[0] = a[0] * b[0];
+          r[1] = a[0] * b[1] + a[1] * b[0];
+          r[2] = a[0] * b[2] + a[2] * b[0];
+          r[3] = a[0] * b[3] + a[3] * b[0] + a[1] * b[2] + a[2] * b[1];
+          dr[0] = da[0] * b[0] + a[0] * db[0];
+          dr[1] = da[0] * b[1] + a[0] * db[1] + da[1] * b[0] + a[1] * db[0];
+          dr[2] = da[0] * b[2] + a[0] * db[2] + da[2] * b[0] + a[2] * db[0];
+          dr[3] = da[0] * b[3] + a[0] * db[3] + da[3] * b[0] + a[3] * db[0] + da[1] * b[2] + a[1] * db[2] +
+                  da[2] * b[1] + a[2] * db[1];
+          for (int m = 0; m < 4; ++m) {
+            a[m] = r[m];
+            da[m] = dr[m];
+          }
+        }
+      }
+    }
+    g[q] = 0.5 * (dc[0][0] * s[0] + dc[0][1] * s[1] + dc[0][2] * s[2] + dc[0][3] * s[3]);
+  }
+}
+
+size_t grad_fast_partials(int nsteps, int nk) { return (size_t)nsteps * (nsteps + 1) / 2 * (nk + 5) + (nk + 5); }
+
+cudaError_t enqueue_grad_fast(const Prob* p, const Prob* eval, int nsteps, int nc_eval, int nplanes, int nk, int extra,
+                              int optimise_noise, long long* fx, double* sums, double* g_out, cudaStream_t s,
+                              long long* nlaunch) {
+  cudaError_t e = ensure_smem_attr((const void*)k_grad_fast, SMEM_GRAD_FAST, GF_SMEM);
+  if (e != cudaSuccess) return e;
+  const int ntiles = nsteps * (nsteps + 1) / 2, nslots = nk + 5;
+  k_grad_fixed<<<dim3((nc_eval + 255) / 256, nplanes), 256, 0, s>>>(eval, fx);
+  k_grad_fast<<<ntiles, 256, GF_SMEM, s>>>(p, eval, fx, nslots, extra);
+  k_grad_fast_reduce<<<nslots, 256, 0, s>>>(p, ntiles, nslots, sums);
+  k_grad_fast_out<<<1, 256, 0, s>>>(p, sums, nslots, optimise_noise ? nk : -1, g_out);
+  if (nlaunch) *nlaunch += 4;
+  return cudaGetLastError();
 }
 
 cudaError_t launch_identity_border(const Prob* p, int nc, cudaStream_t s) {

@@ -157,6 +157,13 @@ __device__ __forceinline__ long long to_fixed62(double x, int e, bool* nonfinite
   return bits < 0 ? -F : F;
 }
 
+// round(x 2^(54 - e)) for |x| < 2^e (a scale break, NaN and infinities are the
+// caller's to have excluded: the same features passed to_fixed55 before)
+__device__ __forceinline__ long long to_fixed54(double x, int e) {
+  bool bad = false;
+  return (to_fixed55(x, e, &bad) + 1) >> 1;
+}
+
 // a diagonal entry: kernel value plus nugget.  NaN becomes negative, which
 // fails that pivot as NaN does in dpotrf.
 __device__ __forceinline__ long long diag_fixed62(double k, double noise, int e, bool* nonfinite) {
