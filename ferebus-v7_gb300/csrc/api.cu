@@ -472,10 +472,9 @@ int enqueue_eval(const Prob* probs_d, int nprob, int max_nsteps, int max_nplanes
   CK(cudaMemsetAsync(status_base, 0, status_bytes, s));
   if (mode == 1) {
     // 128-wide panels; max_nsteps counts 64-column tiles
-    const int nt = max_nsteps / 2, max_nc = max_nsteps * TB;
+    const int nt = max_nsteps / 2;
     CK(cudaMemsetAsync(us->sync_dev, 0, sizeof(int) * us->nsync, s));
-    STAGE(0, launch_prep_planes(probs_d, nprob, max_nc, s));
-    if (us->build_total > 0) STAGE(0, launch_feat_digits(probs_d, nprob, nt, s));
+    STAGE(0, launch_prep(probs_d, nprob, nt, s));
     if (us->dot_builds > 0) STAGE(0, launch_build_dot(probs_d, nprob, max_nsteps, max_nplanes, s));
     if (us->build_total > 0)
       STAGE(0, launch_build_tc(probs_d, nprob, us->build_tiles_dev, us->build_total, us->num_sms, s));

@@ -50,23 +50,6 @@ namespace fgpu {
 
 namespace {
 
-// per-plane feature scale of leaf L: rbf sqrt(exp(theta)), periodic 1/exp(theta)
-__device__ __forceinline__ double plane_weight(const Leaf& L, const double* theta, int k) {
-  return L.type == L_RBF ? exp(0.5 * theta[L.param0 + k]) : 1.0 / exp(theta[L.param0 + k]);
-}
-
-// s with max_k |w_k x_ik| < 2^s over every point (from the per-plane maxima)
-__device__ __forceinline__ int leaf_scale(const Prob& P, const Leaf& L) {
-  const int nf = L.type == L_PERIODIC ? 2 * L.n : L.n;
-  double m = 0.0;
-  for (int k = 0; k < nf; ++k) {
-    const int dim = L.type == L_PERIODIC ? k / 2 : k;
-    m = fmax(m, plane_weight(L, P.theta, dim) * P.plane_max[L.plane0 + k]);
-  }
-  if (m == 0.0) return 0;
-  return (int)((__double_as_longlong(m) >> 52) & 0x7FF) - 1022;
-}
-
 constexpr int NLEV = 8;  // digit-pair levels p + q = 0..7
 
 // W = round(sum_L S_L 2^(u - 16 - 8L)) from the 8 exact level sums (48 <= u <= 63)
@@ -97,58 +80,59 @@ __device__ __forceinline__ long long assemble_w_bits(const uint32_t b[NLEV], int
 }  // namespace
 
 // ---------------------------------------------------------------------------
-// feature digits and exact self dot products; one thread per point
+// preparation of an evaluation, one CTA per 128 points: the features' weights,
+// the problem's scale, the right-hand sides, the scaled features and, for the
+// tensor-core build, their digit planes and exact self products.
 // grid (nt128, nprob) x 128 threads
+//
+// An exponential is ~50 FP64 instructions of 64 cycles each on this GPU, so each
+// weight is formed once per CTA, a thread per parameter, and not by every
+// point (prep and digits as two kernels with an exponential per point and
+// feature, and a serial one per leaf: 13 + 26 us for a lone problem of 500
+// points, 29 + 57 us at N = 4000).
 // ---------------------------------------------------------------------------
-__global__ void __launch_bounds__(128) k_feat_digits(const Prob* __restrict__ probs) {
+__global__ void __launch_bounds__(128) k_prep(const Prob* __restrict__ probs) {
   const Prob& P = probs[blockIdx.y];
   const int rb = blockIdx.x;
   if (P.mode != 1 || rb >= P.nt128) return;
   const Spec& sp = *P.spec;
-  if (!sp.tc_build) return;
-  const int r = threadIdx.x, i = rb * NB + r;
+  const int tid = threadIdx.x, i = rb * NB + tid;
   const size_t nc = (size_t)P.Nc;
-  __shared__ int s_e[2];
-  if (r < sp.ndot) {
-    s_e[r] = leaf_scale(P, sp.leaf[sp.dot_leaf[r]]);
-    if (rb == 0) P.fscale[r] = s_e[r];
+  __shared__ double w[MAX_PARAMS];  // rbf sqrt(exp(theta)), periodic 1 / exp(theta), linear 1 / c, constant theta
+  __shared__ int s_e[2], s_k;
+  for (int q = tid; q < sp.nkparams; q += 128) {
+    int type = L_CONSTANT;
+    for (int l = 0; l < sp.nleaf; ++l) {
+      const int cnt = sp.leaf[l].type == L_CONSTANT ? 1 : sp.leaf[l].n;
+      if (q >= sp.leaf[l].param0 && q < sp.leaf[l].param0 + cnt) type = sp.leaf[l].type;
+    }
+    const double t = P.theta[q];
+    // linear_kernel.f90:70-76, order 0: sum_k 1 / exp(-theta_k); constant.f90:62-68
+    w[q] = type == L_CONSTANT ? t : 1.0;
+    if (type == L_RBF || type == L_PERIODIC || type == L_LINEAR) {
+      const double x = exp(type == L_RBF ? 0.5 * t : (type == L_LINEAR ? -t : t));
+      w[q] = type == L_RBF ? x : 1.0 / x;
+    }
   }
   __syncthreads();
-  bool bad = false;
-  for (int t = 0; t < sp.ndot; ++t) {
-    const Leaf& L = sp.leaf[sp.dot_leaf[t]];
-    const int nf = L.type == L_PERIODIC ? 2 * L.n : L.n;
-    const int e = s_e[t];
-    int S[NLEV] = {0, 0, 0, 0, 0, 0, 0, 0};
-    unsigned char* base = P.slices + (size_t)rb * NSLICE * SLICE_BYTES + (size_t)r * 16;
-    for (int kg = 0; kg < sp.dot_kch[t] * 2; ++kg) {
-      int d[NSLICE][8];
-      for (int kk = 0; kk < 8; ++kk) {
-        const int k = kg * 8 + kk;
-        const double x = (k < nf) ? P.splanes[(size_t)(L.plane0 + k) * nc + i] : 0.0;
-        long long F = to_fixed55(x, e, &bad);
-        for (int p = NSLICE - 1; p >= 1; --p) {
-          const int b = (int)(signed char)(F & 0xFF);
-          d[p][kk] = b;
-          F = (F - b) >> 8;
-        }
-        d[0][kk] = (int)F;
-        for (int p = 0; p < NSLICE; ++p)
-          for (int q = 0; q < NSLICE && p + q < NLEV; ++q) S[p + q] += d[p][kk] * d[q][kk];
-      }
-      const int kgl = sp.dot_koff[t] / 8 + kg;
-      for (int p = 0; p < NSLICE; ++p) {
-        __align__(16) __half h[8];
-        for (int kk = 0; kk < 8; ++kk) h[kk] = __int2half_rn(d[p][kk]);
-        *reinterpret_cast<uint4*>(base + (size_t)p * SLICE_BYTES + (size_t)kgl * 2048) =
-            *reinterpret_cast<const uint4*>(h);
+  if (tid >= 64) {
+    // scale of distance leaf d, 2^s > max |f| over every point (from the per-plane maxima)
+    const int d = (tid - 64) >> 5, lane = tid & 31;
+    if (sp.tc_build && d < sp.ndot) {
+      const Leaf& L = sp.leaf[sp.dot_leaf[d]];
+      const int per = L.type == L_PERIODIC ? 2 : 1;
+      double m = 0.0;
+      for (int k = lane; k < per * L.n; k += 32) m = fmax(m, w[L.param0 + k / per] * P.plane_max[L.plane0 + k]);
+      for (int o = 16; o > 0; o >>= 1) m = fmax(m, __shfl_xor_sync(0xffffffffu, m, o));
+      if (lane == 0) {
+        s_e[d] = m == 0.0 ? 0 : (int)((__double_as_longlong(m) >> 52) & 0x7FF) - 1022;
+        if (rb == 0) P.fscale[d] = s_e[d];
       }
     }
-    P.fnorm[(size_t)t * nc + i] = assemble_w(S, sp.dot_u[t]);
-  }
-  if (bad) atomicOr(&P.status[3], 1);
-  // multilinear coefficients of the kernel expression in the distance leaves
-  if (rb == 0 && r == 0) {
+  } else if (tid == 0) {
+    // the kernel expression in the (at most two) distance leaves of the
+    // tensor-core build, c0 + c1 v0 + c2 v1 + c3 v0 v1; with other leaves only
+    // its value at zero distance, in c0
     double stk[MAX_POST][4];
     int top = 0;
     for (int tk = 0; tk < sp.npost; ++tk) {
@@ -156,37 +140,115 @@ __global__ void __launch_bounds__(128) k_feat_digits(const Prob* __restrict__ pr
       if (tok >= 0) {
         const Leaf& L = sp.leaf[tok];
         double c[4] = {0.0, 0.0, 0.0, 0.0};
-        if (L.type == L_RBF || L.type == L_PERIODIC) {
+        if (L.type == L_LINEAR) {
+          for (int k = 0; k < L.n; ++k) c[0] += w[L.param0 + k];
+        } else if (L.type == L_CONSTANT) {
+          c[0] = w[L.param0];
+        } else if (sp.tc_build) {
           c[tok == sp.dot_leaf[0] ? 1 : 2] = 1.0;
-        } else if (L.type == L_LINEAR) {
-          // linear_kernel.f90:70-76, order 0: sum_k 1 / exp(-theta_k)
-          double a = 0.0;
-          for (int k = 0; k < L.n; ++k) a += 1.0 / exp(-P.theta[L.param0 + k]);
-          c[0] = a;
         } else {
-          c[0] = P.theta[L.param0];  // constant.f90:62-68
+          c[0] = 1.0;
         }
         for (int q = 0; q < 4; ++q) stk[top][q] = c[q];
         ++top;
       } else {
-        const double* b = stk[--top];
-        double* a = stk[top - 1];
+        const double* y = stk[--top];
+        double* x = stk[top - 1];
         if (tok == P_SUM) {
-          for (int q = 0; q < 4; ++q) a[q] += b[q];
-        } else {  // each leaf occurs once: no squared terms
-          const double c0 = a[0] * b[0];
-          const double c1 = a[0] * b[1] + a[1] * b[0];
-          const double c2 = a[0] * b[2] + a[2] * b[0];
-          const double c3 = a[0] * b[3] + a[3] * b[0] + a[1] * b[2] + a[2] * b[1];
-          a[0] = c0;
-          a[1] = c1;
-          a[2] = c2;
-          a[3] = c3;
+          for (int q = 0; q < 4; ++q) x[q] += y[q];
+        } else if (sp.tc_build) {  // each leaf occurs once: no squared terms
+          const double c0 = x[0] * y[0];
+          const double c1 = x[0] * y[1] + x[1] * y[0];
+          const double c2 = x[0] * y[2] + x[2] * y[0];
+          const double c3 = x[0] * y[3] + x[3] * y[0] + x[1] * y[2] + x[2] * y[1];
+          x[0] = c0;
+          x[1] = c1;
+          x[2] = c2;
+          x[3] = c3;
+        } else {
+          x[0] *= y[0];
         }
       }
     }
-    for (int q = 0; q < 4; ++q) P.fcoef[q] = stk[0][q];
+    if (rb == 0 && sp.tc_build)
+      for (int q = 0; q < 4; ++q) P.fcoef[q] = stk[0][q];
+    // the scale 2^e > sqrt(K_ii): the kernels are stationary, so K_ii is one
+    // value, the expression with every distance leaf at 1, plus the nugget
+    const double d = (sp.tc_build ? (stk[0][3] + stk[0][2]) + (stk[0][1] + stk[0][0]) : stk[0][0]) +
+                     (P.optimise_noise ? P.theta[sp.nkparams] : P.noise);
+    int e = 0;
+    if (d > 0.0 && d < 1e300) frexp(sqrt(d) * (1.0 + 0x1p-20), &e);  // sqrt(K_ii) (1 + 2^-20) < 2^e
+    s_k = e;
+    if (rb == 0) P.kscale[0] = e;
   }
+  __syncthreads();
+  {
+    // right-hand sides: y - mu (marginal), or y and 1 (concentrated), in the factor's scale; zero on the padding
+    const double u = ldexp(1.0, -s_k);
+    P.rhs[i] = i < P.N ? u * (P.likelihood == 1 ? P.y[i] : P.y[i] - P.mu[i]) : 0.0;
+    if (P.nrhs > 1) P.rhs[nc + i] = i < P.N ? u : 0.0;
+  }
+  if (!sp.tc_build) {
+    // the dot-product build's scaled planes and rbf norms (the workspace is not
+    // cleared between evaluations: norms of other leaves are zeroed here)
+    for (int l = 0; l < MAX_LEAF; ++l) {
+      double a = 0.0;
+      if (l < sp.nleaf) {
+        const Leaf& L = sp.leaf[l];
+        const int per = L.type == L_PERIODIC ? 2 : 1;
+        const int cnt = L.type == L_LINEAR || L.type == L_CONSTANT ? 0 : per * L.n;
+        for (int k = 0; k < cnt; ++k) {
+          const size_t o = (size_t)(L.plane0 + k) * nc + i;
+          const double u = w[L.param0 + k / per] * P.planes[o];
+          P.splanes[o] = u;
+          if (L.type == L_RBF) a = fma(u, u, a);
+        }
+      }
+      P.norms[(size_t)l * nc + i] = a;
+    }
+    return;
+  }
+  bool bad = false;
+  for (int t = 0; t < sp.ndot; ++t) {
+    const Leaf& L = sp.leaf[sp.dot_leaf[t]];
+    const int per = L.type == L_PERIODIC ? 2 : 1, nf = per * L.n;
+    const int e = s_e[t];
+    int S[NLEV] = {0, 0, 0, 0, 0, 0, 0, 0};
+    unsigned char* base = P.slices + (size_t)rb * NSLICE * SLICE_BYTES + (size_t)tid * 16;
+    for (int kg = 0; kg < sp.dot_kch[t] * 2; ++kg) {
+      long long F[8];
+#pragma unroll
+      for (int kk = 0; kk < 8; ++kk) {
+        const int k = kg * 8 + kk;
+        F[kk] = 0;
+        if (k < nf) {
+          const size_t o = (size_t)(L.plane0 + k) * nc + i;
+          const double x = w[L.param0 + k / per] * P.planes[o];
+          if (P.keep_l) P.splanes[o] = x;  // the adjoint's features
+          F[kk] = to_fixed55(x, e, &bad);
+        }
+        // W_ii's level sums, from the same digits as the products'
+        const long long G = F[kk] + 0x808080808080LL;
+        int d[NSLICE];
+        d[0] = (int)(G >> 48);
+#pragma unroll
+        for (int p = 1; p < NSLICE; ++p) d[p] = (int)((G >> (8 * (6 - p))) & 0xFF) - 128;
+#pragma unroll
+        for (int p = 0; p < NSLICE; ++p)
+#pragma unroll
+          for (int q = p; q < NSLICE; ++q)
+            if (p + q < NLEV) S[p + q] += (p == q ? 1 : 2) * d[p] * d[q];
+      }
+      uint4 out[NSLICE];
+      digits8_of_fixed55(F, out);
+      const int kgl = sp.dot_koff[t] / 8 + kg;
+#pragma unroll
+      for (int p = 0; p < NSLICE; ++p)
+        *reinterpret_cast<uint4*>(base + (size_t)p * SLICE_BYTES + (size_t)kgl * 2048) = out[p];
+    }
+    P.fnorm[(size_t)t * nc + i] = assemble_w(S, sp.dot_u[t]);
+  }
+  if (bad) atomicOr(&P.status[3], 1);
 }
 
 // ---------------------------------------------------------------------------
@@ -471,8 +533,8 @@ __global__ void __launch_bounds__(BLD_THREADS, 1)
 // ---------------------------------------------------------------------------
 // launch helpers
 // ---------------------------------------------------------------------------
-cudaError_t launch_feat_digits(const Prob* probs, int nprob, int max_nt128, cudaStream_t s) {
-  k_feat_digits<<<dim3(max_nt128, nprob), 128, 0, s>>>(probs);
+cudaError_t launch_prep(const Prob* probs, int nprob, int max_nt128, cudaStream_t s) {
+  k_prep<<<dim3(max_nt128, nprob), 128, 0, s>>>(probs);
   return cudaGetLastError();
 }
 

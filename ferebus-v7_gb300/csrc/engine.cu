@@ -230,88 +230,6 @@ __global__ void __launch_bounds__(256) k_build(const Prob* __restrict__ probs) {
 // form for the well separated pairs that dominate, and it vanishes on the
 // diagonal, which is set exactly (x_i = x_j gives a factor 1).
 // ---------------------------------------------------------------------------
-// the kernel expression at zero distance
-__device__ double kernel_diagonal(const Spec& sp, const double* theta) {
-  double stk[MAX_LEAF];
-  int top = 0;
-  for (int t = 0; t < sp.npost; ++t) {
-    const int tok = sp.post[t];
-    if (tok >= 0) {
-      const Leaf& L = sp.leaf[tok];
-      double v = 1.0;
-      if (L.type == L_LINEAR) {
-        v = 0.0;
-        for (int k = 0; k < L.n; ++k) v += 1.0 / transform_param(L_LINEAR, theta[L.param0 + k]);
-      } else if (L.type == L_CONSTANT) {
-        v = theta[L.param0];
-      }
-      stk[top++] = v;
-    } else {
-      const double b = stk[--top];
-      const double a = stk[--top];
-      stk[top++] = (tok == P_SUM) ? a + b : a * b;
-    }
-  }
-  return stk[0];
-}
-
-__global__ void __launch_bounds__(256) k_prep_planes(const Prob* __restrict__ probs) {
-  const Prob& P = probs[blockIdx.z];
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  const int l = blockIdx.y;
-  if (P.mode != 1 || (int)(blockIdx.x * blockDim.x) >= P.Nc) return;
-  const Spec& sp = *P.spec;
-  const size_t nc = (size_t)P.Nc;
-  if (l == 0) {
-    // the scale 2^e > sqrt(K_ii): the kernels are stationary, so K_ii is one
-    // value, the expression with every distance leaf at 1, plus the nugget
-    __shared__ int s_e;
-    if (threadIdx.x == 0) {
-      const double d = kernel_diagonal(sp, P.theta) + (P.optimise_noise ? P.theta[sp.nkparams] : P.noise);
-      int e = 0;
-      if (d > 0.0 && d < 1e300) frexp(sqrt(d) * (1.0 + 0x1p-20), &e);  // sqrt(K_ii) (1 + 2^-20) < 2^e
-      s_e = e;
-      if (blockIdx.x == 0) P.kscale[0] = e;
-    }
-    __syncthreads();
-    // right-hand sides: y - mu (marginal), or y and 1 (concentrated), in the factor's scale; zero on the padding
-    if (i < P.Nc) {
-      const double w = ldexp(1.0, -s_e);
-      P.rhs[i] = i < P.N ? w * (P.likelihood == 1 ? P.y[i] : P.y[i] - P.mu[i]) : 0.0;
-      if (P.nrhs > 1) P.rhs[nc + i] = i < P.N ? w : 0.0;
-    }
-  }
-  if (i >= P.Nc) return;
-  // the workspace is not cleared between evaluations (a batch plan reuses
-  // it across problems): rows of non-rbf leaves are zeroed here
-  if (l >= sp.nleaf || sp.leaf[l].type != L_RBF) P.norms[(size_t)l * nc + i] = 0.0;
-  if (l >= sp.nleaf) return;
-  const Leaf& L = sp.leaf[l];
-  if (L.type == L_RBF) {
-    double a = 0.0;
-    for (int k = 0; k < L.n; ++k) {
-      const double w = exp(0.5 * P.theta[L.param0 + k]);  // sqrt(exp(theta))
-      const double u = w * P.planes[(size_t)(L.plane0 + k) * nc + i];
-      P.splanes[(size_t)(L.plane0 + k) * nc + i] = u;
-      a = fma(u, u, a);
-    }
-    P.norms[(size_t)l * nc + i] = a;
-  } else if (L.type == L_PERIODIC) {
-    for (int k = 0; k < L.n; ++k) {
-      const double w = 1.0 / exp(P.theta[L.param0 + k]);  // sqrt((1 / exp(theta))^2)
-      for (int t = 0; t < 2; ++t) {
-        const size_t o = (size_t)(L.plane0 + 2 * k + t) * nc + i;
-        P.splanes[o] = w * P.planes[o];
-      }
-    }
-  } else if (L.type == L_RBF_CYCLIC) {
-    for (int k = 0; k < L.n; ++k) {
-      const size_t o = (size_t)(L.plane0 + k) * nc + i;
-      P.splanes[o] = P.planes[o];
-    }
-  }
-}
-
 size_t build_dot_smem_bytes(int nplanes) {
   return (size_t)2 * (nplanes + MAX_LEAF) * TB * sizeof(double) + 64;
 }
@@ -781,11 +699,6 @@ cudaError_t launch_build(const Prob* probs, int nprob, int max_nsteps, int max_n
   if (e != cudaSuccess) return e;
   dim3 grid(max_nsteps + 1, max_nsteps, nprob);
   k_build<<<grid, 256, smem, s>>>(probs);
-  return cudaGetLastError();
-}
-
-cudaError_t launch_prep_planes(const Prob* probs, int nprob, int max_nc, cudaStream_t s) {
-  k_prep_planes<<<dim3((max_nc + 255) / 256, MAX_LEAF, nprob), 256, 0, s>>>(probs);
   return cudaGetLastError();
 }
 

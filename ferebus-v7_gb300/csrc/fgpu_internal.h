@@ -131,8 +131,7 @@ int encode_slice_maps(void* host_maps, const void* slices, int nt128);
 // and index it by blockIdx.y; problems whose geometry does not reach the
 // current step exit immediately, so ragged batches share one launch.
 cudaError_t launch_build(const Prob* probs, int nprob, int max_nsteps, int max_nplanes, cudaStream_t s);
-// mode 1: per-evaluation scaled planes, then the dot-product form of the build
-cudaError_t launch_prep_planes(const Prob* probs, int nprob, int max_nc, cudaStream_t s);
+// mode 1: the dot-product form of the build, for kernels the tensor cores do not serve
 cudaError_t launch_build_dot(const Prob* probs, int nprob, int max_nsteps, int max_nplanes, cudaStream_t s);
 size_t build_dot_smem_bytes(int nplanes);
 cudaError_t launch_potf2(const Prob* probs, int nprob, int step, cudaStream_t s);
@@ -181,11 +180,12 @@ cudaError_t launch_panel(const Prob* probs, int step, const int* order, int ndia
 // tiles: the step's trailing tiles, packed (problem << 40 | row tile << 20 | column tile)
 cudaError_t launch_ozaki_update(const Prob* probs, int nprob, int step, int max_nt128,
                                 const unsigned long long* tiles, int total_tiles, int num_sms, cudaStream_t s);
-// Tensor-core kernel-matrix build (build_tc.cu): feature digit planes and
-// exact self products, then the persistent build of the lower triangle.
+// Preparation of an evaluation and the tensor-core kernel-matrix build
+// (build_tc.cu): weights, scale, right-hand sides, scaled features or feature
+// digits; then the persistent build of the lower triangle.
 // tiles: the lower triangle's 128 x 64 tiles of every eligible problem,
 // packed (problem << 40 | row tile << 20 | column tile).
-cudaError_t launch_feat_digits(const Prob* probs, int nprob, int max_nt128, cudaStream_t s);
+cudaError_t launch_prep(const Prob* probs, int nprob, int max_nt128, cudaStream_t s);
 cudaError_t launch_build_tc(const Prob* probs, int nprob, const unsigned long long* tiles, int total_tiles,
                             int num_sms, cudaStream_t s);
 
