@@ -190,6 +190,7 @@ struct Workspace {
   unsigned char* slices = nullptr;
   unsigned char* tmaps = nullptr;  // TMA tensor maps over slices (128-, 64-row boxes; 64 rows, planes stacked)
   double* rhs = nullptr;           // right-hand sides
+  double* ldiag = nullptr;         // the kept factor's diagonal
   PanelBlock* lpub = nullptr;      // the current panel's published diagonal blocks
   PanelZ* zpub = nullptr;          // and solved right-hand-side entries
   double* splanes = nullptr;       // theta-scaled planes (dot-product build)
@@ -357,6 +358,7 @@ void fill_prob(Prob& p, const fgpu_ctx* c, const double* theta_d, const Workspac
   p.tmap_b = ws.tmaps ? ws.tmaps + 128 : nullptr;
   p.tmap_bs = ws.tmaps ? ws.tmaps + 256 : nullptr;
   p.rhs = ws.rhs;
+  p.ldiag = ws.ldiag;
   p.lpub = ws.lpub;
   p.zpub = ws.zpub;
   p.splanes = ws.splanes;
@@ -622,6 +624,7 @@ size_t layout_workspace(const fgpu_ctx* c, unsigned char* base, Workspace& ws, b
   if (c->mode == 1) {
     take(ws.kscale, sizeof(int) * 2);
     take(ws.rhs, sizeof(double) * MAX_RHS * nc);
+    if (keep_l) take(ws.ldiag, sizeof(double) * nc);
     take(ws.lpub, sizeof(PanelBlock) * 8);
     take(ws.zpub, sizeof(PanelZ) * 8);
     take(ws.acc, sizeof(long long) * acc_tiles(c->nt128) * ACC_TILE_ELEMS);
@@ -976,6 +979,10 @@ int fgpu_loglik(fgpu_ctx* ctx, const double* theta, int ntheta, double* ll, int*
   CK(cudaGraphLaunch(w->graph, w->stream));
   t_launches = w->graph_kernels;
   if (alpha) {
+    if (ctx->mode == 1) {
+      CK(launch_factor_doubles(w->prob_d, ctx->nt128, w->stream));
+      ++t_launches;
+    }
     CK(launch_backsolve(w->prob_d, ctx->nsteps, w->bsync, w->stream));
     ++t_launches;
   }
@@ -1143,8 +1150,9 @@ int fgpu_grad(fgpu_ctx* ctx, const double* theta, int ntheta, double* ll, double
     CK(cudaMemcpyAsync(w->theta_d, w->h_stage, sizeof(double) * ntheta, cudaMemcpyHostToDevice, s));
     CK(cudaGraphLaunch(w->graph, s));
     n += w->graph_kernels;
+    CK(launch_factor_doubles(w->prob_d, ctx->nt128, s));
     CK(launch_backsolve(w->prob_d, ctx->nsteps, w->bsync, s));
-    ++n;
+    n += 2;
     if (g->tc)
       CK(enqueue_inverse(w->prob_d, ctx->nt128, g->inv, g->levels, g->num_sms, s, &n));
     else

@@ -59,11 +59,11 @@ struct Spec {
   int dot_u[2];                   // W units: <f_i, f_j> 2^(u - 2 - 2s)
 };
 
-// A 16 x 16 diagonal block of the factor (panel.cu): its entries L'_jc 2^60 as
-// (high, low) 30-bit halves, and 1 / L'_jj = y 2^(sh - 62).
+// A 16 x 16 diagonal block of the factor (panel.cu): its entries L'_jc 2^60 at
+// x[j][c] as (high, low) 30-bit halves, and 1 / L'_jj = y 2^(sh - 62).
 struct alignas(16) PanelBlock {
   int2 x[16][16];
-  unsigned long long y[16];
+  uint2 y[16];  // high, low word
   int sh[16];
 };
 // 16 entries of each solved right-hand side, z = (x as above) 2^-60 scale
@@ -100,7 +100,8 @@ struct Prob {
   double* rhs;                    // MAX_RHS x Nc: right-hand sides times 2^-e, turned into L^-1 r panel by panel
   PanelBlock* lpub;               // 8: the current panel's diagonal blocks, as its diagonal tile publishes them
   PanelZ* zpub;                   // 8: and its solved right-hand-side entries
-  int keep_l;                     // K exists and receives the factor (alpha and the adjoint read it)
+  int keep_l;                     // K exists and receives the factor, as 60-bit fixed point (launch_factor_doubles)
+  double* ldiag;                  // Nc: the factor's diagonal (keep_l)
   // dot-product kernel build (mode 1): planes scaled by sqrt(l_k) per evaluation
   double* splanes;                // nplanes x Nc
   double* norms;                  // MAX_LEAF x Nc: sum_k u_ik^2 of rbf leaves
@@ -141,6 +142,8 @@ cudaError_t launch_trsm(const Prob* probs, int nprob, int step, int max_nsteps, 
 cudaError_t launch_update(const Prob* probs, int nprob, int step, int max_nsteps, cudaStream_t s,
                           int max_rowtiles = 0);
 cudaError_t launch_finalize(const Prob* probs, int nprob, cudaStream_t s);
+// the kept factor of a tensor-core problem to doubles, in place, for alpha and the adjoint
+cudaError_t launch_factor_doubles(const Prob* prob, int nt128, cudaStream_t s);
 // alpha of one problem; sync: two ints of scratch
 cudaError_t launch_backsolve(const Prob* prob, int nsteps, int* sync, cudaStream_t s);
 size_t build_smem_bytes(int nplanes);

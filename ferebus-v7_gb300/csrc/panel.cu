@@ -88,43 +88,91 @@ __device__ __forceinline__ void cp_async16(void* dst, const void* src) {
 }
 __device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_all;" ::: "memory"); }
 
-// 1 / sqrt(D 2^-62), 0 < D < 2^62, as y 2^(sh - 62) with y in [2^62, 2^63): a
-// single-precision estimate refined once in 64-bit fixed point.  With
-// D 2^-62 = m 4^k, 1 <= m < 4 (k < 0, sh = -k - 1), and y0 ~ m^-1/2 (24 bits):
+// 1 / sqrt(D 2^-60), 4 <= D < 2^60, as y 2^(sh - 62) with y = (yh, yl) in [2^62,
+// 2^63): a single-precision estimate refined once in 64-bit fixed point.  With
+// D 2^-60 = m 4^k, 1 <= m < 4 (k < 0, sh = -k - 1), and y0 ~ m^-1/2 (23 bits):
 // e = 1 - m y0^2 is formed to 2^-61 (|e| < 2^-20) and m^-1/2 =
 // y0 (1 - e)^-1/2 = y0 (1 + e/2 + 3 e^2 / 8 + O(2^-61)).  Relative error below
-// 2^-58.  About 130 cycles of integer latency; the library's FP64 rsqrt
-// takes ~380, and 128 of them follow one another in a panel.
-__device__ __forceinline__ void rsqrt_fixed(long long D, unsigned long long& y, int& sh) {
-  const int lz = __clzll(D);
+// 2^-58.  ~50 integer instructions (2 to 3 cycles
+// of issue each on this GPU, ~220 of latency together); the library's FP64
+// rsqrt takes ~380 cycles, and 128 of them follow one another in a panel.
+__device__ __forceinline__ void rsqrt_fixed(long long D, unsigned& yh, unsigned& yl, int& sh) {
+  const unsigned hi = (unsigned)((unsigned long long)D >> 32), lo = (unsigned)D;
+  const int lz = hi ? __clz(hi) : 32 + __clz(lo);
   const unsigned long long A = (unsigned long long)D << (lz & 63);  // leading one at bit 63
-  const int E = 1 - lz, r = E & 1;                                  // D 2^-62 = 1.f 2^E
+  const int E = 3 - lz, r = E & 1;                                  // D 2^-60 = 1.f 2^E
   sh = -(E >> 1) - 1;
-  const unsigned long long M = A >> (1 - r);  // m 2^62
   const float mf = __uint_as_float(((unsigned)(127 + r) << 23) | ((unsigned)(A >> 40) & 0x7FFFFFu));
   float y0;
   asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(y0) : "f"(mf));
-  const unsigned yb = __float_as_uint(fminf(fmaxf(y0, 0.5f), 1.0f));
-  const unsigned Y = ((yb & 0x7FFFFFu) | 0x800000u) << ((yb >> 23) - 126u);  // y0 2^24
+  const unsigned Y = __float_as_uint(y0 + 1.0f) - 0x3F800000u;  // y0 2^23, y0 in [0.5, 1]
   const unsigned long long YY = (unsigned long long)Y * Y;
-  const long long e = (long long)((1ULL << 61) - __umul64hi(M, YY << 15));   // e 2^61
+  const long long e = (long long)((1ULL << 61) - __umul64hi(A, YY << (16 + r)));  // e 2^61
   const int eh = (int)(e >> 10);
-  const unsigned long long e2 = (unsigned long long)((long long)eh * eh);    // e^2 2^102
-  const long long c = (e >> 1) + (long long)((3ULL * e2) >> 44);             // (e/2 + 3 e^2/8) 2^61
-  const unsigned long long v = ((unsigned long long)Y << 39) + (unsigned long long)(((long long)Y * (c >> 2)) >> 20);
-  y = v < 0x7FFFFFFFFFFFFFFFULL ? v : 0x7FFFFFFFFFFFFFFFULL;
+  const unsigned e2 = (unsigned)((unsigned long long)((long long)eh * eh) >> 32);  // e^2 2^70
+  const long long c = (e >> 1) + (long long)((e2 * 3u) >> 12);                    // (e/2 + 3 e^2/8) 2^61
+  // y0 (1 + c) 2^63, less one unit: never 2^63
+  const unsigned long long v =
+      (((unsigned long long)(Y * 256u - 1u) << 32) | 0xFFFFFFFFu) + (unsigned long long)(((long long)Y * (c >> 2)) >> 19);
+  yh = (unsigned)(v >> 32);
+  yl = (unsigned)v;
 }
 
-// X = x 2^60 of x = T 2^-62 / L'_jj, split in Xh 2^30 + Xl.  |x| <= 1 while
-// the matrix is positive semidefinite, i.e. |T| < 2^(62 - sh); a larger |T|
-// clamps to +-1 (which fails the row's pivot).
-__device__ __forceinline__ void scale_entry(long long T, unsigned long long y, int sh, int& Xh, int& Xl) {
-  const int lim = 1 << (30 - sh);
-  const int th = (int)(T >> 32);
-  long long X = __mul64hi(T << sh, (long long)y);
-  if ((unsigned)(th + lim) >= 2u * (unsigned)lim) X = T < 0 ? -(1LL << 60) : 1LL << 60;
-  Xh = min(max((int)((X + (1LL << 29)) >> 30), -(1 << 30)), 1 << 30);
+// X = x 2^60 of x = T 2^-60 / L'_jj, split in Xh 2^30 + Xl.  |x| <= 1 while
+// the matrix is positive semidefinite, i.e. |T| < 2^(60 - sh); a larger |T|
+// clamps, to |x| = 1 up to 2^-28, which fails the row's pivot.
+__device__ __forceinline__ void scale_entry(long long T, unsigned yh, unsigned yl, int sh, int& Xh, int& Xl) {
+  const int lim = 1 << (29 - sh);  // |T| up to twice its bound
+  const unsigned tl = (unsigned)T;
+  const int th = min(max((int)(T >> 32), -lim), lim - 1);
+  // T 2^(sh + 2) y 2^-64: high product, and the two cross products' high parts
+  const int uh = (int)__funnelshift_l(tl, (unsigned)th, sh + 2);
+  const unsigned ul = tl << (sh + 2);
+  const long long X = (long long)uh * (int)yh + (long long)(((unsigned long long)ul * yh) >> 32) +
+                      (((long long)uh * (int)(yl >> 1)) >> 31);
+  const long long Xr = X + (1LL << 29);
+  const int hi = min(max((int)(Xr >> 32), -(1 << 28)), (1 << 28) - 1);
+  Xh = (int)__funnelshift_l((unsigned)Xr, (unsigned)hi, 2);
   Xl = (int)((unsigned)X - ((unsigned)Xh << 30));
+}
+
+// a Schur complement entry from units of 2^-62 to 2^-60, rounded
+__device__ __forceinline__ long long to_unit60(unsigned long long w) { return ((long long)w + 2) >> 2; }
+
+// S + M 2^-30 += x l in units of 2^-60
+__device__ __forceinline__ void mac_entry(long long& S, long long& M, int xh, int xl, int lh, int ll) {
+  S += (long long)xh * lh;
+  M += (long long)xh * ll;
+  M += (long long)xl * lh;
+}
+// B = S - M 2^-30 -= x l, in units of 2^-60
+__device__ __forceinline__ void take_entry(long long& S, long long& M, int xh, int xl, int lh, int ll) {
+  S -= (long long)xh * lh;
+  M += (long long)xh * ll;
+  M += (long long)xl * lh;
+}
+
+// shift a register array down by n: a[i] = a[i + n]
+template <int n, typename T, int N>
+__device__ __forceinline__ void shift_down(T (&a)[N]) {
+#pragma unroll
+  for (int i = 0; i + n < N; ++i) a[i] = a[i + n];
+}
+
+// B = T - M 2^-30 of a row's column k -= sum over c0 <= c < n of x_c l_kc, two
+// block entries a load
+template <int c0>
+__device__ __forceinline__ void take_row(long long& T, long long& M, const int (&Xh)[PW], const int (&Xl)[PW],
+                                         const PanelBlock& Lt, int k, int n) {
+  const int4* l = reinterpret_cast<const int4*>(&Lt.x[k][0]);
+#pragma unroll
+  for (int c = c0; c < PW; c += 2) {
+    if (c < n) {
+      const int4 v = l[c / 2];
+      take_entry(T, M, Xh[c], Xl[c], v.x, v.y);
+      if (c + 1 < n) take_entry(T, M, Xh[c + 1], Xl[c + 1], v.z, v.w);
+    }
+  }
 }
 
 // the digit planes of 8 entries X = x 2^60 of a row
@@ -185,11 +233,12 @@ __global__ void __launch_bounds__(PN_THREADS, 1)
   uint64_t* b_z = b_mma + 2;                                        // its z is in Zs
   uint64_t* b_drained = b_mma + 3;                                  // the row warps hold its couplings in registers
   uint64_t* b_digits = b_mma + 4;                                   // the row warps' digits are in As (and in HBM)
-  uint64_t* b_pub = b_mma + 5;                                      // diagonal tile: the digits are in HBM
-  uint64_t* b_quiet = b_mma + 6;                                    // quiescing before an early exit
+  uint64_t* b_half = b_mma + 5;                                     // the first half of its block's columns is in Ls
+  uint64_t* b_rhs = b_mma + 6;                                      // diagonal tile: the piece's right-hand-side entries are in Rs
+  uint64_t* b_quiet = b_mma + 7;                                    // quiescing before an early exit
   __shared__ int s_tile, s_sub, s_skip, s_stop, s_abort;
   __shared__ uint32_t s_tmem;
-  __shared__ long long s_D[2][PW];  // the pieces' pivots, in the matrix's unit
+  __shared__ long long s_D[2][PW];  // the pieces' pivots, in units of 2^-60
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   if (tid == 0) {
     const int u = atomicAdd(counter, 1);
@@ -212,13 +261,15 @@ __global__ void __launch_bounds__(PN_THREADS, 1)
   const int c0 = s * NB;
   int* fl = flags + PANEL_FLAGS * p;
   const int fbase = s * NPIECE;  // the counters grow through the whole sweep
+  const int np = min(NPIECE, (P.N - c0 + PW - 1) / PW);  // pieces that hold more than identity padding
   if (tid == 0) {
     mbar_init(b_mma, 1);
     mbar_init(b_blk, 1);
     mbar_init(b_z, 1);
     mbar_init(b_drained, nrw);
     mbar_init(b_digits, nrw);
-    mbar_init(b_pub, nrw);
+    mbar_init(b_half, 1);
+    mbar_init(b_rhs, 1);
     mbar_init(b_quiet, 1);
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
@@ -262,22 +313,31 @@ __global__ void __launch_bounds__(PN_THREADS, 1)
       live = r == 0;
       return live;
     };
+    int Xh[PW], Xl[PW];  // this row's entries of the current piece
+    int Ph[PW], Pl[PW];  // and of the previous one
+    // the row's own pivot, once its block is factored (kept here: the shared copies are overwritten two pieces on)
+    long long D_own = 0;
+    unsigned yh_own = 0, yl_own = 0;
+    int sh_own = 0;
 #pragma unroll 1
-    for (int t = 0; t < NPIECE; ++t) {
+    for (int t = 0;; ++t) {
+      const bool tail = t == np;  // only the last piece's leftovers
       const bool done = diag && warp < (t >> 1);  // the diagonal tile: every row of this warp is factored
-      long long T[PW];
-      if (t > 0) {
+      const bool was_done = diag && warp < ((t - 1) >> 1);
+      const bool pivot = diag && warp == (t >> 1);
+      long long T[PW];  // the row's right-hand sides B, in units of 2^-60
+      if (t > 0 && !tail) {
         if (!wait(b_mma, (t - 1) & 1)) break;
         asm volatile("tcgen05.fence::after_thread_sync;");
       }
-      if (!done) {
+      if (tail) {
+      } else if (!done) {
         if (t > 0) {
           // the couplings' 7 level sums: by the magic add where they lie in
           // (-2^22, 2^22) (the sum's exponent bits tell), else by F2I
-          uint32_t off = 0;
 #pragma unroll
           for (int g = 0; g < 2; ++g) {
-            uint32_t v[NSLICE][8];
+            uint32_t v[NSLICE][8], off = 0;
 #pragma unroll
             for (int l = 0; l < NSLICE; ++l) tmem_ld8(v[l], trow + (uint32_t)(l * PW + g * 8));
             asm volatile("tcgen05.wait::ld.sync.aligned;");
@@ -290,22 +350,22 @@ __global__ void __launch_bounds__(PN_THREADS, 1)
               }
 #pragma unroll
             for (int jj = 0; jj < 8; ++jj)
-              T[g * 8 + jj] = (long long)((unsigned long long)wv[g * 8 + jj] - (unsigned long long)level_bits_to_w64(v, jj));
-          }
-          if (__any_sync(0xffffffffu, off >> 23)) {
+              T[g * 8 + jj] = to_unit60((unsigned long long)wv[g * 8 + jj] - (unsigned long long)level_bits_to_w64(v, jj));
+            if (__any_sync(0xffffffffu, off >> 23)) {
 #pragma unroll 1
-            for (int c = 0; c < PW; ++c) {
-              uint32_t v[NSLICE];
+              for (int c = 0; c < 8; ++c) {
+                uint32_t u[NSLICE];
 #pragma unroll
-              for (int l = 0; l < NSLICE; ++l) v[l] = tmem_ld1(trow + (uint32_t)(l * PW + c));
-              asm volatile("tcgen05.wait::ld.sync.aligned;");
-              int S[NSLICE];
+                for (int l = 0; l < NSLICE; ++l) u[l] = tmem_ld1(trow + (uint32_t)(l * PW + g * 8 + c));
+                asm volatile("tcgen05.wait::ld.sync.aligned;");
+                int I[NSLICE];
 #pragma unroll
-              for (int l = 0; l < NSLICE; ++l) S[l] = __float2int_rn(__uint_as_float(v[l]));
-              const unsigned long long W = (unsigned long long)levels_to_w64(S);
+                for (int l = 0; l < NSLICE; ++l) I[l] = __float2int_rn(__uint_as_float(u[l]));
+                const unsigned long long W = (unsigned long long)levels_to_w64(I);
 #pragma unroll
-              for (int k = 0; k < PW; ++k)
-                if (k == c) T[k] = (long long)((unsigned long long)wv[k] - W);
+                for (int k = 0; k < 8; ++k)
+                  if (k == c) T[g * 8 + k] = to_unit60((unsigned long long)wv[g * 8 + k] - W);
+              }
             }
           }
           asm volatile("tcgen05.fence::before_thread_sync;");
@@ -313,51 +373,90 @@ __global__ void __launch_bounds__(PN_THREADS, 1)
           if (lane == 0) mbar_arrive(b_drained);
         } else {
 #pragma unroll
-          for (int c = 0; c < PW; ++c) T[c] = wv[c];
+          for (int c = 0; c < PW; ++c) T[c] = to_unit60((unsigned long long)wv[c]);
         }
-        if (t + 1 < NPIECE) load_piece(t + 1);
-      } else if (t > 0 && lane == 0) {
+        if (t + 1 < np) load_piece(t + 1);
+      } else if (lane == 0) {
         mbar_arrive(b_drained);
       }
       PanelBlock& Lt = Ls[t & 1];
-      long long* Dj = s_D[t & 1];
-      int Xh[PW], Xl[PW];  // this row's solved entries
-      const int c_own = diag ? rl - t * PW : PW;  // this row's index in the piece's block; < 0: above it
-      if (diag && warp == (t >> 1)) {
-        // the 16 x 16 diagonal block, column by column on the whole warp
-        // (rows below the block in the same warp are solved on the way)
+      if (pivot && !tail) {
+        // The 16 x 16 diagonal block on the whole warp (rows below the block in
+        // the same warp are solved on the way), four columns a round: within
+        // the four each entry is taken off the next columns at once (the
+        // pivot rows' entries by shuffles), then the four together off the
+        // columns beyond (from shared memory), which move down by four.  A
+        // rolled loop: unrolled whole, it is 50 KB of code that the
+        // instruction fetch shares with the other warps' (14k cycles a piece
+        // against 9k alone).  A non-positive pivot is remembered and what
+        // follows it is discarded.
         const int base = (t & 1) * PW;
-        if (c_own >= 0 && c_own < PW) {
-          Rs[c_own] = rhs0 - r0;
-          Rs[PW + c_own] = rhs1 - r1;
-        }
-        // no branch per column: a non-positive pivot is remembered and what
-        // follows it is discarded
+        const int c_own = lane - base;  // this row's index in the block; < 0: above, >= 16: below
+        long long M[PW];                // with T: B = T - M 2^-30
+#pragma unroll
+        for (int k = 0; k < PW; ++k) M[k] = 0;
         int fail = PW;
+#pragma unroll 1
+        for (int b = 0; b < 4; ++b) {
+          int xh[4], xl[4];
 #pragma unroll
-        for (int j = 0; j < PW; ++j) {
-          long long S = 0, M = 0;
+          for (int q = 0; q < 4; ++q) {
+            const int j = 4 * b + q;
+            const long long Tj = T[q] - (M[q] >> 30);
+            const long long D = __shfl_sync(0xffffffffu, Tj, base + j);
+            if (D < 4 && fail == PW) fail = j;  // 2^-58 of 2^2e: far below what K's own rounding leaves of a pivot
+            unsigned yh, yl;
+            int sh;
+            rsqrt_fixed(D, yh, yl, sh);
+            sh = min(max(sh, 0), 28);  // discarded columns only
+            scale_entry(Tj, yh, yl, sh, xh[q], xl[q]);
+            if (c_own < j) xh[q] = xl[q] = 0;  // above the diagonal
+            if (c_own == j) {
+              yh_own = yh;
+              yl_own = yl;
+              sh_own = sh;
+              D_own = D;
+              Lt.y[j] = make_uint2(yh, yl);
+              Lt.sh[j] = sh;
+              s_D[t & 1][j] = D;
+            }
 #pragma unroll
-          for (int c = 0; c < j; ++c) {
-            const int lh = __shfl_sync(0xffffffffu, Xh[c], base + j), ll = __shfl_sync(0xffffffffu, Xl[c], base + j);
-            S += (long long)Xh[c] * lh;
-            M += (long long)Xh[c] * ll;
-            M += (long long)Xl[c] * lh;
+            for (int k = q + 1; k < 4; ++k) {
+              const int lh = __shfl_sync(0xffffffffu, xh[q], base + 4 * b + k);
+              const int ll = __shfl_sync(0xffffffffu, xl[q], base + 4 * b + k);
+              take_entry(T[k], M[k], xh[q], xl[q], lh, ll);
+            }
           }
-          const long long Tj = T[j] - (S << 2) - (M >> 28);
-          const long long D = __shfl_sync(0xffffffffu, Tj, base + j);
-          if (D <= 0 && fail == PW) fail = j;
-          unsigned long long y;
-          int sh;
-          rsqrt_fixed(D, y, sh);
-          sh = min(max(sh, 0), 30);  // discarded columns only
-          scale_entry(Tj, y, sh, Xh[j], Xl[j]);
-          if (lane == 0) {
-            Lt.y[j] = y;
-            Lt.sh[j] = sh;
-            Dj[j] = D;
+          if (c_own >= 0 && c_own < PW) {
+            int4* lx = reinterpret_cast<int4*>(&Lt.x[c_own][4 * b]);
+            lx[0] = make_int4(xh[0], xl[0], xh[1], xl[1]);
+            lx[1] = make_int4(xh[2], xl[2], xh[3], xl[3]);
           }
-          if (c_own < j) Xh[j] = Xl[j] = 0;  // above the diagonal
+          shift_down<4>(Xh);
+          shift_down<4>(Xl);
+#pragma unroll
+          for (int q = 0; q < 4; ++q) {
+            Xh[PW - 4 + q] = xh[q];
+            Xl[PW - 4 + q] = xl[q];
+          }
+          __syncwarp();
+          if (b == 1 && lane == 0) mbar_arrive(b_half);
+          const int4* lb = reinterpret_cast<const int4*>(&Lt.x[4 * b + 4][4 * b]);
+#pragma unroll
+          for (int g = 0; g < 3; ++g) {
+            if (b < 3 - g) {  // the columns left: uniform
+#pragma unroll
+              for (int i = 4 * g; i < 4 * g + 4; ++i) {
+                const int4 l0 = lb[i * (PW / 2)], l1 = lb[i * (PW / 2) + 1];
+                T[i] = T[i + 4];
+                M[i] = M[i + 4];
+                take_entry(T[i], M[i], xh[0], xl[0], l0.x, l0.y);
+                take_entry(T[i], M[i], xh[1], xl[1], l0.z, l0.w);
+                take_entry(T[i], M[i], xh[2], xl[2], l1.x, l1.y);
+                take_entry(T[i], M[i], xh[3], xl[3], l1.z, l1.w);
+              }
+            }
+          }
         }
         if (fail < PW) {
           if (lane == 0) {
@@ -370,97 +469,126 @@ __global__ void __launch_bounds__(PN_THREADS, 1)
           live = false;
           break;
         }
-        if (c_own >= 0 && c_own < PW) {
-#pragma unroll
-          for (int c = 0; c < PW; c += 2)
-            *reinterpret_cast<int4*>(&Lt.x[c_own][c]) = make_int4(Xh[c], Xl[c], Xh[c + 1], Xl[c + 1]);
-        }
+        // the right-hand-side warp has taken the previous block: no barrier's
+        // phase can pass a warp that still waits for the one before
+        if (t > 0 && !wait(b_z, (t - 1) & 1)) break;
         __syncwarp();
         if (lane == 0) mbar_arrive(b_blk);
-        {
-          const uint4* src = reinterpret_cast<const uint4*>(&Lt);
-          uint4* dst = reinterpret_cast<uint4*>(P.lpub + t);
-          for (int q = lane; q < (int)PN_LBYTES / 16; q += 32) dst[q] = src[q];
-        }
-        __threadfence();
-        __syncwarp();
-        if (lane == 0) st_release(&fl[FLAG_L], fbase + t + 1);
       }
-      if (!wait(b_blk, t & 1)) break;
-      if (!done && !(diag && warp == (t >> 1))) {
-        // x L'_tt^T = B
+      // Two rounds around one copy of the leftovers' code: the pivot warp writes
+      // its digits first, the others do the leftovers while they wait for the
+      // pivots.
+      bool out = false;
+#pragma unroll 1
+      for (int round = 0; round < 2; ++round) {
+        if ((round == 1) == (pivot && !tail) && t > 0 && !was_done) {
+          // the previous piece's leftovers, which nothing on the pivots' chain
+          // waits for: the factor's entries for alpha and the adjoint, and the
+          // right-hand sides' sum_k L'_ik z_k, z in 60-bit fixed point of the
+          // piece's own scale
+          const int tp = t - 1;
+          if (P.keep_l) {
+            // as they are, X = x 2^60: k_factor_doubles converts them where they are wanted
+            const int c_own = diag ? rl - tp * PW : PW;
+            if (c_own >= 0 && c_own < PW)  // the row's own L_jj = d d^-1/2
+              P.ldiag[i] = fixed62_to_double(D_own, 2) * fixed62_to_double((long long)yh_own << 32 | yl_own, sh_own + kexp);
+            long long* kp = reinterpret_cast<long long*>(krow) + (size_t)(tp * PW) * ld;
 #pragma unroll
-        for (int k = 0; k < PW; ++k) {
-          long long S = 0, M = 0;
-#pragma unroll
-          for (int c = 0; c < k; ++c) {
-            const int2 l = Lt.x[k][c];
-            S += (long long)Xh[c] * l.x;
-            M += (long long)Xh[c] * l.y;
-            M += (long long)Xl[c] * l.x;
+            for (int c = 0; c < PW; ++c) kp[(size_t)c * ld] = (long long)Ph[c] * (1LL << 30) + Pl[c];
           }
-          scale_entry(T[k] - (S << 2) - (M >> 28), Lt.y[k], Lt.sh[k], Xh[k], Xl[k]);
-        }
-      }
-      if (!done) {
-#pragma unroll
-        for (int g = 0; g < 2; ++g) {
-          uint4 d[NSLICE];
-          digits8_packed(&Xh[g * 8], &Xl[g * 8], d);
-#pragma unroll
-          for (int q = 0; q < NSLICE; ++q) {
-            if (t + 1 < NPIECE) *reinterpret_cast<uint4*>(As + t * PN_ACHUNK + q * 4096 + g * 2048 + tid * 16) = d[q];
-            *reinterpret_cast<uint4*>(gdig + (size_t)q * SLICE_BYTES + (size_t)(2 * t + g) * 2048) = d[q];
-            // the diagonal tile's own B operand of the next piece
-            if (diag && (rl >> 4) == t + 1)
-              *reinterpret_cast<uint4*>(Bs + t * PN_BCHUNK + g * (NSLICE * PW * 16) + q * (PW * 16) + (rl & 15) * 16) = d[q];
+          if (!wait(b_z, tp & 1)) {
+            out = true;
+            break;
           }
-        }
-        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");  // digits visible to the tensor cores
-      }
-      __syncwarp();
-      if (lane == 0) mbar_arrive(b_digits);
-      if (diag) {
-        __threadfence();  // digits visible to the device before they are published
-        __syncwarp();
-        if (lane == 0) mbar_arrive(b_pub);
-      }
-      if (!done && P.keep_l) {
-        double ljj = 0.0;  // the row's own L_jj = d d^-1/2
-        if (c_own >= 0 && c_own < PW)
-          ljj = fixed62_to_double(Dj[c_own]) * fixed62_to_double((long long)Lt.y[c_own], Lt.sh[c_own] + kexp);
-#pragma unroll
-        for (int c = 0; c < PW; ++c) {
-          const double x = fixed62_to_double(((long long)Xh[c] * (1LL << 30) + Xl[c]) * 4, kexp);
-          krow[(size_t)(t * PW + c) * ld] = c == c_own ? ljj : x;
-        }
-      }
-      // the right-hand sides: sum_k L'_ik z_k of this piece, z in 60-bit fixed
-      // point of the piece's own scale
-      if (!wait(b_z, t & 1)) break;
-      if (!done) {
-        const PanelZ& Z = Zs[t & 1];
-        long long S = 0, M = 0;
-#pragma unroll
-        for (int c = 0; c < PW; ++c) {
-          const int2 z = Z.x[0][c];
-          S += (long long)Xh[c] * z.x;
-          M += (long long)Xh[c] * z.y;
-          M += (long long)Xl[c] * z.x;
-        }
-        r0 = fma(Z.scale[0], fixed62_to_double((S << 2) + (M >> 28)), r0);
-        if (two) {
-          S = M = 0;
+          const PanelZ& Z = Zs[tp & 1];
+          long long s = 0, m = 0;
 #pragma unroll
           for (int c = 0; c < PW; ++c) {
-            const int2 z = Z.x[1][c];
-            S += (long long)Xh[c] * z.x;
-            M += (long long)Xh[c] * z.y;
-            M += (long long)Xl[c] * z.x;
+            mac_entry(s, m, Ph[c], Pl[c], Z.x[0][c].x, Z.x[0][c].y);
           }
-          r1 = fma(Z.scale[1], fixed62_to_double((S << 2) + (M >> 28)), r1);
+          r0 = fma(Z.scale[0], fixed62_to_double((s << 2) + (m >> 28)), r0);
+          if (two) {
+            s = m = 0;
+#pragma unroll
+            for (int c = 0; c < PW; ++c) {
+              mac_entry(s, m, Ph[c], Pl[c], Z.x[1][c].x, Z.x[1][c].y);
+            }
+            r1 = fma(Z.scale[1], fixed62_to_double((s << 2) + (m >> 28)), r1);
+          }
+        }
+        if (tail) break;
+        if (round == 0) {
+          if (!done && !pivot) {
+            // x L'_tt^T = B: the first 8 columns, their part of the last 8, the last 8
+            if (!wait(b_half, t & 1)) {
+              out = true;
+              break;
+            }
+            constexpr int HW = PW / 2;
+#pragma unroll
+            for (int k = 0; k < HW; ++k) {
+              long long M = 0;
+              take_row<0>(T[k], M, Xh, Xl, Lt, k, k);
+              scale_entry(T[k] - (M >> 30), Lt.y[k].x, Lt.y[k].y, Lt.sh[k], Xh[k], Xl[k]);
+            }
+            long long M2[HW];
+#pragma unroll
+            for (int q = 0; q < HW; ++q) {
+              M2[q] = 0;
+              take_row<0>(T[HW + q], M2[q], Xh, Xl, Lt, HW + q, HW);
+            }
+            if (!wait(b_blk, t & 1)) {
+              out = true;
+              break;
+            }
+#pragma unroll
+            for (int k = HW; k < PW; ++k) {
+              take_row<HW>(T[k], M2[k - HW], Xh, Xl, Lt, k, k);
+              scale_entry(T[k] - (M2[k - HW] >> 30), Lt.y[k].x, Lt.y[k].y, Lt.sh[k], Xh[k], Xl[k]);
+            }
+          }
+          if (!done) {
+            unsigned char* ad = As + t * PN_ACHUNK + tid * 16;
+            unsigned char* gd = gdig + (size_t)(2 * t) * 2048;
+            unsigned char* bd = Bs + t * PN_BCHUNK + (rl & 15) * 16;
+            const bool own_b = diag && (rl >> 4) == t + 1;  // the diagonal tile's own B operand of the next piece
+#pragma unroll
+            for (int g = 0; g < 2; ++g) {
+              uint4 d[NSLICE];
+              digits8_packed(&Xh[g * 8], &Xl[g * 8], d);
+#pragma unroll
+              for (int q = 0; q < NSLICE; ++q) {
+                if (t + 1 < NPIECE) *reinterpret_cast<uint4*>(ad + g * 2048 + q * 4096) = d[q];
+                *reinterpret_cast<uint4*>(gd + (size_t)q * SLICE_BYTES + g * 2048) = d[q];
+                if (own_b) *reinterpret_cast<uint4*>(bd + g * (NSLICE * PW * 16) + q * (PW * 16)) = d[q];
+              }
+            }
+            asm volatile("fence.proxy.async.shared::cta;" ::: "memory");  // digits visible to the tensor cores
+          }
+          __syncwarp();
+          if (lane == 0) mbar_arrive(b_digits);
         }
       }
+      if (out || tail) break;
+      if (pivot) {
+        const int c_own = lane - (t & 1) * PW;
+        if (c_own >= 0 && c_own < PW) {
+          Rs[c_own] = rhs0 - r0;
+          Rs[PW + c_own] = rhs1 - r1;
+        }
+        __syncwarp();
+        if (lane == 0) mbar_arrive(b_rhs);
+      }
+#pragma unroll
+      for (int c = 0; c < PW; ++c) {
+        Ph[c] = Xh[c];
+        Pl[c] = Xl[c];
+      }
+    }
+    if (diag && live && P.keep_l) {
+      // columns of the identity padding, which the pieces leave out
+      for (int c = np * PW; c < NB; ++c) krow[(size_t)c * ld] = 0.0;
+      if (rl >= np * PW) P.ldiag[i] = ldexp(0.5, kexp);
     }
     if (!diag && live) {
       P.rhs[i] = rhs0 - r0;
@@ -499,7 +627,7 @@ __global__ void __launch_bounds__(PN_THREADS, 1)
     };
     int st = 0;  // 1: the problem failed, 2: a wait gave up
 #pragma unroll 1
-    for (int t = 0; t < NPIECE && !st; ++t) {
+    for (int t = 0; t < np && !st; ++t) {
       if (!diag) {
         if ((st = wait_flag(FLAG_L, t))) break;
         const unsigned char* pub = reinterpret_cast<const unsigned char*>(P.lpub + t);
@@ -507,9 +635,12 @@ __global__ void __launch_bounds__(PN_THREADS, 1)
         for (int q = lane; q < (int)PN_LBYTES / 16; q += 32) cp_async16(dst + q * 16, pub + q * 16);
         cp_async_wait();
         __syncwarp();
-        if (lane == 0) mbar_arrive(b_blk);
+        if (lane == 0) {
+          mbar_arrive(b_half);
+          mbar_arrive(b_blk);
+        }
       }
-      if (t + 1 < NPIECE) {
+      if (t + 1 < np) {
         if (t > 0) {
           // earlier chunks against the next piece, while the rows are solved
           if ((st = wait_or_stop(b_mma, (t - 1) & 1, &s_stop))) break;  // the couplings of piece t have read Bs
@@ -535,8 +666,13 @@ __global__ void __launch_bounds__(PN_THREADS, 1)
         if (lane == 0) {
           issue_chunk(t);
           mma_commit(b_mma);
+          // the row warps' digits, written to HBM before they arrived (release:
+          // cumulative over what this warp has observed)
+          if (diag) st_release(&fl[FLAG_D], fbase + t + 1);
         }
         __syncwarp();
+      } else if (!diag) {
+        if ((st = wait_or_stop(b_digits, t & 1, &s_stop))) break;  // the rows have taken the previous z
       }
       if (!diag) {
         if ((st = wait_flag(FLAG_Z, t))) break;
@@ -567,13 +703,22 @@ __global__ void __launch_bounds__(PN_THREADS, 1)
     const int ke = *P.kscale;
     bool ok = true;
 #pragma unroll 1
-    for (int t = 0; t < NPIECE; ++t) {
-      const int w = wait_or_stop(b_blk, t & 1, &s_stop);
+    for (int t = 0; t < np; ++t) {
+      int w = wait_or_stop(b_blk, t & 1, &s_stop);
       if (w == 2) s_abort = s_stop = 1;
       ok = w == 0;
       if (!ok) break;
       const PanelBlock& Lt = Ls[t & 1];
-      double r = have ? Rs[lane] : 0.0, z = 0.0;
+      const long long lb = __double_as_longlong(fixed62_to_double(s_D[t & 1][j], 2));
+      {
+        // publish the block (release: cumulative over what this warp has
+        // observed, the pivot warp's stores before b_blk included)
+        const uint4* src = reinterpret_cast<const uint4*>(&Lt);
+        uint4* dst = reinterpret_cast<uint4*>(P.lpub + t);
+        for (int q = lane; q < (int)PN_LBYTES / 16; q += 32) dst[q] = src[q];
+        __syncwarp();
+        if (lane == 0) st_release(&fl[FLAG_L], fbase + t + 1);
+      }
       // row j of the block, and 1 / L'_jj = y 2^(sh - 62), as doubles
       double lrow[PW];
 #pragma unroll
@@ -581,7 +726,12 @@ __global__ void __launch_bounds__(PN_THREADS, 1)
         const int2 l = Lt.x[j][c];
         lrow[c] = fixed62_to_double(((long long)l.x * (1LL << 30) + l.y) * 4);
       }
-      const double rdj = fixed62_to_double((long long)Lt.y[j], Lt.sh[j]);
+      const double rdj = fixed62_to_double((long long)Lt.y[j].x << 32 | Lt.y[j].y, Lt.sh[j]);
+      w = wait_or_stop(b_rhs, t & 1, &s_stop);
+      if (w == 2) s_abort = s_stop = 1;
+      ok = w == 0;
+      if (!ok) break;
+      double r = have ? Rs[lane] : 0.0, z = 0.0;
 #pragma unroll
       for (int c = 0; c < PW; ++c) {
         const double b = __shfl_sync(0xffffffffu, r * rdj, (lane & 16) + c);
@@ -608,18 +758,16 @@ __global__ void __launch_bounds__(PN_THREADS, 1)
         }
       }
       if (have) P.rhs[(size_t)(lane >> 4) * P.Nc + c0 + t * PW + j] = z;
-      __threadfence();
+      // every row warp has taken the previous z before this one is signalled
+      w = wait_or_stop(b_digits, t & 1, &s_stop);
+      if (w == 2) s_abort = s_stop = 1;
+      ok = w == 0;
+      if (!ok) break;
       __syncwarp();
       if (lane == 0) {
         mbar_arrive(b_z);
         st_release(&fl[FLAG_Z], fbase + t + 1);
       }
-      const int wp = wait_or_stop(b_pub, t & 1, &s_stop);
-      if (wp == 2) s_abort = s_stop = 1;
-      ok = wp == 0;
-      if (!ok) break;
-      if (lane == 0) st_release(&fl[FLAG_D], fbase + t + 1);
-      const long long lb = __double_as_longlong(fixed62_to_double(s_D[t & 1][j]));
       if (c0 + t * PW + j < P.N) {  // not the identity padding
         esum += (int)(lb >> 52) - 1023 + 2 * ke;
         prod *= __longlong_as_double((lb & 0xFFFFFFFFFFFFFLL) | 0x3FF0000000000000LL);
@@ -645,6 +793,32 @@ __global__ void __launch_bounds__(PN_THREADS, 1)
   if (warp == PN_MMA_WARP) __syncwarp();
   if (warp == PN_MMA_WARP)
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "n"(PN_TMEM_COLS));
+}
+
+// ---------------------------------------------------------------------------
+// the factor the panels left in K (lower triangle, X = L' 2^60, its diagonal in
+// ldiag) as doubles, in place: only alpha and the adjoint read it, and on the
+// panels' chain the conversions cost 1.2k cycles a piece.  One CTA per 128 x 128
+// tile
+// ---------------------------------------------------------------------------
+__global__ void __launch_bounds__(256) k_factor_doubles(const Prob* __restrict__ pp) {
+  const Prob& P = *pp;
+  const int ti = blockIdx.x, tj = blockIdx.y;
+  if (ti < tj || P.status[1]) return;
+  const size_t ld = (size_t)P.ld;
+  const int kexp = *P.kscale, i = ti * NB + (threadIdx.x & 127);
+#pragma unroll 8
+  for (int c = threadIdx.x >> 7; c < NB; c += 2) {
+    const int j = tj * NB + c;
+    double* k = P.K + (size_t)j * ld + i;
+    const double x = fixed62_to_double(__double_as_longlong(*k) * 4, kexp);
+    *k = i > j ? x : (i == j ? P.ldiag[i] : 0.0);
+  }
+}
+
+cudaError_t launch_factor_doubles(const Prob* prob, int nt128, cudaStream_t s) {
+  k_factor_doubles<<<dim3(nt128, nt128), 256, 0, s>>>(prob);
+  return cudaGetLastError();
 }
 
 // Rows per CTA: 128, or 64 or 32 while that still gives every tile an SM of

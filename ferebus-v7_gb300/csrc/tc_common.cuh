@@ -218,7 +218,8 @@ __device__ __forceinline__ uint32_t level_bits(uint32_t v) {
 // 2^32; the offsets leave as one constant.
 constexpr unsigned long long LEVEL_BITS_BIAS =
     (1ULL << 22) * 0x0001010101010101ULL + 0x4B000000ULL * ((1ULL << 40) + (1ULL << 24) + (1ULL << 8) + 1ULL);
-__device__ __forceinline__ long long level_bits_to_w64(const uint32_t (&b)[7][8], int jj) {
+template <int N>
+__device__ __forceinline__ long long level_bits_to_w64(const uint32_t (&b)[7][N], int jj) {
   const uint32_t p01 = b[0][jj] * 256u + b[1][jj];
   const uint32_t p23 = b[2][jj] * 256u + b[3][jj];
   const uint32_t p45 = b[4][jj] * 256u + b[5][jj];

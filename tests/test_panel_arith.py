@@ -28,45 +28,63 @@ def rsqrt_fixed(D, ulps):
     """The device function; ``ulps`` perturbs the single-precision estimate."""
     lz = 64 - D.bit_length()
     A = D << lz
-    E = 1 - lz
+    E = 3 - lz
     r = E & 1
     sh = -(E >> 1) - 1
-    M = A >> (1 - r)
     mf = np.uint32(((127 + r) << 23) | ((A >> 40) & 0x7FFFFF)).view(np.float32)
-    yb = int(np.float32(1.0 / math.sqrt(float(mf))).view(np.uint32)) + ulps
-    yb = max(min(yb, 127 << 23), 126 << 23)
-    Y = ((yb & 0x7FFFFF) | 0x800000) << ((yb >> 23) - 126)
-    assert 2 ** 23 <= Y <= 2 ** 24
-    YY = Y * Y
-    assert M < 2 ** 64 and (YY << 15) < 2 ** 64
-    e = (1 << 61) - ((M * (YY << 15)) >> 64)
+    y0 = np.uint32(int(np.float32(1.0 / math.sqrt(float(mf))).view(np.uint32)) + ulps).view(np.float32)
+    Y = int(np.float32(y0 + np.float32(1.0)).view(np.uint32)) - 0x3F800000
+    assert 2 ** 22 <= Y <= 2 ** 23
+    YY = (Y * Y) << (16 + r)
+    assert YY < 2 ** 64
+    e = (1 << 61) - ((A * YY) >> 64)
     assert abs(e) < 2 ** 41
     eh = e >> 10
-    e2 = eh * eh
-    assert 3 * e2 < 2 ** 64
-    c = (e >> 1) + ((3 * e2) >> 44)
+    assert abs(eh) < 2 ** 31
+    e2 = (eh * eh) >> 32
+    assert e2 * 3 < 2 ** 32
+    c = (e >> 1) + ((e2 * 3) >> 12)
     prod = Y * (c >> 2)
     assert abs(prod) < 2 ** 63
-    return min((Y << 39) + (prod >> 20), 2 ** 63 - 1), sh
+    y = (((Y * 256 - 1) << 32) | 0xFFFFFFFF) + (prod >> 19)
+    assert 0 <= y < 2 ** 63
+    return y, sh
 
 
 def test_rsqrt_fixed_within_its_bound():
     rng = random.Random(5)
-    cases = [1, 2, 3, 4, 2 ** 62 - 1, 2 ** 61, 2 ** 61 - 1, 2 ** 61 + 1, 2 ** 60, 2 ** 60 - 1]
-    cases += [rng.getrandbits(rng.randint(2, 62)) | 1 for _ in range(4000)]
+    cases = [4, 5, 7, 2 ** 60 - 1, 2 ** 59, 2 ** 59 - 1, 2 ** 59 + 1, 2 ** 58, 2 ** 58 - 1]
+    cases += [rng.getrandbits(rng.randint(3, 60)) | 4 for _ in range(4000)]
     for D in cases:
-        for ulps in (-2, 0, 2):  # the estimate is within 2 ulp
+        for ulps in (-1, 0, 1):  # the estimate is within 2^-22.9
             y, sh = rsqrt_fixed(D, ulps)
-            assert 0 <= sh <= 30 and 2 ** 62 <= y + 2 ** 4 and y < 2 ** 63
+            assert 0 <= sh <= 28 and 2 ** 62 <= y + 2 ** 5
             got = Fraction(y) * Fraction(2) ** (sh - 62)
             # relative error: got = (1 + t) / sqrt(d), t = (got^2 d - 1) / 2 to first order
-            t = abs(float((got ** 2 * Fraction(D, 2 ** 62) - 1) / 2))
+            t = abs(float((got ** 2 * Fraction(D, 2 ** 60) - 1) / 2))
             assert t <= 2.0 ** -58, (D, ulps, t)
 
 
+def wrap(v, bits=64):
+    assert -(1 << (bits - 1)) <= v < 1 << (bits - 1), v
+    return v
+
+
 def split30(X):
-    h = max(min((X + (1 << 29)) >> 30, 1 << 30), -(1 << 30))
-    return h, X - (h << 30)
+    r = X + (1 << 29)
+    hi = min(max(r >> 32, -(1 << 28)), (1 << 28) - 1)
+    h = (hi << 2) | ((r >> 30) & 3)
+    return h, wrap((X - (h << 30) + (1 << 31)) % (1 << 32) - (1 << 31), 32)
+
+
+def scale_entry(T, y, sh):
+    lim = 1 << (29 - sh)
+    yh, yl = y >> 32, y & 0xFFFFFFFF
+    th = min(max(T >> 32, -lim), lim - 1)
+    u = wrap(((th << 32) | (T & 0xFFFFFFFF)) << (sh + 2))
+    uh, ul = u >> 32, u & 0xFFFFFFFF
+    X = wrap(uh * yh + ((ul * yh) >> 32) + ((uh * (yl >> 1)) >> 31))
+    return split30(X)
 
 
 def substitute(T, L, ys, shs):
@@ -74,28 +92,39 @@ def substitute(T, L, ys, shs):
     the 64-bit range of every sum checked."""
     out = []
     for k in range(16):
-        S = M = 0
+        S, M = T[k], 0
         for c in range(k):
             lh, ll = split30(L[k][c])
             xh, xl = out[c]
-            S += xh * lh
-            M += xh * ll + xl * lh
-            assert abs(S) < 2 ** 61 and abs(M) < 2 ** 63
-        t = T[k] - (S << 2) - (M >> 28)
-        assert abs(t << shs[k]) < 2 ** 63
-        h, low = split30(((t << shs[k]) * ys[k]) >> 64)
+            S = wrap(S - xh * lh)
+            M = wrap(M + xh * ll + xl * lh)
+        h, low = scale_entry(wrap(S - (M >> 30)), ys[k], shs[k])
         assert abs(h) <= 2 ** 30 and -2 ** 29 <= low < 2 ** 29
         out.append((h, low))
     return [(h << 30) + low for h, low in out]
 
 
+def test_scale_entry_clamps_what_a_semidefinite_matrix_cannot_have():
+    """|x| < 1 is exact to a few units; beyond it the high half is that of +-1."""
+    rng = random.Random(4)
+    for _ in range(4000):
+        y, sh = rsqrt_fixed(rng.getrandbits(rng.randint(3, 60)) | 4, 0)
+        T = rng.choice([-1, 1]) * rng.randrange(1 << (60 - sh))
+        h, low = scale_entry(T, y, sh)
+        want = (T * y) >> (62 - sh)
+        if abs(want) < 2 ** 60 - 2 ** 30:
+            assert abs(want - ((h << 30) + low)) <= 3
+        big = rng.choice([-1, 1]) * rng.randrange(1 << (60 - sh), 1 << 62)
+        assert abs(scale_entry(big, y, sh)[0]) >= 2 ** 30 - 4
+
+
 def test_substitution_in_fixed_point():
     """Against exact rational substitution on the same block.  Bound: column
-    k's right-hand side is off by the dropped Xl Ll (at most 15 x 2^58 2^-120),
-    the shifts (2^-62) and the block's own rounding (15 x 2^-61 |x|); the
-    division by L_kk scales that by 1 / L_kk, plus y's 2^-58 relative and
-    2^-60: below 2^-57 (1 + 1 / min L_kk), amplified by the block's
-    conditioning, which max |inv(L)| bounds."""
+    k's right-hand side is off by its rounding (2^-61), the dropped Xl Ll (at
+    most 15 x 2^58 2^-120), the shift (2^-60) and the block's own rounding
+    (15 x 2^-61 |x|); the division by L_kk scales that by 1 / L_kk, plus y's
+    2^-58 relative and 3 x 2^-60: below 2^-56 (1 + 1 / min L_kk), amplified by
+    the block's conditioning, which max |inv(L)| bounds."""
     rng = np.random.default_rng(9)
     for cond in (0.0, 2.0, 6.0, 9.0):
         A = rng.normal(size=(40, 24)) * np.exp(-cond * np.linspace(0, 1, 24))
@@ -104,13 +133,13 @@ def test_substitution_in_fixed_point():
         Lf = np.linalg.cholesky(G)
         blk, row = Lf[:16, :16], Lf[20, :16]
         L = [[round(Fraction(float(v)) * 2 ** 60) for v in r] for r in blk]
-        D = [round(Fraction(float(blk[j, j])) ** 2 * 2 ** 62) for j in range(16)]
+        D = [round(Fraction(float(blk[j, j])) ** 2 * 2 ** 60) for j in range(16)]
         ys, shs = zip(*(rsqrt_fixed(d, 0) for d in D))
-        T = [round(sum(Fraction(float(row[c])) * Fraction(float(blk[k, c])) for c in range(k + 1)) * 2 ** 62)
+        T = [round(sum(Fraction(float(row[c])) * Fraction(float(blk[k, c])) for c in range(k + 1)) * 2 ** 60)
              for k in range(16)]
         got = substitute(T, L, ys, shs)
         inv = np.abs(np.linalg.inv(blk)).max()
-        tol = 2.0 ** -57 * (1 + inv) * (1 + 16 * inv * np.abs(blk).max())
+        tol = 2.0 ** -56 * (1 + inv) * (1 + 16 * inv * np.abs(blk).max())
         for k in range(16):
             assert abs(got[k] / 2.0 ** 60 - row[k]) <= tol, (cond, k, got[k] / 2.0 ** 60 - row[k], tol)
 
