@@ -195,6 +195,7 @@ struct Workspace {
   PanelZ* zpub = nullptr;          // and solved right-hand-side entries
   double* splanes = nullptr;       // theta-scaled planes (dot-product build)
   double* norms = nullptr;
+  DotConst* dotc = nullptr;        // dot-product build: per-evaluation constants
   long long* fnorm = nullptr;      // tensor-core build: W_ii of the distance leaves
   double* fcoef = nullptr;         // tensor-core build: expression coefficients
   int* fscale = nullptr;           // tensor-core build: leaf scales
@@ -363,6 +364,7 @@ void fill_prob(Prob& p, const fgpu_ctx* c, const double* theta_d, const Workspac
   p.zpub = ws.zpub;
   p.splanes = ws.splanes;
   p.norms = ws.norms;
+  p.dotc = ws.dotc;
   p.plane_max = c->plane_max_d;
   p.fnorm = ws.fnorm;
   p.fcoef = ws.fcoef;
@@ -631,6 +633,7 @@ size_t layout_workspace(const fgpu_ctx* c, unsigned char* base, Workspace& ws, b
     take(ws.slices, (size_t)c->nt128 * NSLICE * SLICE_BYTES);
     take(ws.splanes, sizeof(double) * (size_t)std::max(c->spec.nplanes, 1) * nc);
     take(ws.norms, sizeof(double) * (size_t)MAX_LEAF * nc);
+    take(ws.dotc, sizeof(DotConst));
     take(ws.fnorm, sizeof(long long) * 2 * nc);
     take(ws.fcoef, sizeof(double) * 4);
     take(ws.fscale, sizeof(int) * 2);
@@ -838,8 +841,8 @@ int fgpu_create(fgpu_ctx** out, int N, int d, const double* X, const double* y, 
   c->ntheta = c->nkparams + c->optimise_noise;
   // feature planes, plane-major, padded to Nc.  FP64 mode: x, or the
   // half-angle pair sin(x/2), cos(x/2) for periodic dims.  Tensor-core mode
-  // (dot-product build): rbf dims centred on their mean, periodic dims as
-  // the pair cos(x), sin(x), rbf-cyclic dims raw.
+  // rbf and unwrapped rbf-cyclic dims centred on their mean, periodic dims as
+  // the pair cos(x), sin(x), wrapped rbf-cyclic dims as fractions of a turn.
   const int np = c->spec.nplanes;
   std::vector<double> planes((size_t)std::max(np, 1) * c->Nc, 0.0);
   std::vector<int> plane_leaf(np, 0);
@@ -851,7 +854,24 @@ int fgpu_create(fgpu_ctx** out, int N, int d, const double* X, const double* y, 
   for (int p = 0; p < np; ++p) {
     const double* col = X + (size_t)plane_dim[p] * N;  // X(:, dim), column-major
     double* dst = planes.data() + (size_t)p * c->Nc;
-    if (c->mode == 1 && plane_leaf[p] == FGPU_RBF) {
+    if (c->mode == 1 && plane_kind[p] == 3) {
+      // a wrapped rbf-cyclic feature: x / (2 pi) modulo 1 as a 64-bit fraction,
+      // so that differences wrap as integers (the product carries its error,
+      // and 1 / (2 pi) its tail)
+      constexpr double HI = 0.15915494309189535, LO = -9.839338337591243e-18;
+      for (int i = 0; i < N; ++i) {
+        const double q = col[i] * HI, err = std::fma(col[i], HI, -q) + col[i] * LO;
+        unsigned long long u = TURN_NOT_FINITE;
+        if (std::isfinite(q)) {
+          const double f = q - std::floor(q);  // exact
+          u = (unsigned long long)(f * 0x1p63) * 2ULL + (unsigned long long)(long long)std::llrint(std::ldexp(err, 64));
+          if (u == TURN_NOT_FINITE) ++u;  // half a turn, to 2^-64
+        }
+        memcpy(&dst[i], &u, 8);
+      }
+      continue;
+    }
+    if (c->mode == 1 && (plane_leaf[p] == FGPU_RBF || plane_leaf[p] == FGPU_RBF_CYCLIC)) {
       double mean = 0.0;
       for (int i = 0; i < N; ++i) mean += col[i];
       mean /= N;
@@ -882,7 +902,7 @@ int fgpu_create(fgpu_ctx** out, int N, int d, const double* X, const double* y, 
   {
     std::vector<double> pmax(std::max(np, 1), 0.0);
     for (int p = 0; p < np; ++p)
-      for (int i = 0; i < N; ++i) pmax[p] = std::max(pmax[p], std::fabs(planes[(size_t)p * c->Nc + i]));
+      for (int i = 0; i < N && !(c->mode == 1 && plane_kind[p] == 3); ++i) pmax[p] = std::max(pmax[p], std::fabs(planes[(size_t)p * c->Nc + i]));
     CK(cudaMalloc(&c->plane_max_d, pmax.size() * sizeof(double)));
     CK(cudaMemcpy(c->plane_max_d, pmax.data(), pmax.size() * sizeof(double), cudaMemcpyHostToDevice));
   }

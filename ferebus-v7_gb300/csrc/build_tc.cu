@@ -98,8 +98,9 @@ __global__ void __launch_bounds__(128) k_prep(const Prob* __restrict__ probs) {
   const Spec& sp = *P.spec;
   const int tid = threadIdx.x, i = rb * NB + tid;
   const size_t nc = (size_t)P.Nc;
-  __shared__ double w[MAX_PARAMS];  // rbf sqrt(exp(theta)), periodic 1 / exp(theta), linear 1 / c, constant theta
-  __shared__ int s_e[2], s_k;
+  __shared__ double w[MAX_PARAMS];  // rbf, rbf-cyclic sqrt(exp(theta)), periodic 1 / exp(theta), linear 1 / c, constant theta
+  __shared__ int s_e[2], s_k, s_c[MAX_LEAF];
+  __shared__ bool s_huge[MAX_LEAF];
   for (int q = tid; q < sp.nkparams; q += 128) {
     int type = L_CONSTANT;
     for (int l = 0; l < sp.nleaf; ++l) {
@@ -109,9 +110,10 @@ __global__ void __launch_bounds__(128) k_prep(const Prob* __restrict__ probs) {
     const double t = P.theta[q];
     // linear_kernel.f90:70-76, order 0: sum_k 1 / exp(-theta_k); constant.f90:62-68
     w[q] = type == L_CONSTANT ? t : 1.0;
-    if (type == L_RBF || type == L_PERIODIC || type == L_LINEAR) {
-      const double x = exp(type == L_RBF ? 0.5 * t : (type == L_LINEAR ? -t : t));
-      w[q] = type == L_RBF ? x : 1.0 / x;
+    if (type != L_CONSTANT) {
+      const bool half = type == L_RBF || type == L_RBF_CYCLIC;
+      const double x = exp(half ? 0.5 * t : (type == L_LINEAR ? -t : t));
+      w[q] = half ? x : 1.0 / x;
     }
   }
   __syncthreads();
@@ -128,6 +130,37 @@ __global__ void __launch_bounds__(128) k_prep(const Prob* __restrict__ probs) {
         s_e[d] = m == 0.0 ? 0 : (int)((__double_as_longlong(m) >> 52) & 0x7FF) - 1022;
         if (rb == 0) P.fscale[d] = s_e[d];
       }
+    }
+    // the dot-product build's constants; rbf-cyclic leaves get a scale too, a
+    // wrapped feature counting as pi / 2 (its difference is at most pi)
+    for (int l = d; !sp.tc_build && l < sp.nleaf; l += 2) {
+      const Leaf& L = sp.leaf[l];
+      double m = 0.0, c = 0.0;
+      for (int k = lane; k < L.n; k += 32) {
+        const double u = w[L.param0 + k];
+        if (L.type == L_RBF_CYCLIC)
+          m = fmax(m, u * (sp.cyclic[L.plane0 + k] ? 1.5707963267948966 : P.plane_max[L.plane0 + k]));
+        else
+          c += L.type == L_PERIODIC ? u * u : u;
+      }
+      for (int o = 16; o > 0; o >>= 1) {
+        m = fmax(m, __shfl_xor_sync(0xffffffffu, m, o));
+        c += __shfl_xor_sync(0xffffffffu, c, o);
+      }
+      const int s = m == 0.0 ? 0 : (int)((__double_as_longlong(m) >> 52) & 0x7FF) - 1022;
+      if (lane == 0) {
+        s_c[l] = s;
+        s_huge[l] = !(m < 0x1p900);
+        if (rb == 0) {
+          P.dotc->leaf_c[l] = L.type == L_CONSTANT ? w[L.param0] : c;
+          P.dotc->scale[l] = s;
+        }
+      }
+      if (rb == 0 && L.type == L_RBF_CYCLIC)
+        for (int k = lane; k < L.n; k += 32) {
+          const long long f = llrint(ldexp(6.283185307179586 * w[L.param0 + k], 54 - s));  // below 2^57
+          P.dotc->mul[L.plane0 + k] = make_int2((int)(f >> 32), (int)((unsigned)f >> 1));
+        }
     }
   } else if (tid == 0) {
     // the kernel expression in the (at most two) distance leaves of the
@@ -199,6 +232,21 @@ __global__ void __launch_bounds__(128) k_prep(const Prob* __restrict__ probs) {
         const int cnt = L.type == L_LINEAR || L.type == L_CONSTANT ? 0 : per * L.n;
         for (int k = 0; k < cnt; ++k) {
           const size_t o = (size_t)(L.plane0 + k) * nc + i;
+          if (L.type == L_RBF_CYCLIC) {
+            // fixed point 2^(54 - s), or the fraction of a turn as it is; a point
+            // (or a leaf) that is not finite is marked in its norm
+            const double x = P.planes[o];
+            if (sp.cyclic[L.plane0 + k]) {
+              P.splanes[o] = x;
+              if (__double_as_longlong(x) == (long long)TURN_NOT_FINITE) a = 1.0;
+            } else {
+              bool nf = false;
+              P.splanes[o] = __longlong_as_double((to_fixed55(w[L.param0 + k] * x, s_c[l], &nf) + 1) >> 1);
+              if (nf) a = 1.0;
+            }
+            if (s_huge[l]) a = 1.0;
+            continue;
+          }
           const double u = w[L.param0 + k / per] * P.planes[o];
           P.splanes[o] = u;
           if (L.type == L_RBF) a = fma(u, u, a);

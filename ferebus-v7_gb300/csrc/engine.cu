@@ -229,6 +229,16 @@ __global__ void __launch_bounds__(256) k_build(const Prob* __restrict__ probs) {
 // (absolute) on centred features, the size of its own rounding in the direct
 // form for the well separated pairs that dominate, and it vanishes on the
 // diagonal, which is set exactly (x_i = x_j gives a factor 1).
+//
+// An rbf-cyclic leaf (stationary_cyclic_kernel.f90:104-127 on distance_matrix.f90:
+// 95-128, every 3rd feature's difference wrapped to [-pi, pi]) has no inner
+// product to go by; its differences are integers: plain features in 54-bit
+// fixed point of the leaf's scale 2^s, wrapped ones as fractions of a turn,
+// whose 64-bit differences wrap by themselves and are brought to that scale by
+// one multiplication.  D = h 2^27 + l enters the exact sum as h^2 + 2 h l 2^-27 +
+// l^2 2^-54.  ~12 to 25 integer instructions (2 to 3 cycles) per feature and
+// pair, against 3 to ~30 FP64 ones (64 cycles; the wrap goes through fmod): 20
+// problems of N = 1000, d = 24, 2.6 -> 0.5 ms.
 // ---------------------------------------------------------------------------
 size_t build_dot_smem_bytes(int nplanes) {
   return (size_t)2 * (nplanes + MAX_LEAF) * TB * sizeof(double) + 64;
@@ -248,8 +258,7 @@ __global__ void __launch_bounds__(256) k_build_dot(const Prob* __restrict__ prob
   double* Ni = Pj + (size_t)np * TB;                      // nl x 64 norms, row points
   double* Nj = Ni + (size_t)MAX_LEAF * TB;
   uint64_t* bar = reinterpret_cast<uint64_t*>(Nj + (size_t)MAX_LEAF * TB);
-  __shared__ double ls[MAX_PARAMS];
-  __shared__ double leaf_c[MAX_LEAF];  // sum of l (periodic) or sum of 1/c (linear)
+  __shared__ DotConst dc;
   __shared__ int s_fail;
   const int tid = threadIdx.x;
   const int i0 = ti * TB, j0 = tj * TB;
@@ -273,24 +282,8 @@ __global__ void __launch_bounds__(256) k_build_dot(const Prob* __restrict__ prob
       bulk_g2s(Ni + l * TB, P.norms + (size_t)l * nc + i0, per, bar);
     }
   }
-  for (int k = tid; k < sp.nkparams; k += blockDim.x) {
-    int type = L_CONSTANT;
-    for (int l = 0; l < nl; ++l) {
-      const int cnt = sp.leaf[l].type == L_CONSTANT ? 1 : sp.leaf[l].n;
-      if (k >= sp.leaf[l].param0 && k < sp.leaf[l].param0 + cnt) type = sp.leaf[l].type;
-    }
-    ls[k] = transform_param(type, P.theta[k]);
-  }
-  __syncthreads();
-  if (tid < nl) {
-    double acc = 0.0;
-    const Leaf& L = sp.leaf[tid];
-    if (L.type == L_LINEAR)
-      for (int k = 0; k < L.n; ++k) acc += 1.0 / ls[L.param0 + k];
-    else if (L.type == L_PERIODIC)
-      for (int k = 0; k < L.n; ++k) acc += ls[L.param0 + k];
-    leaf_c[tid] = acc;
-  }
+  for (int q = tid; q < (int)sizeof(DotConst) / 4; q += blockDim.x)
+    reinterpret_cast<int*>(&dc)[q] = reinterpret_cast<const int*>(P.dotc)[q];
   if (!mbar_wait(bar, 0)) s_fail = 1;
   __syncthreads();
   if (s_fail) {
@@ -309,46 +302,79 @@ __global__ void __launch_bounds__(256) k_build_dot(const Prob* __restrict__ prob
   long long* A = P.acc + acc_tile(ti >> 1, tj, P.nt128) * ACC_TILE_ELEMS;
   for (int cc = 0; cc < 8; ++cc) {
     const int c = c0 + cc, j = j0 + c;
-    long long v[2];
-    for (int a = 0; a < 2; ++a) {
-      const int r = r0 + a, i = i0 + r;
-      long long val = 0;
-      if (i < P.N && j < P.N) {
-        if (i >= j) {
-          double stk[MAX_LEAF];
-          int top = 0;
-          for (int t = 0; t < sp.npost; ++t) {
-            const int tok = sp.post[t];
-            if (tok >= 0) {
-              const Leaf& L = sp.leaf[tok];
-              double lv;
-              if (L.type == L_RBF) {
-                double dot = 0.0;
-                for (int k = 0; k < L.n; ++k) dot = fma(Pi[(L.plane0 + k) * TB + r], Pj[(L.plane0 + k) * TB + c], dot);
-                const double e = (i == j) ? 0.0 : (Ni[tok * TB + r] + Nj[tok * TB + c]) - 2.0 * dot;
-                lv = iexp_neg(-0.5 * e);
-              } else if (L.type == L_PERIODIC) {
-                double dot = 0.0;
-                for (int k = 0; k < 2 * L.n; ++k)
-                  dot = fma(Pi[(L.plane0 + k) * TB + r], Pj[(L.plane0 + k) * TB + c], dot);
-                lv = (i == j) ? 1.0 : iexp_neg(dot - leaf_c[tok]);
-              } else {
-                lv = leaf_value(L, Pi, Pj, r, c, ls, sp.cyclic, leaf_c[tok]);
+    const int i = i0 + r0;  // this thread's rows i, i + 1
+    long long v[2] = {0, 0};
+    if (i + 1 >= j) {
+      double stk[2][MAX_LEAF];
+      int top = 0;
+      for (int t = 0; t < sp.npost; ++t) {
+        const int tok = sp.post[t];
+        if (tok >= 0) {
+          const Leaf& L = sp.leaf[tok];
+          if (L.type == L_RBF_CYCLIC) {
+            long long H[2] = {0, 0}, M[2] = {0, 0};
+            const longlong2* fi = reinterpret_cast<const longlong2*>(Pi + L.plane0 * TB + r0);
+            const long long* fj = reinterpret_cast<const long long*>(Pj + L.plane0 * TB + c);
+            for (int k = 0; k < L.n; ++k) {
+              const longlong2 f = fi[k * (TB / 2)];
+              const long long g = fj[k * TB];
+              long long D[2] = {(long long)((unsigned long long)f.x - (unsigned long long)g),
+                                (long long)((unsigned long long)f.y - (unsigned long long)g)};
+              if (sp.cyclic[L.plane0 + k]) {  // uniform
+                const int2 m = dc.mul[L.plane0 + k];
+#pragma unroll
+                for (int a = 0; a < 2; ++a) {
+                  const int dh = (int)(D[a] >> 32);
+                  D[a] = (long long)dh * m.x + (long long)(((unsigned long long)(unsigned)D[a] * (unsigned)m.x) >> 32) +
+                         (((long long)dh * m.y) >> 31);
+                }
               }
-              stk[top++] = lv;
-            } else {
-              const double b = stk[--top];
-              const double a2 = stk[--top];
-              stk[top++] = (tok == P_SUM) ? a2 + b : a2 * b;
+#pragma unroll
+              for (int a = 0; a < 2; ++a) {
+                const int hh = (int)((D[a] + (1LL << 26)) >> 27);
+                const int l = (int)((unsigned)D[a] - ((unsigned)hh << 27));
+                H[a] += (long long)hh * hh;
+                M[a] += (long long)hh * l + (((long long)l * l) >> 28);
+              }
             }
+            const IexpScale sc = iexp_scale(2 * dc.scale[tok] - 55);
+            for (int a = 0; a < 2; ++a)
+              stk[a][top] = Ni[tok * TB + r0 + a] != 0.0 || Nj[tok * TB + c] != 0.0
+                                ? nan("")
+                                : iexp_fixed_tab((unsigned long long)(H[a] + (M[a] >> 26)), sc, g_iexp_tab1024, g_iexp_fine1024);
+          } else if (L.type == L_RBF || L.type == L_PERIODIC) {
+            const int nf = L.type == L_PERIODIC ? 2 * L.n : L.n;
+            double dot[2] = {0.0, 0.0};
+            for (int k = 0; k < nf; ++k) {
+              const double2 f = *reinterpret_cast<const double2*>(Pi + (L.plane0 + k) * TB + r0);
+              const double g = Pj[(L.plane0 + k) * TB + c];
+              dot[0] = fma(f.x, g, dot[0]);
+              dot[1] = fma(f.y, g, dot[1]);
+            }
+            for (int a = 0; a < 2; ++a) {
+              if (i + a == j)
+                stk[a][top] = 1.0;
+              else if (L.type == L_RBF)
+                stk[a][top] = iexp_neg(-0.5 * ((Ni[tok * TB + r0 + a] + Nj[tok * TB + c]) - 2.0 * dot[a]));
+              else
+                stk[a][top] = iexp_neg(dot[a] - dc.leaf_c[tok]);
+            }
+          } else {
+            // linear: sum_k (x_ik x_jk)^0 / c_k, independent of (i, j); constant.f90:62-68
+            stk[0][top] = stk[1][top] = dc.leaf_c[tok];
           }
-          val = i == j ? diag_fixed62(stk[0], noise, e2, &nonfinite) : to_fixed62(stk[0], e2, &nonfinite);
+          ++top;
+        } else {
+          --top;
+          for (int a = 0; a < 2; ++a)
+            stk[a][top - 1] = (tok == P_SUM) ? stk[a][top - 1] + stk[a][top] : stk[a][top - 1] * stk[a][top];
         }
-      } else {
-        val = (i == j) ? 1LL << 60 : 0LL;  // identity padding, 1/4 in the matrix's unit
       }
-      v[a] = val;
+      for (int a = 0; a < 2; ++a)
+        v[a] = i + a == j ? diag_fixed62(stk[a][0], noise, e2, &nonfinite) : to_fixed62(stk[a][0], e2, &nonfinite);
     }
+    for (int a = 0; a < 2; ++a)  // identity padding, 1/4 in the matrix's unit; zero above the diagonal
+      if (i + a < j || i + a >= P.N || j >= P.N) v[a] = i + a == j ? 1LL << 60 : 0LL;
     *reinterpret_cast<longlong2*>(A + acc_elem((ti & 1) * TB + r0, c)) = make_longlong2(v[0], v[1]);
   }
   if (nonfinite) atomicOr(&P.status[3], 1);

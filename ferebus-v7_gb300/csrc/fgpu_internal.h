@@ -72,6 +72,17 @@ struct alignas(16) PanelZ {
   double scale[MAX_RHS];
 };
 
+// What the dot-product build (engine.cu) needs per evaluation besides the scaled
+// planes, from k_prep: per leaf the sum of l (periodic) or of 1 / c (linear), or
+// the constant; for rbf-cyclic leaves the fixed-point scale s and per wrapped
+// plane the factor 2 pi sqrt(l) 2^(54 - s) as (high word, low word >> 1).
+constexpr unsigned long long TURN_NOT_FINITE = 1ULL << 63;  // a wrapped feature's plane entry that stands for NaN or infinity
+struct DotConst {
+  double leaf_c[MAX_LEAF];
+  int scale[MAX_LEAF];
+  int2 mul[MAX_PLANES];
+};
+
 // Per-problem descriptor, resident in device memory.
 struct Prob {
   int N, Nc, ld, nsteps, nrhs, likelihood, optimise_noise, nkparams;
@@ -105,6 +116,7 @@ struct Prob {
   // dot-product kernel build (mode 1): planes scaled by sqrt(l_k) per evaluation
   double* splanes;                // nplanes x Nc
   double* norms;                  // MAX_LEAF x Nc: sum_k u_ik^2 of rbf leaves
+  DotConst* dotc;
   // FP64 kernels: number of 64-row tiles when extra border rows follow the
   // right-hand-side tile (the adjoint's identity rows); 0 = nsteps + 1
   int nrt;

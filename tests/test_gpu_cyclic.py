@@ -1,0 +1,55 @@
+"""The rbf-cyclic leaf's fixed-point distances (the tensor-core mode's
+dot-product build) against the oracle: dihedrals wrapped across +-pi, far outside
+[-pi, pi] and at exactly opposite angles, sizes at the edges of its 64-row tiles,
+alone and combined with other leaves.  Tolerance: the well conditioned cases'
+1e-9 relative.  A point that is not finite fails the evaluation, as it does in
+the FP64 mode."""
+import numpy as np
+import pytest
+
+from oracle import gpr_oracle as O
+
+pytestmark = pytest.mark.gpu
+
+
+def _data(n, d, seed):
+    rng = np.random.default_rng(seed)
+    X = rng.normal(2.0, 0.3, size=(n, d))
+    X[:, 2::3] = rng.uniform(-np.pi, np.pi, size=X[:, 2::3].shape)
+    X[: n // 3, 2] += 4 * np.pi          # whole turns away
+    X[n // 2, 2::3] = np.pi              # opposite to the next point's 0
+    X[n // 2 - 1, 2::3] = 0.0
+    y = np.cos(X[:, 0]) + 0.2 * np.sin(X[:, 2]) + 1e-3 * rng.normal(size=n)
+    return X, y
+
+
+@pytest.mark.parametrize("n", [3, 63, 64, 65, 129, 300])
+@pytest.mark.parametrize("spec", ["cyclic", "cyclic_plus_rbf", "cyclic_times_const_plus_linear"])
+def test_cyclic_against_oracle(n, spec, lib):
+    from fgpu import Engine
+    d = 9
+    X, y = _data(n, d, n)
+    cyc = [O.RBF_CYCLIC, d, *range(1, d + 1)]
+    ks = {"cyclic": cyc, "cyclic_plus_rbf": cyc + [O.RBF, 2, 1, 2, O.SUM],
+          "cyclic_times_const_plus_linear": cyc + [O.CONSTANT, 0, O.PROD, O.LINEAR, 1, 2, O.SUM]}[spec]
+    mu = O.mean_vector("constant", X, y)
+    th = np.random.default_rng(1).uniform(0.2, 0.9, size=O.kernel_nparams(ks))
+    e = Engine(X, y, mu, ks, 0, 1e-3, False)
+    ll, info = e.loglik(th)
+    ref, rinfo = O.loglik(ks, th, X, y, mu, 0, 1e-3, False)
+    assert info == rinfo == 0
+    assert abs(ll - ref) <= 1e-9 * abs(ref), (ll, ref)
+
+
+@pytest.mark.parametrize("col", [0, 2])  # a plain and a wrapped feature
+def test_point_that_is_not_finite(col, lib):
+    from fgpu import Engine
+    from fgpu._lib import FgpuError
+    X, y = _data(80, 9, 5)
+    X[40, col] = np.nan
+    e = Engine(X, y, np.zeros(80), [O.RBF_CYCLIC, 9, *range(1, 10)], 0, 1e-3, False)
+    try:
+        ll, info = e.loglik(np.full(9, 0.5))
+    except FgpuError:
+        return
+    assert info > 0 and np.isnan(ll)
