@@ -93,27 +93,33 @@ __device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_al
 // D 2^-60 = m 4^k, 1 <= m < 4 (k < 0, sh = -k - 1), and y0 ~ m^-1/2 (23 bits):
 // e = 1 - m y0^2 is formed to 2^-61 (|e| < 2^-20) and m^-1/2 =
 // y0 (1 - e)^-1/2 = y0 (1 + e/2 + 3 e^2 / 8 + O(2^-61)).  Relative error below
-// 2^-58.  ~50 integer instructions (2 to 3 cycles
+// 2^-57.  ~50 integer instructions (2 to 3 cycles
 // of issue each on this GPU, ~220 of latency together); the library's FP64
 // rsqrt takes ~380 cycles, and 128 of them follow one another in a panel.
 __device__ __forceinline__ void rsqrt_fixed(long long D, unsigned& yh, unsigned& yl, int& sh) {
   const unsigned hi = (unsigned)((unsigned long long)D >> 32), lo = (unsigned)D;
-  const int lz = hi ? __clz(hi) : 32 + __clz(lo);
-  const unsigned long long A = (unsigned long long)D << (lz & 63);  // leading one at bit 63
-  const int E = 3 - lz, r = E & 1;                                  // D 2^-60 = 1.f 2^E
+  // leading one to bit 63 of (ah, al); D 2^-60 = 1.f 2^E
+  const unsigned h1 = hi ? hi : lo, l1 = hi ? lo : 0u;
+  const int z = __clz(h1), E = (hi ? 3 : -29) - z, r = E & 1;
+  const unsigned ah = __funnelshift_l(l1, h1, z), al = l1 << (z & 31);
   sh = -(E >> 1) - 1;
-  const float mf = __uint_as_float(((unsigned)(127 + r) << 23) | ((unsigned)(A >> 40) & 0x7FFFFFu));
+  const float mf = __uint_as_float((ah >> 8) + ((unsigned)(126 + r) << 23));  // the leading one carries into the exponent
   float y0;
   asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(y0) : "f"(mf));
   const unsigned Y = __float_as_uint(y0 + 1.0f) - 0x3F800000u;  // y0 2^23, y0 in [0.5, 1]
-  const unsigned long long YY = (unsigned long long)Y * Y;
-  const long long e = (long long)((1ULL << 61) - __umul64hi(A, YY << (16 + r)));  // e 2^61
+  // e 2^61 = 2^61 - m y0^2 2^61, m 2^62 in (mh, ml), y0^2 2^63 in (qh, ql); the
+  // product of the low words (below 2^-61) is left out
+  const unsigned mh = r ? ah : ah >> 1, ml = r ? al : __funnelshift_r(al, ah, 1);
+  const unsigned long long q = ((unsigned long long)Y * Y) << 17;
+  const unsigned qh = (unsigned)(q >> 32), ql = (unsigned)q;
+  const unsigned long long t1 = (unsigned long long)mh * ql, t2 = (unsigned long long)ml * qh;
+  const long long e = (long long)((1ULL << 61) - (t2 >> 32) - ((unsigned long long)mh * qh + (t1 >> 32)));
   const int eh = (int)(e >> 10);
   const unsigned e2 = (unsigned)((unsigned long long)((long long)eh * eh) >> 32);  // e^2 2^70
-  const long long c = (e >> 1) + (long long)((e2 * 3u) >> 12);                    // (e/2 + 3 e^2/8) 2^61
-  // y0 (1 + c) 2^63, less one unit: never 2^63
-  const unsigned long long v =
-      (((unsigned long long)(Y * 256u - 1u) << 32) | 0xFFFFFFFFu) + (unsigned long long)(((long long)Y * (c >> 2)) >> 19);
+  const unsigned c2 = (e2 * 3u) >> 14;                                             // 3 e^2 / 8 2^59
+  // y0 (1 + e/2 + c2) 2^63, less one unit: never 2^63
+  const unsigned long long v = (((unsigned long long)(Y * 256u - 1u) << 32) | 0xFFFFFFFFu) +
+                               (unsigned long long)(((long long)Y * (e >> 3) + (long long)((unsigned long long)Y * c2)) >> 19);
   yh = (unsigned)(v >> 32);
   yl = (unsigned)v;
 }
@@ -145,13 +151,6 @@ __device__ __forceinline__ void mac_entry(long long& S, long long& M, int xh, in
   M += (long long)xh * ll;
   M += (long long)xl * lh;
 }
-// B = S - M 2^-30 -= x l, in units of 2^-60
-__device__ __forceinline__ void take_entry(long long& S, long long& M, int xh, int xl, int lh, int ll) {
-  S -= (long long)xh * lh;
-  M += (long long)xh * ll;
-  M += (long long)xl * lh;
-}
-
 // shift a register array down by n: a[i] = a[i + n]
 template <int n, typename T, int N>
 __device__ __forceinline__ void shift_down(T (&a)[N]) {
@@ -159,18 +158,17 @@ __device__ __forceinline__ void shift_down(T (&a)[N]) {
   for (int i = 0; i + n < N; ++i) a[i] = a[i + n];
 }
 
-// B = T - M 2^-30 of a row's column k -= sum over c0 <= c < n of x_c l_kc, two
-// block entries a load
+// S + M 2^-30 += sum over c0 <= c < n of x_c l_kc, two block entries a load
 template <int c0>
-__device__ __forceinline__ void take_row(long long& T, long long& M, const int (&Xh)[PW], const int (&Xl)[PW],
-                                         const PanelBlock& Lt, int k, int n) {
+__device__ __forceinline__ void mac_row(long long& S, long long& M, const int (&Xh)[PW], const int (&Xl)[PW],
+                                        const PanelBlock& Lt, int k, int n) {
   const int4* l = reinterpret_cast<const int4*>(&Lt.x[k][0]);
 #pragma unroll
   for (int c = c0; c < PW; c += 2) {
     if (c < n) {
       const int4 v = l[c / 2];
-      take_entry(T, M, Xh[c], Xl[c], v.x, v.y);
-      if (c + 1 < n) take_entry(T, M, Xh[c + 1], Xl[c + 1], v.z, v.w);
+      mac_entry(S, M, Xh[c], Xl[c], v.x, v.y);
+      if (c + 1 < n) mac_entry(S, M, Xh[c + 1], Xl[c + 1], v.z, v.w);
     }
   }
 }
@@ -392,17 +390,17 @@ __global__ void __launch_bounds__(PN_THREADS, 1)
         // follows it is discarded.
         const int base = (t & 1) * PW;
         const int c_own = lane - base;  // this row's index in the block; < 0: above, >= 16: below
-        long long M[PW];                // with T: B = T - M 2^-30
+        long long M[PW];                // with T: B = T + M 2^-30
 #pragma unroll
         for (int k = 0; k < PW; ++k) M[k] = 0;
         int fail = PW;
 #pragma unroll 1
         for (int b = 0; b < 4; ++b) {
-          int xh[4], xl[4];
+          int xh[4], xl[4], nxh[4], nxl[4];
 #pragma unroll
           for (int q = 0; q < 4; ++q) {
             const int j = 4 * b + q;
-            const long long Tj = T[q] - (M[q] >> 30);
+            const long long Tj = T[q] + (M[q] >> 30);
             const long long D = __shfl_sync(0xffffffffu, Tj, base + j);
             if (D < 4 && fail == PW) fail = j;  // 2^-58 of 2^2e: far below what K's own rounding leaves of a pivot
             unsigned yh, yl;
@@ -411,6 +409,8 @@ __global__ void __launch_bounds__(PN_THREADS, 1)
             sh = min(max(sh, 0), 28);  // discarded columns only
             scale_entry(Tj, yh, yl, sh, xh[q], xl[q]);
             if (c_own < j) xh[q] = xl[q] = 0;  // above the diagonal
+            nxh[q] = -xh[q];
+            nxl[q] = -xl[q];
             if (c_own == j) {
               yh_own = yh;
               yl_own = yl;
@@ -424,7 +424,7 @@ __global__ void __launch_bounds__(PN_THREADS, 1)
             for (int k = q + 1; k < 4; ++k) {
               const int lh = __shfl_sync(0xffffffffu, xh[q], base + 4 * b + k);
               const int ll = __shfl_sync(0xffffffffu, xl[q], base + 4 * b + k);
-              take_entry(T[k], M[k], xh[q], xl[q], lh, ll);
+              mac_entry(T[k], M[k], nxh[q], nxl[q], lh, ll);
             }
           }
           if (c_own >= 0 && c_own < PW) {
@@ -450,10 +450,10 @@ __global__ void __launch_bounds__(PN_THREADS, 1)
                 const int4 l0 = lb[i * (PW / 2)], l1 = lb[i * (PW / 2) + 1];
                 T[i] = T[i + 4];
                 M[i] = M[i + 4];
-                take_entry(T[i], M[i], xh[0], xl[0], l0.x, l0.y);
-                take_entry(T[i], M[i], xh[1], xl[1], l0.z, l0.w);
-                take_entry(T[i], M[i], xh[2], xl[2], l1.x, l1.y);
-                take_entry(T[i], M[i], xh[3], xl[3], l1.z, l1.w);
+                mac_entry(T[i], M[i], nxh[0], nxl[0], l0.x, l0.y);
+                mac_entry(T[i], M[i], nxh[1], nxl[1], l0.z, l0.w);
+                mac_entry(T[i], M[i], nxh[2], nxl[2], l1.x, l1.y);
+                mac_entry(T[i], M[i], nxh[3], nxl[3], l1.z, l1.w);
               }
             }
           }
@@ -527,15 +527,17 @@ __global__ void __launch_bounds__(PN_THREADS, 1)
             constexpr int HW = PW / 2;
 #pragma unroll
             for (int k = 0; k < HW; ++k) {
-              long long M = 0;
-              take_row<0>(T[k], M, Xh, Xl, Lt, k, k);
-              scale_entry(T[k] - (M >> 30), Lt.y[k].x, Lt.y[k].y, Lt.sh[k], Xh[k], Xl[k]);
+              long long S = 0, M = 0;
+              mac_row<0>(S, M, Xh, Xl, Lt, k, k);
+              scale_entry(T[k] - S - (M >> 30), Lt.y[k].x, Lt.y[k].y, Lt.sh[k], Xh[k], Xl[k]);
             }
             long long M2[HW];
 #pragma unroll
             for (int q = 0; q < HW; ++q) {
+              long long S = 0;
               M2[q] = 0;
-              take_row<0>(T[HW + q], M2[q], Xh, Xl, Lt, HW + q, HW);
+              mac_row<0>(S, M2[q], Xh, Xl, Lt, HW + q, HW);
+              T[HW + q] -= S;
             }
             if (!wait(b_blk, t & 1)) {
               out = true;
@@ -543,8 +545,9 @@ __global__ void __launch_bounds__(PN_THREADS, 1)
             }
 #pragma unroll
             for (int k = HW; k < PW; ++k) {
-              take_row<HW>(T[k], M2[k - HW], Xh, Xl, Lt, k, k);
-              scale_entry(T[k] - (M2[k - HW] >> 30), Lt.y[k].x, Lt.y[k].y, Lt.sh[k], Xh[k], Xl[k]);
+              long long S = 0;
+              mac_row<HW>(S, M2[k - HW], Xh, Xl, Lt, k, k);
+              scale_entry(T[k] - S - (M2[k - HW] >> 30), Lt.y[k].x, Lt.y[k].y, Lt.sh[k], Xh[k], Xl[k]);
             }
           }
           if (!done) {

@@ -4,9 +4,10 @@ point of the kernel matrix, the substitution in 60-bit fixed point and the
 digits of its results.
 
 Bounds, derived before the first run: the reciprocal square root errs by
-2^-59 relative from the truncated product y0 c, 5/16 e^3 < 2^-61 from the series
-and 2^-60 from e: below 2^-58; each conversion rounds once, so it is within
-half a unit.
+2^-59 from e / 2 and 2^-59 from 3 e^2 / 8 cut to that unit, 3 x 2^-62 from e (the
+low words' product and two high words cut off), 5/16 e^3 < 2^-61 from the series
+and y0 times that again, all relative: below 2^-57; each conversion rounds
+once, so it is within half a unit.
 """
 import math
 import random
@@ -26,25 +27,32 @@ def _double(b):
 
 def rsqrt_fixed(D, ulps):
     """The device function; ``ulps`` perturbs the single-precision estimate."""
-    lz = 64 - D.bit_length()
-    A = D << lz
-    E = 3 - lz
+    hi, lo = D >> 32, D & 0xFFFFFFFF
+    h1, l1 = (hi, lo) if hi else (lo, 0)
+    z = 32 - h1.bit_length()
+    E = (3 if hi else -29) - z
     r = E & 1
+    A = ((h1 << 32) | l1) << z
+    assert A >> 63 == 1 and A < 2 ** 64
+    ah, al = A >> 32, A & 0xFFFFFFFF
     sh = -(E >> 1) - 1
-    mf = np.uint32(((127 + r) << 23) | ((A >> 40) & 0x7FFFFF)).view(np.float32)
+    mf = np.uint32((ah >> 8) + ((126 + r) << 23)).view(np.float32)
+    assert 1 <= mf <= 4
     y0 = np.uint32(int(np.float32(1.0 / math.sqrt(float(mf))).view(np.uint32)) + ulps).view(np.float32)
     Y = int(np.float32(y0 + np.float32(1.0)).view(np.uint32)) - 0x3F800000
     assert 2 ** 22 <= Y <= 2 ** 23
-    YY = (Y * Y) << (16 + r)
-    assert YY < 2 ** 64
-    e = (1 << 61) - ((A * YY) >> 64)
+    q = (Y * Y) << 17
+    assert q < 2 ** 64
+    m = A if r else A >> 1
+    mh, ml, qh, ql = m >> 32, m & 0xFFFFFFFF, q >> 32, q & 0xFFFFFFFF
+    e = (1 << 61) - ((ml * qh) >> 32) - (mh * qh + ((mh * ql) >> 32))
     assert abs(e) < 2 ** 41
     eh = e >> 10
     assert abs(eh) < 2 ** 31
     e2 = (eh * eh) >> 32
     assert e2 * 3 < 2 ** 32
-    c = (e >> 1) + ((e2 * 3) >> 12)
-    prod = Y * (c >> 2)
+    c2 = (e2 * 3) >> 14
+    prod = Y * (e >> 3) + Y * c2
     assert abs(prod) < 2 ** 63
     y = (((Y * 256 - 1) << 32) | 0xFFFFFFFF) + (prod >> 19)
     assert 0 <= y < 2 ** 63
@@ -62,7 +70,7 @@ def test_rsqrt_fixed_within_its_bound():
             got = Fraction(y) * Fraction(2) ** (sh - 62)
             # relative error: got = (1 + t) / sqrt(d), t = (got^2 d - 1) / 2 to first order
             t = abs(float((got ** 2 * Fraction(D, 2 ** 60) - 1) / 2))
-            assert t <= 2.0 ** -58, (D, ulps, t)
+            assert t <= 2.0 ** -57, (D, ulps, t)
 
 
 def wrap(v, bits=64):
@@ -123,7 +131,7 @@ def test_substitution_in_fixed_point():
     k's right-hand side is off by its rounding (2^-61), the dropped Xl Ll (at
     most 15 x 2^58 2^-120), the shift (2^-60) and the block's own rounding
     (15 x 2^-61 |x|); the division by L_kk scales that by 1 / L_kk, plus y's
-    2^-58 relative and 3 x 2^-60: below 2^-56 (1 + 1 / min L_kk), amplified by
+    2^-57 relative and 3 x 2^-60: below 2^-56 (1 + 1 / min L_kk), amplified by
     the block's conditioning, which max |inv(L)| bounds."""
     rng = np.random.default_rng(9)
     for cond in (0.0, 2.0, 6.0, 9.0):
