@@ -171,6 +171,7 @@ struct UpdSched {
   int* sync_dev = nullptr;          // zeroed per evaluation: PANEL_FLAGS ints per problem, a tile counter per step
   size_t flag_ints = 0, nsync = 0;  // offset of the counters, ints in all
   int dot_builds = 0;               // problems the FP64 dot-product build serves
+  bool keep_l = false;              // a worker's: the factor is kept
 };
 
 // One problem's device buffers.  They are carved from one block (`base`,
@@ -358,6 +359,7 @@ void fill_prob(Prob& p, const fgpu_ctx* c, const double* theta_d, const Workspac
   p.tmap_a = ws.tmaps;
   p.tmap_b = ws.tmaps ? ws.tmaps + 128 : nullptr;
   p.tmap_bs = ws.tmaps ? ws.tmaps + 256 : nullptr;
+  p.tmap_b16 = ws.tmaps ? ws.tmaps + 384 : nullptr;
   p.rhs = ws.rhs;
   p.ldiag = ws.ldiag;
   p.lpub = ws.lpub;
@@ -484,7 +486,8 @@ int enqueue_eval(const Prob* probs_d, int nprob, int max_nsteps, int max_nplanes
       STAGE(0, launch_build_tc(probs_d, nprob, us->build_tiles_dev, us->build_total, us->num_sms, s));
     for (int step = 0; step < nt; ++step) {
       STAGE(2, launch_panel(probs_d, step, us->pan_order_dev + us->pan_off[step], us->diag_totals[step],
-                            us->row_totals[step], us->sync_dev + us->flag_ints + step, us->sync_dev, us->num_sms, s));
+                            us->row_totals[step], us->sync_dev + us->flag_ints + step, us->sync_dev, us->keep_l,
+                            us->num_sms, s, &n));
       if (step + 1 < nt)
         STAGE(3, launch_ozaki_update(probs_d, nprob, step, nt, us->tiles_dev + us->tile_off[step],
                                      us->totals[step], us->num_sms, s));
@@ -729,6 +732,7 @@ int make_worker(fgpu_ctx* c, Worker** out) {
   if (c->mode == 1 &&
       (rc = build_sched(std::vector<int>{c->nt128}, std::vector<int>{c->spec.tc_build}, w->sched, nullptr)) != 0)
     return bail(rc);
+  w->sched.keep_l = true;
   if ((rc = capture(w->stream, &w->graph, w->prob_d, 1, c->nsteps, c->spec.nplanes, w->ws.status,
                     sizeof(int) * 4, &w->graph_kernels, nullptr, c->mode, &w->sched)) != 0)
     return bail(rc);

@@ -108,6 +108,7 @@ struct Prob {
   const void* tmap_a;             // TMA tensor map over slices, box 8 x 128 rows x 2 kgroups x 7 planes
   const void* tmap_b;             // same, box of 64 rows
   const void* tmap_bs;            // box of 64 rows landing as [k-group][plane][row]: the 7 planes stacked along N
+  const void* tmap_b16;           // same, box of 16 rows
   double* rhs;                    // MAX_RHS x Nc: right-hand sides times 2^-e, turned into L^-1 r panel by panel
   PanelBlock* lpub;               // 8: the current panel's diagonal blocks, as its diagonal tile publishes them
   PanelZ* zpub;                   // 8: and its solved right-hand-side entries
@@ -134,10 +135,10 @@ struct Prob {
   int* fscale;                    // 2: s of the distance leaves, max |f| < 2^s
 };
 
-// Encode the three 5-D TMA tensor maps of a problem's digit-plane buffer
-// (boxes of 128 and 64 rows, and 64 rows with the planes stacked) into host
-// memory (TMAP_BYTES).  Returns 0 or a CUDA driver error code.
-constexpr size_t TMAP_BYTES = 3 * 128;
+// Encode the four 5-D TMA tensor maps of a problem's digit-plane buffer
+// (boxes of 128 and 64 rows, and 64 and 16 rows with the planes stacked) into
+// host memory (TMAP_BYTES).  Returns 0 or a CUDA driver error code.
+constexpr size_t TMAP_BYTES = 4 * 128;
 int encode_slice_maps(void* host_maps, const void* slices, int nt128);
 
 // Launch helpers (engine.cu).  All kernels take a device array of problems
@@ -189,7 +190,7 @@ constexpr size_t ACC_TILE_ELEMS = (size_t)NB * TB;
 // zeroed once per evaluation.
 constexpr int PANEL_FLAGS = 32;            // one 128-byte line per problem
 cudaError_t launch_panel(const Prob* probs, int step, const int* order, int ndiag, int total_tiles, int* counter,
-                         int* flags, int num_sms, cudaStream_t s);
+                         int* flags, bool keep_l, int num_sms, cudaStream_t s, long long* nlaunch);
 // prefix: device table of nprob + 1 tile offsets for this step (tiles of
 // problem p at step s: m (m + 1), m = nt128_p - s - 1); total_tiles = prefix[nprob].
 // tiles: the step's trailing tiles, packed (problem << 40 | row tile << 20 | column tile)
@@ -260,7 +261,7 @@ cudaError_t enqueue_grad_fast(const Prob* p, const Prob* eval, int nsteps, int n
 // device, or a second thread, sets the attribute for itself.  Devices
 // beyond the first 64 set it on every call.
 enum SmemSlot {
-  SMEM_BUILD, SMEM_BUILD_DOT, SMEM_UPDATE, SMEM_SYRK, SMEM_OZAKI_UPDATE, SMEM_PANEL,
+  SMEM_BUILD, SMEM_BUILD_DOT, SMEM_UPDATE, SMEM_SYRK, SMEM_OZAKI_UPDATE, SMEM_PANEL, SMEM_PANEL_ROWS,
   SMEM_BUILD_TC, SMEM_INV_GEMM, SMEM_GRAD_FAST, SMEM_NSLOTS
 };
 cudaError_t ensure_smem_attr(const void* func, int slot, int bytes);

@@ -205,6 +205,45 @@ __device__ __forceinline__ uint32_t tmem_ld1(uint32_t addr) {
   return v;
 }
 
+// T -= the couplings' exact sums of this warp's 32 rows and 16 columns, from
+// their 7 level sums at `addr` in TMEM: by the magic add where they lie in
+// (-2^22, 2^22) (the sum's exponent bits tell), else by F2I
+__device__ __forceinline__ void drain_couplings(long long (&T)[PW], uint32_t addr) {
+#pragma unroll
+  for (int g = 0; g < 2; ++g) {
+    uint32_t v[NSLICE][8], off = 0;
+#pragma unroll
+    for (int l = 0; l < NSLICE; ++l) tmem_ld8(v[l], addr + (uint32_t)(l * PW + g * 8));
+    asm volatile("tcgen05.wait::ld.sync.aligned;");
+#pragma unroll
+    for (int l = 0; l < NSLICE; ++l)
+#pragma unroll
+      for (int jj = 0; jj < 8; ++jj) {
+        v[l][jj] = level_bits(v[l][jj]);
+        off |= v[l][jj] ^ 0x4B000000u;
+      }
+    if (__any_sync(0xffffffffu, off >> 23)) {
+#pragma unroll 1
+      for (int c = 0; c < 8; ++c) {
+        int I[NSLICE];
+#pragma unroll
+        for (int l = 0; l < NSLICE; ++l) I[l] = (int)tmem_ld1(addr + (uint32_t)(l * PW + g * 8 + c));
+        asm volatile("tcgen05.wait::ld.sync.aligned;");
+#pragma unroll
+        for (int l = 0; l < NSLICE; ++l) I[l] = __float2int_rn(__int_as_float(I[l]));
+        const unsigned long long W = (unsigned long long)levels_to_w64(I);
+#pragma unroll
+        for (int k = 0; k < 8; ++k)
+          if (k == c) T[g * 8 + k] = (long long)((unsigned long long)T[g * 8 + k] - W);
+      }
+    } else {
+#pragma unroll
+      for (int jj = 0; jj < 8; ++jj)
+        T[g * 8 + jj] = (long long)((unsigned long long)T[g * 8 + jj] - (unsigned long long)level_bits_to_w64(v, jj));
+    }
+  }
+}
+
 // one lane polls a problem's counter until it reaches `want` (bounded)
 __device__ __forceinline__ int poll_flag(const int* f, int want) {
   for (int it = 0; it < (1 << 22); ++it) {
@@ -331,48 +370,18 @@ __global__ void __launch_bounds__(PN_THREADS, 1)
       if (tail) {
       } else if (!done) {
         if (t > 0) {
-          // the couplings' 7 level sums: by the magic add where they lie in
-          // (-2^22, 2^22) (the sum's exponent bits tell), else by F2I
 #pragma unroll
-          for (int g = 0; g < 2; ++g) {
-            uint32_t v[NSLICE][8], off = 0;
-#pragma unroll
-            for (int l = 0; l < NSLICE; ++l) tmem_ld8(v[l], trow + (uint32_t)(l * PW + g * 8));
-            asm volatile("tcgen05.wait::ld.sync.aligned;");
-#pragma unroll
-            for (int l = 0; l < NSLICE; ++l)
-#pragma unroll
-              for (int jj = 0; jj < 8; ++jj) {
-                v[l][jj] = level_bits(v[l][jj]);
-                off |= v[l][jj] ^ 0x4B000000u;
-              }
-#pragma unroll
-            for (int jj = 0; jj < 8; ++jj)
-              T[g * 8 + jj] = to_unit60((unsigned long long)wv[g * 8 + jj] - (unsigned long long)level_bits_to_w64(v, jj));
-            if (__any_sync(0xffffffffu, off >> 23)) {
-#pragma unroll 1
-              for (int c = 0; c < 8; ++c) {
-                uint32_t u[NSLICE];
-#pragma unroll
-                for (int l = 0; l < NSLICE; ++l) u[l] = tmem_ld1(trow + (uint32_t)(l * PW + g * 8 + c));
-                asm volatile("tcgen05.wait::ld.sync.aligned;");
-                int I[NSLICE];
-#pragma unroll
-                for (int l = 0; l < NSLICE; ++l) I[l] = __float2int_rn(__uint_as_float(u[l]));
-                const unsigned long long W = (unsigned long long)levels_to_w64(I);
-#pragma unroll
-                for (int k = 0; k < 8; ++k)
-                  if (k == c) T[g * 8 + k] = to_unit60((unsigned long long)wv[g * 8 + k] - W);
-              }
-            }
-          }
+          for (int c = 0; c < PW; ++c) T[c] = wv[c];
+          drain_couplings(T, trow);
           asm volatile("tcgen05.fence::before_thread_sync;");
           __syncwarp();
           if (lane == 0) mbar_arrive(b_drained);
         } else {
 #pragma unroll
-          for (int c = 0; c < PW; ++c) T[c] = to_unit60((unsigned long long)wv[c]);
+          for (int c = 0; c < PW; ++c) T[c] = wv[c];
         }
+#pragma unroll
+        for (int c = 0; c < PW; ++c) T[c] = to_unit60((unsigned long long)T[c]);
         if (t + 1 < np) load_piece(t + 1);
       } else if (lane == 0) {
         mbar_arrive(b_drained);
@@ -799,6 +808,254 @@ __global__ void __launch_bounds__(PN_THREADS, 1)
 }
 
 // ---------------------------------------------------------------------------
+// the rows of a panel whose diagonal tiles are done (batches): the same pieces,
+// arranged for throughput.  A row tile's integer work (~2.1k instructions per
+// piece and warp at 2.5 cycles of issue) keeps one warp per SM quarter only half
+// busy -- it waits for its couplings, loads and barriers -- so two CTAs share
+// an SM.  That leaves 113 KB each: the digits of the current piece stay in
+// shared memory, those of the earlier pieces come back from the L2 by TMA (21
+// chunks of 28 KB per tile) through a 2-stage ring, and are multiplied into the
+// other one of two TMEM accumulators while the rows are solved.  One thread
+// issues the copies and the MMAs.  Every word is the one k_panel computes: the
+// sums are exact integers.  All panels of 40 problems of N = 4000: 9.3 -> 6.4
+// ms, of 16 of N = 10000: 21.8 -> 15.9 ms, of 50 of N = 2000: 3.3 -> 2.5 ms.
+// ---------------------------------------------------------------------------
+namespace {
+constexpr int PR_THREADS = 160;
+constexpr uint32_t PR_STAGE = PN_ACHUNK + PN_BCHUNK;
+constexpr uint32_t PR_OFF_RING = PN_ACHUNK;
+constexpr uint32_t PR_OFF_B = PR_OFF_RING + 2 * PR_STAGE;  // [2]: B operand of the current piece's own chunk
+constexpr uint32_t PR_OFF_L = PR_OFF_B + 2 * PN_BCHUNK;
+constexpr uint32_t PR_OFF_Z = PR_OFF_L + 2 * PN_LBYTES;
+constexpr uint32_t PR_OFF_BAR = PR_OFF_Z + NPIECE * PN_ZBYTES;
+constexpr uint32_t PR_SMEM = PR_OFF_BAR + 96;
+static_assert(2 * (PR_SMEM + 2048) <= 228 * 1024, "two CTAs per SM");
+static_assert(PN_LBYTES % 16 == 0 && PR_OFF_L % 16 == 0 && PR_STAGE % 128 == 0 && PR_OFF_B % 128 == 0, "bulk and TMA alignment");
+}  // namespace
+
+__global__ void __launch_bounds__(PR_THREADS, 2)
+    k_panel_rows(const Prob* __restrict__ probs, int s, const int* __restrict__ order) {
+  extern __shared__ __align__(1024) unsigned char smr[];
+  unsigned char* As = smr;                 // the current piece's digits
+  unsigned char* ring = smr + PR_OFF_RING;  // [2]: an earlier piece's digits and its B operand
+  unsigned char* Bs = smr + PR_OFF_B;
+  PanelBlock* Ls = reinterpret_cast<PanelBlock*>(smr + PR_OFF_L);  // [2]
+  PanelZ* Zs = reinterpret_cast<PanelZ*>(smr + PR_OFF_Z);          // [NPIECE]
+  uint64_t* b_mma = reinterpret_cast<uint64_t*>(smr + PR_OFF_BAR);  // a piece's couplings are in TMEM
+  uint64_t* b_digits = b_mma + 1;                                   // its digits are in As and in HBM, its couplings drained
+  uint64_t* b_quiet = b_mma + 2;                                    // quiescing before an early exit
+  uint64_t* b_blk = b_mma + 3;                                      // [2]: Ls
+  uint64_t* b_own = b_mma + 5;                                      // [2]: Bs
+  uint64_t* full = b_mma + 7;                                       // [2]: ring
+  uint64_t* empty = b_mma + 9;                                      // [2]
+  __shared__ int s_skip, s_stop, s_abort;
+  __shared__ uint32_t s_tmem;
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int id = order[blockIdx.x], p = id >> 16, ti = id & 0xFFFF;
+  const Prob& P = probs[p];
+  if (tid == 0) {
+    s_skip = *(volatile int*)&P.status[1];  // one read: the exit below is block-uniform
+    s_stop = 0;
+    s_abort = 0;
+    mbar_init(b_mma, 1);
+    mbar_init(b_digits, 4);
+    mbar_init(b_quiet, 1);
+    for (int k = 0; k < 2; ++k) {
+      mbar_init(&b_blk[k], 1);
+      mbar_init(&b_own[k], 1);
+      mbar_init(&full[k], 1);
+      mbar_init(&empty[k], 1);
+    }
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+  }
+  for (int q = tid; q < NPIECE * (int)PN_ZBYTES / 16; q += PR_THREADS)
+    reinterpret_cast<uint4*>(Zs)[q] = reinterpret_cast<const uint4*>(P.zpub)[q];
+  __syncthreads();
+  if (s_skip) return;
+  if (warp == 4) {
+    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], 256;" ::"r"(su32(&s_tmem)));
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;");
+  }
+  asm volatile("tcgen05.fence::before_thread_sync;");
+  __syncthreads();
+  asm volatile("tcgen05.fence::after_thread_sync;");
+  const uint32_t tmem = s_tmem;
+  uint32_t issued = 0;  // the issuing thread: ring loads
+
+  if (warp < 4) {
+    // ---------------- row warps: one thread per row ----------------
+    const int rl = tid, i = ti * NB + rl;
+    const long long* acc0 = P.acc + acc_tile(ti, 2 * s, P.nt128) * ACC_TILE_ELEMS + acc_elem(rl, 0);
+    const long long* acc1 = P.acc + acc_tile(ti, 2 * s + 1, P.nt128) * ACC_TILE_ELEMS + acc_elem(rl, 0);
+    unsigned char* gdig = P.slices + (size_t)ti * NSLICE * SLICE_BYTES + (size_t)rl * 16;
+    const uint32_t trow = tmem + ((uint32_t)(warp * 32) << 16);
+    const bool two = P.nrhs > 1;
+    double r0 = 0.0, r1 = 0.0;  // sum_k L'_ik z_k
+    bool live = true;
+    auto wait = [&](uint64_t* bar, int parity) -> bool {
+      const int r = wait_or_stop(bar, (uint32_t)parity, &s_stop);
+      if (r == 2) s_abort = s_stop = 1;
+      live = r == 0;
+      return live;
+    };
+    long long T[PW];
+    auto load_piece = [&](int t) {
+      const long long* a = (t < 4 ? acc0 : acc1) + (size_t)(t & 3) * 2048;  // 16 columns: 2 groups of 8
+#pragma unroll
+      for (int c = 0; c < PW; ++c) T[c] = a[(c >> 3) * 1024 + (c & 7) * 32];
+    };
+    load_piece(0);
+#pragma unroll 1
+    for (int t = 0; t < NPIECE; ++t) {
+      if (t > 0) {
+        if (!wait(b_mma, (t - 1) & 1)) break;
+        asm volatile("tcgen05.fence::after_thread_sync;");
+        drain_couplings(T, trow + (uint32_t)((t & 1) * PN_TMEM_COLS));
+        asm volatile("tcgen05.fence::before_thread_sync;");
+      }
+#pragma unroll
+      for (int c = 0; c < PW; ++c) T[c] = to_unit60((unsigned long long)T[c]);
+      if (!wait(&b_blk[t & 1], (t >> 1) & 1)) break;
+      const PanelBlock& Lt = Ls[t & 1];
+      int Xh[PW], Xl[PW];
+#pragma unroll
+      for (int k = 0; k < PW; ++k) {
+        long long S = 0, M = 0;
+        mac_row<0>(S, M, Xh, Xl, Lt, k, k);
+        scale_entry(T[k] - S - (M >> 30), Lt.y[k].x, Lt.y[k].y, Lt.sh[k], Xh[k], Xl[k]);
+      }
+      if (t + 1 < NPIECE) load_piece(t + 1);
+      unsigned char* ad = As + rl * 16;
+      unsigned char* gd = gdig + (size_t)(2 * t) * 2048;
+#pragma unroll
+      for (int g = 0; g < 2; ++g) {
+        uint4 d[NSLICE];
+        digits8_packed(&Xh[g * 8], &Xl[g * 8], d);
+#pragma unroll
+        for (int q = 0; q < NSLICE; ++q) {
+          if (t + 1 < NPIECE) *reinterpret_cast<uint4*>(ad + g * 2048 + q * 4096) = d[q];
+          *reinterpret_cast<uint4*>(gd + (size_t)q * SLICE_BYTES + g * 2048) = d[q];
+        }
+      }
+      asm volatile("fence.proxy.async;" ::: "memory");  // digits visible to the MMAs and to the TMA reloads
+      __syncwarp();
+      if (lane == 0) mbar_arrive(b_digits);
+      // the right-hand sides: sum_k L'_ik z_k, z in 60-bit fixed point of the piece's scale
+      const PanelZ& Z = Zs[t];
+      long long S = 0, M = 0;
+#pragma unroll
+      for (int c = 0; c < PW; ++c) mac_entry(S, M, Xh[c], Xl[c], Z.x[0][c].x, Z.x[0][c].y);
+      r0 = fma(Z.scale[0], fixed62_to_double((S << 2) + (M >> 28)), r0);
+      if (two) {
+        S = M = 0;
+#pragma unroll
+        for (int c = 0; c < PW; ++c) mac_entry(S, M, Xh[c], Xl[c], Z.x[1][c].x, Z.x[1][c].y);
+        r1 = fma(Z.scale[1], fixed62_to_double((S << 2) + (M >> 28)), r1);
+      }
+    }
+    if (live) {
+      P.rhs[i] -= r0;
+      if (two) P.rhs[P.Nc + i] -= r1;
+    }
+  } else if (lane == 0) {
+    // ---------------- copies and MMA issue ----------------
+    const void* ma = P.tmap_a;
+    const void* mb = P.tmap_b16;
+    asm volatile("fence.proxy.tensormap::generic.acquire.gpu [%0], 128;" ::"l"(ma) : "memory");
+    asm volatile("fence.proxy.tensormap::generic.acquire.gpu [%0], 128;" ::"l"(mb) : "memory");
+    bool ok = true;
+    auto wait = [&](uint64_t* bar, uint32_t parity) -> bool {
+      if (ok) {
+        ok = false;
+        for (int it = 0; it < (1 << 22) && !ok && !*(volatile int*)&s_stop; ++it) ok = mbar_wait_n(bar, parity, 1);
+        if (!ok && !*(volatile int*)&s_stop) s_abort = 1;
+      }
+      return ok;
+    };
+    auto load_block = [&](int t) {
+      mbar_expect_tx(&b_blk[t & 1], PN_LBYTES);
+      bulk_g2s(Ls + (t & 1), P.lpub + t, PN_LBYTES, &b_blk[t & 1]);
+    };
+    // B operand: rows 16 t .. + 15 of the diagonal tile, chunk c
+    auto load_b = [&](unsigned char* dst, int t, int c, uint64_t* bar) {
+      tma_load_5d(dst, mb, (t & 1) * 128, t >> 1, 0, 2 * c, s, bar);
+    };
+    auto issue = [&](uint32_t acc, unsigned char* a, unsigned char* b, bool first) {
+      const uint64_t ad = smem_desc(su32(a), 2048, 128), bd = smem_desc(su32(b), NSLICE * PW * 16, 128);
+#pragma unroll
+      for (int q = 0; q < NSLICE; ++q)
+        mma_f16_desc(acc + (uint32_t)q * PW, ad + (uint64_t)((q * 4096) >> 4), bd,
+                     (1u << 4) | ((uint32_t)(PW * (NSLICE - q) >> 3) << 17) | ((128u >> 4) << 24),
+                     first && q == 0 ? 0u : 1u);
+    };
+    load_block(0);
+    load_block(1);
+    uint32_t g = 0;  // ring loads consumed
+#pragma unroll 1
+    for (int t = 1; t < NPIECE && ok; ++t) {  // the couplings of piece t
+      const uint32_t acc = tmem + (uint32_t)((t & 1) * PN_TMEM_COLS);
+      unsigned char* bo = Bs + (t & 1) * PN_BCHUNK;
+      const int older = t - 1;  // chunks 0 .. t - 2 through the ring, chunk t - 1 from As
+      // the digits of piece t - 2 were waited for: its couplings are drained,
+      // its accumulator and its B slot free
+      mbar_expect_tx(&b_own[t & 1], PN_BCHUNK);
+      load_b(bo, t, t - 1, &b_own[t & 1]);
+      auto load_older = [&](int c) {
+        const uint32_t st = issued & 1;
+        if (issued >= 2 && !wait(&empty[st], ((issued >> 1) & 1) ^ 1)) return;
+        unsigned char* dst = ring + st * PR_STAGE;
+        mbar_expect_tx(&full[st], PR_STAGE);
+        tma_load_5d(dst, ma, 0, 0, 2 * c, 0, ti, &full[st]);
+        load_b(dst + PN_ACHUNK, t, c, &full[st]);
+        ++issued;
+      };
+      if (older > 0) load_older(0);
+      if (older > 1) load_older(1);
+#pragma unroll 1
+      for (int c = 0; c < older && ok; ++c, ++g) {
+        const uint32_t st = g & 1;
+        if (!wait(&full[st], (g >> 1) & 1)) break;
+        asm volatile("tcgen05.fence::after_thread_sync;");
+        issue(acc, ring + st * PR_STAGE, ring + st * PR_STAGE + PN_ACHUNK, c == 0);
+        mma_commit(&empty[st]);
+        if (c + 2 < older) load_older(c + 2);
+      }
+      if (!wait(&b_own[t & 1], (uint32_t)((t - (t & 1 ? 1 : 2)) >> 1) & 1)) break;
+      if (!wait(b_digits, (uint32_t)(t - 1) & 1)) break;
+      asm volatile("tcgen05.fence::after_thread_sync;");
+      asm volatile("fence.proxy.async;" ::: "memory");
+      issue(acc, As, bo, older == 0);
+      mma_commit(b_mma);
+      if (t + 1 < NPIECE) load_block(t + 1);  // the rows are done with block t - 1
+    }
+    if (!ok) s_stop = 1;
+  }
+  __syncthreads();
+  if (s_stop) {
+    // a bounded wait gave up: the copies and MMAs this CTA issued finish
+    // (bounded waits) before it frees its TMEM and exits
+    if (warp == 4 && lane == 0) {
+      drain_ring(full, 2, issued);
+      drain_mmas(b_quiet);
+      for (int k = 0; k < 2; ++k) {
+        // either phase of these two-deep buffers may be the one in flight
+        mbar_wait_n(&b_blk[k], 0, 1 << 16);
+        mbar_wait_n(&b_blk[k], 1, 1 << 16);
+        mbar_wait_n(&b_own[k], 0, 1 << 16);
+        mbar_wait_n(&b_own[k], 1, 1 << 16);
+      }
+    }
+    if (tid == 0 && s_abort) atomicExch(&P.status[2], 1);
+    __syncthreads();
+  }
+  asm volatile("tcgen05.fence::after_thread_sync;");
+  if (warp == 4) {
+    __syncwarp();
+    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, 256;" ::"r"(tmem));
+  }
+}
+
+// ---------------------------------------------------------------------------
 // the factor the panels left in K (lower triangle, X = L' 2^60, its diagonal in
 // ldiag) as doubles, in place: only alpha and the adjoint read it, and on the
 // panels' chain the conversions cost 1.2k cycles a piece.  One CTA per 128 x 128
@@ -825,16 +1082,29 @@ cudaError_t launch_factor_doubles(const Prob* prob, int nt128, cudaStream_t s) {
 }
 
 // Rows per CTA: 128, or 64 or 32 while that still gives every tile an SM of
-// its own.  The FP64 pipe is per SM, so a lone problem's substitution runs up to
-// four times faster on four SMs; once the tiles outnumber the SMs, splitting
-// them only repeats the per-CTA work.
+// its own: a row tile's chain is shorter on four SMs than on one, and once the
+// tiles outnumber the SMs, splitting them only repeats the per-CTA work.  A
+// panel with at least as many row tiles as SMs is a throughput problem: its
+// diagonal tiles go first, alone, and the rows follow two tiles to an SM (not
+// where the factor is kept, which the latency kernel does).  With fewer, one
+// launch overlaps the rows with the pivots: all panels of 5 problems of N =
+// 4000 (155 row tiles, then fewer) 2.64 ms with the rule at 152, 3.01 with it
+// at 100, 2.67 in single launches; of 50 of N = 1000 (350, then fewer) 0.95,
+// 0.96 and 1.08, and 1.03 with it at 304.
 cudaError_t launch_panel(const Prob* probs, int step, const int* order, int ndiag, int total_tiles, int* counter,
-                         int* flags, int num_sms, cudaStream_t s) {
+                         int* flags, bool keep_l, int num_sms, cudaStream_t s, long long* nlaunch) {
   cudaError_t e = ensure_smem_attr((const void*)k_panel, SMEM_PANEL, PN_SMEM);
   if (e != cudaSuccess) return e;
   if (ndiag <= 0) return cudaSuccess;
-  int sh = 0;
   const int rest = total_tiles - ndiag;
+  if (!keep_l && rest >= num_sms) {
+    if ((e = ensure_smem_attr((const void*)k_panel_rows, SMEM_PANEL_ROWS, PR_SMEM)) != cudaSuccess) return e;
+    k_panel<<<ndiag, PN_THREADS, PN_SMEM, s>>>(probs, step, order, ndiag, 0, counter, flags);
+    k_panel_rows<<<rest, PR_THREADS, PR_SMEM, s>>>(probs, step, order + ndiag);
+    if (nlaunch) ++*nlaunch;
+    return cudaGetLastError();
+  }
+  int sh = 0;
   while (sh < 2 && ndiag + (rest << (sh + 1)) <= num_sms) ++sh;
   k_panel<<<ndiag + (rest << sh), PN_THREADS, PN_SMEM, s>>>(probs, step, order, ndiag, sh, counter, flags);
   return cudaGetLastError();
