@@ -385,13 +385,17 @@ int build_sched(const std::vector<int>& nt128, const std::vector<int>& tc_build,
   u.tile_off.assign(std::max(ntmax, 1), 0);
   for (int st = 0; st < ntmax; ++st) {
     u.tile_off[st] = tl.size();
+    auto tile = [&](int p, int ti, int tj) {
+      tl.push_back(((unsigned long long)p << 40) | ((unsigned long long)ti << 20) | (unsigned long long)tj);
+    };
+    for (int p = 0; p < nprob; ++p)
+      if (nt128[p] > st + 1)  // the next diagonal tile first
+        for (int half = 0; half < 2; ++half) tile(p, st + 1, 2 * (st + 1) + half);
     for (int p = 0; p < nprob; ++p) {
       const int m = nt128[p] - st - 1;
       for (int q = 0; q < m; ++q)
         for (int half = 0; half < 2; ++half)
-          for (int ti = st + 1 + q; ti < nt128[p]; ++ti)
-            tl.push_back(((unsigned long long)p << 40) | ((unsigned long long)ti << 20) |
-                         (unsigned long long)(2 * (st + 1) + 2 * q + half));
+          for (int ti = st + 1 + std::max(q, 1); ti < nt128[p]; ++ti) tile(p, ti, 2 * (st + 1) + 2 * q + half);
     }
     u.totals[st] = (int)(tl.size() - u.tile_off[st]);
   }
@@ -449,6 +453,13 @@ int build_sched(const std::vector<int>& nt128, const std::vector<int>& tc_build,
   return 0;
 }
 
+// Update tiles per SM (5.5 us each) from which the next diagonal tiles are
+// factored meanwhile: 20 problems of N = 2000 took 3.67 ms without, 3.30 with
+// it from 2 or 4 tiles, 3.36 from 12; 50 of N = 1000 1.88, 1.74 and 1.78.
+constexpr int LOOKAHEAD_TILES = 4;
+// and what a diagonal tile's factorisation takes, in such tiles
+constexpr int DIAG_TILES = 12;
+
 int mark(StageEvents* pe, int stage, cudaStream_t s, bool begin) {
   if (!pe || (pe->only >= 0 && stage != pe->only)) return 0;
   cudaEvent_t e;
@@ -470,10 +481,27 @@ int mark(StageEvents* pe, int stage, cudaStream_t s, bool begin) {
     ++n;                                       \
   } while (0)
 
+// A second stream of a capture, for the branch that overlaps the main one.
+struct SideStream {
+  cudaStream_t stream = nullptr;
+  cudaEvent_t fork = nullptr, join = nullptr;
+  cudaError_t create() {
+    cudaError_t e = cudaStreamCreateWithFlags(&stream, cudaStreamNonBlocking);
+    if (e == cudaSuccess) e = cudaEventCreateWithFlags(&fork, cudaEventDisableTiming);
+    if (e == cudaSuccess) e = cudaEventCreateWithFlags(&join, cudaEventDisableTiming);
+    return e;
+  }
+  ~SideStream() {
+    if (fork) cudaEventDestroy(fork);
+    if (join) cudaEventDestroy(join);
+    if (stream) cudaStreamDestroy(stream);
+  }
+};
+
 // Enqueue the whole evaluation: reset, build, sweep, epilogue.
 int enqueue_eval(const Prob* probs_d, int nprob, int max_nsteps, int max_nplanes, int* status_base,
                  size_t status_bytes, cudaStream_t s, long long* kernels, StageEvents* pe, int mode = 0,
-                 const UpdSched* us = nullptr) {
+                 const UpdSched* us = nullptr, const SideStream* side = nullptr) {
   long long n = 0;
   CK(cudaMemsetAsync(status_base, 0, status_bytes, s));
   if (mode == 1) {
@@ -484,13 +512,67 @@ int enqueue_eval(const Prob* probs_d, int nprob, int max_nsteps, int max_nplanes
     if (us->dot_builds > 0) STAGE(0, launch_build_dot(probs_d, nprob, max_nsteps, max_nplanes, s));
     if (us->build_total > 0)
       STAGE(0, launch_build_tc(probs_d, nprob, us->build_tiles_dev, us->build_total, us->num_sms, s));
+    // A panel with at least as many row tiles as SMs is a throughput problem:
+    // its diagonal tiles go first, alone, and the rows follow two tiles to an
+    // SM (not where the factor is kept, which the latency kernel does).  With
+    // fewer, one launch overlaps the rows with the pivots: all panels of 5
+    // problems of N = 4000 (155 row tiles, then fewer) 2.64 ms with the rule
+    // at 152, 3.01 with it at 100, 2.67 in single launches; of 50 of N = 1000
+    // (350, then fewer) 0.95, 0.96 and 1.08, and 1.03 with it at 304.
+    auto split = [&](int step) {
+      return !us->keep_l && us->row_totals[step] - us->diag_totals[step] >= us->num_sms;
+    };
+    bool diag_done = false;  // this step's diagonal tiles
     for (int step = 0; step < nt; ++step) {
-      STAGE(2, launch_panel(probs_d, step, us->pan_order_dev + us->pan_off[step], us->diag_totals[step],
-                            us->row_totals[step], us->sync_dev + us->flag_ints + step, us->sync_dev, us->keep_l,
-                            us->num_sms, s, &n));
-      if (step + 1 < nt)
-        STAGE(3, launch_ozaki_update(probs_d, nprob, step, nt, us->tiles_dev + us->tile_off[step],
-                                     us->totals[step], us->num_sms, s));
+      const int* order = us->pan_order_dev + us->pan_off[step];
+      const int ndiag = us->diag_totals[step], nrows = us->row_totals[step] - ndiag;
+      int* count = us->sync_dev + us->flag_ints + step;
+      if (diag_done || split(step)) {
+        if (!diag_done) STAGE(2, launch_panel(probs_d, step, order, ndiag, ndiag, count, us->sync_dev, us->num_sms, s));
+        STAGE(2, launch_panel_rows(probs_d, step, order + ndiag, nrows, s));
+      } else {
+        STAGE(2, launch_panel(probs_d, step, order, ndiag, ndiag + nrows, count, us->sync_dev, us->num_sms, s));
+      }
+      diag_done = false;
+      if (step + 1 >= nt) continue;
+      const unsigned long long* tiles = us->tiles_dev + us->tile_off[step];
+      int total = us->totals[step];
+      // The next diagonal tiles are a chain of ~65 us on a few SMs.  Where
+      // enough tiles are left to fill the others meanwhile, their updates go
+      // first; they are factored on a second stream while the rest of the
+      // update runs on the other SMs, and their SMs then take its last tiles.
+      // It costs a launch of a few us, and the next panel then runs split,
+      // which pays from half a row tile per SM (with the chain hidden, the
+      // rows alone are shorter than the one launch): 50 problems of N = 2000
+      // 6.98 -> 6.49 ms, 40 of N = 4000 27.7 -> 26.5 ms, 4 of N = 4000 4.9 ->
+      // 4.6 ms (4.9 with the split from a whole tile per SM, 4.6 from a third).
+      const int nd = us->diag_totals[step + 1], first = 2 * nd;
+      if ((pe || side) && !us->keep_l && nd < us->num_sms && 2 * (us->row_totals[step + 1] - nd) >= us->num_sms &&
+          total - first >= LOOKAHEAD_TILES * us->num_sms) {
+        STAGE(3, launch_ozaki_update(probs_d, nprob, step, nt, tiles, first, us->num_sms, s));
+        tiles += first;
+        total -= first;
+        // (profiled, the stages are timed one after the other)
+        cudaStream_t s2 = pe ? s : side->stream;
+        if (!pe) {
+          CK(cudaEventRecord(side->fork, s));
+          CK(cudaStreamWaitEvent(s2, side->fork, 0));
+        }
+        STAGE(2, launch_panel(probs_d, step + 1, us->pan_order_dev + us->pan_off[step + 1], nd, nd, count + 1,
+                              us->sync_dev, us->num_sms, s2));
+        // both ways finish together if the diagonal tiles' SMs take DIAG_TILES each fewer
+        const int others = pe ? us->num_sms : us->num_sms - nd;
+        const int late = pe ? 0 : std::max(0, (total - others * DIAG_TILES) / us->num_sms) * nd;
+        STAGE(3, launch_ozaki_update(probs_d, nprob, step, nt, tiles, total - late, others, s));
+        if (late) STAGE(3, launch_ozaki_update(probs_d, nprob, step, nt, tiles + total - late, late, nd, s2));
+        if (!pe) {
+          CK(cudaEventRecord(side->join, s2));
+          CK(cudaStreamWaitEvent(s, side->join, 0));
+        }
+        diag_done = true;
+      } else {
+        STAGE(3, launch_ozaki_update(probs_d, nprob, step, nt, tiles, total, us->num_sms, s));
+      }
     }
     STAGE(4, launch_finalize(probs_d, nprob, s));
     if (kernels) *kernels = n;
@@ -583,13 +665,15 @@ size_t plan_memory_budget() {
 // one graph.
 int capture_plan(fgpu_plan* p, cudaGraphExec_t* exec, long long* kernels, StageEvents* pe) {
   cudaStream_t s = p->stream;
+  SideStream side;  // needed for the capture only: the graph keeps no stream
+  CK(side.create());
   CK(cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal));
   int rc = 0;
   long long total = 0;
   for (PlanWave& w : p->waves) {
     long long n = 0;
     rc = enqueue_eval(p->probs_d + w.first, w.count, w.max_nsteps, w.max_nplanes, p->status_all + 4 * w.first,
-                      sizeof(int) * 4 * w.count, s, &n, pe, p->mode, p->mode == 1 ? &w.sched : nullptr);
+                      sizeof(int) * 4 * w.count, s, &n, pe, p->mode, p->mode == 1 ? &w.sched : nullptr, &side);
     if (rc) break;
     total += n;
   }
@@ -633,7 +717,7 @@ size_t layout_workspace(const fgpu_ctx* c, unsigned char* base, Workspace& ws, b
     take(ws.lpub, sizeof(PanelBlock) * 8);
     take(ws.zpub, sizeof(PanelZ) * 8);
     take(ws.acc, sizeof(long long) * acc_tiles(c->nt128) * ACC_TILE_ELEMS);
-    take(ws.slices, (size_t)c->nt128 * NSLICE * SLICE_BYTES);
+    take(ws.slices, (size_t)(c->nt128 + 1) * NSLICE * SLICE_BYTES);
     take(ws.splanes, sizeof(double) * (size_t)std::max(c->spec.nplanes, 1) * nc);
     take(ws.norms, sizeof(double) * (size_t)MAX_LEAF * nc);
     take(ws.dotc, sizeof(DotConst));

@@ -104,7 +104,8 @@ struct Prob {
   int nt128;                      // Nc / 128 (mode 1)
   int* kscale;                    // [0]: the scale e, K_ii < 2^2e for every i
   long long* acc;                 // lower-triangle 128 x 64 tiles: K, then its Schur complements, value A 2^(2e - 62)
-  unsigned char* slices;          // nt128 x 7 x 32 KB: fp16 digit planes of the current panel
+  unsigned char* slices;          // (nt128 + 1) x 7 x 32 KB: fp16 digit planes of the current panel; the last
+                                  // slot holds its diagonal tile's, which no update reads
   const void* tmap_a;             // TMA tensor map over slices, box 8 x 128 rows x 2 kgroups x 7 planes
   const void* tmap_b;             // same, box of 64 rows
   const void* tmap_bs;            // box of 64 rows landing as [k-group][plane][row]: the 7 planes stacked along N
@@ -190,12 +191,13 @@ constexpr size_t ACC_TILE_ELEMS = (size_t)NB * TB;
 // zeroed once per evaluation.
 constexpr int PANEL_FLAGS = 32;            // one 128-byte line per problem
 cudaError_t launch_panel(const Prob* probs, int step, const int* order, int ndiag, int total_tiles, int* counter,
-                         int* flags, bool keep_l, int num_sms, cudaStream_t s, long long* nlaunch);
+                         int* flags, int num_sms, cudaStream_t s);
+cudaError_t launch_panel_rows(const Prob* probs, int step, const int* order, int ntiles, cudaStream_t s);
 // prefix: device table of nprob + 1 tile offsets for this step (tiles of
 // problem p at step s: m (m + 1), m = nt128_p - s - 1); total_tiles = prefix[nprob].
 // tiles: the step's trailing tiles, packed (problem << 40 | row tile << 20 | column tile)
 cudaError_t launch_ozaki_update(const Prob* probs, int nprob, int step, int max_nt128,
-                                const unsigned long long* tiles, int total_tiles, int num_sms, cudaStream_t s);
+                                const unsigned long long* tiles, int total_tiles, int max_ctas, cudaStream_t s);
 // Preparation of an evaluation and the tensor-core kernel-matrix build
 // (build_tc.cu): weights, scale, right-hand sides, scaled features or feature
 // digits; then the persistent build of the lower triangle.

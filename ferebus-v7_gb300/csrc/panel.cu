@@ -331,7 +331,7 @@ __global__ void __launch_bounds__(PN_THREADS, 1)
     // the accumulators of this row, column 0 of the panel (tiles 2 s and 2 s + 1)
     const long long* acc0 = P.acc + acc_tile(ti, 2 * s, P.nt128) * ACC_TILE_ELEMS + acc_elem(rl, 0);
     const long long* acc1 = P.acc + acc_tile(ti, 2 * s + 1, P.nt128) * ACC_TILE_ELEMS + acc_elem(rl, 0);
-    unsigned char* gdig = P.slices + (size_t)ti * NSLICE * SLICE_BYTES + (size_t)rl * 16;
+    unsigned char* gdig = P.slices + (size_t)(diag ? P.nt128 : ti) * NSLICE * SLICE_BYTES + (size_t)rl * 16;
     long long wv[PW];
     auto load_piece = [&](int t) {
       const long long* a = (t < 4 ? acc0 : acc1) + (size_t)(t & 3) * 2048;  // 16 columns: 2 groups of 8
@@ -622,7 +622,7 @@ __global__ void __launch_bounds__(PN_THREADS, 1)
     };
     // the digits of rows 16 (t + 1) .. + 15 of the diagonal tile, chunk c
     auto load_chunk = [&](int t, int c) {
-      const unsigned char* src = P.slices + (size_t)s * NSLICE * SLICE_BYTES + (size_t)(t + 1) * PW * 16;
+      const unsigned char* src = P.slices + (size_t)P.nt128 * NSLICE * SLICE_BYTES + (size_t)(t + 1) * PW * 16;
       for (int q = lane; q < (int)PN_BCHUNK / 16; q += 32) {
         const int row = q & 15, pl = (q >> 4) % NSLICE, g = (q >> 4) / NSLICE;
         cp_async16(Bs + c * PN_BCHUNK + q * 16, src + (size_t)pl * SLICE_BYTES + (size_t)(2 * c + g) * 2048 + row * 16);
@@ -978,7 +978,7 @@ __global__ void __launch_bounds__(PR_THREADS, 2)
     };
     // B operand: rows 16 t .. + 15 of the diagonal tile, chunk c
     auto load_b = [&](unsigned char* dst, int t, int c, uint64_t* bar) {
-      tma_load_5d(dst, mb, (t & 1) * 128, t >> 1, 0, 2 * c, s, bar);
+      tma_load_5d(dst, mb, (t & 1) * 128, t >> 1, 0, 2 * c, P.nt128, bar);
     };
     auto issue = [&](uint32_t acc, unsigned char* a, unsigned char* b, bool first) {
       const uint64_t ad = smem_desc(su32(a), 2048, 128), bd = smem_desc(su32(b), NSLICE * PW * 16, 128);
@@ -1083,30 +1083,23 @@ cudaError_t launch_factor_doubles(const Prob* prob, int nt128, cudaStream_t s) {
 
 // Rows per CTA: 128, or 64 or 32 while that still gives every tile an SM of
 // its own: a row tile's chain is shorter on four SMs than on one, and once the
-// tiles outnumber the SMs, splitting them only repeats the per-CTA work.  A
-// panel with at least as many row tiles as SMs is a throughput problem: its
-// diagonal tiles go first, alone, and the rows follow two tiles to an SM (not
-// where the factor is kept, which the latency kernel does).  With fewer, one
-// launch overlaps the rows with the pivots: all panels of 5 problems of N =
-// 4000 (155 row tiles, then fewer) 2.64 ms with the rule at 152, 3.01 with it
-// at 100, 2.67 in single launches; of 50 of N = 1000 (350, then fewer) 0.95,
-// 0.96 and 1.08, and 1.03 with it at 304.
+// tiles outnumber the SMs, splitting them only repeats the per-CTA work.
 cudaError_t launch_panel(const Prob* probs, int step, const int* order, int ndiag, int total_tiles, int* counter,
-                         int* flags, bool keep_l, int num_sms, cudaStream_t s, long long* nlaunch) {
+                         int* flags, int num_sms, cudaStream_t s) {
   cudaError_t e = ensure_smem_attr((const void*)k_panel, SMEM_PANEL, PN_SMEM);
   if (e != cudaSuccess) return e;
   if (ndiag <= 0) return cudaSuccess;
   const int rest = total_tiles - ndiag;
-  if (!keep_l && rest >= num_sms) {
-    if ((e = ensure_smem_attr((const void*)k_panel_rows, SMEM_PANEL_ROWS, PR_SMEM)) != cudaSuccess) return e;
-    k_panel<<<ndiag, PN_THREADS, PN_SMEM, s>>>(probs, step, order, ndiag, 0, counter, flags);
-    k_panel_rows<<<rest, PR_THREADS, PR_SMEM, s>>>(probs, step, order + ndiag);
-    if (nlaunch) ++*nlaunch;
-    return cudaGetLastError();
-  }
   int sh = 0;
   while (sh < 2 && ndiag + (rest << (sh + 1)) <= num_sms) ++sh;
   k_panel<<<ndiag + (rest << sh), PN_THREADS, PN_SMEM, s>>>(probs, step, order, ndiag, sh, counter, flags);
+  return cudaGetLastError();
+}
+
+cudaError_t launch_panel_rows(const Prob* probs, int step, const int* order, int ntiles, cudaStream_t s) {
+  cudaError_t e = ensure_smem_attr((const void*)k_panel_rows, SMEM_PANEL_ROWS, PR_SMEM);
+  if (e != cudaSuccess || ntiles <= 0) return e;
+  k_panel_rows<<<ntiles, PR_THREADS, PR_SMEM, s>>>(probs, step, order);
   return cudaGetLastError();
 }
 

@@ -1,6 +1,7 @@
 """Batches whose panels have more row tiles than the GPU has SMs: their diagonal
-tiles go first and the rows follow two tiles to an SM.  The arithmetic is the one
-of the single launch, so every problem's value is bit-identical to its own lone
+tiles go first (beside the previous panel's update, where it has enough tiles) and
+the rows follow two tiles to an SM.  The arithmetic is the one of the single
+launch, so every problem's value is bit-identical to its own lone
 evaluation; the oracle's tolerance is the well conditioned cases' 1e-9 relative."""
 import numpy as np
 import pytest
