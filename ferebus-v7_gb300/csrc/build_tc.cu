@@ -67,14 +67,15 @@ __device__ __forceinline__ long long assemble_w(const int S[NLEV], int u) {
 // constants, one for the top five levels and one for the last three.
 constexpr long long BUILD_BIAS_H = (1LL << 22) * 0x0101010101LL + 0x4B000000LL * ((1LL << 24) + (1LL << 8) + 1);
 constexpr long long BUILD_BIAS_LO = (1LL << 22) * 0x010101LL + 0x4B000000LL * ((1LL << 8) + 1);
+// (the first of them once per row and pass: this is W + (BUILD_BIAS_H << (u - 48)), modulo 2^64)
 __device__ __forceinline__ long long assemble_w_bits(const uint32_t b[NLEV], int u) {
   const uint32_t p01 = b[0] * 256u + b[1];
   const uint32_t p23 = b[2] * 256u + b[3];
   const uint32_t p56 = b[5] * 256u + b[6];
-  const long long H = (long long)(((unsigned long long)p01 << 24) + ((unsigned long long)p23 << 8) + b[4]) -
-                      BUILD_BIAS_H;  // sum_{L<=4} S_L 256^(4-L)
-  const long long Lo = (long long)(((unsigned long long)p56 << 8) + b[7]) - BUILD_BIAS_LO;
-  return (long long)((unsigned long long)H << (u - 48)) + ((Lo + (1LL << (71 - u))) >> (72 - u));
+  // sum_{L<=4} S_L 256^(4-L) + BUILD_BIAS_H
+  const unsigned long long H = ((unsigned long long)p01 << 24) + ((unsigned long long)p23 << 8) + b[4];
+  const long long Lo = (long long)(((unsigned long long)p56 << 8) + b[7]);
+  return (long long)((H << (u - 48)) + (unsigned long long)((Lo + ((1LL << (71 - u)) - BUILD_BIAS_LO)) >> (72 - u)));
 }
 
 }  // namespace
@@ -488,10 +489,18 @@ __global__ void __launch_bounds__(BLD_THREADS, 1)
         // TMEM drained: the next pass's MMAs may start
         asm volatile("tcgen05.fence::before_thread_sync;");
         mbar_arrive(tempty);
-        const IexpScale esc = iexp_scale(2 * P.fscale[d] + 1 - u);
-        const long long wi = P.fnorm[(size_t)d * nc + i];
+        // the squared distances, in the leaf's unit
+        const long long wi = (long long)((unsigned long long)P.fnorm[(size_t)d * nc + i] +
+                                         (small ? (unsigned long long)BUILD_BIAS_H << (u - 47) : 0ULL));
         // W_jj of this thread's 16 columns (the same for the whole warp), two at a time
         const longlong2* wj2 = reinterpret_cast<const longlong2*>(P.fnorm + (size_t)d * nc + j0);
+#pragma unroll
+        for (int q = 0; q < 16; ++q) {
+          const longlong2 w2 = __ldg(wj2 + q / 2);
+          W[q] = (long long)((unsigned long long)wi + (unsigned long long)((q & 1) ? w2.y : w2.x) - 2 * (unsigned long long)W[q]);
+          if (W[q] < 0) W[q] = 0;
+        }
+        const IexpScale esc = iexp_scale(2 * P.fscale[d] + 1 - u);
         // The combination of the leaf values is chosen once per pass, outside
         // the entry loop: a ternary inside it is compiled into both sides,
         // and every FP64 operation costs this part's narrow FP64 pipe.
@@ -500,64 +509,57 @@ __global__ void __launch_bounds__(BLD_THREADS, 1)
         const int e2 = 2 * *P.kscale;
         bool nonfinite = false;
         // entries (i, j0 + q), in the accumulator layout; the lower triangle of
-        // the N x N block, identity padding (1/4 in the matrix's unit) beyond
+        // the N x N block, zeros beyond
         long long* A = P.acc + acc_tile(ti, tj, P.nt128) * ACC_TILE_ELEMS;
+        const int jmax = i < N ? i : -1;
         auto put = [&](int q, long long F) {
-          const int j = j0 + q;
-          if (j > i || i >= N || j >= N) F = i == j ? 1LL << 60 : 0LL;
-          A[acc_elem(r, h * 16 + q)] = F;
-        };
-        auto leaf = [&](int q) {
-          const longlong2 w2 = __ldg(wj2 + q / 2);
-          long long E = wi + ((q & 1) ? w2.y : w2.x) - 2 * W[q];
-          E = E < 0 ? 0 : E;
-          return iexp_fixed_parts((unsigned long long)E, esc, tab, fine);
-        };
-        auto leaf_double = [&](int q) {
-          const longlong2 w2 = __ldg(wj2 + q / 2);
-          long long E = wi + ((q & 1) ? w2.y : w2.x) - 2 * W[q];
-          E = E < 0 ? 0 : E;
-          return iexp_fixed_tab((unsigned long long)E, esc, tab, fine);
+          A[acc_elem(r, h * 16 + q)] = j0 + q <= jmax ? F : 0LL;
         };
         // one leaf, or a plain sum of two: fixed point throughout (K_ii >= 1,
-        // so e2 >= 2 unless the nugget is negative); any other expression
-        // combines in FP64
+        // so e2 >= 2 unless the nugget is negative); any other expression,
+        // and scales outside the exponential's common form, combine in FP64
         const bool sum = ca == 0.0 && cd == 0.0 && cb == 1.0 && (sp.ndot == 1 || cc == 1.0) && e2 >= 2;
         constexpr int tstash = BLD_EPI_WARPS * 32;
-        if (sum) {
+        auto fixed = [&](auto parts) {
           long long* st = reinterpret_cast<long long*>(stash) + tid;  // the first leaf's values, for the second pass
           if (d < sp.ndot - 1) {
 #pragma unroll
-            for (int q = 0; q < 16; ++q) st[q * tstash] = iexp_parts_fixed62(leaf(q), e2);
+            for (int q = 0; q < 16; ++q) st[q * tstash] = iexp_parts_fixed62(parts((unsigned long long)W[q]), e2);
           } else if (d == 0) {
 #pragma unroll
-            for (int q = 0; q < 16; ++q) put(q, iexp_parts_fixed62(leaf(q), e2));
+            for (int q = 0; q < 16; ++q) put(q, iexp_parts_fixed62(parts((unsigned long long)W[q]), e2));
           } else {
 #pragma unroll
-            for (int q = 0; q < 16; ++q) put(q, st[q * tstash] + iexp_parts_fixed62(leaf(q), e2));
+            for (int q = 0; q < 16; ++q) put(q, st[q * tstash] + iexp_parts_fixed62(parts((unsigned long long)W[q]), e2));
           }
+        };
+        if (sum && iexp_common(esc) && esc.F <= 64) {
+          fixed([&](unsigned long long E) { return iexp_common_parts<true>(E, esc, tab, fine); });
+        } else if (sum && iexp_common(esc)) {
+          fixed([&](unsigned long long E) { return iexp_common_parts<false>(E, esc, tab, fine); });
         } else {
+          auto leaf = [&](int q) { return iexp_fixed_tab((unsigned long long)W[q], esc, tab, fine); };
           double* st = stash + tid;
           if (d < sp.ndot - 1) {
 #pragma unroll
-            for (int q = 0; q < 16; ++q) st[q * tstash] = leaf_double(q);
+            for (int q = 0; q < 16; ++q) st[q * tstash] = leaf(q);
           } else if (d == 0) {
 #pragma unroll
-            for (int q = 0; q < 16; ++q) put(q, to_fixed62(fma(cb, leaf_double(q), ca), e2, &nonfinite));
+            for (int q = 0; q < 16; ++q) put(q, to_fixed62(fma(cb, leaf(q), ca), e2, &nonfinite));
           } else {
 #pragma unroll
             for (int q = 0; q < 16; ++q) {
               // second distance leaf: k = (d v0 + c) v1 + (b v0 + a)
               const double v0 = st[q * tstash];
-              put(q, to_fixed62(fma(fma(cd, v0, cc), leaf_double(q), fma(cb, v0, ca)), e2, &nonfinite));
+              put(q, to_fixed62(fma(fma(cd, v0, cc), leaf(q), fma(cb, v0, ca)), e2, &nonfinite));
             }
           }
         }
-        // the diagonal entry (every leaf 1), with the nugget
-        if (d == sp.ndot - 1 && i >= j0 && i < j0 + 16 && i < N) {
+        // the diagonal entry: every leaf 1, with the nugget; identity padding (1/4 in the matrix's unit) beyond N
+        if (d == sp.ndot - 1 && i >= j0 && i < j0 + 16) {
           const double noise = P.optimise_noise ? P.theta[sp.nkparams] : P.noise;
           const double kd = sp.ndot == 1 ? cb + ca : (cd + cc) + (cb + ca);
-          A[acc_elem(r, i - j0 + h * 16)] = diag_fixed62(kd, noise, e2, &nonfinite);
+          A[acc_elem(r, i - j0 + h * 16)] = i < N ? diag_fixed62(kd, noise, e2, &nonfinite) : 1LL << 60;
         }
         if (nonfinite) atomicOr(&P.status[3], 1);
       }

@@ -69,68 +69,75 @@ __device__ __forceinline__ double iexp_fixed(unsigned long long E, int e) {
 // exp(-E 2^e) for exact integers E >= 0 sharing one scale 2^e (the
 // kernel-matrix build's entries of one distance leaf), with the per-entry
 // work cut down:
-//  * y = E 2^e log2(e) is read off the 128-bit product E * C at a fixed
-//    binary point K0, C = log2(e) 2^63 rounded (relative error 2^-64, below
-//    2^-54 absolute in y for y < 1024): no per-entry normalisation;
-//  * the fraction g = m - y (64 bits) splits as j/1024 + k/2^20 + s with
-//    two 1024-entry tables the caller keeps in shared memory, 2^(j/1024)
-//    2^63 and (2^(k/2^20) - 1) 2^64, so t = s ln2 < 2^-20 ln2 and
-//    exp(t) = 1 + t + t^2/2 up to t^3/6 < 2^-64;
-//  * the small products (t^2, (2^(k/2^20) - 1) (exp(t) - 1)) are single
-//    32 x 32-bit multiplies; two 64 x 64-bit high products remain (s ln2
-//    and the final 2^(j/1024) factor);
-//  * one round-to-nearest into the double, subnormals included.
-// Error before the final rounding below 2^-60 relative (CPU model against
-// 60-digit arithmetic: never more than 1 ulp from the correctly rounded
-// value); measured on the GPU through fgpu_diag_exp_fixed.
+//  * x = E 2^e as it stands, 2^-64 its fraction's unit: only m, the number of
+//    halvings, needs log2(e), from 32 bits of x (13 fractional, rounded
+//    up so that m >= x log2(e)), and g = m ln2 - x, 0 < g < ln2 + 2^-12, is one
+//    64 x 32-bit product modulo 2^64 (ln2 rounded at 2^-64: m 2^-65 off);
+//  * the fraction splits as g = j/1024 + (k + 1/2)/2^20 + t, |t| <= 2^-21, with
+//    two 1024-entry tables the caller keeps in shared memory, exp(j/1024)
+//    2^62 and expm1((k + 1/2)/2^20) 2^64, and exp(t) = 1 + t + t^2/2 up to
+//    t^3/6 < 2^-65;
+//  * the small products are single 32 x 32-bit multiplies, and the final one,
+//    exp(j/1024) times a correction below 2^-10, three;
+//  * one round-to-nearest, subnormals included.
+// The integer pipe's wide multiplies bound the build (2.3 cycles each, a
+// 64 x 64-bit high product 26): against y = x log2(e) from a 64 x 128-bit product
+// and two high products, the form before, 40 problems of N = 4000 (two
+// leaves) build in 3.8 instead of 5.5 ms.  Error before the final
+// rounding below 2^-60 relative for x < 8 (at most 14 2^-64 on a CPU model
+// against 60-digit arithmetic, 15 in the form before), the rounding of m
+// ln2 beyond; measured on the GPU through fgpu_diag_exp_fixed.
 struct IexpScale {
-  int K0;  // binary point of y in E * IEXP_L2E64: y = (E C) 2^-K0
+  int F;  // fractional bits of x
 };
-__device__ __forceinline__ IexpScale iexp_scale(int e) { return IexpScale{63 - e}; }
+__device__ __forceinline__ IexpScale iexp_scale(int e) { return IexpScale{-e}; }
 
-// exp(-E 2^e) = Z 2^-62 2^-m, 2^62 <= Z <= 2^63 (m >= 1100: below every double)
+// exp(-E 2^e) = Z 2^-62 2^-m, 2^62 <= Z < 2^63 + 2^52 (m >= 1100: below every double)
 struct IexpParts {
   unsigned long long Z;
   int m;
 };
-__device__ __forceinline__ IexpParts iexp_fixed_parts(unsigned long long E, IexpScale sc,
-                                                      const unsigned long long* __restrict__ tab1024,
-                                                      const unsigned long long* __restrict__ fine1024) {
-  const int K0 = sc.K0;
-  if (E == 0 || K0 >= 192) return IexpParts{1ULL << 62, 0};  // 1, or y < 2^-64: rounds to 1
-  if (K0 < 64) {  // outside this form's range
-    const unsigned long long bits = (unsigned long long)__double_as_longlong(iexp_fixed(E, 63 - K0));
-    const int ef = (int)(bits >> 52);
-    if (ef == 0) return IexpParts{1ULL << 62, 1100};
-    return IexpParts{((bits & 0xFFFFFFFFFFFFFULL) | 0x10000000000000ULL) << 10, 1023 - ef};
-  }
-  const unsigned long long plo = E * IEXP_L2E64, phi = __umul64hi(E, IEXP_L2E64);
-  unsigned long long yi, yf;  // y = yi + yf 2^-64
-  if (K0 >= 128) {
-    yi = 0ULL;
-    yf = K0 == 128 ? phi : (phi >> (K0 - 128));
-  } else {
-    yi = phi >> (K0 - 64);
-    yf = K0 == 64 ? plo : ((plo >> (K0 - 64)) | (phi << (128 - K0)));
-  }
-  const int m = yi >= 1100 ? 1100 : (int)yi + (yf ? 1 : 0);
-  const unsigned long long f = 0ULL - yf;  // (m - y) 2^64
-  const int j = (int)(f >> 54);
-  const int k = (int)(f >> 44) & 1023;
-  const unsigned long long s = f & 0x00000FFFFFFFFFFFULL;
-  const unsigned long long t = __umul64hi(s << 20, IEXP_LN2) >> 20;  // t 2^64 < 2^43.5
-  const unsigned int th = (unsigned int)(t >> 12);
-  const unsigned long long eps = t + (((unsigned long long)th * th) >> 41);  // (exp(t) - 1) 2^64 < 2^44
-  const unsigned long long dk = fine1024[k];                                  // (2^(k/2^20) - 1) 2^64 < 2^53.5
-  const unsigned long long de = ((dk >> 22) * (eps >> 12)) >> 30;            // their product, 2^64
-  const unsigned long long p = (1ULL << 63) + ((dk + eps + de) >> 1);       // 2^(k/2^20) exp(t) 2^63
-  return IexpParts{__umul64hi(tab1024[j], p), m};                           // 2^(g) 2^62
+// x: 13 fractional bits in x13 (saturated), frac = x 2^64 modulo 2^64
+__device__ __forceinline__ IexpParts iexp_parts_core(unsigned x13, unsigned long long frac,
+                                                     const unsigned long long* __restrict__ tab1024,
+                                                     const unsigned long long* __restrict__ fine1024) {
+  const unsigned m = (__umulhi(x13, IEXP_L2E32) + 2u + (1u << 12)) >> 12;
+  const unsigned long long g = (unsigned long long)m * IEXP_LN2 - frac;
+  const unsigned gh = (unsigned)(g >> 32);
+  const unsigned long long dk = *reinterpret_cast<const unsigned long long*>(
+      reinterpret_cast<const char*>(fine1024) + ((gh >> 9) & (1023u << 3)));
+  const unsigned long long T =
+      *reinterpret_cast<const unsigned long long*>(reinterpret_cast<const char*>(tab1024) + ((gh >> 19) & ~7u));
+  const long long t = (long long)((g & 0x00000FFFFFFFFFFFULL) - (1ULL << 43));  // 2^64, |t| <= 2^43
+  const int th = (int)(t >> 12);
+  const long long eps = t + (((long long)th * th) >> 41);                                  // expm1(t) 2^64
+  const long long de = ((long long)(int)(unsigned)(dk >> 23) * (int)(eps >> 13)) >> 28;   // their product, 2^64
+  const unsigned long long d = dk + (unsigned long long)(eps + de);                        // 0 < d < 2^55
+  const unsigned Th = (unsigned)(T >> 32), Tl = (unsigned)T, dh = (unsigned)(d >> 32), dl = (unsigned)d;
+  const unsigned long long mid = (unsigned long long)Th * dl + (3ULL << 30) + (unsigned long long)Tl * dh;
+  return IexpParts{T + (unsigned long long)Th * dh + (mid >> 32), (int)m};  // exp(g) 2^62
 }
+// the scales of every ordinary leaf, uniform over a pass
+__device__ __forceinline__ bool iexp_common(IexpScale sc) { return sc.F >= 20 && sc.F < 128; }
+template <bool COARSE>  // F <= 64
+__device__ __forceinline__ IexpParts iexp_common_parts(unsigned long long E, IexpScale sc,
+                                                       const unsigned long long* __restrict__ tab1024,
+                                                       const unsigned long long* __restrict__ fine1024) {
+  // x below 2^19 (exp is 0 far before): the top word alone decides
+  const unsigned top = sc.F >= 45 ? ~0u : (1u << (sc.F - 13)) - 1u;
+  E = (unsigned long long)min((unsigned)(E >> 32), top) << 32 | (unsigned)E;
+  const unsigned long long frac = COARSE ? E << (64 - sc.F) : E >> (sc.F - 64);
+  return iexp_parts_core((unsigned)(E >> min(sc.F - 13, 63)), frac, tab1024, fine1024);
+}
+// the others (a call: inlined it would cost its callers registers)
+static __device__ __noinline__ double iexp_other(unsigned long long E, IexpScale sc) { return iexp_fixed(E, -sc.F); }
 
 __device__ __forceinline__ double iexp_fixed_tab(unsigned long long E, IexpScale sc,
                                                  const unsigned long long* __restrict__ tab1024,
                                                  const unsigned long long* __restrict__ fine1024) {
-  const IexpParts v = iexp_fixed_parts(E, sc, tab1024, fine1024);
+  if (!iexp_common(sc)) return iexp_other(E, sc);
+  const IexpParts v = sc.F <= 64 ? iexp_common_parts<true>(E, sc, tab1024, fine1024)
+                                 : iexp_common_parts<false>(E, sc, tab1024, fine1024);
   if (v.m >= 1100) return 0.0;
   const int top = (int)(v.Z >> 63);
   const int sh = 10 + top;
@@ -148,6 +155,7 @@ __device__ __forceinline__ double iexp_fixed_tab(unsigned long long E, IexpScale
 // round(exp(-E 2^e) 2^(62 - e2)), e2 >= 1: the value straight in the matrix's
 // fixed-point unit
 __device__ __forceinline__ long long iexp_parts_fixed62(IexpParts v, int e2) {
-  const int sh = v.m + e2;
-  return sh > 63 ? 0LL : (long long)((v.Z + (1ULL << ((sh - 1) & 63))) >> (sh & 63));
+  unsigned long long h;  // the shift gives 0 from 64 on
+  asm("shr.u64 %0, %1, %2;" : "=l"(h) : "l"(v.Z), "r"(v.m + e2 - 1));
+  return (long long)((h + 1) >> 1);
 }
