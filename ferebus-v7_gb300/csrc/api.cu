@@ -151,6 +151,8 @@ void plan_tc_build(Spec& sp) {
     sp.ndot++;
   }
   sp.tc_build = sp.ndot > 0 ? 1 : 0;
+  for (int k = 0; k < sp.npost; ++k)
+    if (sp.ndot == 2 && sp.post[k] == P_PROD) sp.tc_build = 2;
 }
 
 // Per-step tile tables of the persistent tensor-core update: for step s,
@@ -164,6 +166,7 @@ struct UpdSched {
   int num_sms = 0;
   unsigned long long* build_tiles_dev = nullptr;  // tiles of the tensor-core build, packed like `tiles_dev`
   int build_total = 0;
+  bool products = false;  // some of them may be of products of two leaves
   std::vector<int> row_totals;      // per step: 128-row tiles ti >= step over all problems
   int* pan_order_dev = nullptr;     // per step: (problem << 16 | ti) of its row tiles, own row tiles first
   std::vector<size_t> pan_off;      // offset of each step's order
@@ -439,6 +442,7 @@ int build_sched(const std::vector<int>& nt128, const std::vector<int>& tc_build,
       u.dot_builds++;
       continue;
     }
+    u.products |= tc_build[p] == 2;
     for (int q = 0; q < nt128[p]; ++q)
       for (int half = 0; half < 2; ++half)
         for (int ti = q; ti < nt128[p]; ++ti)
@@ -511,7 +515,7 @@ int enqueue_eval(const Prob* probs_d, int nprob, int max_nsteps, int max_nplanes
     STAGE(0, launch_prep(probs_d, nprob, nt, s));
     if (us->dot_builds > 0) STAGE(0, launch_build_dot(probs_d, nprob, max_nsteps, max_nplanes, s));
     if (us->build_total > 0)
-      STAGE(0, launch_build_tc(probs_d, nprob, us->build_tiles_dev, us->build_total, us->num_sms, s));
+      STAGE(0, launch_build_tc(probs_d, nprob, us->build_tiles_dev, us->build_total, us->products, us->num_sms, s));
     // A panel with at least as many row tiles as SMs is a throughput problem:
     // its diagonal tiles go first, alone, and the rows follow two tiles to an
     // SM (not where the factor is kept, which the latency kernel does).  With
@@ -723,7 +727,7 @@ size_t layout_workspace(const fgpu_ctx* c, unsigned char* base, Workspace& ws, b
     take(ws.dotc, sizeof(DotConst));
     take(ws.fnorm, sizeof(long long) * 2 * nc);
     take(ws.fcoef, sizeof(double) * 4);
-    take(ws.fscale, sizeof(int) * 2);
+    take(ws.fscale, sizeof(int) * 3);
   }
   return (off + 255) / 256 * 256;
 }

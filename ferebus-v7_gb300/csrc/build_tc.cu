@@ -36,8 +36,8 @@
 // integer work is what bounds the kernel, so it gets the warps); one pass per
 // distance leaf per 128 x 64 tile, the first leaf's values kept in shared
 // memory for the second pass.  FP64 instructions run at 2 lanes per cycle
-// per SM on this part (FP32: 128), so the entry loop holds none but the one
-// add of a two-leaf sum: the combination is chosen once per pass, and the
+// per SM on this part (FP32: 128), so one leaf, a sum of two and a product of
+// two combine in fixed point (k_prep decides which, once per problem), and the
 // nugget goes onto the one diagonal entry afterwards.
 #include "../../include/fgpu.h"
 #include "fgpu_internal.h"
@@ -51,6 +51,7 @@ namespace fgpu {
 namespace {
 
 constexpr int NLEV = 8;  // digit-pair levels p + q = 0..7
+enum Form { FORM_FP64 = 0, FORM_SUM = 1, FORM_PROD = 2 };  // how the leaves' values combine (Prob::fscale[2])
 
 // W = round(sum_L S_L 2^(u - 16 - 8L)) from the 8 exact level sums (48 <= u <= 63)
 __device__ __forceinline__ long long assemble_w(const int S[NLEV], int u) {
@@ -100,6 +101,7 @@ __global__ void __launch_bounds__(128) k_prep(const Prob* __restrict__ probs) {
   const int tid = threadIdx.x, i = rb * NB + tid;
   const size_t nc = (size_t)P.Nc;
   __shared__ double w[MAX_PARAMS];  // rbf, rbf-cyclic sqrt(exp(theta)), periodic 1 / exp(theta), linear 1 / c, constant theta
+  int form = FORM_FP64;  // thread 0
   __shared__ int s_e[2], s_k, s_c[MAX_LEAF];
   __shared__ bool s_huge[MAX_LEAF];
   for (int q = tid; q < sp.nkparams; q += 128) {
@@ -204,8 +206,13 @@ __global__ void __launch_bounds__(128) k_prep(const Prob* __restrict__ probs) {
         }
       }
     }
+    const double* c = stk[0];
     if (rb == 0 && sp.tc_build)
-      for (int q = 0; q < 4; ++q) P.fcoef[q] = stk[0][q];
+      for (int q = 0; q < 4; ++q) P.fcoef[q] = c[q];
+    form = c[0] != 0.0                                                             ? FORM_FP64
+           : c[3] == 0.0 && c[1] == 1.0 && (sp.ndot == 1 || c[2] == 1.0)           ? FORM_SUM
+           : sp.ndot == 2 && c[1] == 0.0 && c[2] == 0.0 && c[3] == 1.0             ? FORM_PROD
+                                                                                   : FORM_FP64;
     // the scale 2^e > sqrt(K_ii): the kernels are stationary, so K_ii is one
     // value, the expression with every distance leaf at 1, plus the nugget
     const double d = (sp.tc_build ? (stk[0][3] + stk[0][2]) + (stk[0][1] + stk[0][0]) : stk[0][0]) +
@@ -216,6 +223,13 @@ __global__ void __launch_bounds__(128) k_prep(const Prob* __restrict__ probs) {
     if (rb == 0) P.kscale[0] = e;
   }
   __syncthreads();
+  if (rb == 0 && tid == 0 && sp.tc_build) {
+    // fixed point throughout (K_ii >= 1, so e >= 1 unless the nugget is
+    // negative), with scales in the exponential's common form
+    bool fixed = s_k >= 1;
+    for (int l = 0; l < sp.ndot; ++l) fixed &= iexp_common(iexp_scale(2 * s_e[l] + 1 - sp.dot_u[l]));
+    P.fscale[2] = fixed ? form : FORM_FP64;
+  }
   {
     // right-hand sides: y - mu (marginal), or y and 1 (concentrated), in the factor's scale; zero on the padding
     const double u = ldexp(1.0, -s_k);
@@ -311,6 +325,11 @@ constexpr uint32_t BLD_STASH = BLD_TAB + 2 * 1024 * 8;  // the first leaf's 16 v
 constexpr uint32_t BLD_SMEM = BLD_STASH + BLD_EPI_WARPS * 32 * 16 * 8;
 static_assert(BLD_SMEM <= 227 * 1024, "shared memory per CTA");
 
+// PROD: with the fixed-point product of two leaves.  Its own instance, because
+// the loops it adds cost the others up to 18% (40 problems of N = 4000, a sum of
+// two: 3.8 -> 4.5 ms, the compiler's schedule).  Against the FP64
+// combination, the product's build: 7.5 -> 4.1 ms.
+template <bool PROD>
 __global__ void __launch_bounds__(BLD_THREADS, 1)
     k_build_tc(const Prob* __restrict__ probs, int nprob, const unsigned long long* __restrict__ tiles, int total) {
   extern __shared__ __align__(1024) unsigned char smb[];
@@ -442,6 +461,7 @@ __global__ void __launch_bounds__(BLD_THREADS, 1)
       const size_t nc = (size_t)P.Nc;
       const int i = ti * NB + r;
       const int j0 = tj * TB + h * 16;
+      const int form = P.fscale[2];
       bool stop = false;
       for (int d = 0; d < sp.ndot; ++d, ++it) {
         if (!mbar_wait(tfull, it & 1)) {
@@ -501,10 +521,6 @@ __global__ void __launch_bounds__(BLD_THREADS, 1)
           if (W[q] < 0) W[q] = 0;
         }
         const IexpScale esc = iexp_scale(2 * P.fscale[d] + 1 - u);
-        // The combination of the leaf values is chosen once per pass, outside
-        // the entry loop: a ternary inside it is compiled into both sides,
-        // and every FP64 operation costs this part's narrow FP64 pipe.
-        const double ca = P.fcoef[0], cb = P.fcoef[1], cc = P.fcoef[2], cd = P.fcoef[3];
         const int N = P.N;
         const int e2 = 2 * *P.kscale;
         bool nonfinite = false;
@@ -515,29 +531,39 @@ __global__ void __launch_bounds__(BLD_THREADS, 1)
         auto put = [&](int q, long long F) {
           A[acc_elem(r, h * 16 + q)] = j0 + q <= jmax ? F : 0LL;
         };
-        // one leaf, or a plain sum of two: fixed point throughout (K_ii >= 1,
-        // so e2 >= 2 unless the nugget is negative); any other expression,
-        // and scales outside the exponential's common form, combine in FP64
-        const bool sum = ca == 0.0 && cd == 0.0 && cb == 1.0 && (sp.ndot == 1 || cc == 1.0) && e2 >= 2;
+        // One leaf, a plain sum of two or a plain product of two: fixed point
+        // throughout.  Any other expression, and scales outside the
+        // exponential's common form, combine in FP64, 64 cycles an operation
+        // and warp.
+        const bool sum = form == FORM_SUM, prod = PROD && form == FORM_PROD;
         constexpr int tstash = BLD_EPI_WARPS * 32;
         auto fixed = [&](auto parts) {
           long long* st = reinterpret_cast<long long*>(stash) + tid;  // the first leaf's values, for the second pass
           if (d < sp.ndot - 1) {
+            const int unit = PROD && prod ? 0 : e2;  // a product's first factor: v0 2^62
 #pragma unroll
-            for (int q = 0; q < 16; ++q) st[q * tstash] = iexp_parts_fixed62(parts((unsigned long long)W[q]), e2);
+            for (int q = 0; q < 16; ++q) st[q * tstash] = iexp_parts_fixed62(parts((unsigned long long)W[q]), unit);
           } else if (d == 0) {
 #pragma unroll
             for (int q = 0; q < 16; ++q) put(q, iexp_parts_fixed62(parts((unsigned long long)W[q]), e2));
+          } else if (PROD && prod) {
+#pragma unroll
+            for (int q = 0; q < 16; ++q) {
+              IexpParts v = parts((unsigned long long)W[q]);
+              v.Z = __umul64hi((unsigned long long)st[q * tstash], v.Z);  // v0 v1 2^(60 + m)
+              put(q, iexp_parts_fixed62(v, e2 - 2));
+            }
           } else {
 #pragma unroll
             for (int q = 0; q < 16; ++q) put(q, st[q * tstash] + iexp_parts_fixed62(parts((unsigned long long)W[q]), e2));
           }
         };
-        if (sum && iexp_common(esc) && esc.F <= 64) {
+        if ((sum || prod) && iexp_common(esc) && esc.F <= 64) {
           fixed([&](unsigned long long E) { return iexp_common_parts<true>(E, esc, tab, fine); });
-        } else if (sum && iexp_common(esc)) {
+        } else if ((sum || prod) && iexp_common(esc)) {
           fixed([&](unsigned long long E) { return iexp_common_parts<false>(E, esc, tab, fine); });
         } else {
+          const double ca = P.fcoef[0], cb = P.fcoef[1], cc = P.fcoef[2], cd = P.fcoef[3];
           auto leaf = [&](int q) { return iexp_fixed_tab((unsigned long long)W[q], esc, tab, fine); };
           double* st = stash + tid;
           if (d < sp.ndot - 1) {
@@ -558,6 +584,7 @@ __global__ void __launch_bounds__(BLD_THREADS, 1)
         // the diagonal entry: every leaf 1, with the nugget; identity padding (1/4 in the matrix's unit) beyond N
         if (d == sp.ndot - 1 && i >= j0 && i < j0 + 16) {
           const double noise = P.optimise_noise ? P.theta[sp.nkparams] : P.noise;
+          const double ca = P.fcoef[0], cb = P.fcoef[1], cc = P.fcoef[2], cd = P.fcoef[3];
           const double kd = sp.ndot == 1 ? cb + ca : (cd + cc) + (cb + ca);
           A[acc_elem(r, i - j0 + h * 16)] = i < N ? diag_fixed62(kd, noise, e2, &nonfinite) : 1LL << 60;
         }
@@ -589,12 +616,13 @@ cudaError_t launch_prep(const Prob* probs, int nprob, int max_nt128, cudaStream_
 }
 
 cudaError_t launch_build_tc(const Prob* probs, int nprob, const unsigned long long* tiles, int total_tiles,
-                            int num_sms, cudaStream_t s) {
-  cudaError_t e = ensure_smem_attr((const void*)k_build_tc, SMEM_BUILD_TC, BLD_SMEM);
+                            bool products, int num_sms, cudaStream_t s) {
+  auto kernel = products ? k_build_tc<true> : k_build_tc<false>;
+  cudaError_t e = ensure_smem_attr((const void*)kernel, products ? SMEM_BUILD_TC_PROD : SMEM_BUILD_TC, BLD_SMEM);
   if (e != cudaSuccess) return e;
   if (total_tiles <= 0) return cudaSuccess;
   const int grid = total_tiles < num_sms ? total_tiles : num_sms;
-  k_build_tc<<<grid, BLD_THREADS, BLD_SMEM, s>>>(probs, nprob, tiles, total_tiles);
+  kernel<<<grid, BLD_THREADS, BLD_SMEM, s>>>(probs, nprob, tiles, total_tiles);
   return cudaGetLastError();
 }
 

@@ -51,7 +51,7 @@ struct Spec {
   uint8_t cyclic[MAX_PLANES];     // rbf-cyclic: plane's feature index is 3, 6, 9, ... (1-based)
   // tensor-core build (tensor-core mode; leaves rbf / periodic / linear /
   // constant, at most 2 rbf or periodic "distance" leaves, <= 128 digit columns)
-  int tc_build;
+  int tc_build;                   // 0 no, 1 yes, 2 yes and two leaves may be multiplied
   int ndot;                       // distance leaves
   int dot_leaf[2];                // their leaf indices
   int dot_koff[2];                // first digit column (multiple of 16)
@@ -133,7 +133,7 @@ struct Prob {
   const double* plane_max;        // nplanes: max_i |planes[p][i]|
   long long* fnorm;               // 2 x Nc: W_ii of the distance leaves
   double* fcoef;                  // 4: k = a + b v0 + c v1 + d v0 v1
-  int* fscale;                    // 2: s of the distance leaves, max |f| < 2^s
+  int* fscale;                    // 2: s of the distance leaves, max |f| < 2^s; how their values combine
 };
 
 // Encode the four 5-D TMA tensor maps of a problem's digit-plane buffer
@@ -205,7 +205,7 @@ cudaError_t launch_ozaki_update(const Prob* probs, int nprob, int step, int max_
 // packed (problem << 40 | row tile << 20 | column tile).
 cudaError_t launch_prep(const Prob* probs, int nprob, int max_nt128, cudaStream_t s);
 cudaError_t launch_build_tc(const Prob* probs, int nprob, const unsigned long long* tiles, int total_tiles,
-                            int num_sms, cudaStream_t s);
+                            bool products, int num_sms, cudaStream_t s);
 
 // K^-1 of a tensor-core context's factor (inv.cu).  A split task turns a
 // 128 x 128 operand tile into digit planes: kind 0 rows of L', 1 rows of V, 2
@@ -264,7 +264,7 @@ cudaError_t enqueue_grad_fast(const Prob* p, const Prob* eval, int nsteps, int n
 // beyond the first 64 set it on every call.
 enum SmemSlot {
   SMEM_BUILD, SMEM_BUILD_DOT, SMEM_UPDATE, SMEM_SYRK, SMEM_OZAKI_UPDATE, SMEM_PANEL, SMEM_PANEL_ROWS,
-  SMEM_BUILD_TC, SMEM_INV_GEMM, SMEM_GRAD_FAST, SMEM_NSLOTS
+  SMEM_BUILD_TC, SMEM_BUILD_TC_PROD, SMEM_INV_GEMM, SMEM_GRAD_FAST, SMEM_NSLOTS
 };
 cudaError_t ensure_smem_attr(const void* func, int slot, int bytes);
 
