@@ -121,31 +121,36 @@ __global__ void __launch_bounds__(256) k_inv_diag128(const Prob* __restrict__ pp
 }
 
 // sums of squares of the diagonal tiles: per row over groups of 16 columns, per
-// column over groups of 32 rows.  grid nt128 x 128 threads
+// column over groups of 32 rows.  grid (nt128, 8) x 128 threads, 16 columns each
+// (all 128 in one CTA: a chain of 26 us)
 __global__ void __launch_bounds__(128) k_inv_diag_norms(const Prob* __restrict__ pp, const double* __restrict__ V,
                                                         float* __restrict__ rowpart, float* __restrict__ colpart) {
   const Prob& P = *pp;
   if (P.status[1]) return;
-  const int t = blockIdx.x, s0 = t * NB, r = threadIdx.x;
+  const int t = blockIdx.x, g = blockIdx.y, s0 = t * NB, r = threadIdx.x;
   const size_t nc = (size_t)P.Nc;
-  for (int g = 0; g < 8; ++g) {
-    float s = 0.0f;
-    for (int q = 0; q < 16; ++q) {
-      const float x = (float)V[(size_t)(s0 + g * 16 + q) * nc + s0 + r];
-      s = fmaf(x, x, s);
-      float y = x * x;
-      for (int o = 16; o > 0; o >>= 1) y += __shfl_down_sync(0xffffffffu, y, o);
-      if ((r & 31) == 0) colpart[(size_t)(t * 4 + (r >> 5)) * nc + s0 + g * 16 + q] = y;
-    }
-    rowpart[(size_t)(t * 8 + g) * nc + s0 + r] = s;
+  float s = 0.0f;
+#pragma unroll
+  for (int q = 0; q < 16; ++q) {
+    const float x = (float)V[(size_t)(s0 + g * 16 + q) * nc + s0 + r];
+    s = fmaf(x, x, s);
+    float y = x * x;
+    for (int o = 16; o > 0; o >>= 1) y += __shfl_down_sync(0xffffffffu, y, o);
+    if ((r & 31) == 0) colpart[(size_t)(t * 4 + (r >> 5)) * nc + s0 + g * 16 + q] = y;
   }
+  rowpart[(size_t)(t * 8 + g) * nc + s0 + r] = s;
 }
 
 // ---------------------------------------------------------------------------
-// digit planes of one 128 x 128 operand tile: one thread per operand row.
+// digit planes of one 128 x 128 operand tile: four threads per operand row and
+// two CTAs per tile, two groups of 8 entries each.  A row's norm is summed by
+// its four threads.  A level has fewer tiles than the GPU has SMs at N = 1000,
+// and its chain per thread is what it costs: with one thread per row, 51 us a
+// level at N = 1003 and 56 at N = 4000, now 13 and 23.
 // kind 0: rows of L' (norms below 1); 1: rows of V; 2: columns of V; 3: columns of P
+// grid (tasks, 2) x (128, 4) threads
 // ---------------------------------------------------------------------------
-__global__ void __launch_bounds__(128)
+__global__ void __launch_bounds__(512)
     k_inv_split(const Prob* __restrict__ pp, const InvSplit* __restrict__ tasks, const double* __restrict__ V,
                 const double* __restrict__ Pm, const float* __restrict__ rowpart, const float* __restrict__ colpart,
                 const float* __restrict__ colpart_p, int* __restrict__ exps, unsigned char* __restrict__ dr,
@@ -157,22 +162,26 @@ __global__ void __launch_bounds__(128)
   const size_t nc = (size_t)P.Nc;
   bool bad = false;
   int e = 0;
-  if (T.kind > 0) {
+  if (T.kind > 0) {  // block-uniform
+    __shared__ float sum[4][NB];
     const float* part = T.kind == 1 ? rowpart : (T.kind == 2 ? colpart : colpart_p);
     float s = 0.0f;
 #pragma unroll 8
-    for (int g = T.g0; g < T.g1; ++g) s += part[(size_t)g * nc + i];
-    e = norm_exponent(s, &bad);
+    for (int g = T.g0 + threadIdx.y; g < T.g1; g += 4) s += part[(size_t)g * nc + i];
+    sum[threadIdx.y][r] = s;
+    __syncthreads();
+    e = norm_exponent((sum[0][r] + sum[1][r]) + (sum[2][r] + sum[3][r]), &bad);
   }
-  exps[(size_t)T.kind * nc + i] = e;
+  if (blockIdx.y == 0 && threadIdx.y == 0) exps[(size_t)T.kind * nc + i] = e;
   const int es = T.kind == 0 ? *P.kscale : e;
   const bool rows = T.kind <= 1;
   const double* src = T.kind == 0 ? P.K : (T.kind == 3 ? Pm : V);
   const size_t ld = T.kind == 0 ? (size_t)P.ld : nc;
   const int k0 = T.k * NB;
   unsigned char* dst = (T.kind <= 1 ? dr : dc) + (size_t)T.slot * NSLICE * SLICE_BYTES + (size_t)r * 16;
-#pragma unroll 2
-  for (int kg = 0; kg < 16; ++kg) {
+  const int kg0 = (blockIdx.y * 4 + threadIdx.y) * 2;
+#pragma unroll
+  for (int kg = kg0; kg < kg0 + 2; ++kg) {
     long long F[8];
     if (rows) {
 #pragma unroll
@@ -462,10 +471,10 @@ cudaError_t enqueue_inverse(const Prob* p, int nt128, const InvWorkspace& w, con
   long long n = 0;
   k_inv_diag32<<<nt128 * 4, 32, 0, s>>>(p, w.V);
   k_inv_diag128<<<dim3(16, nt128), 256, 0, s>>>(p, w.V);
-  k_inv_diag_norms<<<nt128, 128, 0, s>>>(p, w.V, w.rowpart, w.colpart);
+  k_inv_diag_norms<<<dim3(nt128, 8), 128, 0, s>>>(p, w.V, w.rowpart, w.colpart);
   n += 3;
   auto split = [&](int first, int count) {
-    k_inv_split<<<count, 128, 0, s>>>(p, w.splits + first, w.V, w.kinv, w.rowpart, w.colpart, w.colpart_p, w.exps, w.dr,
+    k_inv_split<<<dim3(count, 2), dim3(NB, 4), 0, s>>>(p, w.splits + first, w.V, w.kinv, w.rowpart, w.colpart, w.colpart_p, w.exps, w.dr,
                                       w.dc);
     ++n;
   };

@@ -1067,9 +1067,9 @@ __global__ void __launch_bounds__(256) k_factor_doubles(const Prob* __restrict__
   if (ti < tj || P.status[1]) return;
   const size_t ld = (size_t)P.ld;
   const int kexp = *P.kscale, i = ti * NB + (threadIdx.x & 127);
-#pragma unroll 8
-  for (int c = threadIdx.x >> 7; c < NB; c += 2) {
-    const int j = tj * NB + c;
+#pragma unroll
+  for (int c = 0; c < 8; ++c) {
+    const int j = tj * NB + blockIdx.z * 16 + (threadIdx.x >> 7) * 8 + c;
     double* k = P.K + (size_t)j * ld + i;
     const double x = fixed62_to_double(__double_as_longlong(*k) * 4, kexp);
     *k = i > j ? x : (i == j ? P.ldiag[i] : 0.0);
@@ -1077,7 +1077,7 @@ __global__ void __launch_bounds__(256) k_factor_doubles(const Prob* __restrict__
 }
 
 cudaError_t launch_factor_doubles(const Prob* prob, int nt128, cudaStream_t s) {
-  k_factor_doubles<<<dim3(nt128, nt128), 256, 0, s>>>(prob);
+  k_factor_doubles<<<dim3(nt128, nt128, NB / 16), 256, 0, s>>>(prob);
   return cudaGetLastError();
 }
 
