@@ -85,7 +85,10 @@ __device__ __forceinline__ long long assemble_w_bits(const uint32_t b[NLEV], int
 // preparation of an evaluation, one CTA per 128 points: the features' weights,
 // the problem's scale, the right-hand sides, the scaled features and, for the
 // tensor-core build, their digit planes and exact self products.
-// grid (nt128, nprob) x 128 threads
+// grid (nt128, nprob) x (128, PREP_Y) threads: the digits of a point's groups of 8
+// features, and the right-hand sides, side by side (one thread per point: 20
+// us for a lone problem of 500 points and 12 features, now 14; 31 with 24
+// features, now 17)
 //
 // An exponential is ~50 FP64 instructions of 64 cycles each on this GPU, so each
 // weight is formed once per CTA, a thread per parameter, and not by every
@@ -93,18 +96,20 @@ __device__ __forceinline__ long long assemble_w_bits(const uint32_t b[NLEV], int
 // feature, and a serial one per leaf: 13 + 26 us for a lone problem of 500
 // points, 29 + 57 us at N = 4000).
 // ---------------------------------------------------------------------------
-__global__ void __launch_bounds__(128) k_prep(const Prob* __restrict__ probs) {
+constexpr int PREP_Y = 4;
+__global__ void __launch_bounds__(NB * PREP_Y) k_prep(const Prob* __restrict__ probs) {
   const Prob& P = probs[blockIdx.y];
   const int rb = blockIdx.x;
   if (P.mode != 1 || rb >= P.nt128) return;
   const Spec& sp = *P.spec;
-  const int tid = threadIdx.x, i = rb * NB + tid;
+  const int tid = threadIdx.x, y = threadIdx.y, i = rb * NB + tid;
   const size_t nc = (size_t)P.Nc;
   __shared__ double w[MAX_PARAMS];  // rbf, rbf-cyclic sqrt(exp(theta)), periodic 1 / exp(theta), linear 1 / c, constant theta
   int form = FORM_FP64;  // thread 0
   __shared__ int s_e[2], s_k, s_c[MAX_LEAF];
   __shared__ bool s_huge[MAX_LEAF];
-  for (int q = tid; q < sp.nkparams; q += 128) {
+  __shared__ int s_lev[2][PREP_Y][NLEV][NB];
+  for (int q = y * NB + tid; q < sp.nkparams; q += NB * PREP_Y) {
     int type = L_CONSTANT;
     for (int l = 0; l < sp.nleaf; ++l) {
       const int cnt = sp.leaf[l].type == L_CONSTANT ? 1 : sp.leaf[l].n;
@@ -120,7 +125,8 @@ __global__ void __launch_bounds__(128) k_prep(const Prob* __restrict__ probs) {
     }
   }
   __syncthreads();
-  if (tid >= 64) {
+  if (y > 0) {
+  } else if (tid >= 64) {
     // scale of distance leaf d, 2^s > max |f| over every point (from the per-plane maxima)
     const int d = (tid - 64) >> 5, lane = tid & 31;
     if (sp.tc_build && d < sp.ndot) {
@@ -223,14 +229,14 @@ __global__ void __launch_bounds__(128) k_prep(const Prob* __restrict__ probs) {
     if (rb == 0) P.kscale[0] = e;
   }
   __syncthreads();
-  if (rb == 0 && tid == 0 && sp.tc_build) {
+  if (rb == 0 && tid == 0 && y == 0 && sp.tc_build) {
     // fixed point throughout (K_ii >= 1, so e >= 1 unless the nugget is
     // negative), with scales in the exponential's common form
     bool fixed = s_k >= 1;
     for (int l = 0; l < sp.ndot; ++l) fixed &= iexp_common(iexp_scale(2 * s_e[l] + 1 - sp.dot_u[l]));
     P.fscale[2] = fixed ? form : FORM_FP64;
   }
-  {
+  if (y == PREP_Y - 1) {
     // right-hand sides: y - mu (marginal), or y and 1 (concentrated), in the factor's scale; zero on the padding
     const double u = ldexp(1.0, -s_k);
     P.rhs[i] = i < P.N ? u * (P.likelihood == 1 ? P.y[i] : P.y[i] - P.mu[i]) : 0.0;
@@ -239,13 +245,14 @@ __global__ void __launch_bounds__(128) k_prep(const Prob* __restrict__ probs) {
   if (!sp.tc_build) {
     // the dot-product build's scaled planes and rbf norms (the workspace is not
     // cleared between evaluations: norms of other leaves are zeroed here)
+    __shared__ double s_norm[PREP_Y][NB];
     for (int l = 0; l < MAX_LEAF; ++l) {
       double a = 0.0;
       if (l < sp.nleaf) {
         const Leaf& L = sp.leaf[l];
         const int per = L.type == L_PERIODIC ? 2 : 1;
         const int cnt = L.type == L_LINEAR || L.type == L_CONSTANT ? 0 : per * L.n;
-        for (int k = 0; k < cnt; ++k) {
+        for (int k = y; k < cnt; k += PREP_Y) {
           const size_t o = (size_t)(L.plane0 + k) * nc + i;
           if (L.type == L_RBF_CYCLIC) {
             // fixed point 2^(54 - s), or the fraction of a turn as it is; a point
@@ -267,7 +274,13 @@ __global__ void __launch_bounds__(128) k_prep(const Prob* __restrict__ probs) {
           if (L.type == L_RBF) a = fma(u, u, a);
         }
       }
-      P.norms[(size_t)l * nc + i] = a;
+      if (l < sp.nleaf) {
+        s_norm[y][tid] = a;
+        __syncthreads();
+        a = (s_norm[0][tid] + s_norm[1][tid]) + (s_norm[2][tid] + s_norm[3][tid]);
+        __syncthreads();
+      }
+      if (y == 0) P.norms[(size_t)l * nc + i] = a;
     }
     return;
   }
@@ -278,7 +291,7 @@ __global__ void __launch_bounds__(128) k_prep(const Prob* __restrict__ probs) {
     const int e = s_e[t];
     int S[NLEV] = {0, 0, 0, 0, 0, 0, 0, 0};
     unsigned char* base = P.slices + (size_t)rb * NSLICE * SLICE_BYTES + (size_t)tid * 16;
-    for (int kg = 0; kg < sp.dot_kch[t] * 2; ++kg) {
+    for (int kg = t == 0 ? y : PREP_Y - 1 - y; kg < sp.dot_kch[t] * 2; kg += PREP_Y) {
       long long F[8];
 #pragma unroll
       for (int kk = 0; kk < 8; ++kk) {
@@ -309,7 +322,19 @@ __global__ void __launch_bounds__(128) k_prep(const Prob* __restrict__ probs) {
       for (int p = 0; p < NSLICE; ++p)
         *reinterpret_cast<uint4*>(base + (size_t)p * SLICE_BYTES + (size_t)kgl * 2048) = out[p];
     }
-    P.fnorm[(size_t)t * nc + i] = assemble_w(S, sp.dot_u[t]);
+#pragma unroll
+    for (int l = 0; l < NLEV; ++l) s_lev[t][y][l][tid] = S[l];
+  }
+  __syncthreads();
+  if (y < sp.ndot) {
+    int S[NLEV];
+#pragma unroll
+    for (int l = 0; l < NLEV; ++l) {
+      S[l] = 0;
+#pragma unroll
+      for (int q = 0; q < PREP_Y; ++q) S[l] += s_lev[y][q][l][tid];
+    }
+    P.fnorm[(size_t)y * nc + i] = assemble_w(S, sp.dot_u[y]);
   }
   if (bad) atomicOr(&P.status[3], 1);
 }
@@ -611,7 +636,7 @@ __global__ void __launch_bounds__(BLD_THREADS, 1)
 // launch helpers
 // ---------------------------------------------------------------------------
 cudaError_t launch_prep(const Prob* probs, int nprob, int max_nt128, cudaStream_t s) {
-  k_prep<<<dim3(max_nt128, nprob), 128, 0, s>>>(probs);
+  k_prep<<<dim3(max_nt128, nprob), dim3(NB, PREP_Y), 0, s>>>(probs);
   return cudaGetLastError();
 }
 
