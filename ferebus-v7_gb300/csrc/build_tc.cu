@@ -79,6 +79,13 @@ __device__ __forceinline__ long long assemble_w_bits(const uint32_t b[NLEV], int
   return (long long)((H << (u - 48)) + (unsigned long long)((Lo + ((1LL << (71 - u)) - BUILD_BIAS_LO)) >> (72 - u)));
 }
 
+__device__ __forceinline__ void tmem_ldw(uint32_t (&v)[8], uint32_t addr) { tmem_ld8(v, addr); }
+__device__ __forceinline__ void tmem_ldw(uint32_t (&v)[4], uint32_t addr) {
+  asm volatile("tcgen05.ld.sync.aligned.32x32b.x4.b32 {%0,%1,%2,%3}, [%4];"
+               : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3])
+               : "r"(addr));
+}
+
 }  // namespace
 
 // ---------------------------------------------------------------------------
@@ -354,7 +361,11 @@ static_assert(BLD_SMEM <= 227 * 1024, "shared memory per CTA");
 // the loops it adds cost the others up to 18% (40 problems of N = 4000, a sum of
 // two: 3.8 -> 4.5 ms, the compiler's schedule).  Against the FP64
 // combination, the product's build: 7.5 -> 4.1 ms.
-template <bool PROD>
+// NC: columns per epilogue thread.  A tile takes 16; where a problem has so few
+// tiles that its parts still fit one wave, a CTA takes 4 NC of a tile's 64
+// columns (and all of its products): the epilogue's chain is what a small
+// build costs.  A lone N = 59 34 -> 18 us, N = 500 25 -> 16.5.
+template <bool PROD, int NC>
 __global__ void __launch_bounds__(BLD_THREADS, 1)
     k_build_tc(const Prob* __restrict__ probs, int nprob, const unsigned long long* __restrict__ tiles, int total) {
   extern __shared__ __align__(1024) unsigned char smb[];
@@ -365,6 +376,8 @@ __global__ void __launch_bounds__(BLD_THREADS, 1)
   uint64_t* drain = tfull + 2;  // quiescing after a give-up
   uint32_t* slot = reinterpret_cast<uint32_t*>(tfull + 3);
   __shared__ int s_abort;
+  constexpr int SUB = 16 / NC;      // CTAs per tile
+  constexpr int GW = NC < 8 ? NC : 8;  // columns drained together
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   uint32_t issued = 0;  // producer lane: k-chunks whose operand copies were issued
   if (tid == 0) {
@@ -396,7 +409,7 @@ __global__ void __launch_bounds__(BLD_THREADS, 1)
   __syncthreads();
   // tile t: (problem << 40 | 128-row tile << 20 | 64-column tile), host-built
   auto tile_of = [&](int t, int& p, int& ti, int& tj) {
-    const unsigned long long e = tiles[t];
+    const unsigned long long e = tiles[t / SUB];
     p = (int)(e >> 40);
     ti = (int)((e >> 20) & 0xFFFFF);
     tj = (int)(e & 0xFFFFF);
@@ -406,7 +419,7 @@ __global__ void __launch_bounds__(BLD_THREADS, 1)
     // ---------------- TMA producer: digit planes of each leaf's k chunks ----------------
     if (lane == 0) {
       uint32_t g = 0;
-      for (int t = blockIdx.x; t < total && !s_abort; t += gridDim.x) {
+      for (int t = blockIdx.x; t < total * SUB && !s_abort; t += gridDim.x) {
         int p, ti, tj;
         tile_of(t, p, ti, tj);
         const Prob& P = probs[p];
@@ -437,7 +450,7 @@ __global__ void __launch_bounds__(BLD_THREADS, 1)
       uint32_t g = 0, it = 0;
       const uint64_t adesc0 = smem_desc(su32(smb), 2048, 128);
       const uint64_t bdesc0 = smem_desc(su32(smb) + A_STAGE, 1024, 128);
-      for (int t = blockIdx.x; t < total && !s_abort; t += gridDim.x) {
+      for (int t = blockIdx.x; t < total * SUB && !s_abort; t += gridDim.x) {
         int p, ti, tj;
         tile_of(t, p, ti, tj);
         const Spec& sp = *probs[p].spec;
@@ -475,17 +488,18 @@ __global__ void __launch_bounds__(BLD_THREADS, 1)
   } else {
     // ---------------- epilogue (warps 0-15) ----------------
     const int r = (warp & 3) * 32 + lane;  // TMEM lane = tile row
-    const int h = warp >> 2;               // group of 16 columns
+    const int h = warp >> 2;               // group of NC columns
     const uint32_t lane_base = (uint32_t)((warp & 3) * 32) << 16;
     uint32_t it = 0;
-    for (int t = blockIdx.x; t < total; t += gridDim.x) {
+    for (int t = blockIdx.x; t < total * SUB; t += gridDim.x) {
       int p, ti, tj;
       tile_of(t, p, ti, tj);
       const Prob& P = probs[p];
       const Spec& sp = *P.spec;
       const size_t nc = (size_t)P.Nc;
       const int i = ti * NB + r;
-      const int j0 = tj * TB + h * 16;
+      const int cb0 = (t % SUB * 4 + h) * NC;  // this thread's columns of the tile
+      const int j0 = tj * TB + cb0;
       const int form = P.fscale[2];
       bool stop = false;
       for (int d = 0; d < sp.ndot; ++d, ++it) {
@@ -495,7 +509,7 @@ __global__ void __launch_bounds__(BLD_THREADS, 1)
           break;
         }
         asm volatile("tcgen05.fence::after_thread_sync;");
-        long long W[16];
+        long long W[NC];
         const int u = sp.dot_u[d];
         // level sums of a leaf with at most 36 features stay below 2^22 (7
         // digit pairs x 36 terms x 2^14): converted by the exact magic add
@@ -503,31 +517,28 @@ __global__ void __launch_bounds__(BLD_THREADS, 1)
         const Leaf& LF = sp.leaf[sp.dot_leaf[d]];
         const bool small = (LF.type == L_PERIODIC ? 2 * LF.n : LF.n) <= 36;
 #pragma unroll
-        for (int gq = 0; gq < 2; ++gq) {
-          uint32_t v[NLEV][8];
+        for (int gq = 0; gq < NC / GW; ++gq) {
+          uint32_t v[NLEV][GW];
 #pragma unroll
           for (int l = 0; l < NLEV; ++l) {
-            asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
-                         : "=r"(v[l][0]), "=r"(v[l][1]), "=r"(v[l][2]), "=r"(v[l][3]), "=r"(v[l][4]),
-                           "=r"(v[l][5]), "=r"(v[l][6]), "=r"(v[l][7])
-                         : "r"(tbase + lane_base + (uint32_t)(l * 64 + h * 16 + gq * 8)));
+            tmem_ldw(v[l], tbase + lane_base + (uint32_t)(l * 64 + cb0 + gq * GW));
           }
           asm volatile("tcgen05.wait::ld.sync.aligned;");
           if (small) {
 #pragma unroll
-            for (int jj = 0; jj < 8; ++jj) {
+            for (int jj = 0; jj < GW; ++jj) {
               uint32_t b[NLEV];
 #pragma unroll
               for (int l = 0; l < NLEV; ++l) b[l] = level_bits(v[l][jj]);
-              W[gq * 8 + jj] = assemble_w_bits(b, u);
+              W[gq * GW + jj] = assemble_w_bits(b, u);
             }
           } else {
 #pragma unroll
-            for (int jj = 0; jj < 8; ++jj) {
+            for (int jj = 0; jj < GW; ++jj) {
               int S[NLEV];
 #pragma unroll
               for (int l = 0; l < NLEV; ++l) S[l] = __float2int_rn(__uint_as_float(v[l][jj]));
-              W[gq * 8 + jj] = assemble_w(S, u);
+              W[gq * GW + jj] = assemble_w(S, u);
             }
           }
         }
@@ -537,10 +548,10 @@ __global__ void __launch_bounds__(BLD_THREADS, 1)
         // the squared distances, in the leaf's unit
         const long long wi = (long long)((unsigned long long)P.fnorm[(size_t)d * nc + i] +
                                          (small ? (unsigned long long)BUILD_BIAS_H << (u - 47) : 0ULL));
-        // W_jj of this thread's 16 columns (the same for the whole warp), two at a time
+        // W_jj of this thread's NC columns (the same for the whole warp), two at a time
         const longlong2* wj2 = reinterpret_cast<const longlong2*>(P.fnorm + (size_t)d * nc + j0);
 #pragma unroll
-        for (int q = 0; q < 16; ++q) {
+        for (int q = 0; q < NC; ++q) {
           const longlong2 w2 = __ldg(wj2 + q / 2);
           W[q] = (long long)((unsigned long long)wi + (unsigned long long)((q & 1) ? w2.y : w2.x) - 2 * (unsigned long long)W[q]);
           if (W[q] < 0) W[q] = 0;
@@ -554,7 +565,7 @@ __global__ void __launch_bounds__(BLD_THREADS, 1)
         long long* A = P.acc + acc_tile(ti, tj, P.nt128) * ACC_TILE_ELEMS;
         const int jmax = i < N ? i : -1;
         auto put = [&](int q, long long F) {
-          A[acc_elem(r, h * 16 + q)] = j0 + q <= jmax ? F : 0LL;
+          A[acc_elem(r, cb0 + q)] = j0 + q <= jmax ? F : 0LL;
         };
         // One leaf, a plain sum of two or a plain product of two: fixed point
         // throughout.  Any other expression, and scales outside the
@@ -567,20 +578,20 @@ __global__ void __launch_bounds__(BLD_THREADS, 1)
           if (d < sp.ndot - 1) {
             const int unit = PROD && prod ? 0 : e2;  // a product's first factor: v0 2^62
 #pragma unroll
-            for (int q = 0; q < 16; ++q) st[q * tstash] = iexp_parts_fixed62(parts((unsigned long long)W[q]), unit);
+            for (int q = 0; q < NC; ++q) st[q * tstash] = iexp_parts_fixed62(parts((unsigned long long)W[q]), unit);
           } else if (d == 0) {
 #pragma unroll
-            for (int q = 0; q < 16; ++q) put(q, iexp_parts_fixed62(parts((unsigned long long)W[q]), e2));
+            for (int q = 0; q < NC; ++q) put(q, iexp_parts_fixed62(parts((unsigned long long)W[q]), e2));
           } else if (PROD && prod) {
 #pragma unroll
-            for (int q = 0; q < 16; ++q) {
+            for (int q = 0; q < NC; ++q) {
               IexpParts v = parts((unsigned long long)W[q]);
               v.Z = __umul64hi((unsigned long long)st[q * tstash], v.Z);  // v0 v1 2^(60 + m)
               put(q, iexp_parts_fixed62(v, e2 - 2));
             }
           } else {
 #pragma unroll
-            for (int q = 0; q < 16; ++q) put(q, st[q * tstash] + iexp_parts_fixed62(parts((unsigned long long)W[q]), e2));
+            for (int q = 0; q < NC; ++q) put(q, st[q * tstash] + iexp_parts_fixed62(parts((unsigned long long)W[q]), e2));
           }
         };
         if ((sum || prod) && iexp_common(esc) && esc.F <= 64) {
@@ -593,13 +604,13 @@ __global__ void __launch_bounds__(BLD_THREADS, 1)
           double* st = stash + tid;
           if (d < sp.ndot - 1) {
 #pragma unroll
-            for (int q = 0; q < 16; ++q) st[q * tstash] = leaf(q);
+            for (int q = 0; q < NC; ++q) st[q * tstash] = leaf(q);
           } else if (d == 0) {
 #pragma unroll
-            for (int q = 0; q < 16; ++q) put(q, to_fixed62(fma(cb, leaf(q), ca), e2, &nonfinite));
+            for (int q = 0; q < NC; ++q) put(q, to_fixed62(fma(cb, leaf(q), ca), e2, &nonfinite));
           } else {
 #pragma unroll
-            for (int q = 0; q < 16; ++q) {
+            for (int q = 0; q < NC; ++q) {
               // second distance leaf: k = (d v0 + c) v1 + (b v0 + a)
               const double v0 = st[q * tstash];
               put(q, to_fixed62(fma(fma(cd, v0, cc), leaf(q), fma(cb, v0, ca)), e2, &nonfinite));
@@ -607,11 +618,11 @@ __global__ void __launch_bounds__(BLD_THREADS, 1)
           }
         }
         // the diagonal entry: every leaf 1, with the nugget; identity padding (1/4 in the matrix's unit) beyond N
-        if (d == sp.ndot - 1 && i >= j0 && i < j0 + 16) {
+        if (d == sp.ndot - 1 && i >= j0 && i < j0 + NC) {
           const double noise = P.optimise_noise ? P.theta[sp.nkparams] : P.noise;
           const double ca = P.fcoef[0], cb = P.fcoef[1], cc = P.fcoef[2], cd = P.fcoef[3];
           const double kd = sp.ndot == 1 ? cb + ca : (cd + cc) + (cb + ca);
-          A[acc_elem(r, i - j0 + h * 16)] = i < N ? diag_fixed62(kd, noise, e2, &nonfinite) : 1LL << 60;
+          A[acc_elem(r, i - j0 + cb0)] = i < N ? diag_fixed62(kd, noise, e2, &nonfinite) : 1LL << 60;
         }
         if (nonfinite) atomicOr(&P.status[3], 1);
       }
@@ -642,11 +653,16 @@ cudaError_t launch_prep(const Prob* probs, int nprob, int max_nt128, cudaStream_
 
 cudaError_t launch_build_tc(const Prob* probs, int nprob, const unsigned long long* tiles, int total_tiles,
                             bool products, int num_sms, cudaStream_t s) {
-  auto kernel = products ? k_build_tc<true> : k_build_tc<false>;
-  cudaError_t e = ensure_smem_attr((const void*)kernel, products ? SMEM_BUILD_TC_PROD : SMEM_BUILD_TC, BLD_SMEM);
+  // the parts of the tiles fill one wave at most
+  const int sub = 4 * total_tiles <= num_sms ? 4 : (2 * total_tiles <= num_sms ? 2 : 1);
+  using Kernel = void (*)(const Prob*, int, const unsigned long long*, int);
+  const Kernel kernels[2][3] = {{k_build_tc<false, 16>, k_build_tc<false, 8>, k_build_tc<false, 4>},
+                                {k_build_tc<true, 16>, k_build_tc<true, 8>, k_build_tc<true, 4>}};
+  const Kernel kernel = kernels[products][sub / 2];
+  cudaError_t e = ensure_smem_attr((const void*)kernel, SMEM_BUILD_TC + products * 3 + sub / 2, BLD_SMEM);
   if (e != cudaSuccess) return e;
   if (total_tiles <= 0) return cudaSuccess;
-  const int grid = total_tiles < num_sms ? total_tiles : num_sms;
+  const int grid = total_tiles * sub < num_sms ? total_tiles * sub : num_sms;
   kernel<<<grid, BLD_THREADS, BLD_SMEM, s>>>(probs, nprob, tiles, total_tiles);
   return cudaGetLastError();
 }

@@ -52,6 +52,15 @@ def test_two_leaves(n, op, lib):
     _check(X, y, ks, n % 2)
 
 
+# 30, 42 and 90 tiles: a CTA takes a quarter, half and the whole of one
+@pytest.mark.parametrize("n", [600, 700, 1100])
+@pytest.mark.parametrize("op", ["sum", "prod"])
+def test_parts_of_tiles(n, op, lib):
+    X, y = _data(n, n)
+    ks = [O.RBF, 4, 1, 2, 3, 4, O.PERIODIC, 1, 5, O.SUM if op == "sum" else O.PROD]
+    _check(X, y, ks, 1)
+
+
 @pytest.mark.parametrize("spread", [0.0, 1e-15, 1e9])
 @pytest.mark.parametrize("op", ["sum", "prod"])
 @pytest.mark.parametrize("first", [True, False])
