@@ -1306,7 +1306,7 @@ int fgpu_grad(fgpu_ctx* ctx, const double* theta, int ntheta, double* ll, double
   }
   if (g->fast)
     CK(enqueue_grad_fast(g->prob_d, w->prob_d, g->nsteps, ctx->Nc, ctx->spec.nplanes, ctx->nkparams, g->extra,
-                         ctx->optimise_noise, g->fx, g->sums, g->g_d, s, &n));
+                         ctx->optimise_noise, g->fx, g->sums, g->g_d, g->num_sms, s, &n));
   else
     CK(enqueue_grad_passes(g->prob_d, g->nsteps, ctx->nkparams, ctx->optimise_noise, g->g_d, s, &n));
   double* h_out = g->h_stage;

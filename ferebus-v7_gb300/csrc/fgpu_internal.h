@@ -254,7 +254,7 @@ constexpr int GRAD_SLOTS = 33;  // parameters per fused pass + noise slot
 // grad_fast_partials: doubles of partial and total sums.
 size_t grad_fast_partials(int nsteps, int nk);
 cudaError_t enqueue_grad_fast(const Prob* p, const Prob* eval, int nsteps, int nc_eval, int nplanes, int nk, int extra,
-                              int optimise_noise, long long* fx, double* sums, double* g_out, cudaStream_t s,
+                              int optimise_noise, long long* fx, double* sums, double* g_out, int num_sms, cudaStream_t s,
                               long long* nlaunch);
 
 // Opt kernel `func` into `bytes` of dynamic shared memory on the CURRENT
@@ -264,7 +264,7 @@ cudaError_t enqueue_grad_fast(const Prob* p, const Prob* eval, int nsteps, int n
 // beyond the first 64 set it on every call.
 enum SmemSlot {
   SMEM_BUILD, SMEM_BUILD_DOT, SMEM_UPDATE, SMEM_SYRK, SMEM_OZAKI_UPDATE, SMEM_PANEL, SMEM_PANEL_ROWS,
-  SMEM_BUILD_TC, SMEM_BUILD_TC_LAST = SMEM_BUILD_TC + 5, SMEM_INV_GEMM, SMEM_GRAD_FAST, SMEM_NSLOTS
+  SMEM_BUILD_TC, SMEM_BUILD_TC_LAST = SMEM_BUILD_TC + 5, SMEM_INV_GEMM, SMEM_GRAD_FAST, SMEM_GRAD_FAST2, SMEM_NSLOTS
 };
 cudaError_t ensure_smem_attr(const void* func, int slot, int bytes);
 

@@ -257,7 +257,7 @@ __global__ void k_grad_reduce(const Prob* __restrict__ pp, int nblocks, int q0, 
 // D = h 2^27 + l squared as h^2 + 2 h l 2^-27 + l^2 2^-54 on the integer
 // multiply-add pipe, and the fixed-point exponential.  One CTA per 64 x 64 lower
 // tile, 2 rows x 8 columns per thread, the features staged 16 planes at a time.
-// N = 4000, d = 24: 2.1 ms, against 4.9 ms for k_grad (all FP64, leaf values and
+// N = 4000, d = 24: 1.6 ms, against 4.9 ms for k_grad (all FP64, leaf values and
 // differences formed twice) and 0.34 ms for its one-block reduction.
 // ---------------------------------------------------------------------------
 namespace {
@@ -279,7 +279,13 @@ __global__ void __launch_bounds__(256) k_grad_fixed(const Prob* __restrict__ pe,
   }
 }
 
-__global__ void __launch_bounds__(256)
+// PER_SM: CTAs per SM.  With more tiles than SMs, two: the tile's integer and
+// FP64 halves follow one another behind barriers, and a second CTA fills the
+// pipe the first leaves idle, which is worth the 128 registers (N = 4000: 2.08 ->
+// 1.57 ms).  With fewer, one CTA with all the registers it wants (N = 1003: 163
+// us, and 168 with 128).
+template <int PER_SM>
+__global__ void __launch_bounds__(256, PER_SM)
     k_grad_fast(const Prob* __restrict__ pp, const Prob* __restrict__ pe, const long long* __restrict__ fx,
                 int nslots, int extra) {
   const Prob& P = *pp;   // adjoint: planes, alpha, K^-1
@@ -541,13 +547,15 @@ __global__ void __launch_bounds__(256)
 size_t grad_fast_partials(int nsteps, int nk) { return (size_t)nsteps * (nsteps + 1) / 2 * (nk + 5) + (nk + 5); }
 
 cudaError_t enqueue_grad_fast(const Prob* p, const Prob* eval, int nsteps, int nc_eval, int nplanes, int nk, int extra,
-                              int optimise_noise, long long* fx, double* sums, double* g_out, cudaStream_t s,
+                              int optimise_noise, long long* fx, double* sums, double* g_out, int num_sms, cudaStream_t s,
                               long long* nlaunch) {
-  cudaError_t e = ensure_smem_attr((const void*)k_grad_fast, SMEM_GRAD_FAST, GF_SMEM);
-  if (e != cudaSuccess) return e;
   const int ntiles = nsteps * (nsteps + 1) / 2, nslots = nk + 5;
+  const bool two = ntiles > num_sms;
+  const auto kernel = two ? k_grad_fast<2> : k_grad_fast<1>;
+  const cudaError_t e = ensure_smem_attr((const void*)kernel, two ? SMEM_GRAD_FAST2 : SMEM_GRAD_FAST, GF_SMEM);
+  if (e != cudaSuccess) return e;
   k_grad_fixed<<<dim3((nc_eval + 255) / 256, nplanes), 256, 0, s>>>(eval, fx);
-  k_grad_fast<<<ntiles, 256, GF_SMEM, s>>>(p, eval, fx, nslots, extra);
+  kernel<<<ntiles, 256, GF_SMEM, s>>>(p, eval, fx, nslots, extra);
   k_grad_fast_reduce<<<nslots, 256, 0, s>>>(p, ntiles, nslots, sums);
   k_grad_fast_out<<<1, 256, 0, s>>>(p, sums, nslots, optimise_noise ? nk : -1, g_out);
   if (nlaunch) *nlaunch += 4;

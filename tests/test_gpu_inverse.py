@@ -1,6 +1,7 @@
 """The adjoint's K^-1 on the tensor cores (csrc/inv.cu) at the edges of its
 block recursion: one tile, one column past it, block counts that are not a
-power of two.  Same tolerance as the other gradient tests: 1e-6 relative to
+power of two; the last three around the size from which the dK/dtheta pass runs two
+CTAs per SM.  Same tolerance as the other gradient tests: 1e-6 relative to
 the oracle's FP64 gradient, 1e-9 of its largest component for those that
 cancel."""
 import numpy as np
@@ -11,7 +12,7 @@ from oracle import gpr_oracle as O
 pytestmark = pytest.mark.gpu
 
 
-@pytest.mark.parametrize("n", [127, 128, 129, 257, 385, 640, 897])
+@pytest.mark.parametrize("n", [127, 128, 129, 257, 385, 640, 897, 1024, 1025, 1200])
 @pytest.mark.parametrize("lik", [0, 1])
 def test_gradient_at_block_edges(n, lik, lib):
     from fgpu import Engine
