@@ -742,7 +742,7 @@ size_t workspace_bytes(const fgpu_ctx* c, bool keep_l) {
 int write_tmaps(const fgpu_ctx* c, const Workspace& ws, unsigned char* dst) {
   if (c->mode != 1) return 0;
   alignas(64) unsigned char maps[TMAP_BYTES];
-  const int er = encode_slice_maps(maps, ws.slices, c->nt128);
+  const int er = encode_slice_maps(maps, ws.slices, c->nt128 + 1);
   if (er != 0) return fail(FGPU_ECUDA, "cuTensorMapEncodeTiled failed (%d)", er);
   CK(cudaMemcpy(dst, maps, TMAP_BYTES, cudaMemcpyHostToDevice));
   return 0;

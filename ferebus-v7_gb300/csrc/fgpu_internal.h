@@ -140,7 +140,7 @@ struct Prob {
 // (boxes of 128 and 64 rows, and 64 and 16 rows with the planes stacked) into
 // host memory (TMAP_BYTES).  Returns 0 or a CUDA driver error code.
 constexpr size_t TMAP_BYTES = 4 * 128;
-int encode_slice_maps(void* host_maps, const void* slices, int nt128);
+int encode_slice_maps(void* host_maps, const void* slices, int tiles);
 
 // Launch helpers (engine.cu).  All kernels take a device array of problems
 // and index it by blockIdx.y; problems whose geometry does not reach the

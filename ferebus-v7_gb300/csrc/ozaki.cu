@@ -308,7 +308,7 @@ __global__ void __launch_bounds__(UPD_THREADS, 1)
 // buffer layout: [row tile nt128][plane 7][k-group 16][row 128][8 fp16]; a (k-group, plane)
 // block is 2 KB contiguous
 // ---------------------------------------------------------------------------
-int encode_slice_maps(void* host_maps, const void* slices, int nt128) {
+int encode_slice_maps(void* host_maps, const void* slices, int tiles) {
   static PFN_cuTensorMapEncodeTiled_v12000 fn = nullptr;
   static std::mutex mu;
   {
@@ -325,7 +325,7 @@ int encode_slice_maps(void* host_maps, const void* slices, int nt128) {
   }
   // A (k-group, plane) block of 128 rows x 16 B is 2 KB contiguous: describe it
   // as 4 rows of 256 fp16 (512 B) so each TMA request moves 512 B.
-  const cuuint64_t dims[5] = {256, 4, 16, (cuuint64_t)NSLICE, (cuuint64_t)nt128 + 1};
+  const cuuint64_t dims[5] = {256, 4, 16, (cuuint64_t)NSLICE, (cuuint64_t)tiles};
   const cuuint64_t strides[4] = {512, 2048, (cuuint64_t)SLICE_BYTES, (cuuint64_t)NSLICE * SLICE_BYTES};
   const cuuint32_t boxA[5] = {256, 4, 2, NSLICE, 1};   // 128 rows
   const cuuint32_t boxB[5] = {256, 2, 2, NSLICE, 1};   // 64 rows
@@ -342,7 +342,7 @@ int encode_slice_maps(void* host_maps, const void* slices, int nt128) {
   // a box of 64 rows with the plane and k-group dimensions swapped: it lands
   // as [k-group][plane][row], so the 7 planes of a k-group are one operand of
   // 7 x 64 rows (the stacked-N MMAs of the trailing update)
-  const cuuint64_t dimsS[5] = {256, 4, (cuuint64_t)NSLICE, 16, (cuuint64_t)nt128 + 1};
+  const cuuint64_t dimsS[5] = {256, 4, (cuuint64_t)NSLICE, 16, (cuuint64_t)tiles};
   const cuuint64_t stridesS[4] = {512, (cuuint64_t)SLICE_BYTES, 2048, (cuuint64_t)NSLICE * SLICE_BYTES};
   const cuuint32_t boxS[5] = {256, 2, NSLICE, 2, 1};
   r = fn(&m[2], CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 5, const_cast<void*>(slices), dimsS, stridesS, boxS, es,
