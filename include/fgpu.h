@@ -114,11 +114,13 @@ int fgpu_loglik_batch(fgpu_ctx* const* ctxs, int nprob, const double* const* the
                       double* ll, int* info);
 
 /* Log-likelihood and its gradient d logL / d theta (including the noise
- * parameter when optimise_noise is set) by the FP64 adjoint
+ * parameter when optimise_noise is set) by the adjoint
  * 1/2 tr((alpha alpha^T / s - K^-1) dK/dtheta), s = 1 (marginal) or sigma^2
  * (concentrated).  The factor is the evaluation's own (on a tensor-core
  * context the same factor, log-likelihood and alpha as fgpu_loglik), K^-1
- * comes from it in FP64, and dK is recomputed tile by tile.  The reference
+ * comes from it (on a tensor-core context by split-integer products, otherwise
+ * or where that workspace does not fit in FP64), and dK is recomputed tile by
+ * tile.  The reference
  * has no analytic likelihood gradient (negative_log_likelihood,
  * gpr.f90:258-289, accepts but ignores gradient=.true.); this is the
  * optional gradient polish.  dll_dtheta has fgpu_nparams(ctx) entries. */
@@ -195,8 +197,9 @@ int fgpu_loglik_noalloc(int N, int d, const double* X_dev, const double* y_dev, 
 
 /* Stage timing for roofline accounting.  When enabled, the plan's graph is
  * re-captured with CUDA event nodes around every launch (enable = 1) or
- * around the trailing-update launches only (enable = 2, which leaves the
- * rest of the graph as it runs unprofiled); after a run,
+ * around the trailing-update launches only (enable = 2), its launches one
+ * after the other (unprofiled, a batch's next diagonal tiles are factored
+ * beside the trailing update); after a run,
  * fgpu_plan_stage_times fills ms[k] with the summed device time of stage k
  * during the LAST replay and count[k] with its launches (k: 0 build,
  * 1 diagonal factor, 2 panel solve, 3 trailing update, 4 likelihood
