@@ -616,7 +616,7 @@ __global__ void __launch_bounds__(256) k_finalize(const Prob* __restrict__ probs
 // owns the 64-row block b = nsteps - 1 - k, adds up L_rb^T alpha_r as the blocks
 // r > b below it are published, and solves its own triangle.  Whoever waits
 // for a block holds a later ticket than it, so that block's CTA is running.
-// The chain is nsteps triangles of 64 dependent FP64 steps, ~6 us each; the
+// The chain is nsteps triangles of 64 dependent FP64 steps, ~8 us each; the
 // tiles of L are read beside it.  (Two launches per block, with a division per
 // step and everything re-read in order, took 34 us per block.)
 // sync[0]: ticket, sync[1]: blocks solved; both zeroed before the launch.

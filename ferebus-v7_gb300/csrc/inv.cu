@@ -18,8 +18,9 @@
 // Against the FP64 sweep over identity rows and the FP64 product (N^3 / 3
 // multiply-adds on a 1.05 TFLOP/s pipe: 51 ms at N = 4000) this is 24 k
 // 128 x 64 x 128 tile products at the trailing update's rate (about 1 ms) and
-// four launches per doubling of the block size: a gradient takes 13.6 ms
-// instead of 62.4 at N = 4000, 2.8 instead of 6.6 at N = 1003, with the same
+// four launches per doubling of the block size: 1.6 ms at N = 4000 and 0.35 at
+// N = 1003 (a gradient took 13.6 ms instead of 62.4, and 2.8 instead of 6.6,
+// with this; 6.9 and 1.4 with what else has changed since), with the same
 // errors against extended precision (7 kernels and data sets, ratio 0.7 to 1.2).
 #include "fgpu_internal.h"
 #include "tc_common.cuh"

@@ -45,8 +45,9 @@
 // digit chunks the couplings read (28 KB each) stay in shared memory, hence
 // one CTA per SM.  Measured, against the FP64 panel in ten launches
 // (conversion of the integer sums, 32-column factors, solves and couplings,
-// right-hand-side update) that this replaces: a lone problem 250 -> 95 us
-// per panel (N = 4000, 32 panels), a swarm of 40 at N = 4000 20.7 -> 9.8 ms.
+// right-hand-side update) that this replaces: a lone problem 250 -> 75 us
+// per panel (N = 4000, 32 panels), a swarm of 40 at N = 4000 20.7 -> 9.3 ms
+// (6.4 with k_panel_rows below).
 #include "fgpu_internal.h"
 #include "tc_common.cuh"
 
