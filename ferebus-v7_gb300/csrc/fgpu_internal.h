@@ -263,8 +263,11 @@ cudaError_t enqueue_grad_fast(const Prob* p, const Prob* eval, int nsteps, int n
 // device, or a second thread, sets the attribute for itself.  Devices
 // beyond the first 64 set it on every call.
 enum SmemSlot {
-  SMEM_BUILD, SMEM_BUILD_DOT, SMEM_UPDATE, SMEM_SYRK, SMEM_OZAKI_UPDATE, SMEM_PANEL, SMEM_PANEL_ROWS,
-  SMEM_BUILD_TC, SMEM_BUILD_TC_LAST = SMEM_BUILD_TC + 5, SMEM_INV_GEMM, SMEM_GRAD_FAST, SMEM_GRAD_FAST2, SMEM_NSLOTS
+  SMEM_BUILD, SMEM_BUILD_DOT, SMEM_UPDATE, SMEM_SYRK, SMEM_PANEL, SMEM_PANEL_ROWS, SMEM_INV_GEMM, SMEM_GRAD_FAST,
+  SMEM_GRAD_FAST2,
+  SMEM_OZAKI_UPDATE, SMEM_OZAKI_UPDATE_LAST = SMEM_OZAKI_UPDATE + 2,  // one slot per instance
+  SMEM_BUILD_TC, SMEM_BUILD_TC_LAST = SMEM_BUILD_TC + 5,
+  SMEM_NSLOTS
 };
 cudaError_t ensure_smem_attr(const void* func, int slot, int bytes);
 

@@ -84,6 +84,12 @@ static_assert(UPD_SMEM <= 227 * 1024, "shared memory per CTA");
 __host__ __device__ constexpr int upd_level_warp(int) { return 0; }
 static_assert(UPD_MMA_WARPS == 1, "the update epilogue converts all 7 levels of a column group in one pass");
 
+//
+// KSH: a tile's 8 k-chunks are shared by 2^KSH CTAs, each of which subtracts
+// its part (the same integers).  Where a step has so few tiles that the parts
+// still fit one wave, the loads and MMAs of one tile are what it costs: the
+// updates of a lone N = 500 39 -> 28 us, of N = 1501 138 -> 116.
+template <int KSH>
 __global__ void __launch_bounds__(UPD_THREADS, 1)
     k_ozaki_update(const Prob* __restrict__ probs, int nprob, int s, const unsigned long long* __restrict__ tiles,
                    int total) {
@@ -119,7 +125,7 @@ __global__ void __launch_bounds__(UPD_THREADS, 1)
   const uint32_t tbase = *slot;
   // tile t of the step: one load instead of a search over the problems
   auto tile_of = [&](int t, int& p, int& ti, int& tj) {
-    const unsigned long long e = tiles[t];
+    const unsigned long long e = tiles[t >> KSH];
     p = (int)(e >> 40);
     ti = (int)((e >> 20) & 0xFFFFF);
     tj = (int)(e & 0xFFFFF);
@@ -137,23 +143,23 @@ __global__ void __launch_bounds__(UPD_THREADS, 1)
     // ---------------- TMA producer ----------------
     if (lane == 0) {
       uint32_t g = 0;
-      for (int t = blockIdx.x; t < total; t += gridDim.x) {
+      for (int t = blockIdx.x; t < total << KSH; t += gridDim.x) {
         int p, ti, tj;
         tile_of(t, p, ti, tj);
         const Prob& P = probs[p];
         if (failed(P)) continue;
         asm volatile("fence.proxy.tensormap::generic.acquire.gpu [%0], 128;" ::"l"(P.tmap_a) : "memory");
         asm volatile("fence.proxy.tensormap::generic.acquire.gpu [%0], 128;" ::"l"(P.tmap_bs) : "memory");
-        for (int c = 0; c < CH; ++c, ++g) {
-          const int st = g % NSTAGE;
+        for (int c = 0; c < CH >> KSH; ++c, ++g) {
+          const int st = g % NSTAGE, kc = c + (t & ((1 << KSH) - 1)) * (CH >> KSH);
           if (!mbar_wait(&empty[st], ((g / NSTAGE) & 1) ^ 1)) {
             s_abort = 1;
             break;
           }
           unsigned char* As = smu + st * STAGE;
           mbar_expect_tx(&full[st], STAGE);
-          tma_load_5d(As, P.tmap_a, 0, 0, 2 * c, 0, ti, &full[st]);
-          tma_load_5d(As + A_STAGE, P.tmap_bs, 0, (tj & 1) * 2, 0, 2 * c, tj >> 1, &full[st]);
+          tma_load_5d(As, P.tmap_a, 0, 0, 2 * kc, 0, ti, &full[st]);
+          tma_load_5d(As + A_STAGE, P.tmap_bs, 0, (tj & 1) * 2, 0, 2 * kc, tj >> 1, &full[st]);
           issued = g + 1;
         }
         if (s_abort) break;
@@ -166,7 +172,7 @@ __global__ void __launch_bounds__(UPD_THREADS, 1)
       uint32_t g = 0, it = 0;
       const uint64_t adesc0 = smem_desc(su32(smu), 2048, 128);
       const uint64_t bdesc0 = smem_desc(su32(smu) + A_STAGE, NSLICE * 1024, 128);  // [k-group][plane][row]
-      for (int t = blockIdx.x; t < total; t += gridDim.x) {
+      for (int t = blockIdx.x; t < total << KSH; t += gridDim.x) {
         int p, ti, tj;
         tile_of(t, p, ti, tj);
         if (failed(probs[p])) continue;
@@ -176,7 +182,7 @@ __global__ void __launch_bounds__(UPD_THREADS, 1)
         }
         asm volatile("tcgen05.fence::after_thread_sync;");
         bool ok = true;
-        for (int c = 0; c < CH; ++c, ++g) {
+        for (int c = 0; c < CH >> KSH; ++c, ++g) {
           const int st = g % NSTAGE;
           if (!mbar_wait(&full[st], (g / NSTAGE) & 1)) {
             ok = false;
@@ -200,7 +206,7 @@ __global__ void __launch_bounds__(UPD_THREADS, 1)
     const int h = warp >> 2;  // column group of UPD_COLS; TMEM lanes (tile rows) 32 (warp & 3) + lane
     const uint32_t lane_base = (uint32_t)((warp & 3) * 32) << 16;
     uint32_t it = 0;
-    for (int t = blockIdx.x; t < total; t += gridDim.x) {
+    for (int t = blockIdx.x; t < total << KSH; t += gridDim.x) {
       int p, ti, tj;
       tile_of(t, p, ti, tj);
       const Prob& P = probs[p];
@@ -362,11 +368,13 @@ int encode_slice_maps(void* host_maps, const void* slices, int tiles) {
 // ---------------------------------------------------------------------------
 cudaError_t launch_ozaki_update(const Prob* probs, int nprob, int step, int max_nt128,
                                 const unsigned long long* tiles, int total_tiles, int max_ctas, cudaStream_t s) {
-  cudaError_t e = ensure_smem_attr((const void*)k_ozaki_update, SMEM_OZAKI_UPDATE, UPD_SMEM);
-  if (e != cudaSuccess) return e;
   if (max_nt128 - step - 1 <= 0 || total_tiles <= 0) return cudaSuccess;
-  const int grid = total_tiles < max_ctas ? total_tiles : max_ctas;
-  k_ozaki_update<<<grid, UPD_THREADS, UPD_SMEM, s>>>(probs, nprob, step, tiles, total_tiles);
+  const int ksh = 4 * total_tiles <= max_ctas ? 2 : (2 * total_tiles <= max_ctas ? 1 : 0);
+  const auto kernel = ksh == 2 ? k_ozaki_update<2> : (ksh == 1 ? k_ozaki_update<1> : k_ozaki_update<0>);
+  const cudaError_t e = ensure_smem_attr((const void*)kernel, SMEM_OZAKI_UPDATE + ksh, UPD_SMEM);
+  if (e != cudaSuccess) return e;
+  const int units = total_tiles << ksh, grid = units < max_ctas ? units : max_ctas;
+  kernel<<<grid, UPD_THREADS, UPD_SMEM, s>>>(probs, nprob, step, tiles, total_tiles);
   return cudaGetLastError();
 }
 
