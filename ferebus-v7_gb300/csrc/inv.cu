@@ -20,7 +20,7 @@
 // 128 x 64 x 128 tile products at the trailing update's rate (about 1 ms) and
 // four launches per doubling of the block size: 1.6 ms at N = 4000 and 0.35 at
 // N = 1003 (a gradient took 13.6 ms instead of 62.4, and 2.8 instead of 6.6,
-// with this; 6.9 and 1.4 with what else has changed since), with the same
+// with this; 6.8 and 1.3 with what else has changed since), with the same
 // errors against extended precision (7 kernels and data sets, ratio 0.7 to 1.2).
 #include "fgpu_internal.h"
 #include "tc_common.cuh"
@@ -51,33 +51,38 @@ __device__ __forceinline__ int norm_exponent(float s, bool* bad) {
 }  // namespace
 
 // ---------------------------------------------------------------------------
-// 32 x 32 diagonal inverses: one warp per block, a column per lane (496
-// multiply-adds at 64 cycles each: 16 us, all blocks side by side).  Written to
-// V's diagonal blocks; grid (nt128 * 4)
+// 32 x 32 diagonal inverses: a column per lane, every fourth row per warp, the
+// solved rows handed over in shared memory (one warp alone issues 496
+// multiply-adds at 64 cycles each: 30 us, all blocks side by side; now 17).
+// Written to V's diagonal blocks; grid (nt128 * 4) x (32, 4) threads
 // ---------------------------------------------------------------------------
-__global__ void __launch_bounds__(32) k_inv_diag32(const Prob* __restrict__ pp, double* __restrict__ V) {
+__global__ void __launch_bounds__(128) k_inv_diag32(const Prob* __restrict__ pp, double* __restrict__ V) {
   const Prob& P = *pp;
   if (P.status[1]) return;
-  const int c0 = blockIdx.x * 32, lane = threadIdx.x;
+  const int c0 = blockIdx.x * 32, lane = threadIdx.x, q = threadIdx.y;
   const size_t ld = (size_t)P.ld, nc = (size_t)P.Nc;
   const double w = ldexp(1.0, -*P.kscale);
   __shared__ double L[32][33];  // L[row][col]
-  __shared__ double rd[32];
-  for (int k = 0; k < 32; ++k) L[lane][k] = k <= lane ? P.K[(size_t)(c0 + k) * ld + c0 + lane] * w : 0.0;
-  __syncwarp();
-  rd[lane] = 1.0 / L[lane][lane];
-  __syncwarp();
-  double v[32];
+  __shared__ double rd[32], xs[32][32];
 #pragma unroll
-  for (int i = 0; i < 32; ++i) v[i] = i == lane ? 1.0 : 0.0;
+  for (int k = q; k < 32; k += 4) L[lane][k] = k <= lane ? P.K[(size_t)(c0 + k) * ld + c0 + lane] * w : 0.0;
+  __syncthreads();
+  if (q == 0) rd[lane] = 1.0 / L[lane][lane];
+  __syncthreads();
+  double v[8];  // rows q, q + 4, ..
+#pragma unroll
+  for (int m = 0; m < 8; ++m) v[m] = 4 * m + q == lane ? 1.0 : 0.0;
 #pragma unroll
   for (int k = 0; k < 32; ++k) {
-    v[k] *= rd[k];
+    if (q == (k & 3)) xs[k][lane] = v[k >> 2] *= rd[k];
+    __syncthreads();
+    const double x = xs[k][lane];
 #pragma unroll
-    for (int i = k + 1; i < 32; ++i) v[i] = fma(-L[i][k], v[k], v[i]);
+    for (int m = k >> 2; m < 8; ++m)
+      if (4 * m + q > k) v[m] = fma(-L[4 * m + q][k], x, v[m]);  // uniform in a warp
   }
 #pragma unroll
-  for (int i = 0; i < 32; ++i) V[(size_t)(c0 + lane) * nc + c0 + i] = v[i];
+  for (int m = 0; m < 8; ++m) V[(size_t)(c0 + lane) * nc + c0 + 4 * m + q] = v[m];
 }
 
 // ---------------------------------------------------------------------------
@@ -470,7 +475,7 @@ cudaError_t enqueue_inverse(const Prob* p, int nt128, const InvWorkspace& w, con
   const unsigned char* map_ca = w.tmaps + TMAP_BYTES;      // D_C as the A operand
   const unsigned char* map_cb = w.tmaps + TMAP_BYTES + 256;  // D_C as the stacked B operand
   long long n = 0;
-  k_inv_diag32<<<nt128 * 4, 32, 0, s>>>(p, w.V);
+  k_inv_diag32<<<nt128 * 4, dim3(32, 4), 0, s>>>(p, w.V);
   k_inv_diag128<<<dim3(16, nt128), 256, 0, s>>>(p, w.V);
   k_inv_diag_norms<<<dim3(nt128, 8), 128, 0, s>>>(p, w.V, w.rowpart, w.colpart);
   n += 3;
