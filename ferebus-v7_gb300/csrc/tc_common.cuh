@@ -164,15 +164,19 @@ __device__ __forceinline__ long long to_fixed54(double x, int e) {
   return (to_fixed55(x, e, &bad) + 1) >> 1;
 }
 
-// a diagonal entry: kernel value plus nugget.  NaN becomes negative, which
-// fails that pivot as NaN does in dpotrf.
+// a diagonal entry: kernel value plus nugget, exact up to the matrix's unit.  The
+// scale is their sum's: where they cancel (a nugget below zero) neither need
+// fit it, and what is converted is their sum and its rounding error.  NaN
+// becomes negative, which fails that pivot as NaN does in dpotrf.
 __device__ __forceinline__ long long diag_fixed62(double k, double noise, int e, bool* nonfinite) {
   const double d = k + noise;
   if (d != d) {
     *nonfinite = true;
     return -(1LL << 61);
   }
-  return to_fixed62(k, e, nonfinite) + to_fixed62(noise, e, nonfinite);
+  if (fmax(fabs(k), fabs(noise)) < ldexp(1.0, e)) return to_fixed62(k, e, nonfinite) + to_fixed62(noise, e, nonfinite);
+  const double t = d - k;
+  return to_fixed62(d, e, nonfinite) + to_fixed62((k - (d - t)) + (noise - t), e, nonfinite);
 }
 
 // T 2^(e - 62) rounded to the nearest double (ties away from zero), T a signed
