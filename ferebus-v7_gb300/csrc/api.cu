@@ -194,6 +194,7 @@ struct Workspace {
   unsigned char* slices = nullptr;
   unsigned char* tmaps = nullptr;  // TMA tensor maps over slices (128-, 64-row boxes; 64 rows, planes stacked)
   double* rhs = nullptr;           // right-hand sides
+  int* rowsq = nullptr;            // the factor rows' sums of squares
   double* ldiag = nullptr;         // the kept factor's diagonal
   PanelBlock* lpub = nullptr;      // the current panel's published diagonal blocks
   PanelZ* zpub = nullptr;          // and solved right-hand-side entries
@@ -364,6 +365,7 @@ void fill_prob(Prob& p, const fgpu_ctx* c, const double* theta_d, const Workspac
   p.tmap_bs = ws.tmaps ? ws.tmaps + 256 : nullptr;
   p.tmap_b16 = ws.tmaps ? ws.tmaps + 384 : nullptr;
   p.rhs = ws.rhs;
+  p.rowsq = ws.rowsq;
   p.ldiag = ws.ldiag;
   p.lpub = ws.lpub;
   p.zpub = ws.zpub;
@@ -717,6 +719,7 @@ size_t layout_workspace(const fgpu_ctx* c, unsigned char* base, Workspace& ws, b
   if (c->mode == 1) {
     take(ws.kscale, sizeof(int) * 2);
     take(ws.rhs, sizeof(double) * MAX_RHS * nc);
+    take(ws.rowsq, sizeof(int) * nc);
     if (keep_l) take(ws.ldiag, sizeof(double) * nc);
     take(ws.lpub, sizeof(PanelBlock) * 8);
     take(ws.zpub, sizeof(PanelZ) * 8);

@@ -248,6 +248,7 @@ __global__ void __launch_bounds__(NB * PREP_Y) k_prep(const Prob* __restrict__ p
     const double u = ldexp(1.0, -s_k);
     P.rhs[i] = i < P.N ? u * (P.likelihood == 1 ? P.y[i] : P.y[i] - P.mu[i]) : 0.0;
     if (P.nrhs > 1) P.rhs[nc + i] = i < P.N ? u : 0.0;
+    P.rowsq[i] = 0;
   }
   if (!sp.tc_build) {
     // the dot-product build's scaled planes and rbf norms (the workspace is not

@@ -111,6 +111,7 @@ struct Prob {
   const void* tmap_bs;            // box of 64 rows landing as [k-group][plane][row]: the 7 planes stacked along N
   const void* tmap_b16;           // same, box of 16 rows
   double* rhs;                    // MAX_RHS x Nc: right-hand sides times 2^-e, turned into L^-1 r panel by panel
+  int* rowsq;                     // Nc: sums of squares of the factor's rows so far (panel.cu)
   PanelBlock* lpub;               // 8: the current panel's diagonal blocks, as its diagonal tile publishes them
   PanelZ* zpub;                   // 8: and its solved right-hand-side entries
   int keep_l;                     // K exists and receives the factor, as 60-bit fixed point (launch_factor_doubles)

@@ -37,6 +37,10 @@
 // The dropped Xl Ll and the final shifts err by a few 2^-61, well below the
 // 2^-56 to which x is rounded for the trailing update.  The 64-bit sums cannot
 // overflow: rows of L' have norm at most 1, so sum |Xh Ll| <= 2^30 2^29 4.
+// That holds while K is positive definite.  Schur complements are kept modulo 4 in
+// the matrix's unit, so a row of an indefinite matrix, whose entries' squares
+// add up far beyond K_ii, could come round to a positive pivot: every row
+// keeps the sum of its squares (rowsq), and one that is beyond K_ii fails the pivot.
 // Only the right-hand sides' substitution (32 operations per piece, off the
 // critical path) and their running sums (one per row and piece) are FP64.
 //
@@ -172,6 +176,26 @@ __device__ __forceinline__ void mac_row(long long& S, long long& M, const int (&
       if (c + 1 < n) mac_entry(S, M, Xh[c + 1], Xl[c + 1], v.z, v.w);
     }
   }
+}
+
+// A row's sum of squares, sum_{k <= i} x_ik^2 = K_ii < 1 where the leading minors are
+// positive, in units of 2^-SQ_BITS, cut off every 8 entries (16 2^-22 a panel).  The
+// pivot K_ii - sum_{k < i} is formed modulo 4: one that came round shows in the
+// sum, and one that did not is negative where the matrix is not positive
+// definite.  That holds whatever the row's entries were: until one of them clamps
+// they are exact, right-hand sides beyond the range +-2 (but below 1 +
+// SQ_LIMIT^1/2 = 2.2) come round to ones that clamp, and a clamped entry adds 1.
+// 8 multiply-adds and 3 instructions per 8 entries, off the pivots' chain but for
+// the diagonal block's rows.
+constexpr int SQ_BITS = 22;
+constexpr int SQ_LIMIT = (1 << SQ_BITS) + (1 << (SQ_BITS - 2));  // 1.25
+constexpr int SQ_MAX = 1 << 30;                                  // where the stored sum saturates
+template <int c0>
+__device__ __forceinline__ int squares8(const int (&Xh)[PW]) {
+  unsigned long long q = 0;  // 2^-60; at most 8
+#pragma unroll
+  for (int c = c0; c < c0 + 8; ++c) q += (unsigned long long)((long long)Xh[c] * Xh[c]);
+  return (int)(q >> (60 - SQ_BITS));
 }
 
 // the digit planes of 8 entries X = x 2^60 of a row
@@ -344,6 +368,7 @@ __global__ void __launch_bounds__(PN_THREADS, 1)
     double r0 = 0.0, r1 = 0.0;  // sum_k L_ik z_k; the diagonal tile: the entries themselves
     const bool two = P.nrhs > 1;
     const double rhs0 = P.rhs[i], rhs1 = two ? P.rhs[P.Nc + i] : 0.0;
+    int sq = P.rowsq[i];  // the row's squares so far
     bool live = true;
     auto wait = [&](uint64_t* bar, int parity) -> bool {
       const int r = wait_or_stop(bar, (uint32_t)parity, &s_stop);
@@ -468,6 +493,10 @@ __global__ void __launch_bounds__(PN_THREADS, 1)
             }
           }
         }
+        // the block's rows, their own entries included: K_ii, or 4 and more beyond it if the pivot came round
+        sq += squares8<0>(Xh) + squares8<8>(Xh);
+        const unsigned over = (__ballot_sync(0xffffffffu, sq > SQ_LIMIT) >> base) & 0xFFFF;
+        if (over) fail = min(fail, __ffs(over) - 1);
         if (fail < PW) {
           if (lane == 0) {
             P.status[0] = c0 + t * PW + fail + 1;  // LAPACK info: 1-based column
@@ -580,6 +609,7 @@ __global__ void __launch_bounds__(PN_THREADS, 1)
           }
           __syncwarp();
           if (lane == 0) mbar_arrive(b_digits);
+          if (!done && !pivot) sq += squares8<0>(Xh) + squares8<8>(Xh);
         }
       }
       if (out || tail) break;
@@ -604,6 +634,7 @@ __global__ void __launch_bounds__(PN_THREADS, 1)
       if (rl >= np * PW) P.ldiag[i] = ldexp(0.5, kexp);
     }
     if (!diag && live) {
+      P.rowsq[i] = min(sq, SQ_MAX);
       P.rhs[i] = rhs0 - r0;
       if (two) P.rhs[P.Nc + i] = rhs1 - r1;
     }
@@ -892,6 +923,7 @@ __global__ void __launch_bounds__(PR_THREADS, 2)
     const uint32_t trow = tmem + ((uint32_t)(warp * 32) << 16);
     const bool two = P.nrhs > 1;
     double r0 = 0.0, r1 = 0.0;  // sum_k L'_ik z_k
+    int sq = 0;                 // the row's squares
     bool live = true;
     auto wait = [&](uint64_t* bar, int parity) -> bool {
       const int r = wait_or_stop(bar, (uint32_t)parity, &s_stop);
@@ -941,6 +973,7 @@ __global__ void __launch_bounds__(PR_THREADS, 2)
       asm volatile("fence.proxy.async;" ::: "memory");  // digits visible to the MMAs and to the TMA reloads
       __syncwarp();
       if (lane == 0) mbar_arrive(b_digits);
+      sq += squares8<0>(Xh) + squares8<8>(Xh);
       // the right-hand sides: sum_k L'_ik z_k, z in 60-bit fixed point of the piece's scale
       const PanelZ& Z = Zs[t];
       long long S = 0, M = 0;
@@ -955,6 +988,7 @@ __global__ void __launch_bounds__(PR_THREADS, 2)
       }
     }
     if (live) {
+      P.rowsq[i] = min(P.rowsq[i] + sq, SQ_MAX);
       P.rhs[i] -= r0;
       if (two) P.rhs[P.Nc + i] -= r1;
     }
