@@ -231,7 +231,7 @@ __global__ void __launch_bounds__(NB * PREP_Y) k_prep(const Prob* __restrict__ p
     const double d = (sp.tc_build ? (stk[0][3] + stk[0][2]) + (stk[0][1] + stk[0][0]) : stk[0][0]) +
                      (P.optimise_noise ? P.theta[sp.nkparams] : P.noise);
     int e = 0;
-    if (d > 0.0 && d < 1e300) frexp(sqrt(d) * (1.0 + 0x1p-20), &e);  // sqrt(K_ii) (1 + 2^-20) < 2^e
+    if (d > 0.0 && d < INFINITY) frexp(sqrt(d) * (1.0 + 0x1p-20), &e);  // sqrt(K_ii) (1 + 2^-20) < 2^e
     s_k = e;
     if (rb == 0) P.kscale[0] = e;
   }

@@ -167,12 +167,13 @@ __device__ __forceinline__ long long to_fixed54(double x, int e) {
 // a diagonal entry: kernel value plus nugget, exact up to the matrix's unit.  The
 // scale is their sum's: where they cancel (a nugget below zero) neither need
 // fit it, and what is converted is their sum and its rounding error.  NaN
-// becomes negative, which fails that pivot as NaN does in dpotrf.
+// becomes negative, which fails that pivot as NaN does in dpotrf; infinity only
+// sets *nonfinite.
 __device__ __forceinline__ long long diag_fixed62(double k, double noise, int e, bool* nonfinite) {
   const double d = k + noise;
-  if (d != d) {
+  if (!(fabs(d) < INFINITY)) {
     *nonfinite = true;
-    return -(1LL << 61);
+    return d > 0.0 ? (1LL << 62) - 1 : -(1LL << 61);
   }
   if (fmax(fabs(k), fabs(noise)) < ldexp(1.0, e)) return to_fixed62(k, e, nonfinite) + to_fixed62(noise, e, nonfinite);
   const double t = d - k;

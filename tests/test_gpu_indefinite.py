@@ -97,3 +97,23 @@ def test_row_beyond_its_diagonal(layout, m, lib):
     for k, (got, info) in enumerate(want * reps):
         assert ib[k] == info
         assert lb[k] == got or (info and np.isnan(lb[k]))
+
+
+@pytest.mark.parametrize("nugget", [1e200, 1e299, 1e301, 1.5e308])
+@pytest.mark.parametrize("n", [20, 150])
+def test_huge_diagonal(nugget, n, lib):
+    """The scale follows K_ii through the whole range of doubles; an infinite K_ii fails."""
+    from fgpu import Engine
+    from fgpu._lib import FgpuError
+    rng = np.random.default_rng(3)
+    X, y = rng.normal(size=(n, 3)), rng.normal(size=n)
+    ks, th = [O.RBF, 3, 1, 2, 3], np.zeros(3)
+    ref, _ = O.loglik(ks, th, X, y, np.zeros(n), 0, nugget, False)
+    ll, info = Engine(X, y, np.zeros(n), ks, 0, nugget, False).loglik(th)
+    assert info == 0
+    assert abs(ll - ref) <= 1e-9 * abs(ref), (ll, ref)
+    try:
+        ll, info = Engine(X, y, np.zeros(n), ks, 0, np.inf, False).loglik(th)
+    except FgpuError:
+        return
+    assert info > 0 and np.isnan(ll)
