@@ -85,8 +85,9 @@ __device__ __forceinline__ int ld_acquire(const int* p) {
   asm volatile("ld.acquire.gpu.global.s32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
   return v;
 }
-__device__ __forceinline__ void st_release(int* p, int v) {
-  asm volatile("st.release.gpu.global.s32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
+// raise a counter to v: FLAG_FAIL stays, whatever the diagonal tile's other warps still publish
+__device__ __forceinline__ void publish(int* p, int v) {
+  asm volatile("red.release.gpu.global.max.s32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
 }
 __device__ __forceinline__ void cp_async16(void* dst, const void* src) {
   asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(su32(dst)), "l"(src) : "memory");
@@ -503,7 +504,7 @@ __global__ void __launch_bounds__(PN_THREADS, 1)
             P.status[1] = 1;
             s_stop = 1;
             __threadfence();
-            for (int f = 0; f < 3; ++f) st_release(&fl[f], FLAG_FAIL);
+            for (int f = 0; f < 3; ++f) publish(&fl[f], FLAG_FAIL);
           }
           live = false;
           break;
@@ -712,7 +713,7 @@ __global__ void __launch_bounds__(PN_THREADS, 1)
           mma_commit(b_mma);
           // the row warps' digits, written to HBM before they arrived (release:
           // cumulative over what this warp has observed)
-          if (diag) st_release(&fl[FLAG_D], fbase + t + 1);
+          if (diag) publish(&fl[FLAG_D], fbase + t + 1);
         }
         __syncwarp();
       } else if (!diag) {
@@ -761,7 +762,7 @@ __global__ void __launch_bounds__(PN_THREADS, 1)
         uint4* dst = reinterpret_cast<uint4*>(P.lpub + t);
         for (int q = lane; q < (int)PN_LBYTES / 16; q += 32) dst[q] = src[q];
         __syncwarp();
-        if (lane == 0) st_release(&fl[FLAG_L], fbase + t + 1);
+        if (lane == 0) publish(&fl[FLAG_L], fbase + t + 1);
       }
       // row j of the block, and 1 / L'_jj = y 2^(sh - 62), as doubles
       double lrow[PW];
@@ -810,7 +811,7 @@ __global__ void __launch_bounds__(PN_THREADS, 1)
       __syncwarp();
       if (lane == 0) {
         mbar_arrive(b_z);
-        st_release(&fl[FLAG_Z], fbase + t + 1);
+        publish(&fl[FLAG_Z], fbase + t + 1);
       }
       if (c0 + t * PW + j < P.N) {  // not the identity padding
         esum += (int)(lb >> 52) - 1023 + 2 * ke;
@@ -831,7 +832,7 @@ __global__ void __launch_bounds__(PN_THREADS, 1)
     // a bounded wait gave up: report, and release the problem's other CTAs
     atomicExch(&P.status[2], 1);
     __threadfence();
-    for (int f = 0; f < 3; ++f) st_release(&fl[f], FLAG_FAIL);
+    for (int f = 0; f < 3; ++f) publish(&fl[f], FLAG_FAIL);
   }
   asm volatile("tcgen05.fence::after_thread_sync;");
   if (warp == PN_MMA_WARP) __syncwarp();
