@@ -668,6 +668,7 @@ __global__ void __launch_bounds__(PN_THREADS, 1)
         const int v = poll_flag(&fl[f], fbase + t + 1);
         r = v < 0 ? 2 : (v >= FLAG_FAIL ? 1 : 0);
       }
+      __syncwarp();  // the other lanes' reads come after lane 0's acquire too
       return __shfl_sync(0xffffffffu, r, 0);
     };
     int st = 0;  // 1: the problem failed, 2: a wait gave up
