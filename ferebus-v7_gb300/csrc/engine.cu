@@ -631,7 +631,6 @@ __device__ __forceinline__ void bar_arrive(int id, int n) {
 }
 __global__ void __launch_bounds__(256) k_backsolve(const Prob* __restrict__ pp, int* __restrict__ sync) {
   const Prob& P = *pp;
-  if (P.status[1] || P.status[2]) return;
   extern __shared__ __align__(16) double Ms[];  // [c][r], c > r: L_cr / L_rr
   __shared__ double rd[TB], xs[TB], part_sum[4][TB];
   __shared__ int s_b, s_done[2], s_fail;
@@ -639,11 +638,15 @@ __global__ void __launch_bounds__(256) k_backsolve(const Prob* __restrict__ pp, 
   // of the threads (group) wait for their half of a block's rows only
   const int tid = threadIdx.x, c = tid & 63, part = tid >> 6, group = tid >> 7, lane = tid & 31;
   if (tid == 0) {
-    s_b = P.nsteps - 1 - atomicAdd(&sync[0], 1);
+    // one read of the status, which another CTA's give-up may set meanwhile: the
+    // whole CTA leaves or stays
+    const volatile int* st = P.status;
+    s_b = st[1] || st[2] ? -1 : P.nsteps - 1 - atomicAdd(&sync[0], 1);
     s_fail = 0;
   }
   __syncthreads();
   const int b = s_b;
+  if (b < 0) return;
   const size_t ld = (size_t)P.ld;
   const double* Ld = P.K + (size_t)(b * TB) * ld + b * TB;
   if (tid < TB) rd[tid] = 1.0 / Ld[(size_t)tid * ld + tid];
