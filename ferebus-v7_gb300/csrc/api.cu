@@ -740,6 +740,14 @@ size_t workspace_bytes(const fgpu_ctx* c, bool keep_l) {
   return layout_workspace(c, nullptr, tmp, keep_l);
 }
 
+// cudaMemcpy from pageable memory returns once the data are staged, and the copy to
+// the device may follow later; the evaluations run on streams that do not wait
+// for the legacy stream it is in.  Called at the end of whatever sets a context, a
+// worker or a plan up, so that no kernel reads a descriptor, a table or a
+// tensor map that has not arrived (with six processes on one GPU every
+// fifth first call did).
+cudaError_t uploads_done() { return cudaStreamSynchronize(cudaStreamLegacy); }
+
 // Encode the problem's TMA tensor maps over ws.slices into the TMAP_BYTES
 // device bytes at `dst` (tensor-core mode only).
 int write_tmaps(const fgpu_ctx* c, const Workspace& ws, unsigned char* dst) {
@@ -823,6 +831,7 @@ int make_worker(fgpu_ctx* c, Worker** out) {
   if (c->mode == 1 &&
       (rc = build_sched(std::vector<int>{c->nt128}, std::vector<int>{c->spec.tc_build}, w->sched, nullptr)) != 0)
     return bail(rc);
+  if (uploads_done() != cudaSuccess) return bail(fail(FGPU_ECUDA, "worker uploads"));
   w->sched.keep_l = true;
   if ((rc = capture(w->stream, &w->graph, w->prob_d, 1, c->nsteps, c->spec.nplanes, w->ws.status,
                     sizeof(int) * 4, &w->graph_kernels, nullptr, c->mode, &w->sched)) != 0)
@@ -1022,6 +1031,7 @@ int fgpu_create(fgpu_ctx** out, int N, int d, const double* X, const double* y, 
   CK(cudaMemcpy(c->mu_d, mv.data(), c->Nc * sizeof(double), cudaMemcpyHostToDevice));
   CK(cudaMalloc(&c->spec_d, sizeof(Spec)));
   CK(cudaMemcpy(c->spec_d, &c->spec, sizeof(Spec), cudaMemcpyHostToDevice));
+  CK(uploads_done());
   *out = c.release();
   return 0;
 }
@@ -1212,6 +1222,7 @@ int make_grad_ws(fgpu_ctx* c, bool tc, GradWS** out) {
   p.ldkinv = tc ? c->Nc : g->Nc;
   p.gpart = g->gpart;
   CK(cudaMemcpy(g->prob_d, &p, sizeof(Prob), cudaMemcpyHostToDevice));
+  CK(uploads_done());
   *out = g.release();
   return 0;
 }
@@ -1433,6 +1444,7 @@ int fgpu_plan_create(fgpu_plan** out, fgpu_ctx* const* ctxs, int nprob, int ldth
       if ((rc = build_sched(nts, tcs, w.sched, &p->allocations)) != 0) return bail(rc);
     }
   }
+  PL_CK(uploads_done());
 #undef PL_CK
   if ((rc = capture_plan(p.get(), &p->graph, &p->graph_kernels, nullptr)) != 0) return bail(rc);
   *out = p.release();
