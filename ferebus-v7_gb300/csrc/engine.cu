@@ -312,7 +312,8 @@ __global__ void __launch_bounds__(256) k_build_dot(const Prob* __restrict__ prob
         if (tok >= 0) {
           const Leaf& L = sp.leaf[tok];
           if (L.type == L_RBF_CYCLIC) {
-            long long H[2] = {0, 0}, M[2] = {0, 0};
+            unsigned long long H[2] = {0, 0};  // 192 features' 2^56: not within 63 bits
+            long long M[2] = {0, 0};
             const longlong2* fi = reinterpret_cast<const longlong2*>(Pi + L.plane0 * TB + r0);
             const long long* fj = reinterpret_cast<const long long*>(Pj + L.plane0 * TB + c);
             for (int k = 0; k < L.n; ++k) {
@@ -333,7 +334,7 @@ __global__ void __launch_bounds__(256) k_build_dot(const Prob* __restrict__ prob
               for (int a = 0; a < 2; ++a) {
                 const int hh = (int)((D[a] + (1LL << 26)) >> 27);
                 const int l = (int)((unsigned)D[a] - ((unsigned)hh << 27));
-                H[a] += (long long)hh * hh;
+                H[a] += (unsigned long long)((long long)hh * hh);
                 M[a] += (long long)hh * l + (((long long)l * l) >> 28);
               }
             }
@@ -341,7 +342,7 @@ __global__ void __launch_bounds__(256) k_build_dot(const Prob* __restrict__ prob
             for (int a = 0; a < 2; ++a)
               stk[a][top] = Ni[tok * TB + r0 + a] != 0.0 || Nj[tok * TB + c] != 0.0
                                 ? nan("")
-                                : iexp_fixed_tab((unsigned long long)(H[a] + (M[a] >> 26)), sc, g_iexp_tab1024, g_iexp_fine1024);
+                                : iexp_fixed_tab(H[a] + (unsigned long long)(M[a] >> 26), sc, g_iexp_tab1024, g_iexp_fine1024);
           } else if (L.type == L_RBF || L.type == L_PERIODIC) {
             const int nf = L.type == L_PERIODIC ? 2 * L.n : L.n;
             double dot[2] = {0.0, 0.0};

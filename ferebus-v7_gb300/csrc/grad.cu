@@ -318,9 +318,10 @@ __global__ void __launch_bounds__(256, PER_SM)
     if (d < sp.ndot) {
       const Leaf& L = sp.leaf[sp.dot_leaf[d]];
       const int nf = L.type == L_PERIODIC ? 2 * L.n : L.n;
-      long long H[16], M[16];
+      unsigned long long H[16];  // 128 features' 2^56
+      long long M[16];
 #pragma unroll
-      for (int e = 0; e < 16; ++e) H[e] = M[e] = 0;
+      for (int e = 0; e < 16; ++e) H[e] = 0, M[e] = 0;
       for (int k0 = 0; k0 < nf; k0 += GF_CH) {
         const int kn = min(GF_CH, nf - k0);
         __syncthreads();
@@ -340,7 +341,7 @@ __global__ void __launch_bounds__(256, PER_SM)
               const long long D = (a ? fi.y : fi.x) - fj;
               const int h = (int)((D + (1LL << 26)) >> 27);
               const int l = (int)D - (int)((unsigned)h << 27);
-              H[c * 2 + a] += (long long)h * h;
+              H[c * 2 + a] += (unsigned long long)((long long)h * h);
               M[c * 2 + a] += (long long)h * l + (((long long)l * l) >> 28);
             }
           }
@@ -350,7 +351,7 @@ __global__ void __launch_bounds__(256, PER_SM)
       const IexpScale sc = iexp_scale(2 * Q.fscale[d] - 55);
 #pragma unroll
       for (int e = 0; e < 16; ++e)
-        v[d][e] = iexp_fixed_tab((unsigned long long)(H[e] + (M[e] >> 26)), sc, g_iexp_tab1024, g_iexp_fine1024);
+        v[d][e] = iexp_fixed_tab(H[e] + (unsigned long long)(M[e] >> 26), sc, g_iexp_tab1024, g_iexp_fine1024);
     }
   }
   // weights: w dk/dv_d v_d, and the sums the linear and constant leaves need

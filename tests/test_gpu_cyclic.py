@@ -53,3 +53,22 @@ def test_point_that_is_not_finite(col, lib):
     except FgpuError:
         return
     assert info > 0 and np.isnan(ll)
+
+
+def test_squared_distance_beyond_63_bits(lib):
+    """192 features at the opposite ends of their scale: the sum of the squares takes
+    64 bits."""
+    from fgpu import Engine
+    d, n = 192, 70
+    rng = np.random.default_rng(3)
+    X = np.where(np.arange(n)[:, None] % 2, 0.9999, -0.9999) * np.ones((n, d))
+    X[:, 2::3] = np.where(np.arange(n)[:, None] % 2, np.pi, 0.0)
+    X[:, 0] = rng.uniform(-0.9, 0.9, size=n)
+    y = rng.normal(size=n)
+    ks = [O.RBF_CYCLIC, d, *range(1, d + 1)]
+    for t in (0.0, -0.91, -8.0):  # -0.91: the wrapped differences fill their scale
+        th = np.full(d, t)
+        ll, info = Engine(X, y, np.zeros(n), ks, 0, 1e-2, False).loglik(th)
+        ref, rinfo = O.loglik(ks, th, X, y, np.zeros(n), 0, 1e-2, False)
+        assert info == rinfo == 0
+        assert abs(ll - ref) <= 1e-9 * abs(ref), (t, ll, ref)
