@@ -152,8 +152,10 @@ __global__ void __launch_bounds__(NB * PREP_Y) k_prep(const Prob* __restrict__ p
     for (int l = d; !sp.tc_build && l < sp.nleaf; l += 2) {
       const Leaf& L = sp.leaf[l];
       double m = 0.0, c = 0.0;
+      bool huge = false;  // or NaN, which fmax passes over
       for (int k = lane; k < L.n; k += 32) {
         const double u = w[L.param0 + k];
+        huge |= !(u < 0x1p900);
         if (L.type == L_RBF_CYCLIC)
           m = fmax(m, u * (sp.cyclic[L.plane0 + k] ? 1.5707963267948966 : P.plane_max[L.plane0 + k]));
         else
@@ -164,9 +166,10 @@ __global__ void __launch_bounds__(NB * PREP_Y) k_prep(const Prob* __restrict__ p
         c += __shfl_xor_sync(0xffffffffu, c, o);
       }
       const int s = m == 0.0 ? 0 : (int)((__double_as_longlong(m) >> 52) & 0x7FF) - 1022;
+      huge = __any_sync(0xffffffffu, huge || !(m < 0x1p900));
       if (lane == 0) {
         s_c[l] = s;
-        s_huge[l] = !(m < 0x1p900);
+        s_huge[l] = huge;
         if (rb == 0) {
           P.dotc->leaf_c[l] = L.type == L_CONSTANT ? w[L.param0] : c;
           P.dotc->scale[l] = s;

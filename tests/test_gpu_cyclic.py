@@ -72,3 +72,22 @@ def test_squared_distance_beyond_63_bits(lib):
         ref, rinfo = O.loglik(ks, th, X, y, np.zeros(n), 0, 1e-2, False)
         assert info == rinfo == 0
         assert abs(ll - ref) <= 1e-9 * abs(ref), (t, ll, ref)
+
+
+@pytest.mark.parametrize("value", [np.nan, np.inf, 2000.0])
+@pytest.mark.parametrize("col", [0, 2])
+def test_weight_that_is_not_usable(col, value, lib):
+    """A plan takes theta as it is: NaN and weights beyond any scale fail the problem they belong to,
+    whichever feature they are of."""
+    from fgpu import Engine, Plan
+    from fgpu._lib import FgpuError
+    X, y = _data(80, 9, 5)
+    e = Engine(X, y, np.zeros(80), [O.RBF_CYCLIC, 9, *range(1, 10)], 0, 1e-3, False)
+    th = np.full((2, 9), 0.5)
+    th[1, col] = value
+    try:
+        ll, info = Plan([e, e]).run(th)
+    except FgpuError:
+        return
+    assert info[1] > 0 and np.isnan(ll[1])
+    assert info[0] == 0 and ll[0] == e.loglik(th[0])[0]
