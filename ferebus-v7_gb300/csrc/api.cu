@@ -894,6 +894,52 @@ void free_grad_ws(GradWS* g) {
   if (g->stream) cudaStreamDestroy(g->stream);
   delete g;
 }
+// A feature of an rbf-cyclic leaf as 64-bit integers u (in dst's bits), so that
+// differences are exact: x_i - x_j = (u_i - u_j) 2^-64 g, and the return value is g.
+// Wrapped ones are fractions of a turn, modulo 1, g = 2 pi (the double that the
+// reference wraps by, distance_matrix.f90:95-128), the others distances from the
+// finite values' mean, |u| <= 2^62, g the power of two that takes.  A value that
+// is not finite becomes TURN_NOT_FINITE, which none of the others is.
+double fixed_feature(const double* x, int N, bool wrapped, double* dst) {
+  auto put = [&](int i, unsigned long long u) { memcpy(&dst[i], &u, 8); };
+  if (wrapped) {
+    // 1 / g in two parts; a fraction is below 1, and its product's error known
+    constexpr double g = 6.283185307179586, HI = 0.15915494309189535, LO = -3.635205175920738e-18;
+    for (int i = 0; i < N; ++i) {
+      if (!std::isfinite(x[i])) {
+        put(i, TURN_NOT_FINITE);
+        continue;
+      }
+      const double r = std::fmod(x[i], g), q = r * HI, err = std::fma(r, HI, -q) + r * LO;
+      const double h = q * 0x1p63;  // |q| < 1 + 2^-52
+      const long long t = (long long)std::max(std::min(h, 0x1.fffffffffffffp62), -0x1p63);
+      unsigned long long u = 2ULL * (unsigned long long)t + (unsigned long long)std::llrint(2.0 * (h - (double)t) + std::ldexp(err, 64));
+      if (u == TURN_NOT_FINITE) ++u;  // half a turn, to 2^-64
+      put(i, u);
+    }
+    return g;
+  }
+  double mean = 0.0, top = 0.0;
+  int n = 0;
+  for (int i = 0; i < N; ++i)
+    if (std::isfinite(x[i])) mean += x[i], ++n;
+  mean = n ? mean / n : 0.0;
+  if (!std::isfinite(mean)) mean = 0.0;
+  for (int i = 0; i < N; ++i)
+    if (std::isfinite(x[i])) top = std::max(top, std::fabs(x[i] - mean));
+  int r = 0;
+  std::frexp(top * (1.0 + 0x1p-50), &r);  // |x - mean| < 2^r
+  for (int i = 0; i < N; ++i) {
+    const double d = x[i] - mean, t = d - x[i], err = (x[i] - (d - t)) - (mean + t);
+    if (!std::isfinite(d)) {
+      put(i, TURN_NOT_FINITE);
+      continue;
+    }
+    put(i, (unsigned long long)(std::llrint(std::ldexp(d, 62 - r)) + std::llrint(std::ldexp(err, 62 - r))));
+  }
+  return top == 0.0 ? 0.0 : std::ldexp(1.0, r + 2);
+}
+
 struct GradWSDeleter {
   void operator()(GradWS* g) const { free_grad_ws(g); }
 };
@@ -944,12 +990,13 @@ int fgpu_create(fgpu_ctx** out, int N, int d, const double* X, const double* y, 
   c->nkparams = c->spec.nkparams;
   c->ntheta = c->nkparams + c->optimise_noise;
   // feature planes, plane-major, padded to Nc.  FP64 mode: x, or the
-  // half-angle pair sin(x/2), cos(x/2) for periodic dims.  Tensor-core mode
-  // rbf and unwrapped rbf-cyclic dims centred on their mean, periodic dims as
-  // the pair cos(x), sin(x), wrapped rbf-cyclic dims as fractions of a turn.
+  // half-angle pair sin(x/2), cos(x/2) for periodic dims.  Tensor-core mode:
+  // rbf dims centred on their mean, periodic dims as the pair cos(x), sin(x),
+  // rbf-cyclic dims as 64-bit integers.
   const int np = c->spec.nplanes;
   std::vector<double> planes((size_t)std::max(np, 1) * c->Nc, 0.0);
   std::vector<int> plane_leaf(np, 0);
+  std::vector<double> cyclic_range(np, 0.0);
   for (int l = 0; l < c->spec.nleaf; ++l) {
     const Leaf& L = c->spec.leaf[l];
     const int cnt = L.type == FGPU_PERIODIC ? 2 * L.n : (L.type == FGPU_LINEAR || L.type == FGPU_CONSTANT ? 0 : L.n);
@@ -958,24 +1005,11 @@ int fgpu_create(fgpu_ctx** out, int N, int d, const double* X, const double* y, 
   for (int p = 0; p < np; ++p) {
     const double* col = X + (size_t)plane_dim[p] * N;  // X(:, dim), column-major
     double* dst = planes.data() + (size_t)p * c->Nc;
-    if (c->mode == 1 && plane_kind[p] == 3) {
-      // a wrapped rbf-cyclic feature: x / (2 pi) modulo 1 as a 64-bit fraction,
-      // so that differences wrap as integers (the product carries its error,
-      // and 1 / (2 pi) its tail)
-      constexpr double HI = 0.15915494309189535, LO = -9.839338337591243e-18;
-      for (int i = 0; i < N; ++i) {
-        const double q = col[i] * HI, err = std::fma(col[i], HI, -q) + col[i] * LO;
-        unsigned long long u = TURN_NOT_FINITE;
-        if (std::isfinite(q)) {
-          const double f = q - std::floor(q);  // exact
-          u = (unsigned long long)(f * 0x1p63) * 2ULL + (unsigned long long)(long long)std::llrint(std::ldexp(err, 64));
-          if (u == TURN_NOT_FINITE) ++u;  // half a turn, to 2^-64
-        }
-        memcpy(&dst[i], &u, 8);
-      }
+    if (c->mode == 1 && plane_leaf[p] == FGPU_RBF_CYCLIC) {
+      cyclic_range[p] = fixed_feature(col, N, plane_kind[p] == 3, dst);
       continue;
     }
-    if (c->mode == 1 && (plane_leaf[p] == FGPU_RBF || plane_leaf[p] == FGPU_RBF_CYCLIC)) {
+    if (c->mode == 1 && plane_leaf[p] == FGPU_RBF) {
       double mean = 0.0;
       for (int i = 0; i < N; ++i) mean += col[i];
       mean /= N;
@@ -1005,8 +1039,13 @@ int fgpu_create(fgpu_ctx** out, int N, int d, const double* X, const double* y, 
   CK(cudaMemcpy(c->planes_d, planes.data(), planes.size() * sizeof(double), cudaMemcpyHostToDevice));
   {
     std::vector<double> pmax(std::max(np, 1), 0.0);
-    for (int p = 0; p < np; ++p)
-      for (int i = 0; i < N && !(c->mode == 1 && plane_kind[p] == 3); ++i) pmax[p] = std::max(pmax[p], std::fabs(planes[(size_t)p * c->Nc + i]));
+    for (int p = 0; p < np; ++p) {
+      if (c->mode == 1 && plane_leaf[p] == FGPU_RBF_CYCLIC) {
+        pmax[p] = cyclic_range[p];
+        continue;
+      }
+      for (int i = 0; i < N; ++i) pmax[p] = std::max(pmax[p], std::fabs(planes[(size_t)p * c->Nc + i]));
+    }
     CK(cudaMalloc(&c->plane_max_d, pmax.size() * sizeof(double)));
     CK(cudaMemcpy(c->plane_max_d, pmax.data(), pmax.size() * sizeof(double), cudaMemcpyHostToDevice));
   }

@@ -113,8 +113,9 @@ __global__ void __launch_bounds__(NB * PREP_Y) k_prep(const Prob* __restrict__ p
   const size_t nc = (size_t)P.Nc;
   __shared__ double w[MAX_PARAMS];  // rbf, rbf-cyclic sqrt(exp(theta)), periodic 1 / exp(theta), linear 1 / c, constant theta
   int form = FORM_FP64;  // thread 0
-  __shared__ int s_e[2], s_k, s_c[MAX_LEAF];
+  __shared__ int s_e[2], s_k;
   __shared__ bool s_huge[MAX_LEAF];
+  __shared__ long long s_mul[MAX_PLANES];
   __shared__ int s_lev[2][PREP_Y][NLEV][NB];
   for (int q = y * NB + tid; q < sp.nkparams; q += NB * PREP_Y) {
     int type = L_CONSTANT;
@@ -147,8 +148,9 @@ __global__ void __launch_bounds__(NB * PREP_Y) k_prep(const Prob* __restrict__ p
         if (rb == 0) P.fscale[d] = s_e[d];
       }
     }
-    // the dot-product build's constants; rbf-cyclic leaves get a scale too, a
-    // wrapped feature counting as pi / 2 (its difference is at most pi)
+    // the dot-product build's constants.  rbf-cyclic: |weighted difference| <= m <
+    // 2^q; in units of 2^-t, t = 56 while that leaves the factors below 2^62
+    // (q <= 5, i.e. weights e^theta up to 100 for a wrapped feature)
     for (int l = d; !sp.tc_build && l < sp.nleaf; l += 2) {
       const Leaf& L = sp.leaf[l];
       double m = 0.0, c = 0.0;
@@ -157,7 +159,7 @@ __global__ void __launch_bounds__(NB * PREP_Y) k_prep(const Prob* __restrict__ p
         const double u = w[L.param0 + k];
         huge |= !(u < 0x1p900);
         if (L.type == L_RBF_CYCLIC)
-          m = fmax(m, u * (sp.cyclic[L.plane0 + k] ? 1.5707963267948966 : P.plane_max[L.plane0 + k]));
+          m = fmax(m, u * (0.5 * P.plane_max[L.plane0 + k]));
         else
           c += L.type == L_PERIODIC ? u * u : u;
       }
@@ -165,20 +167,26 @@ __global__ void __launch_bounds__(NB * PREP_Y) k_prep(const Prob* __restrict__ p
         m = fmax(m, __shfl_xor_sync(0xffffffffu, m, o));
         c += __shfl_xor_sync(0xffffffffu, c, o);
       }
-      const int s = m == 0.0 ? 0 : (int)((__double_as_longlong(m) >> 52) & 0x7FF) - 1022;
+      const int q = m == 0.0 ? 0 : (int)((__double_as_longlong(m) >> 52) & 0x7FF) - 1022;
+      const int t = 56 - max(0, q - 5);
       huge = __any_sync(0xffffffffu, huge || !(m < 0x1p900));
       if (lane == 0) {
-        s_c[l] = s;
         s_huge[l] = huge;
         if (rb == 0) {
           P.dotc->leaf_c[l] = L.type == L_CONSTANT ? w[L.param0] : c;
-          P.dotc->scale[l] = s;
+          P.dotc->unit[l] = t;
+          P.dotc->clamp[l] = q > 4;
         }
       }
-      if (rb == 0 && L.type == L_RBF_CYCLIC)
+      if (L.type == L_RBF_CYCLIC)
         for (int k = lane; k < L.n; k += 32) {
-          const long long f = llrint(ldexp(6.283185307179586 * w[L.param0 + k], 54 - s));  // below 2^57
-          P.dotc->mul[L.plane0 + k] = make_int2((int)(f >> 32), (int)((unsigned)f >> 1));
+          // sqrt(l) to l's own rounding, its product with g to the factor's unit
+          const double u = w[L.param0 + k], g = P.plane_max[L.plane0 + k], ug = u * g;
+          const double l = exp(P.theta[L.param0 + k]);
+          const double e = u > 0.0 && l < INFINITY ? fma(fma(-u, u, l) / (2.0 * u), g, fma(u, g, -ug)) : 0.0;
+          const long long f = llrint(ldexp(ug, t)) + llrint(ldexp(e, t));
+          s_mul[L.plane0 + k] = f;
+          if (rb == 0) P.dotc->mul[L.plane0 + k] = make_int2((int)(f >> 32), (int)((unsigned)f >> 1));
         }
     }
   } else if (tid == 0) {
@@ -266,18 +274,12 @@ __global__ void __launch_bounds__(NB * PREP_Y) k_prep(const Prob* __restrict__ p
         for (int k = y; k < cnt; k += PREP_Y) {
           const size_t o = (size_t)(L.plane0 + k) * nc + i;
           if (L.type == L_RBF_CYCLIC) {
-            // fixed point 2^(54 - s), or the fraction of a turn as it is; a point
-            // (or a leaf) that is not finite is marked in its norm
-            const double x = P.planes[o];
-            if (sp.cyclic[L.plane0 + k]) {
-              P.splanes[o] = x;
-              if (__double_as_longlong(x) == (long long)TURN_NOT_FINITE) a = 1.0;
-            } else {
-              bool nf = false;
-              P.splanes[o] = __longlong_as_double((to_fixed55(w[L.param0 + k] * x, s_c[l], &nf) + 1) >> 1);
-              if (nf) a = 1.0;
-            }
-            if (s_huge[l]) a = 1.0;
+            // integers: fractions of a turn as they are, the others in the leaf's unit; a
+            // point (or a leaf) that is not finite is marked in its norm
+            const long long u = __double_as_longlong(P.planes[o]), f = s_mul[L.plane0 + k];
+            const long long F = __mul64hi(u, f) + (long long)(((unsigned long long)u * (unsigned long long)f) >> 63);
+            P.splanes[o] = __longlong_as_double(sp.cyclic[L.plane0 + k] ? u : F);
+            if (u == (long long)TURN_NOT_FINITE || s_huge[l]) a = 1.0;
             continue;
           }
           const double u = w[L.param0 + k / per] * P.planes[o];

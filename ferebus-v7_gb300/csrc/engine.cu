@@ -232,16 +232,27 @@ __global__ void __launch_bounds__(256) k_build(const Prob* __restrict__ probs) {
 //
 // An rbf-cyclic leaf (stationary_cyclic_kernel.f90:104-127 on distance_matrix.f90:
 // 95-128, every 3rd feature's difference wrapped to [-pi, pi]) has no inner
-// product to go by; its differences are integers: plain features in 54-bit
-// fixed point of the leaf's scale 2^s, wrapped ones as fractions of a turn,
-// whose 64-bit differences wrap by themselves and are brought to that scale by
-// one multiplication.  D = h 2^27 + l enters the exact sum as h^2 + 2 h l 2^-27 +
-// l^2 2^-54.  ~12 to 25 integer instructions (2 to 3 cycles) per feature and
-// pair, against 3 to ~30 FP64 ones (64 cycles; the wrap goes through fmod): 20
-// problems of N = 1000, d = 24, 2.6 -> 0.5 ms.
+// product to go by; its differences are integers, in the unit 2^-t (t = 56 for
+// ordinary weights): of weighted features, or, where they wrap, of fractions of a
+// turn, whose 64-bit differences do so by themselves and are then weighted by
+// one multiplication.  D = h 2^32 + l enters the sum as h^2 + 2 h l 2^-32 + l^2 2^-64, which
+// is then E = |f_i - f_j|^2 in units of 2^-55.  The value's error against exact
+// arithmetic, on a model: at most 4e-17 for theta up to 6 and 3e-16 up to 9 (FP64
+// differences: 10^-15 and 10^-14, from the wrap's additions of pi).  ~10 to 20 integer
+// instructions (2 to 3 cycles) per feature and pair, against 3 to ~30 FP64 ones (64
+// cycles; the wrap goes through fmod): 20 problems of N = 1000, d = 24, 2.6 -> 0.5 ms.
 // ---------------------------------------------------------------------------
 size_t build_dot_smem_bytes(int nplanes) {
   return (size_t)2 * (nplanes + MAX_LEAF) * TB * sizeof(double) + 64;
+}
+
+// E 2^55 of an rbf-cyclic pair from its sums in units of 2^(64 - 2t) and 2^(33 - 2t); from
+// E = 256 on exp(-E / 2) is below 3e-56 and E need not be told apart
+__device__ __forceinline__ unsigned long long cyclic_square(unsigned long long H, long long M, int t) {
+  const int hs = 119 - 2 * t, ms = 2 * t - 88;
+  if (ms > 0) return H >> (63 - hs) ? ~0ULL : (H << hs) + (unsigned long long)((M + (1LL << (ms - 1))) >> ms);
+  const double e = ldexp((double)H, hs) + ldexp((double)M, -ms);  // weights above 10^10
+  return e < 0x1p63 ? (unsigned long long)e : ~0ULL;
 }
 
 __global__ void __launch_bounds__(256) k_build_dot(const Prob* __restrict__ probs) {
@@ -313,36 +324,39 @@ __global__ void __launch_bounds__(256) k_build_dot(const Prob* __restrict__ prob
           const Leaf& L = sp.leaf[tok];
           if (L.type == L_RBF_CYCLIC) {
             unsigned long long H[2] = {0, 0};  // 192 features' 2^56: not within 63 bits
-            long long M[2] = {0, 0};
+            long long M[2] = {0, 0};           // wraps only where H says E > 256
             const longlong2* fi = reinterpret_cast<const longlong2*>(Pi + L.plane0 * TB + r0);
             const long long* fj = reinterpret_cast<const long long*>(Pj + L.plane0 * TB + c);
-            for (int k = 0; k < L.n; ++k) {
+            auto feature = [&](int k, bool clamp) {
               const longlong2 f = fi[k * (TB / 2)];
-              const long long g = fj[k * TB];
-              long long D[2] = {(long long)((unsigned long long)f.x - (unsigned long long)g),
-                                (long long)((unsigned long long)f.y - (unsigned long long)g)};
+              const unsigned long long g = (unsigned long long)fj[k * TB];
+              long long D[2] = {(long long)((unsigned long long)f.x - g), (long long)((unsigned long long)f.y - g)};
               if (sp.cyclic[L.plane0 + k]) {  // uniform
                 const int2 m = dc.mul[L.plane0 + k];
 #pragma unroll
                 for (int a = 0; a < 2; ++a) {
-                  const int dh = (int)(D[a] >> 32);
-                  D[a] = (long long)dh * m.x + (long long)(((unsigned long long)(unsigned)D[a] * (unsigned)m.x) >> 32) +
-                         (((long long)dh * m.y) >> 31);
+                  const int uh = (int)(D[a] >> 32);
+                  D[a] = (long long)uh * m.x + (long long)(((unsigned long long)(unsigned)D[a] * (unsigned)m.x) >> 32) +
+                         (((long long)uh * m.y) >> 31);
                 }
               }
 #pragma unroll
               for (int a = 0; a < 2; ++a) {
-                const int hh = (int)((D[a] + (1LL << 26)) >> 27);
-                const int l = (int)((unsigned)D[a] - ((unsigned)hh << 27));
-                H[a] += (unsigned long long)((long long)hh * hh);
-                M[a] += (long long)hh * l + (((long long)l * l) >> 28);
+                if (clamp) D[a] = max(min(D[a], 1LL << 60), -(1LL << 60));
+                const int l = (int)D[a], h = (int)(D[a] >> 32) + (l < 0);
+                H[a] += (unsigned long long)((long long)h * h);
+                M[a] += (long long)h * l + (((long long)l * l) >> 33);
               }
-            }
-            const IexpScale sc = iexp_scale(2 * dc.scale[tok] - 55);
+            };
+            if (dc.clamp[tok])  // uniform
+              for (int k = 0; k < L.n; ++k) feature(k, true);
+            else
+              for (int k = 0; k < L.n; ++k) feature(k, false);
             for (int a = 0; a < 2; ++a)
               stk[a][top] = Ni[tok * TB + r0 + a] != 0.0 || Nj[tok * TB + c] != 0.0
                                 ? nan("")
-                                : iexp_fixed_tab(H[a] + (unsigned long long)(M[a] >> 26), sc, g_iexp_tab1024, g_iexp_fine1024);
+                                : iexp_fixed_tab(cyclic_square(H[a], M[a], dc.unit[tok]), iexp_scale(-56), g_iexp_tab1024,
+                                                 g_iexp_fine1024);
           } else if (L.type == L_RBF || L.type == L_PERIODIC) {
             const int nf = L.type == L_PERIODIC ? 2 * L.n : L.n;
             double dot[2] = {0.0, 0.0};

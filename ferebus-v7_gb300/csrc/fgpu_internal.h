@@ -74,12 +74,13 @@ struct alignas(16) PanelZ {
 
 // What the dot-product build (engine.cu) needs per evaluation besides the scaled
 // planes, from k_prep: per leaf the sum of l (periodic) or of 1 / c (linear), or
-// the constant; for rbf-cyclic leaves the fixed-point scale s and per wrapped
-// plane the factor 2 pi sqrt(l) 2^(54 - s) as (high word, low word >> 1).
-constexpr unsigned long long TURN_NOT_FINITE = 1ULL << 63;  // a wrapped feature's plane entry that stands for NaN or infinity
+// the constant; for rbf-cyclic leaves the unit 2^-t of the weighted differences,
+// whether they may pass 2^60 of it, and per plane the factor sqrt(l) g 2^t from
+// differences in units of 2^-64 g, as (high word, low word >> 1), where they wrap.
+constexpr unsigned long long TURN_NOT_FINITE = 1ULL << 63;  // an rbf-cyclic feature's plane entry that stands for NaN or infinity
 struct DotConst {
   double leaf_c[MAX_LEAF];
-  int scale[MAX_LEAF];
+  int unit[MAX_LEAF], clamp[MAX_LEAF];
   int2 mul[MAX_PLANES];
 };
 
@@ -131,7 +132,7 @@ struct Prob {
   int ldkinv;
   double* gpart;                  // adjoint: per-CTA partial sums
   // tensor-core build
-  const double* plane_max;        // nplanes: max_i |planes[p][i]|
+  const double* plane_max;        // nplanes: max_i |planes[p][i]|; rbf-cyclic: g (DotConst)
   long long* fnorm;               // 2 x Nc: W_ii of the distance leaves
   double* fcoef;                  // 4: k = a + b v0 + c v1 + d v0 v1
   int* fscale;                    // 2: s of the distance leaves, max |f| < 2^s; how their values combine

@@ -91,3 +91,61 @@ def test_weight_that_is_not_usable(col, value, lib):
         return
     assert info[1] > 0 and np.isnan(ll[1])
     assert info[0] == 0 and ll[0] == e.loglik(th[0])[0]
+
+
+def _exact_loglik(E, nugget):
+    """logL at y = mu = 0 from the squared distances E, in extended precision."""
+    K = np.exp(-E / 2) + np.eye(len(E), dtype=np.longdouble) * np.longdouble(nugget)
+    ld, n = np.longdouble(0), len(E)
+    for j in range(n):  # outer-product Cholesky
+        ld += np.log(K[j, j])
+        K[j + 1:, j + 1:] -= np.outer(K[j + 1:, j], K[j + 1:, j]) / K[j, j]
+    return -ld / 2 - np.longdouble(n) / 2 * np.log(2 * np.longdouble(np.pi))
+
+
+@pytest.mark.parametrize("theta", [0.5, 3.0, 5.5, 8.0])
+@pytest.mark.parametrize("wrapped", [False, True])
+def test_precision_of_close_points(theta, wrapped, lib):
+    """Pairs at E = 1e-4 (K_ij = 1 - 5e-5) among points far apart: log(1 - K_ij^2) shows
+    E's absolute error.  Allowed: E to 3e-16 relative and 6e-17 (the weight and the
+    units of the distances), K_ij to 2^-53 + 2^-61 (its rounding, and the matrix's),
+    over a pair's 1 - K_ij^2 = 1e-4; the conversions' few ulps of logL."""
+    from fgpu import Engine
+    n, d = 60, 3
+    rng = np.random.default_rng(int(10 * theta))
+    step = 12.0 / np.sqrt(np.exp(theta))  # one pair from the next
+    X = np.zeros((n, d))
+    X[:, 0] = 0.3 + (np.arange(n) // 2) * step
+    X[:, 2] = 2.0
+    col = 2 if wrapped else 1
+    if wrapped:
+        X[::4, 2] = np.pi - 0.001 * np.arange(len(X[::4]))
+    else:
+        X[::2, 1] = rng.uniform(-1.5, 1.5, size=n // 2)
+    gap = np.sqrt(1e-4 / np.exp(theta))
+    X[1::2, col] = X[::2, col] + gap * rng.uniform(0.9, 1.1, size=n // 2)
+    ks, th = [O.RBF_CYCLIC, d, 1, 2, 3], np.full(d, theta)
+    ld = np.longdouble
+    D = X.astype(ld)[:, None] - X.astype(ld)[None]
+    C, P = ld(2.0 * np.pi), ld(np.pi)  # the doubles the reference wraps by
+    D[..., 2] = np.abs(D[..., 2]) + P
+    D[..., 2] = np.fmod(D[..., 2], C) - P
+    want = _exact_loglik((np.exp(ld(theta)) * D * D).sum(-1), 0.0)
+    ll, info = Engine(X, np.zeros(n), np.zeros(n), ks, 0, 0.0, False).loglik(th)
+    tol = n // 2 * ((3e-16 * 1e-4 + 6e-17) / 2 + 2.0 ** -53 + 2.0 ** -61) / 1e-4 / 0.8 + 4 * np.spacing(abs(float(want)))
+    assert info == 0
+    assert abs(ll - want) <= tol, (ll, float(want), float(abs(ll - want)), tol)
+
+
+def test_angles_far_beyond_the_integers(lib):
+    """Wrapped features around 1e17: their differences are exact, and so is the wrap."""
+    from fgpu import Engine
+    n = 40
+    rng = np.random.default_rng(8)
+    X = rng.normal(2.0, 0.3, size=(n, 3))
+    X[:, 2] = 1e17 + 16.0 * np.arange(n)
+    y = rng.normal(size=n)
+    ks, th = [O.RBF_CYCLIC, 3, 1, 2, 3], np.full(3, 0.3)
+    ll, info = Engine(X, y, np.zeros(n), ks, 0, 1e-2, False).loglik(th)
+    ref, _ = O.loglik(ks, th, X, y, np.zeros(n), 0, 1e-2, False)
+    assert info == 0 and abs(ll - ref) <= 1e-9 * abs(ref), (ll, ref)
