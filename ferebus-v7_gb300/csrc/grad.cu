@@ -347,11 +347,17 @@ __global__ void __launch_bounds__(256, PER_SM)
           }
         }
       }
-      // |f_i - f_j|^2 = (H + M 2^-26) 2^(2 s - 54)
-      const IexpScale sc = iexp_scale(2 * Q.fscale[d] - 55);
+      // |f_i - f_j|^2 = (H + M 2^-26) 2^(2 s - 54), in units of 2^-55 or finer: with
+      // those of 2^(2 s - 54) the leaf values of close pairs were 10^-13 off for
+      // weights of 50 (s = 6); beyond 2^62 of the unit (128) they are below 2e-28
+      const int s2 = 2 * Q.fscale[d], up = max(0, min(26, s2 + 1));
+      const IexpScale sc = iexp_scale(s2 - 55 - up);
 #pragma unroll
-      for (int e = 0; e < 16; ++e)
-        v[d][e] = iexp_fixed_tab(H[e] + (unsigned long long)(M[e] >> 26), sc, g_iexp_tab1024, g_iexp_fine1024);
+      for (int e = 0; e < 16; ++e) {
+        const unsigned long long E =
+            H[e] >> (62 - up) && up ? ~0ULL : (H[e] << up) + (unsigned long long)(M[e] >> (26 - up));
+        v[d][e] = iexp_fixed_tab(E, sc, g_iexp_tab1024, g_iexp_fine1024);
+      }
     }
   }
   // weights: w dk/dv_d v_d, and the sums the linear and constant leaves need
