@@ -155,11 +155,12 @@ void plan_tc_build(Spec& sp) {
     if (sp.ndot == 2 && sp.post[k] == P_PROD) sp.tc_build = 2;
 }
 
-// Per-step tile tables of the persistent tensor-core update: for step s,
-// prefix[s * (nprob + 1) + p] = tiles of problems < p.
+// Host-built work lists of the factorisation's steps.
 struct UpdSched {
   // trailing-update tiles of every step, packed (problem << 40 | row tile
-  // << 20 | column tile), problem by problem, column tile major
+  // << 20 | column tile): first the next diagonal tile of every problem (its two
+  // column halves; the look-ahead counts on that), then the others problem by
+  // problem, column tile major
   unsigned long long* tiles_dev = nullptr;
   std::vector<size_t> tile_off;  // first tile of each step
   std::vector<int> totals;       // tiles per step
@@ -173,7 +174,7 @@ struct UpdSched {
   std::vector<int> diag_totals;     // per step: problems with a panel there
   int* sync_dev = nullptr;          // zeroed per evaluation: PANEL_FLAGS ints per problem, a tile counter per step
   size_t flag_ints = 0, nsync = 0;  // offset of the counters, ints in all
-  int dot_builds = 0;               // problems the FP64 dot-product build serves
+  int dot_builds = 0;               // problems the dot-product build serves
   bool keep_l = false;              // a worker's: the factor is kept
 };
 
@@ -1157,7 +1158,7 @@ int fgpu_loglik(fgpu_ctx* ctx, const double* theta, int ntheta, double* ll, int*
   CK(cudaStreamSynchronize(w->stream));
   if (w->h_status[2]) return fail(FGPU_ETIMEOUT, "a bounded wait in a kernel gave up (copy or MMA)");
   if (w->h_status[3] && !w->h_status[1])
-    return fail(FGPU_ECUDA, "panel value outside its row scale bound (split-integer update)");
+    return fail(FGPU_ECUDA, "a kernel value or feature is not finite, or outside its scale");
   *info = w->h_status[0];
   *ll = (*info == 0) ? h_out[0] : std::nan("");
   return 0;
@@ -1372,7 +1373,7 @@ int fgpu_grad(fgpu_ctx* ctx, const double* theta, int ntheta, double* ll, double
   t_launches = n;
   if (h_status[2]) return fail(FGPU_ETIMEOUT, "a bounded wait in a kernel gave up");
   if (h_status[3] && !h_status[1])
-    return fail(FGPU_ECUDA, "panel value outside its row scale bound (split-integer update)");
+    return fail(FGPU_ECUDA, "a kernel value or feature is not finite, or outside its scale");
   *info = h_status[0];
   *ll = (*info == 0) ? h_out[0] : std::nan("");
   for (int k = 0; k < ntheta; ++k) dll[k] = (*info == 0) ? h_g[k] : std::nan("");
@@ -1397,8 +1398,8 @@ int fgpu_plan_create(fgpu_plan** out, fgpu_ctx* const* ctxs, int nprob, int ldth
     p->ctxs.push_back(ctxs[i]);
   }
   if (ldtheta < maxth) return fail(FGPU_EINVAL, "ldtheta=%d < max nparams %d", ldtheta, maxth);
-  // the panels' row-tile order packs (problem << 16 | row tile) into a
-  // non-negative int (a negative entry ends a CTA's work)
+  // the panels' row-tile order packs (problem << 16 | row tile) into an int, and
+  // the kernels take the problem back by an arithmetic shift
   if (ctxs[0]->mode == 1 && nprob > 32767)
     return fail(FGPU_EINVAL, "a tensor-core plan holds at most 32767 problems (%d given)", nprob);
   p->ldtheta = ldtheta;
@@ -1612,7 +1613,7 @@ int fgpu_plan_run(fgpu_plan* p, const double* theta_host, double* ll_host, int* 
   memcpy(info_host, p->h_info, sizeof(int) * p->nprob);
   for (int i = 0; i < p->nprob; ++i) {
     if (info_host[i] == -1) return fail(FGPU_ETIMEOUT, "problem %d: a bounded wait in a kernel gave up", i);
-    if (info_host[i] < 0) return fail(FGPU_ECUDA, "problem %d: panel value outside its row scale bound", i);
+    if (info_host[i] < 0) return fail(FGPU_ECUDA, "problem %d: a kernel value or feature is not finite, or outside its scale", i);
   }
   return 0;
 }

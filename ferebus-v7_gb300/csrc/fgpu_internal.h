@@ -195,9 +195,8 @@ constexpr int PANEL_FLAGS = 32;            // one 128-byte line per problem
 cudaError_t launch_panel(const Prob* probs, int step, const int* order, int ndiag, int total_tiles, int* counter,
                          int* flags, int num_sms, cudaStream_t s);
 cudaError_t launch_panel_rows(const Prob* probs, int step, const int* order, int ntiles, cudaStream_t s);
-// prefix: device table of nprob + 1 tile offsets for this step (tiles of
-// problem p at step s: m (m + 1), m = nt128_p - s - 1); total_tiles = prefix[nprob].
-// tiles: the step's trailing tiles, packed (problem << 40 | row tile << 20 | column tile)
+// Trailing update of `total_tiles` of the step's tiles, packed (problem << 40 | row
+// tile << 20 | column tile), by at most max_ctas CTAs.
 cudaError_t launch_ozaki_update(const Prob* probs, int nprob, int step, int max_nt128,
                                 const unsigned long long* tiles, int total_tiles, int max_ctas, cudaStream_t s);
 // Preparation of an evaluation and the tensor-core kernel-matrix build

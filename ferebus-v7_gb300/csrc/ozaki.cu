@@ -80,11 +80,8 @@ static_assert(UPD_COLS % 8 == 0 && UPD_EPI_WARPS % 4 == 0, "epilogue column grou
 constexpr uint32_t UPD_SMEM = NSTAGE * STAGE + UPD_EPI_WARPS * UPD_PIECE + 256;
 static_assert(UPD_SMEM <= 227 * 1024, "shared memory per CTA");
 
-// MMA-issuing warp of digit level l (one warp issues all levels)
-__host__ __device__ constexpr int upd_level_warp(int) { return 0; }
 static_assert(UPD_MMA_WARPS == 1, "the update epilogue converts all 7 levels of a column group in one pass");
 
-//
 // KSH: a tile's 8 k-chunks are shared by 2^KSH CTAs, each of which subtracts
 // its part (the same integers).  Where a step has so few tiles that the parts
 // still fit one wave, the loads and MMAs of one tile are what it costs: the

@@ -68,7 +68,7 @@ class Engine:
         return ll.value, info.value
 
     def grad(self, theta):
-        """Returns ``(ll, dll_dtheta, info)`` from the FP64 adjoint."""
+        """Returns ``(ll, dll_dtheta, info)`` from the adjoint."""
         th = np.ascontiguousarray(theta, dtype=np.float64)
         ll, info = C.c_double(), C.c_int()
         g = np.empty(self.ntheta)
@@ -137,6 +137,8 @@ class Plan:
         mode = 2 if enable == "update" else (1 if enable else 0)
         _lib.check(self.lib.fgpu_plan_set_profiling(self.handle, mode))
 
+    # by stage index; in tensor-core mode "trsm" is the whole panel, and the last
+    # four are of an earlier form of it and stay 0
     STAGES = ("build", "potf2", "trsm", "update", "finalize", "panel_prep", "split", "border", "coupling")
 
     def stage_times(self):

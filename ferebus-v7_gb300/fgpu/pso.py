@@ -24,7 +24,7 @@ trajectories match the reference in distribution, not bit for bit.
 
 Gradient polish (``SwarmConfig.polish_steps > 0``; off by default, and then
 nothing below runs): after the last iteration each swarm's global best is
-refined by projected gradient ascent on logL with the engine's FP64 adjoint
+refined by projected gradient ascent on logL with the engine's adjoint
 (``fgpu_grad``), in box-normalised coordinates u = (theta - lo) / (hi - lo)
 so that the linear noise parameter (box [1e-12, 1e-6]) and the kernel
 parameters move on the same scale.  Each step tries a move of at most

@@ -87,8 +87,9 @@ int fgpu_set_trailing_update(int mode);
  * default; returns the previous setting): FGPU_BUILD_TC (default) forms the
  * exact distances on the tensor cores where the kernel allows it (leaves
  * rbf / periodic / linear / constant, at most two rbf-or-periodic leaves);
- * FGPU_BUILD_FP64 keeps the FP64 dot-product build.  The environment
- * variable FGPU_BUILD=fp64 selects FP64 at load.  Both give the likelihood
+ * FGPU_BUILD_FP64 keeps the dot-product build (FP64, but for rbf-cyclic
+ * leaves' integer distances).  The environment variable FGPU_BUILD=fp64,
+ * read once, selects it.  Both give the likelihood
  * to the parity tolerance; the autotuner picks between them per shape.  No
  * counterpart in the reference. */
 #define FGPU_BUILD_FP64 0
@@ -141,8 +142,8 @@ int fgpu_grad(fgpu_ctx* ctx, const double* theta, int ntheta, double* ll,
  * that share one workspace arena, still as one graph replay per run; a single
  * problem larger than the budget is FGPU_ENOMEM.  After fgpu_plan_run_device,
  * info_dev[p] < 0 means -1: a bounded device wait gave up (fgpu_plan_run
- * returns FGPU_ETIMEOUT for it), -2: a panel value broke its row-scale bound
- * (fgpu_plan_run returns FGPU_ECUDA); ll_dev[p] is then NaN.  No counterpart
+ * returns FGPU_ETIMEOUT for it), -2: a kernel value or feature is not finite,
+ * or outside its scale (fgpu_plan_run returns FGPU_ECUDA); ll_dev[p] is then NaN.  No counterpart
  * in the reference (its particles are evaluated one per OpenMP thread,
  * src/optimiser/pso/pso.f90:419-452). */
 int fgpu_plan_create(fgpu_plan** plan, fgpu_ctx* const* ctxs, int nprob, int ldtheta);
@@ -184,7 +185,7 @@ void fgpu_destroy(fgpu_ctx* ctx);
  * for it; read ll/info after synchronising with the stream.  *info_dev is 0,
  * a LAPACK-style pivot column > 0 (non-positive-definite K, ll NaN), or
  * negative: -1 a bounded device wait gave up (what other entry points report
- * as FGPU_ETIMEOUT), -2 a panel value broke its row-scale bound (FGPU_ECUDA).
+ * as FGPU_ETIMEOUT), -2 a value is not finite or outside its scale (FGPU_ECUDA).
  * The first call on a device resolves the array's address
  * (cudaGetSymbolAddress) -- make it before any stream capture.  Every call
  * shares the array and finds the previous call's contents there: calls
