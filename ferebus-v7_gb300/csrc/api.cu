@@ -175,6 +175,7 @@ struct UpdSched {
   int* sync_dev = nullptr;          // zeroed per evaluation: PANEL_FLAGS ints per problem, a tile counter per step
   size_t flag_ints = 0, nsync = 0;  // offset of the counters, ints in all
   int dot_builds = 0;               // problems the dot-product build serves
+  bool dot_cyclic = false;          // some of them have an rbf-cyclic leaf
   bool keep_l = false;              // a worker's: the factor is kept
 };
 
@@ -379,7 +380,14 @@ void fill_prob(Prob& p, const fgpu_ctx* c, const double* theta_d, const Workspac
   p.fscale = ws.fscale;
 }
 
-int build_sched(const std::vector<int>& nt128, const std::vector<int>& tc_build, UpdSched& u,
+// How a problem's matrix is built: Spec::tc_build, or -1 for the dot-product build with an rbf-cyclic leaf.
+int build_kind(const Spec& sp) {
+  for (int l = 0; l < sp.nleaf; ++l)
+    if (sp.leaf[l].type == FGPU_RBF_CYCLIC) return -1;
+  return sp.tc_build;
+}
+
+int build_sched(const std::vector<int>& nt128, const std::vector<int>& build, UpdSched& u,
                 std::vector<void*>* track) {
   const int nprob = (int)nt128.size();
   int ntmax = 0;
@@ -441,11 +449,12 @@ int build_sched(const std::vector<int>& nt128, const std::vector<int>& tc_build,
   // 128 x 64 per eligible problem, column-tile pair major, row tile minor
   std::vector<unsigned long long> bl;
   for (int p = 0; p < nprob; ++p) {
-    if (!tc_build[p]) {
+    if (build[p] <= 0) {
       u.dot_builds++;
+      u.dot_cyclic |= build[p] < 0;
       continue;
     }
-    u.products |= tc_build[p] == 2;
+    u.products |= build[p] == 2;
     for (int q = 0; q < nt128[p]; ++q)
       for (int half = 0; half < 2; ++half)
         for (int ti = q; ti < nt128[p]; ++ti)
@@ -516,7 +525,7 @@ int enqueue_eval(const Prob* probs_d, int nprob, int max_nsteps, int max_nplanes
     const int nt = max_nsteps / 2;
     CK(cudaMemsetAsync(us->sync_dev, 0, sizeof(int) * us->nsync, s));
     STAGE(0, launch_prep(probs_d, nprob, nt, s));
-    if (us->dot_builds > 0) STAGE(0, launch_build_dot(probs_d, nprob, max_nsteps, max_nplanes, s));
+    if (us->dot_builds > 0) STAGE(0, launch_build_dot(probs_d, nprob, max_nsteps, max_nplanes, us->dot_cyclic, s));
     if (us->build_total > 0)
       STAGE(0, launch_build_tc(probs_d, nprob, us->build_tiles_dev, us->build_total, us->products, us->num_sms, s));
     // A panel with at least as many row tiles as SMs is a throughput problem:
@@ -830,7 +839,7 @@ int make_worker(fgpu_ctx* c, Worker** out) {
   if (cudaMemcpy(w->prob_d, &p, sizeof(Prob), cudaMemcpyHostToDevice) != cudaSuccess)
     return bail(fail(FGPU_ECUDA, "desc copy"));
   if (c->mode == 1 &&
-      (rc = build_sched(std::vector<int>{c->nt128}, std::vector<int>{c->spec.tc_build}, w->sched, nullptr)) != 0)
+      (rc = build_sched(std::vector<int>{c->nt128}, std::vector<int>{build_kind(c->spec)}, w->sched, nullptr)) != 0)
     return bail(rc);
   if (uploads_done() != cudaSuccess) return bail(fail(FGPU_ECUDA, "worker uploads"));
   w->sched.keep_l = true;
@@ -1479,7 +1488,7 @@ int fgpu_plan_create(fgpu_plan** out, fgpu_ctx* const* ctxs, int nprob, int ldth
       std::vector<int> nts, tcs;
       for (int k = w.first; k < w.first + w.count; ++k) {
         nts.push_back(ctxs[p->order[k]]->nt128);
-        tcs.push_back(ctxs[p->order[k]]->spec.tc_build);
+        tcs.push_back(build_kind(ctxs[p->order[k]]->spec));
       }
       if ((rc = build_sched(nts, tcs, w.sched, &p->allocations)) != 0) return bail(rc);
     }

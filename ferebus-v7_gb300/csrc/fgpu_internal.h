@@ -149,7 +149,8 @@ int encode_slice_maps(void* host_maps, const void* slices, int tiles);
 // current step exit immediately, so ragged batches share one launch.
 cudaError_t launch_build(const Prob* probs, int nprob, int max_nsteps, int max_nplanes, cudaStream_t s);
 // mode 1: the dot-product form of the build, for kernels the tensor cores do not serve
-cudaError_t launch_build_dot(const Prob* probs, int nprob, int max_nsteps, int max_nplanes, cudaStream_t s);
+// (cyclic: some of them have an rbf-cyclic leaf)
+cudaError_t launch_build_dot(const Prob* probs, int nprob, int max_nsteps, int max_nplanes, bool cyclic, cudaStream_t s);
 size_t build_dot_smem_bytes(int nplanes);
 cudaError_t launch_potf2(const Prob* probs, int nprob, int step, cudaStream_t s);
 // max_rowtiles: 64-row tiles of the tallest problem (0 = max_nsteps + 1)
@@ -264,7 +265,8 @@ cudaError_t enqueue_grad_fast(const Prob* p, const Prob* eval, int nsteps, int n
 // device, or a second thread, sets the attribute for itself.  Devices
 // beyond the first 64 set it on every call.
 enum SmemSlot {
-  SMEM_BUILD, SMEM_BUILD_DOT, SMEM_UPDATE, SMEM_SYRK, SMEM_PANEL, SMEM_PANEL_ROWS, SMEM_INV_GEMM, SMEM_GRAD_FAST,
+  SMEM_BUILD, SMEM_UPDATE, SMEM_SYRK, SMEM_PANEL, SMEM_PANEL_ROWS, SMEM_INV_GEMM, SMEM_GRAD_FAST,
+  SMEM_BUILD_DOT, SMEM_BUILD_DOT_LAST = SMEM_BUILD_DOT + 1,  // one slot per instance, as below
   SMEM_GRAD_FAST2,
   SMEM_OZAKI_UPDATE, SMEM_OZAKI_UPDATE_LAST = SMEM_OZAKI_UPDATE + 2,  // one slot per instance
   SMEM_BUILD_TC, SMEM_BUILD_TC_LAST = SMEM_BUILD_TC + 5,
