@@ -51,7 +51,7 @@
 // (conversion of the integer sums, 32-column factors, solves and couplings,
 // right-hand-side update) that this replaces: a lone problem 250 -> 75 us
 // per panel (N = 4000, 32 panels), a swarm of 40 at N = 4000 20.7 -> 9.3 ms
-// (6.4 with k_panel_rows below).
+// (6.8 with k_panel_rows below).
 #include "fgpu_internal.h"
 #include "tc_common.cuh"
 
@@ -853,8 +853,8 @@ __global__ void __launch_bounds__(PN_THREADS, 1)
 // chunks of 28 KB per tile) through a 2-stage ring, and are multiplied into the
 // other one of two TMEM accumulators while the rows are solved.  One thread
 // issues the copies and the MMAs.  Every word is the one k_panel computes: the
-// sums are exact integers.  All panels of 40 problems of N = 4000: 9.3 -> 6.4
-// ms, of 16 of N = 10000: 21.8 -> 15.9 ms, of 50 of N = 2000: 3.3 -> 2.5 ms.
+// sums are exact integers.  All panels of 40 problems of N = 4000: 9.3 -> 6.8
+// ms, of 16 of N = 10000: 21.8 -> 16.6 ms, of 50 of N = 2000: 3.3 -> 2.6 ms.
 // ---------------------------------------------------------------------------
 namespace {
 constexpr int PR_THREADS = 160;
